@@ -91,6 +91,7 @@ struct stg_ctx {
     // adapters run the general-coefficient form (general.cu); gtmp: its finest-size scratch
     bool gen = false;
     stg::d4* gtmp[3] = {nullptr, nullptr, nullptr};
+    bool fixed_cells2d = false;  // 2D: the boundary fixes cells (identity rows among the pressures)
     // the coarse levels hold the solver's own penalties (flow rule of kernels.cu k_coarsen)
     // rather than the reference's sums, which the component adapters reproduce
     bool hier_flow = false;

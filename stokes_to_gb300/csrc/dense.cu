@@ -7,12 +7,13 @@
 // entries are never recorded (as in the reference); with `closed` the pressure block
 // gets +1 everywhere (:605-608). Unknowns that exist only as padding in the reference
 // layout are identity rows decoupled from the rest, so the dense system here keeps the
-// unknowns that exist. It is inverted once per set-up by Gauss-Jordan elimination with
-// partial pivoting on [A | I] (double-buffered in L2; all pivot steps in one cooperative
-// launch with a grid-wide barrier between them), and the inverse is applied as a GEMV
-// inside each V-cycle.
+// unknowns that exist. It is inverted once per set-up by block elimination
+// (k_inv_blocks), or, where that does not apply, by Gauss-Jordan elimination with partial
+// pivoting on [A | I] (double-buffered in L2); either is one cooperative launch with a
+// grid-wide barrier between its steps. The inverse is applied as a GEMV inside each V-cycle.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "kernels.h"
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(TPB) k_gj_step(int nd, int k, const double* in
 // launch gaps of nd dependent kernels were most of the set-up time): the operations of
 // k_gj_step in the same order, so the same inverse bit for bit. Step k reads buffer k mod
 // 2 and writes the other.
-__global__ void __launch_bounds__(TPB) k_gj_all(int nd, double* a, double* b, int* info) {
+__device__ __forceinline__ void gj_all(int nd, double* a, double* b, int* info) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
     for (int k = 0; k < nd; k++) {
@@ -209,6 +210,261 @@ __global__ void __launch_bounds__(TPB) k_gj_all(int nd, double* a, double* b, in
         gj_rows(nd, k, p, in, out, info, blockIdx.x, gridDim.x);
         grid.sync();
     }
+}
+__global__ void __launch_bounds__(TPB) k_gj_all(int nd, double* a, double* b, int* info) { gj_all(nd, a, b, info); }
+
+// ---------------------------------------------------------------- block inversion
+// The coarsest matrix is a saddle point [K B^T; B C]: K (faces) symmetric positive
+// definite, C (cells) the cell penalties plus, on a closed domain, ones everywhere. With
+// the ones moved to one bordering unknown l,
+//   M = [K B^T 0; B C0 e; 0 e^T -1],   C0 = C - e e^T  (its Schur complement over l is A),
+// elimination in the order faces, cells, l meets positive pivots on the faces and negative
+// ones on the cells, which is stable without a pivot search; only the last block, which
+// holds l and the last cells, pivots inside itself. So the inverse is formed block by block:
+// for a diagonal block k of B unknowns, D = M_kk^-1 and M_ij -= M_ik D M_kj, in place: 2 N^3
+// FP64 operations instead of 4 nd^3, no pivot search over a strided column, and one grid
+// barrier a step. The faces of different axes are uncoupled until cells are eliminated, so
+// one step eliminates a block of every axis at once (S blocks), and tiles that are zero are
+// skipped. Every block of the grid inverts the M_kk for itself (a warp each, the tile in
+// registers), which saves a second barrier. A pivot of the wrong sign (a negative penalty)
+// or faces that are coupled across axes (open boundaries) end the attempt, in every block
+// alike, and the pivoted elimination above runs on the untouched [A | I] instead.
+//
+// Bound: for nd = 304 the chain of 10 barriers and 16 x 16 inversions (whole set-up of a
+// 16^3 handle 2.2 -> 0.42 ms against the pivoted elimination, one pivot per barrier), for nd =
+// 2112 the FP64 pipe, two FMAs per SM and clock (set-up at 96^2 276 -> 14.6 ms; 2 nd^3
+// operations take 15 ms, the skipped zero tiles save a third of them). Tile width: 16 keeps
+// the chain of small inversions short, 32 halves the panel traffic where the products dominate.
+template <int B>
+__device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], bool local_pivot, bool positive) {
+    // one warp; lane: row lane / LPR, columns CE (lane % LPR) .. of the tile
+    constexpr int LPR = 32 / B, CE = B / LPR;
+    const int lane = threadIdx.x & 31, r = lane / LPR, h = lane % LPR;
+    double a[CE];
+#pragma unroll
+    for (int c = 0; c < CE; c++) a[c] = s[r][h * CE + c];
+    int col = 0;  // lane q: the pivot row of step q
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+        double f = __shfl_sync(0xffffffffu, a[q % CE], r * LPR + q / CE);  // column q of the own row
+        int p = q;
+        if (local_pivot) {
+            double best = (r >= q) ? fabs(f) : -1.0;
+            int bi = r;
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ob > best || (ob == best && oi < bi)) {
+                    best = ob;
+                    bi = oi;
+                }
+            }
+            p = bi;
+            if (p != q) {  // exchange rows p and q
+                const int src = (r == q ? p : r == p ? q : r) * LPR + h;
+#pragma unroll
+                for (int c = 0; c < CE; c++) a[c] = __shfl_sync(0xffffffffu, a[c], src);
+                f = __shfl_sync(0xffffffffu, f, src);
+            }
+            if (lane == q) col = p;
+        }
+        const double piv = __shfl_sync(0xffffffffu, f, q * LPR);
+        // NaN and infinity fail as well
+        const double want = local_pivot ? fabs(piv) : (positive ? piv : -piv);
+        ok = ok && want > 0.0 && want < 1e300;
+        const double inv = 1.0 / piv;
+        const double g = r == q ? -inv : f * inv;
+#pragma unroll
+        for (int c = 0; c < CE; c++) {
+            const double row = __shfl_sync(0xffffffffu, a[c], q * LPR + h);
+            a[c] = (r == q ? 0.0 : a[c]) - g * row;
+        }
+        if (h == q / CE) a[q % CE] = -g;
+    }
+    if (local_pivot) {  // undo the row exchanges on the columns, last first
+#pragma unroll
+        for (int c = 0; c < CE; c++) s[r][h * CE + c] = a[c];
+        __syncwarp();
+        for (int q = B - 1; q >= 0; q--) {
+            const int p = __shfl_sync(0xffffffffu, col, q);
+            if (p != q && h == 0) {
+                const double t = s[r][q];
+                s[r][q] = s[r][p];
+                s[r][p] = t;
+            }
+            __syncwarp();
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < CE; c++) s[r][h * CE + c] = a[c];
+    }
+    return ok;
+}
+
+// perm[q], q < N: the unknown at position q, -1 for a decoupled filler, -2 for l. The
+// positions hold S face sections of TF tiles each (one axis a section), then the cells' tiles.
+// ws: N^2 + 4 S B N doubles (the pivoted elimination's second buffer). R: tiles of one column
+// a block updates with one product D M_kj.
+template <int B, int R, int S>
+__global__ void __launch_bounds__(TPB) k_inv_blocks(int nd, int N, int TF, const int* __restrict__ perm, int closed, double* a,
+                                                    double* ws, int* info) {
+    namespace cg = cooperative_groups;
+    cg::grid_group grid = cg::this_grid();
+    __shared__ double sD[S][B][B + 1], sE[S][B][B + 1], sA[B][B + 1];
+    __shared__ int s_bad;
+    const int T = N / B, tid = threadIdx.x, TC = S * TF, cell0 = TC * B;
+    constexpr int EPT = B * B / TPB;  // tile elements of a thread: rows r0 + e (TPB / B), column c0
+    const int c0 = tid % B, r0 = tid / B;
+    constexpr int RS = TPB / B;
+    double* M = ws;
+    // pivot tiles of step k: s TF + k for the sections s < S while k < TF, then TC + (k - TF)
+    const int steps = TF + (T - TC);
+    auto pivots = [&](int k) { return k < TF ? S : 1; };
+    auto pivot = [&](int k, int q) { return k < TF ? q * TF + k : TC + (k - TF); };
+    // panels of step k: column tiles M_ip (w = 0) and row tiles M_pj (w = 1) of pivot q
+    auto panel = [&](int k, int w, int q) { return ws + (long long)N * N + (long long)(((k & 1) * 2 + w) * S + q) * B * N; };
+    auto put = [&](int i, int j, int r, int k, double v) {  // element (r, c0) of tile (i, j), and the panels of step k
+        M[(long long)(i * B + r) * N + j * B + c0] = v;
+        const int o = r * B + c0;
+        for (int q = 0; q < pivots(k); q++) {
+            const int pv = pivot(k, q);
+            if (j == pv) panel(k, 0, q)[(long long)i * B * B + o] = v;
+            if (i == pv) panel(k, 1, q)[(long long)j * B * B + o] = v;
+        }
+    };
+    auto in_panel = [&](int i, int j, int k) {
+        for (int q = 0; q < pivots(k); q++)
+            if (i == pivot(k, q) || j == pivot(k, q)) return true;
+        return false;
+    };
+    // the bordered matrix in the elimination order; *info counts faces coupled across axes
+    for (int t = blockIdx.x; t < T * T; t += gridDim.x) {
+        const int i = t / T, j = t % T;
+        const bool apart = i < TC && j < TC && i / TF != j / TF;
+#pragma unroll
+        for (int e = 0; e < EPT; e++) {
+            const int r = r0 + e * RS, x = i * B + r, y = j * B + c0;
+            const int px = __ldg(perm + x), py = __ldg(perm + y);
+            double v;
+            if (px >= 0 && py >= 0)
+                v = a[(long long)px * 2 * nd + py] - (closed && x >= cell0 && y >= cell0 ? 1.0 : 0.0);
+            else if (x == y)
+                v = x >= cell0 ? -1.0 : 1.0;  // l, or a filler with its section's sign
+            else
+                v = (closed && ((px == -2 && py >= 0 && y >= cell0) || (py == -2 && px >= 0 && x >= cell0))) ? 1.0 : 0.0;
+            if (apart && v != 0.0) atomicExch(info, -1);
+            put(i, j, r, 0, v);
+        }
+    }
+    grid.sync();
+    const int G = (T + R - 1) / R;
+    bool good = __ldcg(info) == 0;
+    for (int k = 0; k < steps && good; k++) {
+        const int np = pivots(k);
+        const bool last = k == steps - 1;
+        auto load = [&](double (&s)[B][B + 1], const double* tile) {  // false: all zero
+            bool nz = false;
+#pragma unroll
+            for (int e = 0; e < EPT; e++) {
+                const int r = r0 + e * RS;
+                const double v = __ldcg(tile + r * B + c0);
+                nz = nz || v != 0.0;
+                s[r][c0] = v;
+            }
+            return __syncthreads_or(nz) != 0;
+        };
+        auto product = [&](const double (&x)[B][B + 1], const double (&y)[B][B + 1], int r) {
+            double acc = 0.0;
+#pragma unroll
+            for (int q = 0; q < B; q++) acc += x[r][q] * y[q][c0];
+            return acc;
+        };
+        if (tid == 0) s_bad = 0;
+        for (int q = 0; q < np; q++) load(sD[q], panel(k, 0, q) + (long long)pivot(k, q) * B * B);
+        if (tid < 32 * np) {
+            const bool ok = tile_inverse<B>(sD[tid / 32], last, k < TF);
+            if (!__all_sync(0xffffffffu, ok) && (tid & 31) == 0) atomicExch(&s_bad, 1);
+        }
+        __syncthreads();
+        good = s_bad == 0;
+        if (!good) break;
+        for (int item = blockIdx.x; item < T * G; item += gridDim.x) {
+            const int j = item % T, g0 = (item / T) * R;
+            int jp = -1;  // j is pivot tile jp of this step
+            for (int q = 0; q < np; q++)
+                if (j == pivot(k, q)) jp = q;
+            unsigned enz = 0;  // bit q: D_q M_pj is not zero
+            if (jp < 0) {
+#pragma unroll
+                for (int q = 0; q < S; q++) {
+                    if (q >= np) break;
+                    if (load(sA, panel(k, 1, q) + (long long)j * B * B)) {
+                        enz |= 1u << q;
+#pragma unroll
+                        for (int e = 0; e < EPT; e++) sE[q][r0 + e * RS][c0] = product(sD[q], sA, r0 + e * RS);
+                    }
+                    __syncthreads();
+                }
+            }
+            for (int i = g0; i < g0 + R && i < T; i++) {
+                const bool keep = last || in_panel(i, j, k + 1);  // written even when unchanged
+                int ip = -1;
+                for (int q = 0; q < np; q++)
+                    if (i == pivot(k, q)) ip = q;
+                if (jp < 0 && ip < 0 && !enz && !keep) continue;
+                double v[EPT];
+                bool changed = true;
+                if (jp >= 0) {
+                    if (ip == jp) {
+#pragma unroll
+                        for (int e = 0; e < EPT; e++) v[e] = sD[jp][r0 + e * RS][c0];
+                    } else {  // (another pivot's row: zero, and stays zero)
+                        load(sA, panel(k, 0, jp) + (long long)i * B * B);
+#pragma unroll
+                        for (int e = 0; e < EPT; e++) v[e] = -product(sA, sD[jp], r0 + e * RS);
+                    }
+                } else if (ip >= 0) {
+#pragma unroll
+                    for (int e = 0; e < EPT; e++) v[e] = (enz >> ip & 1) ? sE[ip][r0 + e * RS][c0] : 0.0;
+                } else {
+                    changed = keep;
+#pragma unroll
+                    for (int e = 0; e < EPT; e++) v[e] = M[(long long)(i * B + r0 + e * RS) * N + j * B + c0];
+#pragma unroll
+                    for (int q = 0; q < S; q++) {
+                        if (q >= np) break;
+                        if (!(enz >> q & 1)) continue;
+                        if (load(sA, panel(k, 0, q) + (long long)i * B * B)) {
+                            changed = true;
+#pragma unroll
+                            for (int e = 0; e < EPT; e++) v[e] -= product(sA, sE[q], r0 + e * RS);
+                        }
+                        __syncthreads();
+                    }
+                }
+                if (changed) {
+#pragma unroll
+                    for (int e = 0; e < EPT; e++) {
+                        const int r = r0 + e * RS;
+                        if (!last) {
+                            put(i, j, r, k + 1, v[e]);
+                            continue;
+                        }
+                        const int px = __ldg(perm + i * B + r), py = __ldg(perm + j * B + c0);
+                        if (px >= 0 && py >= 0) a[(long long)px * 2 * nd + nd + py] = v[e];
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (!last) grid.sync();
+    }
+    if (good) return;
+    grid.sync();  // every block has left the workspace
+    if (blockIdx.x == 0 && tid == 0) *info = 0;
+    grid.sync();
+    gj_all(nd, a, ws, info);
 }
 
 template <class V>
@@ -271,6 +527,10 @@ int dense_init(DenseCoarse& D, const Geom& g) {
     STG_CK(cudaMalloc(&D.probe, sizeof(d4) * g.nslot));
     STG_CK(cudaMalloc(&D.image, sizeof(d4) * g.nslot));
     STG_CK(cudaMalloc(&D.rd, sizeof(double) * nd));
+    std::vector<std::vector<int>> faces(3);
+    std::vector<int> cells;
+    for (int q = 0; q < D.nd; q++) (comp_of[q] ? faces[comp_of[q] - 1] : cells).push_back(q);
+    STG_TRY(inv_order(D.order, faces, cells));
     STG_CK(cudaMemcpy(D.slot_of, slot_of.data(), sizeof(int) * nd, cudaMemcpyHostToDevice));
     STG_CK(cudaMemcpy(D.comp_of, comp_of.data(), sizeof(int) * nd, cudaMemcpyHostToDevice));
     STG_CK(cudaMemcpy(D.dense_of, dense_of.data(), sizeof(int) * dense_of.size(), cudaMemcpyHostToDevice));
@@ -290,6 +550,7 @@ void dense_free(DenseCoarse& D) {
     cudaFree(D.probe);
     cudaFree(D.image);
     cudaFree(D.rd);
+    inv_order_free(D.order);
     D = DenseCoarse();
 }
 
@@ -367,6 +628,64 @@ int gj_invert(cudaStream_t st, int nd, double* a, double* b, int* info, const do
         b = t;
     }
     *inv = a + nd;  // right half of the final buffer, row stride 2 nd
+    return STG_OK;
+}
+
+// Elimination order of k_inv_blocks: every axis's faces padded to whole tiles, fillers, the
+// cells and l at the end.
+static int inv_tile(int nd) { return nd <= 512 ? 16 : 32; }
+
+int inv_order(InvOrder& O, const std::vector<std::vector<int>>& faces, const std::vector<int>& cells) {
+    int nd = (int)cells.size(), most = 0;
+    for (auto& f : faces) {
+        nd += (int)f.size();
+        most = std::max(most, (int)f.size());
+    }
+    const int B = inv_tile(nd);
+    O.S = (int)faces.size();
+    O.TF = (most + B - 1) / B;
+    std::vector<int> perm;
+    for (int d = 0; d < O.S; d++) {
+        perm.insert(perm.end(), faces[d].begin(), faces[d].end());
+        perm.resize((size_t)(d + 1) * O.TF * B, -1);
+    }
+    const size_t c = (cells.size() + 1 + B - 1) / B * B;
+    perm.resize(perm.size() + c - 1 - cells.size(), -1);
+    perm.insert(perm.end(), cells.begin(), cells.end());
+    perm.push_back(-2);
+    O.N = (int)perm.size();
+    STG_CK(cudaMalloc(&O.perm, sizeof(int) * O.N));
+    STG_CK(cudaMemcpy(O.perm, perm.data(), sizeof(int) * O.N, cudaMemcpyHostToDevice));
+    return STG_OK;
+}
+
+void inv_order_free(InvOrder& O) {
+    cudaFree(O.perm);
+    O = InvOrder();
+}
+
+int inv_blocks(cudaStream_t st, int nd, const InvOrder& O, int closed, double* a, double* b, int* info, const double** inv) {
+    const int B = inv_tile(nd), R = B == 16 ? 3 : 8;
+    int dev = 0, sms = 0, per_sm = 0, N = O.N, TF = O.TF;
+    STG_CK(cudaGetDevice(&dev));
+    STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // tiles per work item: one round of items over the SMs at nd = 304 (three tiles), an
+    // eighth of the products spent on D M_kj at larger sizes
+    const void* fn = O.S == 3 ? (B == 16 ? (const void*)k_inv_blocks<16, 3, 3> : (const void*)k_inv_blocks<32, 8, 3>)
+                              : (B == 16 ? (const void*)k_inv_blocks<16, 3, 2> : (const void*)k_inv_blocks<32, 8, 2>);
+    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, 0));
+    // the pivoted elimination leaves its result in the first buffer for an even nd (the cells
+    // and padded faces of a grid whose size is a multiple of 4 are always even in number)
+    const bool fits = (long long)N * N + 4ll * O.S * B * N <= 2ll * nd * nd && (nd & 1) == 0;
+    if (!fits || per_sm < 1 || sms < 1 || O.S < 2 || O.S > 3) return gj_invert(st, nd, a, b, info, inv, true);
+    STG_CK(cudaMemsetAsync(info, 0, sizeof(int), st));
+    const int T = N / B, items = T * ((T + R - 1) / R);
+    const int g = items < sms ? items : sms;
+    const int* perm = O.perm;
+    void* args[] = {&nd, &N, &TF, &perm, &closed, &a, &b, &info};
+    STG_CK(cudaLaunchCooperativeKernel(fn, dim3((unsigned)g), dim3(TPB), args, 0, st));
+    add_launches(1);
+    *inv = a + nd;
     return STG_OK;
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <functional>
+#include <vector>
 
 #include "internal.cuh"
 
@@ -136,6 +137,12 @@ int reduce_parts(cudaStream_t st, const double* parts, int nparts, double* out);
 int dot64(cudaStream_t st, long long n4, const d4* a, const d4* b, double* out, double* scratch);
 
 // ---------------------------------------------------------------- coarsest dense solve (dense.cu)
+// Elimination order of the coarsest matrix for inv_blocks (device): S sections of TF tiles
+// with one axis's faces each, then the cells and the bordering unknown (-2); -1: fillers
+struct InvOrder {
+    int N = 0, S = 0, TF = 0;
+    int* perm = nullptr;
+};
 struct DenseCoarse {
     int nd = 0;                // number of unknowns present at the coarsest level
     int* slot_of = nullptr;    // dense index -> slot
@@ -149,6 +156,7 @@ struct DenseCoarse {
     d4* probe = nullptr;       // probe vector and its image (slots)
     d4* image = nullptr;
     double* rd = nullptr;      // gathered right-hand side (nd)
+    InvOrder order;
 };
 int dense_init(DenseCoarse& D, const Geom& g);
 void dense_free(DenseCoarse& D);
@@ -167,6 +175,13 @@ int dense_setup_v(cudaStream_t st, DenseCoarse& D, const Geom& g, const d4* V, c
 // all steps in one cooperative launch (not capturable in a CUDA graph), else one launch
 // per pivot; the two give the same inverse bit for bit.
 int gj_invert(cudaStream_t st, int nd, double* a, double* b, int* info, const double** inv, bool coop = false);
+// The same inverse by blocks in the order O, without a pivot search (dense.cu
+// k_inv_blocks), for the matrices of dense_setup and of the 2D coarsest level; closed: ones
+// were added to the cell-cell block. Falls back to gj_invert's elimination, inside the same
+// launch, where a pivot has the wrong sign. Not capturable in a CUDA graph.
+int inv_order(InvOrder& O, const std::vector<std::vector<int>>& faces, const std::vector<int>& cells);
+void inv_order_free(InvOrder& O);
+int inv_blocks(cudaStream_t st, int nd, const InvOrder& O, int closed, double* a, double* b, int* info, const double** inv);
 // x = A^-1 r on the slots (FP32 in/out, FP64 inside)
 int dense_apply32(cudaStream_t st, const DenseCoarse& D, const Geom& g, const float4* r, float4* x);
 int dense_apply64(cudaStream_t st, const DenseCoarse& D, const Geom& g, const d4* r, d4* x);

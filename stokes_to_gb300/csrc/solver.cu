@@ -171,7 +171,7 @@ int update(stg_t* h) {
     // low words of the finest penalty for the double-float residual (P32 holds the high)
     PROF(h, 8, 0.0, split64(h->st, fine(h).g.nslot, fine(h).P64, nullptr, h->Plo));
     // the coarsest matrix's assembly (27 small launches) reads and writes fixed buffers:
-    // replayed as a CUDA graph; its Gauss-Jordan inversion is one cooperative launch
+    // replayed as a CUDA graph; its inversion is one cooperative launch
     GraphCache& G = h->sgraph;
     PROF(h, 8, 0.0,
          graphed(h, G, h->closed ? 2 : 1,
@@ -180,7 +180,7 @@ int update(stg_t* h) {
                                         false);
                  },
                  [](bool) {}));
-    PROF(h, 8, 0.0, gj_invert(h->st, h->dense.nd, h->dense.A, h->dense.Ainv, h->dense.info, &h->dense.inv, true));
+    PROF(h, 8, 0.0, inv_blocks(h->st, h->dense.nd, h->dense.order, h->closed ? 1 : 0, h->dense.A, h->dense.Ainv, h->dense.info, &h->dense.inv));
     h->updated = true;
     return STG_OK;
 }
@@ -1071,6 +1071,8 @@ int stg_set_boundary(stg_t* h, const double* cell_vol, const int32_t* cell_fixed
         for (int d = 0; d < 2; d++)
             STG_CK(cudaMemcpyAsync(ist + h->ncell + d * h->nface, face_fixed[d], sizeof(int) * h->nface, cudaMemcpyHostToDevice,
                                    h->st));
+        h->fixed_cells2d = false;
+        for (size_t q = 0; cell_fixed && q < h->ncell && !h->fixed_cells2d; q++) h->fixed_cells2d = cell_fixed[q] != 0;
         STG_TRY(set_boundary2d(h, dc, cell_fixed ? ist : nullptr, df[0], df[1], ist + h->ncell, ist + h->ncell + h->nface));
         h->closed = closed != 0;
         h->have_boundary = true;

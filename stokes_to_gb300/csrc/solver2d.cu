@@ -504,6 +504,7 @@ struct Ctx2 {
     double *aug0 = nullptr, *aug1 = nullptr;
     const double* inv = nullptr;
     int* info = nullptr;
+    stg::InvOrder order;
 };
 
 namespace stg {
@@ -601,7 +602,7 @@ int setup2(stg_t* h) {
     }
     auto& lv = h->c2->lv;
     // coarsening and the analytic coarsest matrix touch fixed buffers only: replayed as a
-    // CUDA graph; the Gauss-Jordan inverse follows as one cooperative launch
+    // CUDA graph; the inverse follows as one cooperative launch
     auto body = [&]() -> int {
         for (int i = (int)lv.size() - 2; i >= 0; i--) {
             Level2 &c = lv[i], &f = lv[i + 1];
@@ -622,7 +623,12 @@ int setup2(stg_t* h) {
     GraphCache& G = h->sgraph;
     STG_TRY(graphed(h, G, (h->closed ? 2 : 1) | (h->hier_flow ? 4 : 0), body, [](bool) {}));
     // the inversion: one cooperative launch, outside the graph
-    STG_TRY(gj_invert(h->st, lv[0].g.size(), h->c2->aug0, h->c2->aug1, h->c2->info, &h->c2->inv, true));
+    // fixed cells are identity rows among the pressures, which the block elimination's sign
+    // rule does not cover: the pivoted elimination takes them
+    if (h->fixed_cells2d)
+        STG_TRY(gj_invert(h->st, lv[0].g.size(), h->c2->aug0, h->c2->aug1, h->c2->info, &h->c2->inv, true));
+    else
+        STG_TRY(inv_blocks(h->st, lv[0].g.size(), h->c2->order, h->closed ? 1 : 0, h->c2->aug0, h->c2->aug1, h->c2->info, &h->c2->inv));
     h->updated = true;
     return STG_OK;
 }
@@ -694,6 +700,10 @@ int create2d(stg_t* h) {
     STG_TRY(dalloc(&h->c2->aug0, 2ull * nd * nd));
     STG_TRY(dalloc(&h->c2->aug1, 2ull * nd * nd));
     STG_TRY(dalloc(&h->c2->info, 1));
+    std::vector<std::vector<int>> faces(2);
+    std::vector<int> cells;
+    for (int q = 0; q < nd; q++) (q < lv[0].g.off(0) ? cells : faces[q >= lv[0].g.off(1)]).push_back(q);
+    STG_TRY(inv_order(h->c2->order, faces, cells));
     Level2& F = lv.back();
     h->L = L;
     h->n4 = F.g.size() / 4;
@@ -722,6 +732,7 @@ void destroy2d(stg_t* h) {
     cudaFree(h->c2->aug0);
     cudaFree(h->c2->aug1);
     cudaFree(h->c2->info);
+    inv_order_free(h->c2->order);
     delete h->c2;
     h->c2 = nullptr;
 }
