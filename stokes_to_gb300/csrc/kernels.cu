@@ -254,8 +254,10 @@ __global__ void k_to_bf16(Geom g, const float4* __restrict__ x, __nv_bfloat16* _
     h[1] = __floats2bfloat162_rn(v.z, v.w);
 }
 
-// y = FP16(x / *scale) on the box slots (the sweeps' staged penalty copy)
-__global__ void k_to_f16(Geom g, const float4* __restrict__ x, const float* __restrict__ scale, __half* __restrict__ y) {
+// y = FP16(x / *scale) on the box slots (the sweeps' staged penalty copy); infinity on fixed
+// faces, which tells the sweep by cells that they are fixed (scaled penalties stay below 2^15)
+__global__ void k_to_f16(Geom g, const float4* __restrict__ x, const uint8_t* __restrict__ m, const float* __restrict__ scale,
+                         __half* __restrict__ y) {
     long long t = (long long)blockIdx.x * TPB + threadIdx.x;
     if (t >= g.box()) return;
     int i, j, k;
@@ -264,8 +266,9 @@ __global__ void k_to_f16(Geom g, const float4* __restrict__ x, const float* __re
     const float4 v = __ldg(x + s);
     const float inv = 1.f / __ldg(scale);
     __half2* h = reinterpret_cast<__half2*>(y + 4ll * s);
-    h[0] = __floats2half2_rn(v.x * inv, v.y * inv);
-    h[1] = __floats2half2_rn(v.z * inv, v.w * inv);
+    const uint8_t mm = __ldg(m + s);
+    h[0] = __floats2half2_rn(v.x * inv, (mm & MU) ? INFINITY : v.y * inv);
+    h[1] = __floats2half2_rn((mm & MV) ? INFINITY : v.z * inv, (mm & MW) ? INFINITY : v.w * inv);
 }
 
 // largest |x| over the box slots, as the bits of a non-negative float (atomicMax on them
@@ -847,8 +850,8 @@ int prolong_add_bf16(cudaStream_t st, const Geom& gf, const Geom& gc, const __nv
     return STG_OK;
 }
 
-int to_f16(cudaStream_t st, const Geom& g, const float4* x, const float* scale, __half* y) {
-    k_to_f16<<<grid_for(g.box(), TPB), TPB, 0, st>>>(g, x, scale, y);
+int to_f16(cudaStream_t st, const Geom& g, const float4* x, const uint8_t* m, const float* scale, __half* y) {
+    k_to_f16<<<grid_for(g.box(), TPB), TPB, 0, st>>>(g, x, m, scale, y);
     STG_LAUNCH_CK();
     return STG_OK;
 }

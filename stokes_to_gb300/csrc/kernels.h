@@ -64,7 +64,7 @@ int prolong_add_bf16(cudaStream_t st, const Geom& gf, const Geom& gc, const __nv
 int to_bf16(cudaStream_t st, const Geom& g, const float4* x, __nv_bfloat16* y);
 // y = FP16(x / *scale) on the box slots; the per-level scales (level 0 coarsest) from the
 // finest level's penalties: scale[l] = 8^(nlev-1-l) x the power of two that keeps them below 2^15
-int to_f16(cudaStream_t st, const Geom& g, const float4* x, const float* scale, __half* y);
+int to_f16(cudaStream_t st, const Geom& g, const float4* x, const uint8_t* m, const float* scale, __half* y);
 int penalty_scales(cudaStream_t st, const Geom& fine, const float4* P, int nlev, unsigned* scratch, float* scale);
 // coarse descriptor from the fine one (updateSubSystem + finish); flow: velocity penalties
 // by 8 x the smallest free child instead of the sum (the solver's own hierarchy)

@@ -167,7 +167,7 @@ int update(stg_t* h) {
     // FP16 copies of the penalties for the solver's own sweeps, each level divided by a scale
     // that keeps it in FP16's range (11 significant bits: the V-cycle count is the FP32 one)
     PROF(h, 8, 0.0, penalty_scales(h->st, fine(h).g, fine(h).P32, h->L, h->d_pmax, h->d_pscale));
-    for (int i = 0; i < h->L; i++) PROF(h, 8, 0.0, to_f16(h->st, h->lv[i].g, h->lv[i].P32, h->d_pscale + i, h->lv[i].P16));
+    for (int i = 0; i < h->L; i++) PROF(h, 8, 0.0, to_f16(h->st, h->lv[i].g, h->lv[i].P32, h->lv[i].m, h->d_pscale + i, h->lv[i].P16));
     // low words of the finest penalty for the double-float residual (P32 holds the high)
     PROF(h, 8, 0.0, split64(h->st, fine(h).g.nslot, fine(h).P64, nullptr, h->Plo));
     // the coarsest matrix's assembly (27 small launches) reads and writes fixed buffers:
@@ -209,22 +209,22 @@ int sweep(stg_t* h, Level& L, const float4* r, int flag, bool first, Level* C = 
     const float* psc = h->d_pscale + (&L - h->lv.data());
     if (first) {
         // x = 0: the residual is r itself
-        PROF(h, cls, 41.0 * L.g.box(), sweep32(h->st, L.g, vol, r, nullptr, L.x(), L.m, L.P32, flag, fast(h, L), P16, psc));
+        PROF(h, cls, 40.0 * L.g.box(), sweep32(h->st, L.g, vol, r, nullptr, L.x(), L.m, L.P32, flag, fast(h, L), P16, psc));
         return STG_OK;
     }
     if (C) {  // with the coarse correction injected as x is staged: 2 B a slot more
-        PROF(h, cls, 59.0 * L.g.box(),
+        PROF(h, cls, 58.0 * L.g.box(),
              sweep32(h->st, L.g, vol, r, L.x(), L.other(), L.m, L.P32, flag, fast(h, L), P16, psc, C->x(), &C->g));
         L.cur ^= 1;
         return STG_OK;
     }
-    PROF(h, cls, 57.0 * L.g.box(), sweep32(h->st, L.g, vol, r, L.x(), L.other(), L.m, L.P32, flag, fast(h, L), P16, psc));
+    PROF(h, cls, 56.0 * L.g.box(), sweep32(h->st, L.g, vol, r, L.x(), L.other(), L.m, L.P32, flag, fast(h, L), P16, psc));
     L.cur ^= 1;
     return STG_OK;
 }
 
 // The prolongation (injection) can ride on the first post-smoothing sweep: FP32 coarse
-// correction, the solver's own uniform-form sweeps (TMA, FP16 penalty) with x present.
+// correction, the solver's own uniform-form sweeps (FP16 penalty) with x present.
 bool fuse_prolong(const stg_t* h, const Level& F) {
     return !h->reference_cycle && h->opts.method != STG_METHOD_MIXED && h->opts.prolong != 1 && fast(h, F) && F.P16 &&
            sweep_tma_available();

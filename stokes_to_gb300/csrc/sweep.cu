@@ -650,24 +650,10 @@ __global__ void __launch_bounds__(NT, 3) k_sweep_lap(Geom g, float vol, const fl
 // mbarrier counting the bytes, instead of every thread issuing 16-byte copies. The boxes
 // read zero outside the allocation, as the copies did. Everything else is k_sweep_lap.
 constexpr int RNP = 344;  // r / P ring slot in float4s: RN padded to 128 bytes (TMA destinations)
-constexpr int RNP16 = 352;  // P ring slot in FP16 quadruples (8 bytes): RN padded to 128 bytes
-constexpr unsigned XBYTES = XN * 16, RBYTES = RN * 16, RBYTES16 = RN * 8;
+constexpr unsigned XBYTES = XN * 16, RBYTES = RN * 16;
 static_assert(RNP >= RN && (RNP * 16) % 128 == 0 && (XN * 16) % 128 == 0, "TMA ring slots must be 128-byte aligned");
-static_assert(RNP16 >= RN && (RNP16 * 8) % 128 == 0, "TMA ring slots must be 128-byte aligned");
 
-// PB = false: P in FP32, separate rings for r and the computed residual rr (the adapters,
-// which reproduce the reference smoother to FP32 rounding). PB = true (the solver's own
-// sweeps): P staged from the level's FP16 copy (divided by a per-level power-of-two scale,
-// multiplied back on reading), and rr written over r in place in a three-slot ring (rr(i),
-// r(i+1) turning into rr(i+1), r(i+2) in flight): 68.4 -> 55.2 KB of shared memory, so
-// four blocks (32 warps) share an SM instead of three. The kernel is latency- and
-// issue-bound, and the extra warps hide the per-plane barriers. The smoother works with P
-// to 2^-11 relative, which keeps the FP32 smoother's V-cycle count (BF16's 2^-8 did not);
-// the V-cycle is a preconditioner inside FP64 refinement.
-template <bool PB>
-struct SmemT;
-template <>
-struct SmemT<false> {
+struct SmemT {
     float4 x[4 * XN];
     float4 P[3 * RNP];
     float4 r[2 * RNP];
@@ -677,24 +663,6 @@ struct SmemT<false> {
     uint8_t m[4 * XN];
     unsigned long long bar;
 };
-template <>
-struct SmemT<true> {
-    float4 x[4 * XN];
-    uint2 P[3 * RNP16];
-    float4 r[3 * RNP];  // r and rr in one ring
-    float dp[DJ * DK];
-    float dpp[SJ * SK];
-    uint8_t m[4 * XN];
-    unsigned long long bar;
-};
-
-// a staged penalty quadruple as float4: FP32 as it is, or four FP16 values (x, y in the
-// first word, z, w in the second, low half first) times the level's scale
-__device__ __forceinline__ float4 ldv(const float4& v, float) { return v; }
-__device__ __forceinline__ float4 ldv(const uint2& v, float sc) {
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
-    return make_float4(a.x * sc, a.y * sc, b.x * sc, b.y * sc);
-}
 
 // 3D box load of the tensor map at coordinates (c0, c1, c2) into shared memory, counted on bar
 __device__ __forceinline__ void tma3(unsigned dst, const CUtensorMap* map, int c0, int c1, int c2, unsigned bar) {
@@ -731,29 +699,15 @@ __device__ __forceinline__ void fail(int* err) {
     if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(err, 1);
 }
 
-// PRO (with HAS_X and PB): the sweep also applies the coarse-grid correction, x_in = x +
-// inject(xc) (k_prolong_add32's injection: each unmasked unknown of a box slot adds its
-// parent coarse slot's value), to every x plane as it lands in shared memory, so the
-// first post-smoothing sweep replaces the prolongation pass; xout = x_in + the update.
-template <bool HAS_X, bool PB, bool PRO = false>
-__global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_constant__ CUtensorMap tmx,
-                                                             const __grid_constant__ CUtensorMap tmr,
-                                                             const __grid_constant__ CUtensorMap tmp, Geom g, float vol,
-                                                             float4* __restrict__ xout, const uint8_t* __restrict__ m, int flag,
-                                                             int chunk, int* __restrict__ err, const float* __restrict__ pscale,
-                                                             const float4* __restrict__ xc, int c_plane, int c_sz) {
-    static_assert(!PRO || (HAS_X && PB), "the fused prolongation needs x and the FP16 penalty ring");
+// (the adapters' sweep: the reference smoother to FP32 rounding)
+template <bool HAS_X>
+__global__ void __launch_bounds__(NT, 3) k_sweep_tma(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmr,
+                                                    const __grid_constant__ CUtensorMap tmp, Geom g, float vol,
+                                                    float4* __restrict__ xout, const uint8_t* __restrict__ m, int flag, int chunk,
+                                                    int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    SmemT<PB>& S = *reinterpret_cast<SmemT<PB>*>(smem_raw);
-    float4* RR;  // the residual ring: its own array, or the r ring itself
-    if constexpr (PB)
-        RR = S.r;
-    else
-        RR = S.rr;
-    constexpr int PSTR = PB ? RNP16 : RNP;               // P ring slot, elements
-    constexpr unsigned PESZ = PB ? 8u : 16u;             // P element bytes
-    constexpr unsigned PBYTES = PB ? RBYTES16 : RBYTES;  // bytes one P box load delivers
-    const float psc = PB ? __ldg(pscale) : 1.f;          // the FP16 copy's scale
+    SmemT& S = *reinterpret_cast<SmemT*>(smem_raw);
+    float4* RR = S.rr;
     const int n = g.n;
     const int tk = threadIdx.x, tj = threadIdx.y, tid = tj * SK + tk;
     const int k0 = blockIdx.x * SK, j0 = blockIdx.y * SJ, i0 = blockIdx.z * chunk;
@@ -797,7 +751,7 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
     auto tma_x = [&](int slot, int p) { tma3(sx + 16u * slot, &tmx, 4 * (k0 - 1), j0 - 1, p + 1, bar); };
     auto tma_r = [&](unsigned base, int slot, int p, const CUtensorMap* tm) { tma3(base + 16u * slot, tm, 4 * k0, j0, p + 1, bar); };
-    auto tma_p = [&](int slot, int p) { tma3(sP + PESZ * slot, &tmp, 4 * k0, j0, p + 1, bar); };
+    auto tma_p = [&](int slot, int p) { tma3(sP + 16u * slot, &tmp, 4 * k0, j0, p + 1, bar); };
     uint32_t phase = 0;
     // every thread waits for the current phase; a wait that gives up (about a second) makes
     // the whole block record the error and leave at the next barrier
@@ -805,47 +759,6 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         const bool ok = wait_phase(bar, phase);
         phase ^= 1u;
         return ok;
-    };
-    // fused prolongation: the thread's two staged x elements, whether they lie in the
-    // box's (j, k) range, and their parents' offsets in a coarse plane
-    bool pin0 = false, pin1 = false;
-    int cofs0 = 0, cofs1 = 0;
-    if (PRO) {
-        auto setup = [&](const Stage& X, int e, bool& pin, int& cofs) {
-            const int jj = j0 - 2 + e / XK, kk = k0 - 2 + e % XK;
-            pin = X.s >= 0 && jj >= 0 && jj <= n && kk >= 0 && kk <= n;
-            cofs = pin ? ((jj >> 1) + 1) * c_sz + ((kk >> 1) + 1) : 0;
-        };
-        setup(X0, tid, pin0, cofs0);
-        setup(X1, tid + NT, pin1, cofs1);
-    }
-    // the coarse values of plane p for the thread's two elements (zero outside the box)
-    auto coarse = [&](int p, float4& v0, float4& v1) {
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        v0 = v1 = z;
-        if (!PRO || p < 0 || p > n) return;
-        const float4* cp = xc + (long long)((p >> 1) + 1) * c_plane;
-        if (pin0) v0 = __ldg(cp + cofs0);
-        if (pin1) v1 = __ldg(cp + cofs1);
-    };
-    // x plane p in ring slot xs += the coarse values v0, v1, with the masks ma, mb
-    auto inject = [&](int xs, int p, const float4& v0, const float4& v1, uint8_t ma, uint8_t mb) {
-        if (!PRO || p < 0 || p > n) return;
-        auto add = [&](int idx, const float4& v, uint8_t mm) {
-            float4 x = S.x[xs + idx];
-            if (!(mm & MP)) x.x += v.x;
-            if (!(mm & MU)) x.y += v.y;
-            if (!(mm & MV)) x.z += v.z;
-            if (!(mm & MW)) x.w += v.w;
-            S.x[xs + idx] = x;
-        };
-        if (pin0) add(X0.s, v0, ma);
-        if (pin1) add(X1.s, v1, mb);
-    };
-    auto prolong = [&](int xs, int p, uint8_t ma, uint8_t mb) {
-        float4 v0, v1;
-        coarse(p, v0, v1);
-        inject(xs, p, v0, v1, ma, mb);
     };
     uint8_t mr0 = MALL, mr1 = MALL;
     auto fetch_m = [&](int p, const uint8_t* src) {
@@ -870,7 +783,7 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
                         const float4 v = S.x[idx];
                         return Q4<float>{v.x, v.y, v.z, v.w};
                     };
-                    const float4 pv = ldv(S.P[ps + e], psc);
+                    const float4 pv = S.P[ps + e];
                     float o[4];
                     lap_core<float>(q(xb + xi), q(xa + xi), q(xc + xi), q(xb + xi - XK), q(xb + xi + XK), q(xb + xi - 1),
                                     q(xb + xi + 1), Q4<float>{pv.x, pv.y, pv.z, pv.w}, vol, o);
@@ -896,12 +809,12 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         if (!(b ? pok1 : pok0) || p < 0 || p >= n) return;
         const int dk = b ? pdk1 : pdk0;
         const int ri = pdj * RK + dk, xi = (pdj + 1) * XK + (dk + 1);
-        const float4 rc = RR[rr0 + ri], pc = ldv(S.P[p0 + ri], psc);
+        const float4 rc = RR[rr0 + ri], pc = S.P[p0 + ri];
         const uint8_t mo = S.m[m0s + xi];
         const float rL[3] = {rc.y, rc.z, rc.w}, pL[3] = {pc.y, pc.z, pc.w};
         const uint8_t mhi[3] = {S.m[m1s + xi], S.m[m0s + xi + XK], S.m[m0s + xi + 1]};
         const float rh[3] = {RR[rr1 + ri].y, RR[rr0 + ri + RK].z, RR[rr0 + ri + 1].w};
-        const float ph[3] = {ldv(S.P[p1 + ri], psc).y, ldv(S.P[p0 + ri + RK], psc).z, ldv(S.P[p0 + ri + 1], psc).w};
+        const float ph[3] = {S.P[p1 + ri].y, S.P[p0 + ri + RK].z, S.P[p0 + ri + 1].w};
         const uint8_t bit[3] = {MU, MV, MW};
         float num = rc.x, den = 2.f * pc.x;
 #pragma unroll
@@ -916,13 +829,9 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
 
     // ring slots as element offsets (rotated each plane)
     int xm1 = 0 * XN, x0 = 1 * XN, x1 = 2 * XN, x2 = 3 * XN;  // x(i-1), x(i), x(i+1), x(i+2)
-    int pm1 = 0 * PSTR, p0 = 1 * PSTR, p1 = 2 * PSTR;         // P(i-1), P(i), P(i+1)
+    int pm1 = 0 * RNP, p0 = 1 * RNP, p1 = 2 * RNP;         // P(i-1), P(i), P(i+1)
     int r0 = 0 * RNP, r1 = 1 * RNP;                           // r(i), r(i+1)
     int rrm1 = 0 * RN, rr0 = 1 * RN;                          // rr(i-1), rr(i)
-    if constexpr (PB) {  // rr written over r in place: one ring of three slots
-        rrm1 = r0;
-        rr0 = r1;
-    }
     int mm1 = 0 * XN, m0 = 1 * XN, m1 = 2 * XN, m2 = 3 * XN;  // masks of planes i-1 .. i+2
 
     // new x of slot (i, jj, kk) of the current plane (x / mask index xi, rr / P index ri,
@@ -933,7 +842,7 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
     // thread's own (j, k).
     auto update = [&](int i, int jj, int kk, int xi, int ri, int di, float4* dst) {
         float4 xo = HAS_X ? S.x[x0 + xi] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 rv = RR[rr0 + ri], pv = ldv(S.P[p0 + ri], psc);
+        const float4 rv = RR[rr0 + ri], pv = S.P[p0 + ri];
         const uint8_t mo = S.m[m0 + xi];
         const bool jkc = jj < n && kk < n;
         const bool own_col = ((i + jj + kk + flag) & 1) == 0;
@@ -969,7 +878,7 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
     }
     __syncthreads();
     if (tid == 0) {
-        arm_tx(bar, (HAS_X ? 4 * XBYTES : 0) + 3 * PBYTES + 2 * RBYTES);
+        arm_tx(bar, (HAS_X ? 4 * XBYTES : 0) + 3 * RBYTES + 2 * RBYTES);
         if (HAS_X) {
             tma_x(xm1, i0 - 2);
             tma_x(x0, i0 - 1);
@@ -993,18 +902,6 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
     fetch_m(i0 + 2, gm + 3 * plane);
     store_m(m2);
     if (__syncthreads_or(!wait_loads())) return fail(err);
-    if (PRO) {
-        // planes i0-1 .. i0+1 take their masks from the ring (the thread's own entries), i0-2
-        // from memory
-        auto ms = [&](int slot, const Stage& X) { return X.s >= 0 ? S.m[slot + X.s] : (uint8_t)MALL; };
-        const uint8_t* g2 = m + (long long)(i0 - 1) * plane;  // plane i0-2
-        const bool ok2 = i0 - 2 >= 0;
-        prolong(xm1, i0 - 2, ok2 && X0.jk >= 0 ? __ldg(g2 + X0.jk) : (uint8_t)MALL, ok2 && X1.jk >= 0 ? __ldg(g2 + X1.jk) : (uint8_t)MALL);
-        prolong(x0, i0 - 1, ms(mm1, X0), ms(mm1, X1));
-        prolong(x1, i0, ms(m0, X0), ms(m0, X1));
-        prolong(x2, i0 + 1, ms(m1, X0), ms(m1, X1));
-        __syncthreads();
-    }
     // residual of i0-1: x(i0-2, i0-1, i0) = slots (xm1, x0, x1), r(i0-1) = r0, P(i0-1) = pm1, mask(i0-1) = mm1
     residual(i0 - 1, xm1, x0, x1, r0, pm1, mm1, rrm1);
     __syncthreads();
@@ -1012,7 +909,7 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         arm_tx(bar, (HAS_X ? XBYTES : 0) + RBYTES);
         if (HAS_X) tma_x(xm1, i0 + 2);  // x(i0+2) replaces x(i0-2)
-        tma_r(sr, PB ? 2 * RNP : r0, i0 + 1, &tmr);  // r(i0+1): the third slot, or replaces r(i0-1)
+        tma_r(sr, r0, i0 + 1, &tmr);    // r(i0+1) replaces r(i0-1)
     }
     // residual of i0: x(i0-1, i0, i0+1) = (x0, x1, x2), r(i0) = r1, P(i0) = p0, mask(i0) = m0
     residual(i0, x0, x1, x2, r1, p0, m0, rr0);
@@ -1021,10 +918,6 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
     __syncthreads();
     S.dpp[tid] = S.dp[odi];
     if (__syncthreads_or(!wait_loads())) return fail(err);
-    if (PRO) {  // x(i0+2) landed in slot xm1; its masks are in ring slot m2
-        prolong(xm1, i0 + 2, X0.s >= 0 ? S.m[m2 + X0.s] : (uint8_t)MALL, X1.s >= 0 ? S.m[m2 + X1.s] : (uint8_t)MALL);
-        __syncthreads();
-    }
     // rotate to the loop's view at i = i0: x(i0-1..i0+2) = (x0, x1, x2, xm1), r(i0) = r1,
     // r(i0+1) = r0, rr(i0-1) = rrm1, rr(i0) = rr0, P(i0-1) = pm1, masks i0-1 .. i0+2 unchanged
     {
@@ -1033,15 +926,9 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         x0 = x1;
         x1 = x2;
         x2 = t;
-        if constexpr (PB) {  // rr(i0) in slot 1, r(i0+1) in slot 2, slot 0 (rr(i0-1)) free
-            r0 = 0;
-            r1 = rrm1 = 2 * RNP;
-            rr0 = RNP;
-        } else {
-            t = r0;
-            r0 = r1;
-            r1 = t;
-        }
+        t = r0;
+        r0 = r1;
+        r1 = t;
     }
     gm += 4 * plane;  // plane i0+3
     float4* gout = xout + (i0 + 1) * plane + out_jk;
@@ -1050,16 +937,12 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         // stream x(i+3) into the slot of x(i-1), P(i+2) into P(i-1), r(i+2) into r(i)
         if (tid == 0) {
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            arm_tx(bar, (HAS_X ? XBYTES : 0) + PBYTES + RBYTES);
+            arm_tx(bar, (HAS_X ? XBYTES : 0) + RBYTES + RBYTES);
             if (HAS_X) tma_x(xm1, i + 3);
             tma_p(pm1, i + 2);
             tma_r(sr, r0, i + 2, &tmr);
         }
         fetch_m(i + 3, gm);
-        // the coarse values for x(i+3) are loaded now and injected once it has landed, so
-        // their latency hides behind this plane's work
-        float4 pc0, pc1;
-        coarse(i + 3, pc0, pc1);
         residual(i + 1, x0, x1, x2, r1, p1, m1, rrm1);
         __syncthreads();
         pressure(i, rr0, rrm1, p0, p1, m0, m1);
@@ -1075,10 +958,6 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         store_m(mm1);  // mask (i+3) into the slot of mask (i-1)
         if (__syncthreads_or(!wait_loads())) return fail(err);
         S.dpp[tid] = S.dp[odi];
-        if (PRO) {  // x(i+3) landed in slot xm1; its masks are still in registers
-            inject(xm1, i + 3, pc0, pc1, mr0, mr1);
-            __syncthreads();
-        }
         // rotate the rings and advance the plane pointers
         {
             int t = xm1;
@@ -1090,19 +969,12 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
             pm1 = p0;
             p0 = p1;
             p1 = t;
-            if constexpr (PB) {  // (rr(i), r(i+1), free) <- (r(i+1) now rr(i+1), r(i+2), rr(i))
-                t = rr0;
-                rr0 = r1;
-                r1 = rrm1 = r0;
-                r0 = t;
-            } else {
-                t = r0;
-                r0 = r1;
-                r1 = t;
-                t = rrm1;
-                rrm1 = rr0;
-                rr0 = t;
-            }
+            t = r0;
+            r0 = r1;
+            r1 = t;
+            t = rrm1;
+            rrm1 = rr0;
+            rr0 = t;
             t = mm1;
             mm1 = m0;
             m0 = m1;
@@ -1111,6 +983,287 @@ __global__ void __launch_bounds__(NT, PB ? 4 : 3) k_sweep_tma(const __grid_const
         }
         gm += plane;
         gout += plane;
+    }
+}
+
+// ---------------------------------------------------------------- sweep by cells
+// The solver's own Laplacian-form sweep (FP16 penalty copy), one thread per red cell: the
+// cell's pressure and six faces are exactly the unknowns its block solve changes, and every
+// face belongs to one red cell, so a thread forms the seven residuals, solves and updates
+// without exchanging residuals or pressure updates with other threads, without a halo of
+// redundant residuals, and without the black pressures' rows, which nothing uses.
+//
+// A block covers TK (k) x TJ (j) slots, TK TJ = 512, and marches along i; a thread owns the
+// slot pair (k0 + 2 kk, k0 + 2 kk + 1) of its row, one red and one black slot in every plane.
+// Planes of x (one slot more on the low and two on the high side), r and P are staged by one
+// TMA box load each, a plane ahead of their use (x ring of five planes, r and P of three).
+// Neighbouring lanes work on neighbouring rows, whose red slots have opposite k parity, so a
+// warp's 16-byte loads of its red cells (every second slot of two rows) and of any one
+// neighbour of theirs fall into distinct banks.
+//
+// Output: the red slot leaves with its cell. The black slot gets u from the thread's own red
+// cell of the plane before, v and w from its neighbours' cells through shared memory, and is
+// written a plane later, after the barrier. Faces on the tile's and the chunk's high side
+// belong to another block's black slot: they are stored alone, and that block leaves the
+// component out. Slots at i, j or k = n hold fixed faces only: 0.
+//
+// MODE 0: x = 0 (the first sweep: the residual is r); 1: x from memory; 2: x + the parent
+// coarse value (the injection: a fine fixed unknown's parent is fixed, so its value is 0),
+// added to every plane of x once it has landed.
+//
+// Bound: HBM at 256^3 (MODE 1 moves 0.98 GB in 185 us, 5.3 TB/s or 0.78 of the measured copy;
+// the form with one thread a slot, residuals exchanged through shared memory and 17 instead of
+// 5.7 warp instructions a slot took 290 us; MODE 0 131 us, MODE 2 204 us), shared-memory loads
+// next (19 of x a cell, 70 % of the L1 rate). Staging x by component instead, with 4-byte
+// asynchronous copies (255 us) or through registers (270 us), was slower: the transposing
+// stores and the scattered loads of r and P then bound it.
+template <int TK>
+struct CellTile {
+    static constexpr int TJ = 512 / TK, LR = TK / 2;       // rows, pairs of a row
+    static constexpr int PW = LR < 16 ? LR : 16;           // pairs of a row in one warp
+    static constexpr int XW = TK + 4, XR = TJ + 3;         // staged x: k0 - 2 .. k0 + TK + 1, j0 - 1 .. j0 + TJ + 1
+    static constexpr int RW = TK + 2, RR = TJ + 1;         // staged r and P: k0 .. (P: k0 - 1 ..), j0 .. j0 + TJ
+    static constexpr int XPL = (XW * XR + 7) / 8 * 8;      // ring slots, 128-byte multiples (in slots)
+    static constexpr int RPL = (RW * RR + 7) / 8 * 8, PPL = (RW * RR + 15) / 16 * 16;
+    static constexpr unsigned XB = XW * XR * 16, RB = RW * RR * 16, PB = RW * RR * 8;  // box bytes
+    static constexpr int NX = (XW * XR + NT - 1) / NT;     // staged x slots of a thread (MODE 2)
+    static constexpr int XRING = 5, RRING = 3;
+    static constexpr int VN = 2 * (TJ + 1) * LR, WN = (2 * TJ * (LR + 1) + 1) / 2 * 2;  // sv, sw (floats)
+    static constexpr int smem(bool x) { return (x ? XRING * XPL * 16 : 0) + RRING * (RPL * 16 + PPL * 8) + 4 * (VN + WN) + 8; }
+    static_assert((RRING * PPL * 8 + 4 * VN) % 8 == 0, "the mbarrier lies on an 8-byte boundary");
+};
+
+template <int TK, int MODE>
+__global__ void __launch_bounds__(NT, 2) k_sweep_cell(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmr,
+                                                      const __grid_constant__ CUtensorMap tmp, Geom g, float vol,
+                                                      float4* __restrict__ xout, const float* __restrict__ pscale, int flag,
+                                                      int chunk, int* __restrict__ err, const float4* __restrict__ xc, int c_plane,
+                                                      int c_sz) {
+    using C = CellTile<TK>;
+    constexpr int TJ = C::TJ, XW = C::XW, RW = C::RW;
+    // (no static shared memory: the TMA destinations start at the window's aligned origin)
+    extern __shared__ __align__(1024) unsigned char cell_smem[];
+    float4* sx = reinterpret_cast<float4*>(cell_smem);
+    float4* sr = sx + (MODE ? C::XRING * C::XPL : 0);
+    uint2* sp = reinterpret_cast<uint2*>(sr + C::RRING * C::RPL);
+    float (*sv)[TJ + 1][C::LR] = reinterpret_cast<float (*)[TJ + 1][C::LR]>(sp + C::RRING * C::PPL);  // [2]
+    float (*sw)[TJ][C::LR + 1] = reinterpret_cast<float (*)[TJ][C::LR + 1]>(reinterpret_cast<float*>(sv) + C::VN);  // [2]
+    unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(reinterpret_cast<float*>(sw) + C::WN);
+    const int n = g.n, tid = threadIdx.x, lane = tid & 31, pr = lane >> 1;
+    constexpr int WR = 32 / C::PW, WK = C::LR / C::PW;  // rows of a warp, warps side by side in k
+    const int wid = tid >> 5;
+    const int tj = (wid / WK) * WR + 2 * (pr / C::PW) + (lane & 1), kk = (wid % WK) * C::PW + pr % C::PW;
+    const int k0 = blockIdx.x * TK, j0 = blockIdx.y * TJ, i0 = blockIdx.z * chunk;
+    const int i1 = min(i0 + chunk, n);
+    const int j = j0 + tj, kp0 = k0 + 2 * kk;
+    const bool live = j < n && kp0 < n;
+    const int plane = g.sy * g.sz;
+    const float psc = __ldg(pscale), v6 = 6.f * vol;
+
+    // box loads counted on one mbarrier; plane p of the box sits at p + 1 in the arrays, row j
+    // at j + 1, slot k at k + 1 (coordinates in 8-byte units along k)
+    const unsigned bar = (unsigned)__cvta_generic_to_shared(s_bar);
+    const unsigned bx = (unsigned)__cvta_generic_to_shared(sx), br = (unsigned)__cvta_generic_to_shared(sr),
+                   bp_ = (unsigned)__cvta_generic_to_shared(sp);
+    auto xslot = [&](int p) { return ((p + C::XRING) % C::XRING) * C::XPL; };
+    auto load_x = [&](int p) { tma3(bx + 16u * xslot(p), &tmx, 2 * (k0 - 1), j0, p + 1, bar); };
+    auto load_rp = [&](int p) {
+        const int s = p % C::RRING;
+        tma3(br + 16u * (s * C::RPL), &tmr, 2 * (k0 + 1), j0 + 1, p + 1, bar);
+        tma3(bp_ + 8u * (s * C::PPL), &tmp, k0, j0 + 1, p + 1, bar);
+    };
+    unsigned phase = 0;
+    auto wait_loads = [&]() {
+        const bool ok = wait_phase(bar, phase);
+        phase ^= 1u;
+        return ok;
+    };
+
+    // MODE 2: the parent values of the thread's share of a staged plane, and adding them
+    float4 cv[C::NX];
+    int co[C::NX];  // offset in a coarse plane, -1: none
+    if (MODE == 2) {
+#pragma unroll
+        for (int q = 0; q < C::NX; q++) {
+            const int e = tid + q * NT, jj = j0 - 1 + e / XW, k = k0 - 2 + e % XW;
+            co[q] = e < XW * C::XR && k >= -1 && jj <= n + 1 && k <= n + 1 ? ((jj >> 1) + 1) * c_sz + ((k >> 1) + 1) : -1;
+        }
+    }
+    auto fetch_coarse = [&](int p) {
+        const float4* src = xc + (long long)((p >> 1) + 1) * c_plane;
+#pragma unroll
+        for (int q = 0; q < C::NX; q++)
+            if (co[q] >= 0)  // (volatile: issued here, not where the values are used)
+                asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                             : "=f"(cv[q].x), "=f"(cv[q].y), "=f"(cv[q].z), "=f"(cv[q].w)
+                             : "l"(src + co[q]));
+    };
+    auto add_coarse = [&](int p) {
+        float4* dst = sx + xslot(p) + tid;
+#pragma unroll
+        for (int q = 0; q < C::NX; q++) {
+            if (co[q] < 0) continue;
+            float4 v = dst[q * NT];
+            v.x += cv[q].x;
+            v.y += cv[q].y;
+            v.z += cv[q].z;
+            v.w += cv[q].w;
+            dst[q * NT] = v;
+        }
+    };
+
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (tid == 0) {
+        arm_tx(bar, (MODE ? 4 * C::XB : 0) + 2 * (C::RB + C::PB));
+        if (MODE)
+            for (int p = i0 - 1; p <= i0 + 2; p++) load_x(p);
+        load_rp(i0);
+        load_rp(i0 + 1);
+    }
+    if (MODE == 2) fetch_coarse(i0 - 1);
+    if (__syncthreads_or(!wait_loads())) return fail(err);
+    if (MODE == 2) {
+        for (int p = i0 - 1; p <= i0 + 2; p++) {
+            if (p > i0 - 1 && ((p & 1) == 0)) fetch_coarse(p);  // planes 2 P and 2 P + 1 share their parents
+            add_coarse(p);
+        }
+        __syncthreads();
+    }
+
+    float ukeep = 0.f;               // u of this plane's black slot: the last plane's cell's high face
+    float bp = 0.f, bu = 0.f;        // p and u of the last plane's black slot
+    const bool own_v = tj > 0 || j0 == 0;  // the black slots' v is this block's
+    auto write_black = [&](int i) {  // black slot of plane i
+        const int q = (i + j + flag) & 1;
+        const int s = g.slot(i, j, kp0 + 1 - q);
+        const bool own_u = i > i0 || i0 == 0, own_w = q == 0 || kk > 0 || k0 == 0;
+        const float bv = tj > 0 ? sv[i & 1][tj][kk] : 0.f;
+        const float bw = sw[i & 1][tj][q == 0 ? kk + 1 : kk];
+        if (own_u && own_v && own_w) {
+            xout[s] = make_float4(bp, bu, bv, q == 0 || kk > 0 ? bw : 0.f);
+        } else {
+            float* o = reinterpret_cast<float*>(xout + s);
+            o[0] = bp;
+            if (own_u) o[1] = bu;
+            if (own_v) o[2] = bv;
+            if (own_w) o[3] = q == 0 || kk > 0 ? bw : 0.f;
+        }
+    };
+
+    int base = xslot(i0), rs = i0 % C::RRING;  // ring slots of plane i
+    for (int i = i0; i < i1; i++) {
+        const bool more = i + 1 < i1;
+        // x(i + 3) into the slot of x(i - 2), r and P of i + 2 into those of i - 1
+        if (more && tid == 0) {
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            arm_tx(bar, (MODE ? C::XB : 0) + C::RB + C::PB);
+            if (MODE) load_x(i + 3);
+            load_rp(i + 2);
+        }
+        if (MODE == 2 && more && ((i + 3) & 1) == 0) fetch_coarse(i + 3);  // an odd plane's parents are the last plane's
+        if (i > i0 && live) write_black(i - 1);
+        const int rn = rs + 1 < C::RRING ? rs + 1 : 0;  // ring slot of r and P of plane i + 1
+        if (live) {
+            const int q = (i + j + flag) & 1;  // red: (i + j + k + flag) even, k0 even
+            const int ro = tj * RW + 2 * kk + q;
+            const float4* R = sr + rs * C::RPL + ro;
+            const uint2* Q = sp + rs * C::PPL + ro + 1;
+            const uint2 po = *Q;
+            const __half* Qn = reinterpret_cast<const __half*>(sp + rn * C::PPL + ro + 1);
+            const __half* Qh = reinterpret_cast<const __half*>(Q);
+            const float2 pa = __half22float2(*reinterpret_cast<const __half2*>(&po.x)),
+                         pz = __half22float2(*reinterpret_cast<const __half2*>(&po.y));
+            // a fixed face's copy is infinite: its e below is 0, and x is 0 there, so any finite
+            // penalty gives the same residual
+            const float raw[7] = {pa.x * psc, pa.y * psc, pz.x * psc, pz.y * psc,
+                                  __half2float(Qn[1]) * psc, __half2float(Qh[4 * RW + 2]) * psc, __half2float(Qh[4 + 3]) * psc};
+            const float4 r0 = *R;
+            float res[7] = {r0.x, r0.y, r0.z, r0.w, sr[rn * C::RPL + ro].y, R[RW].z, R[1].w};
+            float p0 = 0.f, pb = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+            if (MODE) {
+                constexpr int XP = C::XPL, XL = (C::XRING - 1) * XP;
+                const float4* B = sx + base + (tj + 1) * XW + 2 * kk + q + 2;
+                const float4* A = B + (base >= XP ? -XP : XL);                             // plane i - 1
+                const float4* D = B + (base < XL ? XP : -XL);                              // plane i + 1
+                const float4* E = B + (base < XL - XP ? 2 * XP : -(C::XRING - 2) * XP);    // plane i + 2
+                // the rows of stencil.cuh lap_core, low face at the cell's slot, high face one on
+                const float4 c = B[0], xm = A[0], xp = D[0], ym = B[-XW], yp = B[XW], zm = B[-1], zp = B[1];
+                const float4 xy = D[XW], xz = D[1], yz = B[XW + 1];
+                p0 = c.x;
+                pb = q ? zm.x : zp.x;
+                lo[0] = c.y;
+                lo[1] = c.z;
+                lo[2] = c.w;
+                hi[0] = xp.y;
+                hi[1] = yp.z;
+                hi[2] = zp.w;
+                const float lu = 6.f * c.y - (xm.y + xp.y) - (ym.y + yp.y) - (zm.y + zp.y);
+                const float hu = 6.f * xp.y - (c.y + E[0].y) - (D[-XW].y + xy.y) - (D[-1].y + xz.y);
+                const float lv = 6.f * c.z - (xm.z + xp.z) - (ym.z + yp.z) - (zm.z + zp.z);
+                const float hv = 6.f * yp.z - (A[XW].z + xy.z) - (c.z + B[2 * XW].z) - (B[XW - 1].z + yz.z);
+                const float lw = 6.f * c.w - (xm.w + xp.w) - (ym.w + yp.w) - (zm.w + zp.w);
+                const float hw = 6.f * zp.w - (A[1].w + xz.w) - (B[1 - XW].w + yz.w) - (c.w + B[2].w);
+                float pen[7];
+#pragma unroll
+                for (int d = 0; d < 7; d++) pen[d] = fminf(raw[d], 1e38f);
+                res[0] -= vol * ((hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2])) + pen[0] * p0;
+                res[1] -= vol * (lu - (p0 - xm.x)) + pen[1] * lo[0];
+                res[2] -= vol * (lv - (p0 - ym.x)) + pen[2] * lo[1];
+                res[3] -= vol * (lw - (p0 - zm.x)) + pen[3] * lo[2];
+                res[4] -= vol * (hu - (xp.x - p0)) + pen[4] * hi[0];
+                res[5] -= vol * (hv - (yp.x - p0)) + pen[5] * hi[1];
+                res[6] -= vol * (hw - (zp.x - p0)) + pen[6] * hi[2];
+            }
+            // block solve: e = 1 / diagonal of the free faces (6 vol + P), 0 on fixed ones
+            float el[3], eh[3], num = res[0], den = 2.f * raw[0];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                el[d] = __fdividef(1.f, v6 + raw[1 + d]);
+                eh[d] = __fdividef(1.f, v6 + raw[4 + d]);
+                num += vol * (res[1 + d] * el[d] - res[4 + d] * eh[d]);
+                den -= vol * vol * (el[d] + eh[d]);
+            }
+            const float dp = den != 0.f ? __fdividef(num, den) : 0.f, vdp = vol * dp;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                lo[d] += (res[1 + d] + vdp) * el[d];
+                hi[d] += (res[4 + d] - vdp) * eh[d];
+            }
+            const int k = kp0 + q;
+            const int s = g.slot(i, j, k);
+            xout[s] = make_float4(p0 + dp, lo[0], lo[1], lo[2]);
+            // high faces that lie in another block's slots
+            if (!more && i1 < n) reinterpret_cast<float*>(xout + s + plane)[1] = hi[0];
+            if (tj == TJ - 1 && j + 1 < n) reinterpret_cast<float*>(xout + s + g.sz)[2] = hi[1];
+            if (q && kk == C::LR - 1 && k + 1 < n) reinterpret_cast<float*>(xout + s + 1)[3] = hi[2];
+            sv[i & 1][tj + 1][kk] = hi[1];
+            sw[i & 1][tj][kk + 1] = hi[2];
+            bp = pb;
+            bu = ukeep;
+            ukeep = hi[0];
+        }
+        base = base < (C::XRING - 1) * C::XPL ? base + C::XPL : 0;
+        rs = rn;
+        if (!more) break;
+        const bool ok = wait_loads();
+        if (MODE == 2) add_coarse(i + 3);
+        if (__syncthreads_or(!ok)) return fail(err);
+    }
+    __syncthreads();
+    if (live) write_black(i1 - 1);
+    // the slots at k, j and i = n
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool end_k = k0 + TK >= n, end_j = j0 + TJ >= n;
+    const int ie = i1 == n ? n : i1 - 1;  // the last chunk also takes plane n
+    for (int i = i0; i <= ie; i++) {
+        if (i == n && live) xout[g.slot(n, j, kp0)] = xout[g.slot(n, j, kp0 + 1)] = z;
+        if (end_k && kk == 0 && j < n) xout[g.slot(i, j, n)] = z;
+        if (end_j && tj == 0 && kp0 < n) xout[g.slot(i, n, kp0)] = xout[g.slot(i, n, kp0 + 1)] = z;
+        if (end_k && end_j && tid == 0) xout[g.slot(i, n, n)] = z;
     }
 }
 
@@ -1148,42 +1301,77 @@ bool slot_map(EncodeTiled enc, CUtensorMap* map, const void* base, const Geom& g
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// the same for an FP16 slot array (four 2-byte values per slot)
-bool slot_map16(EncodeTiled enc, CUtensorMap* map, const void* base, const Geom& g, int bk, int bj) {
-    const cuuint64_t dims[3] = {(cuuint64_t)g.sz * 4, (cuuint64_t)g.sy, (cuuint64_t)g.sx};
-    const cuuint64_t strides[2] = {(cuuint64_t)g.sz * 8, (cuuint64_t)g.sy * g.sz * 8};
-    const cuuint32_t box[3] = {(cuuint32_t)(4 * bk), (cuuint32_t)bj, 1}, es[3] = {1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // per device: kernel attributes set, and the flag a TMA sweep sets when its wait gave up
 bool g_attr_set[MAX_DEVICES] = {}, g_tattr_set[MAX_DEVICES] = {};
 int* g_sweep_err[MAX_DEVICES] = {};
 int g_sms[MAX_DEVICES] = {};
 
-// Planes per block of the TMA sweep on an n^3 box. On large boxes a block marches through
-// its chunk plane after plane (plus about three planes of prologue), and the blocks run in
-// waves of SMs x resident blocks, so the chunk minimises waves x (chunk + 3), the longest
-// chain of planes an SM works through (at n = 256: 37 planes, 2.9 waves, 2 % faster than
-// 32 planes and 3.4 waves). On the coarse levels, where the blocks are few and latency
-// sets the time, that choice measured 2 % slower than the fixed lengths kept there.
-int tma_chunk(int dev, int n, bool fp16_pen) {
-    if (n < 192) return n >= 96 ? 8 : n >= 48 ? 4 : n >= 24 ? 2 : 1;
+// Planes per block of the sweep by cells on an n^3 box: a block marches through its chunk
+// plane after plane (its prologue costs about four), and the blocks run in waves of SMs x
+// resident blocks, so the chunk minimises waves x (chunk + 4), the longest chain of planes an
+// SM works through (n = 256: 37 planes in three waves, n = 128: 15 in one, n = 64: 2 in one).
+int cell_chunk(int dev, int n, int tk, int resident) {
     if (!g_sms[dev] && cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sms[dev] = 0;
-    const long long slots = (long long)(g_sms[dev] > 0 ? g_sms[dev] : 152) * (fp16_pen ? 4 : 3);
-    const long long plane_blocks = (long long)((n + SK - 1) / SK) * ((n + SJ - 1) / SJ);
+    const long long slots = (long long)resident * (g_sms[dev] > 0 ? g_sms[dev] : 152);
+    const int tj = 512 / tk;
+    const long long plane_blocks = (long long)((n + tk - 1) / tk) * ((n + tj - 1) / tj);
     int best = 1;
     long long best_cost = -1;
     for (int c = 1; c <= n; c++) {
         const long long blocks = plane_blocks * ((n + c - 1) / c);
-        const long long cost = ((blocks + slots - 1) / slots) * (c + 3);
+        const long long cost = ((blocks + slots - 1) / slots) * (c + 4);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = c;
         }
     }
     return best;
+}
+
+// tensor map of an array of `per`-word slots (8-byte words: 2 for FP32 slots, 1 for FP16
+// ones), box bk slots x bj rows x 1 plane; parts of a box outside the array read as zero
+bool cell_map(EncodeTiled enc, CUtensorMap* map, const void* base, const Geom& g, int per, int bk, int bj) {
+    const cuuint64_t dims[3] = {(cuuint64_t)g.sz * per, (cuuint64_t)g.sy, (cuuint64_t)g.sx};
+    const cuuint64_t strides[2] = {(cuuint64_t)g.sz * per * 8, (cuuint64_t)g.sy * g.sz * per * 8};
+    const cuuint32_t box[3] = {(cuuint32_t)(per * bk), (cuuint32_t)bj, 1}, es[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int TK>
+int launch_cell(cudaStream_t st, int dev, EncodeTiled enc, const Geom& g, float vol, const float4* r, const float4* xin, float4* xout,
+                const __half* P16, const float* psc, int flag, const float4* xc, const Geom* gc, bool* done) {
+    using C = CellTile<TK>;
+    static bool set[MAX_DEVICES] = {};
+    if (!set[dev]) {
+        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(false)));
+        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(true)));
+        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(true)));
+        set[dev] = true;
+    }
+    CUtensorMap mx{}, mr{}, mp{};
+    *done = cell_map(enc, &mr, r, g, 2, C::RW, C::RR) && cell_map(enc, &mp, P16, g, 1, C::RW, C::RR) &&
+            (!xin || cell_map(enc, &mx, xin, g, 2, C::XW, C::XR));
+    if (!*done) return STG_OK;
+    const int chunk = cell_chunk(dev, g.n, TK, xin ? 2 : 4);
+    const dim3 grid((g.n + TK - 1) / TK, (g.n + C::TJ - 1) / C::TJ, (g.n + chunk - 1) / chunk);
+    int* err = g_sweep_err[dev];
+    if (!xin)
+        k_sweep_cell<TK, 0><<<grid, NT, C::smem(false), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+    else if (!xc)
+        k_sweep_cell<TK, 1><<<grid, NT, C::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+    else
+        k_sweep_cell<TK, 2><<<grid, NT, C::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, xc, gc->sy * gc->sz, gc->sz);
+    STG_LAUNCH_CK();
+    return STG_OK;
+}
+
+// the flag a TMA sweep sets when its wait gave up, per device
+int sweep_err_init(int dev) {
+    if (g_sweep_err[dev]) return STG_OK;
+    STG_CK(cudaMalloc((void**)&g_sweep_err[dev], sizeof(int)));
+    STG_CK(cudaMemset(g_sweep_err[dev], 0, sizeof(int)));
+    return STG_OK;
 }
 
 }  // namespace
@@ -1214,58 +1402,45 @@ int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const fl
         STG_CK(cudaFuncSetAttribute(k_sweep_lap<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_l));
         g_attr_set[dev] = true;
     }
+    if (lap && P16 && p16_scale && encoder()) {
+        // the solver's own sweeps; narrower tiles (with more rows) where a row has fewer slots
+        STG_TRY(sweep_err_init(dev));
+        bool done = false;
+        const auto go = g.n > 32 ? launch_cell<64> : g.n > 16 ? launch_cell<32> : launch_cell<16>;
+        STG_TRY(go(st, dev, encoder(), g, vol, r, xin, xout, P16, p16_scale, flag, xc, gc, &done));
+        if (done) return STG_OK;
+    }
+    if (xc) {
+        set_error("sweep32: the fused prolongation needs the TMA sweep by cells");
+        return STG_E_UNSUPPORTED;
+    }
     // planes per block: long marches on big grids (prologue amortised), short ones on the
     // coarse levels, where the sequential march, not bandwidth, sets the time
     const int chunk = g.n >= 192 ? 32 : g.n >= 96 ? 8 : g.n >= 48 ? 4 : g.n >= 24 ? 2 : 1;
     dim3 grid((g.n + SK) / SK, (g.n + SJ) / SJ, (g.n + chunk) / chunk), block(SK, SJ);
     // the TMA sweep's tiles and chunks cover [0, n) and take the high-side slots (k, j or
-    // i = n) with the last ones (at n = 256: 8 x 32 x 7 blocks of 37 planes)
-    const int chunk_t = tma_chunk(dev, g.n, P16 != nullptr);
-    const dim3 grid_t((g.n + SK - 1) / SK, (g.n + SJ - 1) / SJ, (g.n + chunk_t - 1) / chunk_t);
+    // i = n) with the last ones
+    const dim3 grid_t((g.n + SK - 1) / SK, (g.n + SJ - 1) / SJ, (g.n + chunk - 1) / chunk);
     if (lap && encoder()) {
-        const int smem_t = (int)sizeof(SmemT<false>), smem_b = (int)sizeof(SmemT<true>);
+        const int smem_t = (int)sizeof(SmemT);
         if (!g_tattr_set[dev]) {
-            STG_CK(cudaFuncSetAttribute(k_sweep_tma<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
-            STG_CK(cudaFuncSetAttribute(k_sweep_tma<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
-            STG_CK(cudaFuncSetAttribute(k_sweep_tma<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_b));
-            STG_CK(cudaFuncSetAttribute(k_sweep_tma<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_b));
-            STG_CK(cudaFuncSetAttribute(k_sweep_tma<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_b));
-            STG_CK(cudaMalloc((void**)&g_sweep_err[dev], sizeof(int)));
-            STG_CK(cudaMemset(g_sweep_err[dev], 0, sizeof(int)));
+            STG_CK(cudaFuncSetAttribute(k_sweep_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
+            STG_CK(cudaFuncSetAttribute(k_sweep_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
+            STG_TRY(sweep_err_init(dev));
             g_tattr_set[dev] = true;
         }
         CUtensorMap mx{}, mr{}, mp{};
         const EncodeTiled enc = encoder();
-        if (P16 && !p16_scale) P16 = nullptr;  // the FP16 copy needs its scale
-        const bool ok = (!xin || slot_map(enc, &mx, xin, g, XK, XJ)) && slot_map(enc, &mr, r, g, RK, RJ) &&
-                        (P16 ? slot_map16(enc, &mp, P16, g, RK, RJ) : slot_map(enc, &mp, P, g, RK, RJ));
+        const bool ok = (!xin || slot_map(enc, &mx, xin, g, XK, XJ)) && slot_map(enc, &mr, r, g, RK, RJ) && slot_map(enc, &mp, P, g, RK, RJ);
         if (ok) {
             int* err = g_sweep_err[dev];
-            if (xc && P16 && xin) {
-                k_sweep_tma<true, true, true><<<grid_t, block, smem_b, st>>>(mx, mr, mp, g, vol, xout, m, flag, chunk_t, err, p16_scale,
-                                                                             xc, gc->sy * gc->sz, gc->sz);
-                STG_LAUNCH_CK();
-                return STG_OK;
-            }
-            if (xc) {
-                set_error("sweep32: the fused prolongation needs x and the FP16 penalty");
-                return STG_E_UNSUPPORTED;
-            }
-            if (P16 && xin)
-                k_sweep_tma<true, true><<<grid_t, block, smem_b, st>>>(mx, mr, mp, g, vol, xout, m, flag, chunk_t, err, p16_scale, nullptr, 0, 0);
-            else if (P16)
-                k_sweep_tma<false, true><<<grid_t, block, smem_b, st>>>(mr, mr, mp, g, vol, xout, m, flag, chunk_t, err, p16_scale, nullptr, 0, 0);
-            else if (xin)
-                k_sweep_tma<true, false><<<grid_t, block, smem_t, st>>>(mx, mr, mp, g, vol, xout, m, flag, chunk_t, err, nullptr, nullptr, 0, 0);
+            if (xin)
+                k_sweep_tma<true><<<grid_t, block, smem_t, st>>>(mx, mr, mp, g, vol, xout, m, flag, chunk, err);
             else
-                k_sweep_tma<false, false><<<grid_t, block, smem_t, st>>>(mr, mr, mp, g, vol, xout, m, flag, chunk_t, err, nullptr, nullptr, 0, 0);
+                k_sweep_tma<false><<<grid_t, block, smem_t, st>>>(mr, mr, mp, g, vol, xout, m, flag, chunk, err);
             STG_LAUNCH_CK();
             return STG_OK;
         }
-    }
-    if (xc) {
-        set_error("sweep32: the fused prolongation needs the TMA sweep");
-        return STG_E_UNSUPPORTED;
     }
     if (xin && lap)
         k_sweep_lap<true><<<grid, block, smem_l, st>>>(g, vol, r, xin, xout, m, P, flag, chunk);
