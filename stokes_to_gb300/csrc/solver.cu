@@ -1073,6 +1073,23 @@ int stg_set_boundary(stg_t* h, const double* cell_vol, const int32_t* cell_fixed
                                    h->st));
         h->fixed_cells2d = false;
         for (size_t q = 0; cell_fixed && q < h->ncell && !h->fixed_cells2d; q++) h->fixed_cells2d = cell_fixed[q] != 0;
+        // Laplacian form: boundary faces and no cell fixed, one vol on the free faces
+        bool lap = !h->fixed_cells2d;
+        double fv = NAN;
+        const int n2 = h->n;
+        for (int d = 0; d < 2 && lap; d++)
+            for (size_t q = 0; q < h->nface && lap; q++) {
+                const size_t c = d == 0 ? q / n2 : q % (n2 + 1);  // coordinate along d
+                if (face_fixed[d][q]) continue;
+                if (c == 0 || c == (size_t)n2) lap = false;
+                if (std::isnan(fv)) fv = face_vol[d][q];
+                if (!(face_vol[d][q] == fv)) lap = false;
+            }
+        h->lap2d = lap && !std::isnan(fv);
+        if (h->lap2d && fv != h->vol2d) {
+            h->vol2d = fv;
+            h->vol2d_changes++;
+        }
         STG_TRY(set_boundary2d(h, dc, cell_fixed ? ist : nullptr, df[0], df[1], ist + h->ncell, ist + h->ncell + h->nface));
         h->closed = closed != 0;
         h->have_boundary = true;

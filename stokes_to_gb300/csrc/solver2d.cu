@@ -13,6 +13,8 @@
 //   coarsest   stoke/StokeFlowDirectSolve.cpp:6-133 (analytic dense matrix), inverted on
 //              the GPU by Gauss-Jordan and applied as a GEMV
 //   V-cycle    common_cpx/MultigridSolve.cpp:73-106 in FP32; Krylov as in 3D (solve_core).
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <vector>
 
@@ -484,6 +486,239 @@ __global__ void k2_update(int n, const float* __restrict__ p, const float* __res
 
 unsigned g1(long long n) { return (unsigned)((n + TPB - 1) / TPB); }
 
+// ------------------------------------------------------------------ Laplacian-form V-cycle
+// Where every boundary face is fixed, no cell is and the free faces share one vol, A is vol x
+// (the 5-point face Laplacian - grad p) + penalty on vectors that are zero on fixed faces (the
+// edge-diagonal terms of grad-div and curl-curl cancel, as in 3D), so the solver's own V-cycle
+// runs the smoother in correction form, x <- x + P_c (r - A x), one thread per cell of the
+// colour: its pressure and four faces are exactly the unknowns the box solve changes. A level
+// takes five passes (two sweeps, the restricted residual, two sweeps of which the first adds
+// the prolonged correction on reading) instead of 28 kernels, copies and memsets.
+//
+// Vectors are row-major with a zero halo, by component (p, u, v), so neighbours lie at fixed
+// offsets: value (x, y) of a component at (y + 1) S + x + 1. The finest right-hand side and
+// result are converted on the way in and out.
+struct Lv2 {
+    int n, S, NS;  // cells per axis, row stride, component stride
+    float vol, lap;
+    const float* P;    // penalties (3 NS; 0 on fixed faces)
+    const uint8_t* m;  // NS: bit 0 u fixed, bit 1 v fixed
+    float *r, *xa, *xb;  // 3 NS each
+    __device__ int at(int x, int y) const { return (y + 1) * S + x + 1; }
+};
+constexpr int MAXL2 = 12;
+struct V2 {
+    Lv2 lv[MAXL2];
+    G2d fine, coarse;
+    int L;
+    const double* inv;  // coarsest inverse, row stride ld, blocked coarse order
+    int nd, ld;
+    const int* map;     // blocked coarse index -> padded offset (-1: padding)
+};
+
+// padded offset (component included) of blocked index t, or -1
+__device__ __forceinline__ int pad_index(const G2d& g, const Lv2& L, int t) {
+    int kind, x, y;
+    g.decode(t, kind, x, y);
+    if (kind >= 0 && !g.face_ok(x, y, kind)) return -1;
+    return (kind + 1) * L.NS + L.at(x, y);
+}
+__global__ void k2_pad_index(G2d g, Lv2 L, int* __restrict__ map) {
+    const int t = blockIdx.x * TPB + threadIdx.x;
+    if (t < g.size()) map[t] = pad_index(g, L, t);
+}
+__global__ void k2_pad_coef(G2d g, Lv2 L, const float* __restrict__ pen, const uint8_t* __restrict__ fixed, float* __restrict__ P,
+                            uint8_t* __restrict__ m) {
+    const int t = blockIdx.x * TPB + threadIdx.x;
+    if (t >= L.n * L.n) return;  // the faces at x, y = n are fixed: 0 penalty (as allocated), never updated
+    const int x = t % L.n, y = t / L.n, a = L.at(x, y);
+    const int f0 = g.face(x, y, 0), f1 = g.face(x, y, 1);
+    P[a] = pen[g.cell(x, y)];
+    P[L.NS + a] = pen[f0];
+    P[2 * L.NS + a] = pen[f1];
+    m[a] = (uint8_t)((fixed[f0] ? 1 : 0) | (fixed[f1] ? 2 : 0));
+}
+
+// x and r change while the one-launch V-cycle runs: read through L2
+__device__ __forceinline__ float ldv2(const float* p) { return __ldcg(p); }
+
+// One colour of the smoother, cells t0, t0 + step, ...: xo = x + P_c (r - A x); HX false: x = 0.
+// PRO: x is first corrected by the parent values of xc on level C (a fixed face's parent is
+// fixed, so its value is 0). The other colour's pressures are copied.
+template <bool HX, bool PRO>
+__device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, const Lv2& C, const float* xc, float* xo, int t0,
+                                       int step) {
+    const int h = L.n >> 1, S = L.S, NS = L.NS;
+    for (int t = t0; t < L.n * h; t += step) {
+        const int y = t / h, xx = 2 * (t - y * h) + ((y + flag) & 1);
+        const int i = L.at(xx, y);
+        const int ob = (xx & 1) ? i - 1 : i + 1;  // the pair's other cell
+        auto V = [&](int c, int a, int b) {
+            float v = ldv2(x + c * NS + i + b * S + a);
+            if (PRO) v += ldv2(xc + c * C.NS + C.at((xx + a) >> 1, (y + b) >> 1));
+            return v;
+        };
+        const uint8_t m0 = __ldg(L.m + i), m1 = __ldg(L.m + i + 1), m2 = __ldg(L.m + i + S);
+        const bool fa = m0 & 1, fb = (m1 & 1) || xx + 1 == L.n, fc = m0 & 2, fd = (m2 & 2) || y + 1 == L.n;
+        const float Pp = __ldg(L.P + i), Pa = __ldg(L.P + NS + i), Pb = __ldg(L.P + NS + i + 1), Pc = __ldg(L.P + 2 * NS + i),
+                    Pd = __ldg(L.P + 2 * NS + i + S);
+        float rp = ldv2(L.r + i), ra = ldv2(L.r + NS + i), rb = ldv2(L.r + NS + i + 1), rc = ldv2(L.r + 2 * NS + i),
+              rd = ldv2(L.r + 2 * NS + i + S);
+        float p = 0.f, ua = 0.f, ub = 0.f, vc = 0.f, vd = 0.f, pb = 0.f;
+        if (HX) {
+            p = V(0, 0, 0);
+            const float pl = V(0, -1, 0), pr = V(0, 1, 0), pd = V(0, 0, -1), pu = V(0, 0, 1);
+            pb = (xx & 1) ? pl : pr;
+            ua = V(1, 0, 0);
+            ub = V(1, 1, 0);
+            vc = V(2, 0, 0);
+            vd = V(2, 0, 1);
+            const float la = 4.f * ua - (V(1, -1, 0) + ub) - (V(1, 0, -1) + V(1, 0, 1));
+            const float lb = 4.f * ub - (ua + V(1, 2, 0)) - (V(1, 1, -1) + V(1, 1, 1));
+            const float lc = 4.f * vc - (V(2, -1, 0) + V(2, 1, 0)) - (V(2, 0, -1) + vd);
+            const float ld = 4.f * vd - (V(2, -1, 1) + V(2, 1, 1)) - (vc + V(2, 0, 2));
+            rp -= L.vol * ((ub - ua) + (vd - vc)) + Pp * p;
+            ra -= L.vol * (la - (p - pl)) + Pa * ua;
+            rb -= L.vol * (lb - (pr - p)) + Pb * ub;
+            rc -= L.vol * (lc - (p - pd)) + Pc * vc;
+            rd -= L.vol * (ld - (pu - p)) + Pd * vd;
+        }
+        if (fa) ra = 0.f;
+        if (fb) rb = 0.f;
+        if (fc) rc = 0.f;
+        if (fd) rd = 0.f;
+        // the box solve of k2_smooth
+        const SymInv2 Kx(4.f * L.lap + Pa, 4.f * L.lap + Pb, (fa || fb) ? 0.f : L.lap);
+        const SymInv2 Ky(4.f * L.lap + Pc, 4.f * L.lap + Pd, (fc || fd) ? 0.f : L.lap);
+        const float ga = fa ? 0.f : -L.vol, gb = fb ? 0.f : L.vol, gc = fc ? 0.f : -L.vol, gd = fd ? 0.f : L.vol;
+        float za, zb, zc, zd, wa, wb, wc, wd;
+        Kx.apply(ra, rb, za, zb);
+        Ky.apply(rc, rd, zc, zd);
+        Kx.apply(ga, gb, wa, wb);
+        Ky.apply(gc, gd, wc, wd);
+        const float schur = Pp - (ga * wa + gb * wb + gc * wc + gd * wd);
+        const float num = rp - (ga * za + gb * zb + gc * zc + gd * zd);
+        const float dp = schur != 0.f ? num / schur : 0.f;  // a cell between four fixed faces keeps its pressure
+        xo[i] = p + dp;
+        xo[ob] = pb;
+        xo[NS + i] = ua + (za - dp * wa);
+        xo[NS + i + 1] = ub + (zb - dp * wb);
+        xo[2 * NS + i] = vc + (zc - dp * wc);
+        xo[2 * NS + i + S] = vd + (zd - dp * wd);
+    }
+}
+
+// C.r = the 4-child sums of r - A x, 0 on fixed coarse faces; one coarse cell and its two low
+// faces a thread (the faces at X, Y = n are fixed: 0, as allocated)
+__device__ __forceinline__ void restrict2(const Lv2& L, const float* x, const Lv2& C, int t0, int step) {
+    const int S = L.S, NS = L.NS;
+    for (int t = t0; t < C.n * C.n; t += step) {
+        const int Y = t / C.n, X = t - Y * C.n, o = C.at(X, Y);
+        float sp = 0.f, su = 0.f, sw = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int i = L.at(2 * X + (q & 1), 2 * Y + (q >> 1));
+            const uint8_t m = __ldg(L.m + i);
+            const float *xp = x + i, *xu = x + NS + i, *xv = x + 2 * NS + i;
+            const float p = ldv2(xp), u = ldv2(xu), v = ldv2(xv), ub = ldv2(xu + 1), vd = ldv2(xv + S);
+            const float lu = 4.f * u - (ldv2(xu - 1) + ub) - (ldv2(xu - S) + ldv2(xu + S));
+            const float lv = 4.f * v - (ldv2(xv - 1) + ldv2(xv + 1)) - (ldv2(xv - S) + vd);
+            sp += ldv2(L.r + i) - (L.vol * ((ub - u) + (vd - v)) + __ldg(L.P + i) * p);
+            if (!(m & 1)) su += ldv2(L.r + NS + i) - (L.vol * (lu - (p - ldv2(xp - 1))) + __ldg(L.P + NS + i) * u);
+            if (!(m & 2)) sw += ldv2(L.r + 2 * NS + i) - (L.vol * (lv - (p - ldv2(xp - S))) + __ldg(L.P + 2 * NS + i) * v);
+        }
+        const uint8_t mc = __ldg(C.m + o);
+        C.r[o] = sp;
+        C.r[C.NS + o] = (mc & 1) ? 0.f : su;
+        C.r[2 * C.NS + o] = (mc & 2) ? 0.f : sw;
+    }
+}
+
+__device__ __forceinline__ void pad_in(const V2& v, const Lv2& L, const float* rhs, int t0, int step) {
+    for (int t = t0; t < v.fine.size(); t += step) {
+        const int a = pad_index(v.fine, L, t);
+        if (a >= 0) L.r[a] = __ldg(rhs + t);
+    }
+}
+__device__ __forceinline__ void pad_out(const V2& v, const Lv2& L, const float* x, float* out, int t0, int step) {
+    for (int t = t0; t < v.fine.size(); t += step) {
+        const int a = pad_index(v.fine, L, t);
+        out[t] = a >= 0 ? ldv2(x + a) : 0.f;
+    }
+}
+
+// levels too large for the one-launch part, a pass per launch
+template <bool HX, bool PRO>
+__global__ void __launch_bounds__(TPB) k2v_sweep(Lv2 L, int flag, const float* x, Lv2 C, const float* xc, float* xo) {
+    sweep2<HX, PRO>(L, flag, x, C, xc, xo, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+__global__ void __launch_bounds__(TPB) k2v_restrict(Lv2 L, const float* x, Lv2 C) {
+    restrict2(L, x, C, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+__global__ void __launch_bounds__(TPB) k2v_in(const __grid_constant__ V2 v, const float* __restrict__ rhs) {
+    pad_in(v, v.lv[v.L - 1], rhs, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+__global__ void __launch_bounds__(TPB) k2v_out(const __grid_constant__ V2 v, float* __restrict__ out) {
+    pad_out(v, v.lv[v.L - 1], v.L == 1 ? v.lv[0].xa : v.lv[v.L - 1].xb, out, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+__device__ __forceinline__ void gemv_row2(const V2& v, int row, int lane) {
+    const Lv2& L = v.lv[0];
+    double s = 0;
+    for (int c = lane; c < v.nd; c += 32) {
+        const int a = __ldg(v.map + c);
+        if (a >= 0) s += __ldg(v.inv + (long long)row * v.ld + c) * (double)ldv2(L.r + a);
+    }
+    s = warp_sum(s);
+    const int a = __ldg(v.map + row);
+    if (lane == 0 && a >= 0) L.xa[a] = (float)s;
+}
+__global__ void __launch_bounds__(TPB) k2v_gemv(const __grid_constant__ V2 v) {
+    const int row = (blockIdx.x * TPB + threadIdx.x) >> 5;
+    if (row < v.nd) gemv_row2(v, row, threadIdx.x & 31);
+}
+
+// The V-cycle of levels top .. 0 by one thread-block cluster, a cluster barrier between the
+// passes (about 1 us a pass against 2 to 4 us for a kernel of a graph): parts 1 the way down, 2
+// the coarsest solve, 4 the way up. rhs / out: blocked finest vectors when top is the finest.
+// A level's passes are a few loads deep for each thread, so latency bounds it. 64^2 (levels to
+// 8^2, 18 passes): a design iteration with about 34 V-cycles 12.2 -> 5.65 ms; 512^2, two levels
+// above the cluster's: a solve of 46 V-cycles 22.3 -> 8.7 ms.
+constexpr int VT = 512;  // threads of a cluster's block
+__global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, int top, int parts, const float* rhs, float* out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int t0 = blockIdx.x * VT + threadIdx.x, step = gridDim.x * VT;
+    if (parts & 1) {
+        if (rhs) {
+            pad_in(v, v.lv[top], rhs, t0, step);
+            cl.sync();
+        }
+        for (int i = top; i >= 1; i--) {
+            const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
+            sweep2<false, false>(L, 0, nullptr, C, nullptr, L.xa, t0, step);
+            cl.sync();
+            sweep2<true, false>(L, 1, L.xa, C, nullptr, L.xb, t0, step);
+            cl.sync();
+            restrict2(L, L.xb, C, t0, step);
+            cl.sync();
+        }
+    }
+    if (parts & 2) {
+        for (int row = t0 >> 5; row < v.nd; row += step >> 5) gemv_row2(v, row, threadIdx.x & 31);
+        cl.sync();
+    }
+    if (parts & 4) {
+        for (int i = 1; i <= top; i++) {
+            const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
+            sweep2<true, true>(L, 1, L.xb, C, i == 1 ? C.xa : C.xb, L.xa, t0, step);
+            cl.sync();
+            sweep2<true, false>(L, 0, L.xa, C, nullptr, L.xb, t0, step);
+            cl.sync();
+        }
+        if (out) pad_out(v, v.lv[top], top == 0 ? v.lv[0].xa : v.lv[top].xb, out, t0, step);
+    }
+}
+
 }  // namespace
 
 // ====================================================================== 2D handle state
@@ -505,6 +740,13 @@ struct Ctx2 {
     const double* inv = nullptr;
     int* info = nullptr;
     stg::InvOrder order;
+    // Laplacian-form V-cycle: padded vectors, coefficients and the coarsest index map (one
+    // allocation each, created with the handle); clusters: blocks of a cluster that can run
+    stg::V2 v{};
+    float* pad = nullptr;
+    uint8_t* padm = nullptr;
+    int* map = nullptr;
+    int cluster = 0;
 };
 
 namespace stg {
@@ -614,6 +856,13 @@ int setup2(stg_t* h) {
                                                                        c.pen32);
             STG_LAUNCH_CK();
         }
+        V2& v = h->c2->v;
+        for (int i = 0; i < v.L && h->lap2d; i++) {
+            k2_pad_coef<<<g1((long long)v.lv[i].n * v.lv[i].n), TPB, 0, h->st>>>(lv[i].g, v.lv[i], lv[i].pen32, lv[i].fixed,
+                                                                                const_cast<float*>(v.lv[i].P),
+                                                                                const_cast<uint8_t*>(v.lv[i].m));
+            STG_LAUNCH_CK();
+        }
         Level2& C = lv[0];
         const int nd = C.g.size();
         k2_calcA<<<g1((long long)nd * nd), TPB, 0, h->st>>>(C.g, C.vol, C.pen, C.fixed, C.lap, h->closed ? 1 : 0, h->c2->aug0);
@@ -621,7 +870,7 @@ int setup2(stg_t* h) {
         return STG_OK;
     };
     GraphCache& G = h->sgraph;
-    STG_TRY(graphed(h, G, (h->closed ? 2 : 1) | (h->hier_flow ? 4 : 0), body, [](bool) {}));
+    STG_TRY(graphed(h, G, (h->closed ? 2 : 1) | (h->hier_flow ? 4 : 0) | (h->lap2d ? 8 : 0), body, [](bool) {}));
     // the inversion: one cooperative launch, outside the graph
     // fixed cells are identity rows among the pressures, which the block elimination's sign
     // rule does not cover: the pivoted elimination takes them
@@ -629,7 +878,89 @@ int setup2(stg_t* h) {
         STG_TRY(gj_invert(h->st, lv[0].g.size(), h->c2->aug0, h->c2->aug1, h->c2->info, &h->c2->inv, true));
     else
         STG_TRY(inv_blocks(h->st, lv[0].g.size(), h->c2->order, h->closed ? 1 : 0, h->c2->aug0, h->c2->aug1, h->c2->info, &h->c2->inv));
+    V2& v = h->c2->v;
+    v.inv = h->c2->inv;
+    for (int i = 0; i < v.L; i++) {  // a face's vol doubles a level down, as lap does
+        v.lv[i].lap = (float)lv[i].lap;
+        v.lv[i].vol = (float)std::ldexp(h->vol2d, v.L - 1 - i);
+    }
     h->updated = true;
+    return STG_OK;
+}
+
+// The solver's V-cycle in the Laplacian form. Levels of at most 128 cells an axis, and the
+// coarsest solve when its inverse is small, run in one cluster launch (128^2: 8192 cells a
+// colour, one for each thread of 16 blocks; at 256^2 a pass of one cluster would take longer
+// than a launch of the whole GPU); larger ones a launch a pass, replayed as a CUDA graph.
+constexpr int CLUSTER_N = 128, CLUSTER_ND = 512;
+
+int launch_cluster2(stg_t* h, int top, int parts, const float* rhs, float* out) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)h->c2->cluster);
+    cfg.blockDim = dim3(VT);
+    cfg.stream = h->st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)h->c2->cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    STG_CK(cudaLaunchKernelEx(&cfg, k2v_cluster, h->c2->v, top, parts, rhs, out));
+    count_launch();
+    return STG_OK;
+}
+
+int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
+    const V2& v = h->c2->v;
+    const int fine = v.L - 1;
+    const unsigned gs = g1(v.fine.size());
+    int top = fine;  // finest level of the cluster part
+    while (top > 0 && v.lv[top].n > CLUSTER_N) top--;
+    const bool whole = top == fine, small = v.nd <= CLUSTER_ND;
+    if (whole && small) return launch_cluster2(h, top, 7, rhs, out);
+    if (!whole || top == 0) {
+        k2v_in<<<gs, TPB, 0, h->st>>>(v, rhs);
+        STG_LAUNCH_CK();
+    }
+    auto body = [&]() -> int {
+        for (int i = fine; i > top; i--) {
+            const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
+            const unsigned gb = g1((long long)L.n * L.n / 2);
+            k2v_sweep<false, false><<<gb, TPB, 0, h->st>>>(L, 0, nullptr, C, nullptr, L.xa);
+            STG_LAUNCH_CK();
+            k2v_sweep<true, false><<<gb, TPB, 0, h->st>>>(L, 1, L.xa, C, nullptr, L.xb);
+            STG_LAUNCH_CK();
+            k2v_restrict<<<g1((long long)C.n * C.n), TPB, 0, h->st>>>(L, L.xb, C);
+            STG_LAUNCH_CK();
+        }
+        if (small) {
+            STG_TRY(launch_cluster2(h, top, 7, nullptr, nullptr));
+        } else {
+            if (top > 0) STG_TRY(launch_cluster2(h, top, 1, nullptr, nullptr));
+            k2v_gemv<<<g1(32ll * v.nd), TPB, 0, h->st>>>(v);
+            STG_LAUNCH_CK();
+            if (top > 0) STG_TRY(launch_cluster2(h, top, 4, nullptr, nullptr));
+        }
+        for (int i = top + 1; i <= fine; i++) {
+            const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
+            const unsigned gb = g1((long long)L.n * L.n / 2);
+            k2v_sweep<true, true><<<gb, TPB, 0, h->st>>>(L, 1, L.xb, C, i == 1 ? C.xa : C.xb, L.xa);
+            STG_LAUNCH_CK();
+            k2v_sweep<true, false><<<gb, TPB, 0, h->st>>>(L, 0, L.xa, C, nullptr, L.xb);
+            STG_LAUNCH_CK();
+        }
+        return STG_OK;
+    };
+    if (whole && top > 0) {  // the levels fit a cluster, the coarsest inverse does not
+        STG_TRY(launch_cluster2(h, top, 1, rhs, nullptr));
+        k2v_gemv<<<g1(32ll * v.nd), TPB, 0, h->st>>>(v);
+        STG_LAUNCH_CK();
+        return launch_cluster2(h, top, 4, nullptr, out);
+    }
+    // the vol of the levels is a kernel argument: part of the key through a counter of changes
+    STG_TRY(graphed(h, h->vgraph, 2 + 2 * (long long)h->vol2d_changes + (v.inv == h->c2->aug0 + v.nd), body, [](bool) {}));
+    k2v_out<<<gs, TPB, 0, h->st>>>(v, out);
+    STG_LAUNCH_CK();
     return STG_OK;
 }
 
@@ -646,6 +977,10 @@ int resid2(stg_t* h, const d4* b, const d4* x, d4* r, double* nrm2_host) {
 }
 
 int precond2(stg_t* h, const float4* rhs, float4* out) {
+    if (h->lap2d && h->c2->cluster) {
+        PROF(h, 1, 0.0, vcycle2_lap(h, reinterpret_cast<const float*>(rhs), reinterpret_cast<float*>(out)));
+        return STG_OK;
+    }
     Level2& F = fine2(h);
     const int n = F.g.size();
     STG_CK(cudaMemcpyAsync(F.r, rhs, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->st));
@@ -704,6 +1039,50 @@ int create2d(stg_t* h) {
     std::vector<int> cells;
     for (int q = 0; q < nd; q++) (q < lv[0].g.off(0) ? cells : faces[q >= lv[0].g.off(1)]).push_back(q);
     STG_TRY(inv_order(h->c2->order, faces, cells));
+    if (L <= MAXL2) {
+        V2& v = h->c2->v;
+        size_t nf = 0, nm = 0;
+        for (auto& q : lv) nf += 12ull * (q.g.n + 4) * (q.g.n + 3), nm += (size_t)(q.g.n + 4) * (q.g.n + 3);
+        STG_TRY(dalloc(&h->c2->pad, nf));
+        STG_TRY(dalloc(&h->c2->padm, nm));
+        STG_TRY(dalloc(&h->c2->map, (size_t)nd));
+        v.L = L;
+        v.fine = lv[L - 1].g;
+        v.coarse = lv[0].g;
+        v.nd = nd;
+        v.ld = 2 * nd;
+        v.map = h->c2->map;
+        float* f = h->c2->pad;
+        uint8_t* m = h->c2->padm;
+        for (int i = 0; i < L; i++) {
+            Lv2& q = v.lv[i];
+            q.n = lv[i].g.n;
+            q.S = q.n + 4;
+            q.NS = q.S * (q.n + 3);
+            float** to[4] = {const_cast<float**>(&q.P), &q.r, &q.xa, &q.xb};
+            for (auto t : to) *t = f, f += 3 * q.NS;
+            q.m = m;
+            m += q.NS;
+        }
+        k2_pad_index<<<g1(nd), TPB, 0, h->st>>>(lv[0].g, v.lv[0], h->c2->map);
+        STG_LAUNCH_CK();
+        // blocks of one cluster: 16 where the device grants it, else the portable 8
+        STG_CK(cudaFuncSetAttribute(k2v_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (int c = 16; c >= 8 && !h->c2->cluster; c /= 2) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)c);
+            cfg.blockDim = dim3(VT);
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = (unsigned)c;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int can = 0;
+            if (cudaOccupancyMaxActiveClusters(&can, k2v_cluster, &cfg) == cudaSuccess && can > 0) h->c2->cluster = c;
+            cudaGetLastError();
+        }
+    }
     Level2& F = lv.back();
     h->L = L;
     h->n4 = F.g.size() / 4;
@@ -733,6 +1112,9 @@ void destroy2d(stg_t* h) {
     cudaFree(h->c2->aug1);
     cudaFree(h->c2->info);
     inv_order_free(h->c2->order);
+    cudaFree(h->c2->pad);
+    cudaFree(h->c2->padm);
+    cudaFree(h->c2->map);
     delete h->c2;
     h->c2 = nullptr;
 }
