@@ -69,6 +69,47 @@ __device__ __forceinline__ void block_sums_df(const float (&v)[NV], float2* out)
     }
 }
 
+// Where a reduction's sums go: the last block of the grid to store its partials adds columns
+// col0 .. col1 of the table up in a fixed order (one warp a column), so no second kernel runs.
+// Column q goes to out[q], the last one to *last when that is not null; every value also goes
+// to the host mirror, a pinned copy of the array that starts at dev, so the host reads it
+// after a stream synchronisation without a copy. sig2 (optional): 1 / the last column, or 1
+// where that is outside [1e-8, 1e8] (the caller then renormalises the vector).
+struct Fin {
+    unsigned* counter;  // blocks done, 0 between launches; null: partials only
+    double* out;
+    double* last;
+    const double* dev;
+    double* host;
+    double* sig2;
+    int col0, col1;
+};
+
+__device__ __forceinline__ void finish_cols(const float2* part, int stride, const Fin& f) {
+    if (!f.counter) return;
+    __shared__ bool mine;
+    __threadfence();  // this block's partials before its count
+    __syncthreads();
+    if (threadIdx.x == 0) mine = atomicAdd(f.counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!mine) return;
+    __threadfence();
+    const int lane = threadIdx.x & 31;
+    for (int q = f.col0 + (threadIdx.x >> 5); q <= f.col1; q += TPB / 32) {
+        float2 s = make_float2(0.f, 0.f);
+        for (int p = lane; p < (int)gridDim.x; p += 32) s = df_add(s, __ldcg(part + (long long)p * stride + q));
+        s = warp_sum_df(s);
+        if (lane == 0) {
+            const double v = (double)s.x + (double)s.y;
+            double* dst = (f.last && q == f.col1) ? f.last : f.out + q;
+            *dst = v;
+            if (f.host) f.host[dst - f.dev] = v;
+            if (f.sig2 && q == f.col1) *f.sig2 = v >= 1e-8 && v <= 1e8 ? 1.0 / v : 1.0;
+        }
+    }
+    if (threadIdx.x == 0) *f.counter = 0;
+}
+
 // FP16 copies of basis vectors (four halves per slot, the vector times its scale)
 struct TabH {
     const uint2* p[MAXV];
@@ -219,7 +260,7 @@ __global__ void __launch_bounds__(TPB) k_axpy_multi_32to64(long long n4, Tab z, 
 // pipe cannot keep up with HBM for these streams); block and grid sums are double-float.
 // With WW the pass also returns <w, w> in column NV.
 template <int NV, bool WW>
-__global__ void __launch_bounds__(TPB) k_multidot32(long long n4, Tab v, const float4* __restrict__ w, float2* __restrict__ part) {
+__global__ void __launch_bounds__(TPB) k_multidot32(long long n4, Tab v, const float4* __restrict__ w, float2* __restrict__ part, Fin fin) {
     float acc[NV + 1];
 #pragma unroll
     for (int q = 0; q <= NV; q++) acc[q] = 0.f;
@@ -233,6 +274,7 @@ __global__ void __launch_bounds__(TPB) k_multidot32(long long n4, Tab v, const f
         if (WW) acc[NV] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
     }
     block_sums_df<NV + 1>(acc, part + (long long)blockIdx.x * (MAXV + 1));
+    finish_cols(part, MAXV + 1, fin);
 }
 
 // The FGMRES operator fused with the first multi-dot of the Arnoldi step, in the
@@ -247,7 +289,7 @@ __global__ void __launch_bounds__(TPB) k_multidot32(long long n4, Tab v, const f
 template <int NV, bool H16>
 __global__ void __launch_bounds__(TPB) k_shift_dots(Geom g, float vol, const float4* __restrict__ v, const float4* __restrict__ z,
                                                     const uint8_t* __restrict__ m, const float4* __restrict__ P, Tab V, TabH VH,
-                                                    const float* __restrict__ sc, float4* __restrict__ w, float2* __restrict__ part) {
+                                                    const float* __restrict__ sc, float4* __restrict__ w, float2* __restrict__ part, Fin fin) {
     float acc[NV + 1];
 #pragma unroll
     for (int q = 0; q <= NV; q++) acc[q] = 0.f;
@@ -278,31 +320,7 @@ __global__ void __launch_bounds__(TPB) k_shift_dots(Geom g, float vol, const flo
         for (int q = 0; q < NV; q++) acc[q] *= __frcp_rn(__ldg(sc + q));
     }
     block_sums_df<NV + 1>(acc, part + (long long)blockIdx.x * (MAXV + 1));
-}
-
-// w -= sum_q h[q] v_q ; partial ||w||^2 per block (computed after the update)
-template <int NV>
-__global__ void __launch_bounds__(TPB) k_multiaxpy32(long long n4, Tab v, const double* __restrict__ h, float4* __restrict__ w,
-                                                     float2* __restrict__ part, int want_norm) {
-    float c[NV];
-#pragma unroll
-    for (int q = 0; q < NV; q++) c[q] = (float)h[q];
-    float accf = 0.f;
-    for (long long t = (long long)blockIdx.x * TPB + threadIdx.x; t < n4; t += (long long)gridDim.x * TPB) {
-        float4 a = w[t];
-#pragma unroll
-        for (int q = 0; q < NV; q++) {
-            float4 b = __ldg(v.p[q] + t);
-            a.x -= c[q] * b.x;
-            a.y -= c[q] * b.y;
-            a.z -= c[q] * b.z;
-            a.w -= c[q] * b.w;
-        }
-        w[t] = a;
-        if (want_norm) accf += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
-    }
-    const float acc[1] = {accf};
-    if (want_norm) block_sums_df<1>(acc, part + blockIdx.x);
+    finish_cols(part, MAXV + 1, fin);
 }
 
 // Projection step of classical Gram-Schmidt on unnormalised basis vectors:
@@ -315,7 +333,7 @@ __global__ void __launch_bounds__(TPB) k_multiaxpy32(long long n4, Tab v, const 
 template <int NV, bool DOTS>
 __global__ void __launch_bounds__(TPB) k_proj32(long long n4, Tab v, const double* __restrict__ d, const double* __restrict__ sig2,
                                                 const float4* w, float4* out, float2* __restrict__ part, uint2* __restrict__ out16,
-                                                const double* __restrict__ nest, float* __restrict__ sc_out) {
+                                                const double* __restrict__ nest, float* __restrict__ sc_out, Fin fin) {
     // the coefficients and the FP16 scale in FP64 once per block (FP64 is slow on GB300)
     __shared__ float csh[NV + 1];
     if (threadIdx.x < NV) csh[threadIdx.x] = (float)(sig2[threadIdx.x] * d[threadIdx.x]);
@@ -349,6 +367,7 @@ __global__ void __launch_bounds__(TPB) k_proj32(long long n4, Tab v, const doubl
         acc[NV] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
     }
     block_sums_df<NV + 1>(acc, part + (long long)blockIdx.x * (MAXV + 1));
+    finish_cols(part, MAXV + 1, fin);
 }
 
 // sc (optional): the scale of x's FP16 copy, which keeps representing the scaled vector
@@ -379,22 +398,6 @@ __global__ void k_reduce_cols(const double* __restrict__ part, int nparts, int s
             out[q] = r;
         }
         __syncthreads();
-    }
-}
-
-// Sums column q of a [nparts][stride] table of double-float partials in a fixed order, one
-// warp per column (no block barriers): columns 0 .. ncols-2 go to out[q], the last to
-// *out_last (or to out[ncols-1] when out_last is null).
-__global__ void k_reduce_cols_df(const float2* __restrict__ part, int nparts, int stride, int ncols, double* __restrict__ out,
-                                 double* __restrict__ out_last) {
-    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (q >= ncols) return;
-    float2 s = make_float2(0.f, 0.f);
-    for (int p = lane; p < nparts; p += 32) s = df_add(s, part[(long long)p * stride + q]);
-    s = warp_sum_df(s);
-    if (lane == 0) {
-        double* dst = (out_last && q == ncols - 1) ? out_last : out + q;
-        *dst = (double)s.x + (double)s.y;
     }
 }
 
@@ -438,9 +441,9 @@ int f32_to_f64(cudaStream_t st, long long n4, const float4* a, d4* out) {
     return STG_OK;
 }
 
-// column sums of a table of double-float partials (the Krylov kernels' scratch, 8 bytes an entry)
-static void rcols_df(cudaStream_t st, const double* scratch, int nparts, int stride, int ncols, double* out, double* out_last = nullptr) {
-    k_reduce_cols_df<<<1, 32 * ncols, 0, st>>>(reinterpret_cast<const float2*>(scratch), nparts, stride, ncols, out, out_last);
+// the sums of columns col0 .. col1 of a pass over the basis (Fin)
+static Fin fin_of(const Reduce& R, int col0, int col1, double* out, double* last, double* sig2 = nullptr) {
+    return Fin{R.counter, out, last, R.dev, R.host, sig2, col0, col1};
 }
 
 int reduce_parts(cudaStream_t st, const double* parts, int nparts, double* out) {
@@ -481,21 +484,21 @@ struct AxpyL {
 };
 template <int NV>
 struct DotL {
-    static void run(cudaStream_t st, long long n4, const Tab& t, const float4* w, double* part, bool ww) {
+    static void run(cudaStream_t st, long long n4, const Tab& t, const float4* w, double* part, bool ww, const Fin& fin) {
         if (ww)
-            k_multidot32<NV, true><<<rgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part));
+            k_multidot32<NV, true><<<rgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part), fin);
         else
-            k_multidot32<NV, false><<<rgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part));
+            k_multidot32<NV, false><<<rgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part), fin);
     }
 };
 template <int NV>
 struct ProjL {
     static void run(cudaStream_t st, long long n4, const Tab& t, const double* d, const double* sig2, const float4* w, float4* out,
-                    double* part, bool dots, uint2* out16, const double* nest, float* sc_out) {
+                    double* part, bool dots, uint2* out16, const double* nest, float* sc_out, const Fin& fin) {
         if (dots)
-            k_proj32<NV, true><<<rgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out);
+            k_proj32<NV, true><<<rgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out, fin);
         else
-            k_proj32<NV, false><<<rgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out);
+            k_proj32<NV, false><<<rgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out, fin);
     }
 };
 
@@ -526,16 +529,17 @@ int axpy_multi_32to64(cudaStream_t st, long long n4, const float4* const* z, con
 template <int NV>
 struct ShiftL {
     static void run(cudaStream_t st, const Geom& g, float vol, const float4* v, const float4* z, const uint8_t* m, const float4* P,
-                    const Tab& t, const TabH& th, const float* sc, float4* w, double* part) {
+                    const Tab& t, const TabH& th, const float* sc, float4* w, double* part, const Fin& fin) {
+        const unsigned nb = rgrid(g.box());
         if (sc)
-            k_shift_dots<NV, true><<<RGRID, TPB, 0, st>>>(g, vol, v, z, m, P, t, th, sc, w, reinterpret_cast<float2*>(part));
+            k_shift_dots<NV, true><<<nb, TPB, 0, st>>>(g, vol, v, z, m, P, t, th, sc, w, reinterpret_cast<float2*>(part), fin);
         else
-            k_shift_dots<NV, false><<<RGRID, TPB, 0, st>>>(g, vol, v, z, m, P, t, th, sc, w, reinterpret_cast<float2*>(part));
+            k_shift_dots<NV, false><<<nb, TPB, 0, st>>>(g, vol, v, z, m, P, t, th, sc, w, reinterpret_cast<float2*>(part), fin);
     }
 };
 
 int shift_multidot32(cudaStream_t st, const Geom& g, float vol, const float4* v, const float4* z, const uint8_t* m, const float4* P,
-                     long long n4, const float4* const* V, int nv, float4* w, double* h, double* scratch, double* ww,
+                     long long n4, const float4* const* V, int nv, float4* w, double* h, const Reduce& R, double* ww,
                      const uint2* const* V16, const float* sc) {
     const int nb = nv < MAXV ? nv : MAXV;
     Tab t{};
@@ -544,74 +548,41 @@ int shift_multidot32(cudaStream_t st, const Geom& g, float vol, const float4* v,
         t.p[q] = V[q];
         th.p[q] = V16 ? V16[q] : nullptr;
     }
-    dispatch_nv<ShiftL>(nb, st, g, vol, v, z, m, P, t, th, V16 ? sc : nullptr, w, scratch);
-    STG_LAUNCH_CK();
-    rcols_df(st, scratch, RGRID, MAXV + 1, nb + 1, h, ww);  // the dots, and <w, w> in column nb
+    // the dots, and <w, w> in column nb
+    dispatch_nv<ShiftL>(nb, st, g, vol, v, z, m, P, t, th, V16 ? sc : nullptr, w, R.part, fin_of(R, 0, nb, h, ww));
     STG_LAUNCH_CK();
     // basis vectors past the first MAXV: a plain multi-dot pass over the written w
-    if (nv > MAXV) STG_TRY(multidot32(st, n4, V + MAXV, nv - MAXV, w, h + MAXV, scratch, nullptr));
+    if (nv > MAXV) STG_TRY(multidot32(st, n4, V + MAXV, nv - MAXV, w, h + MAXV, R, nullptr));
     return STG_OK;
 }
 
-int multidot32(cudaStream_t st, long long n4, const float4* const* v, int nv, const float4* w, double* h, double* scratch,
-               double* ww) {
-    unsigned g = rgrid(n4);
+int multidot32(cudaStream_t st, long long n4, const float4* const* v, int nv, const float4* w, double* h, const Reduce& R,
+               double* ww, double* sig2) {
     for (int j0 = 0; j0 < nv; j0 += MAXV) {
         int nb = nv - j0 < MAXV ? nv - j0 : MAXV;
         bool want_ww = ww && j0 == 0;
         Tab t{};
         for (int q = 0; q < nb; q++) t.p[q] = v[j0 + q];
-        dispatch_nv<DotL>(nb, st, n4, t, w, scratch, want_ww);
-        STG_LAUNCH_CK();
-        rcols_df(st, scratch, (int)g, MAXV + 1, want_ww ? nb + 1 : nb, h + j0, want_ww ? ww : nullptr);
-        STG_LAUNCH_CK();
-    }
-    return STG_OK;
-}
-
-template <int NV>
-struct MaxpyL {
-    static void run(cudaStream_t st, long long n4, const Tab& t, const double* h, float4* w, double* part, int want) {
-        k_multiaxpy32<NV><<<rgrid(n4), TPB, 0, st>>>(n4, t, h, w, reinterpret_cast<float2*>(part), want);
-    }
-};
-
-int multiaxpy32_norm(cudaStream_t st, long long n4, const float4* const* v, int nv, const double* h, float4* w, double* nrm2,
-                     double* scratch) {
-    if (nv < 1) {
-        set_error("multiaxpy32_norm: empty basis");
-        return STG_E_INVALID;
-    }
-    unsigned g = rgrid(n4);
-    for (int j0 = 0; j0 < nv; j0 += MAXV) {
-        int nb = nv - j0 < MAXV ? nv - j0 : MAXV;
-        int last = j0 + nb >= nv;
-        Tab t{};
-        for (int q = 0; q < nb; q++) t.p[q] = v[j0 + q];
-        dispatch_nv<MaxpyL>(nb, st, n4, t, h + j0, w, scratch, last);
+        dispatch_nv<DotL>(nb, st, n4, t, w, R.part, want_ww,
+                          fin_of(R, 0, want_ww ? nb : nb - 1, h + j0, want_ww ? ww : nullptr, want_ww ? sig2 : nullptr));
         STG_LAUNCH_CK();
     }
-    rcols_df(st, scratch, (int)g, 1, 1, nrm2);
-    STG_LAUNCH_CK();
     return STG_OK;
 }
 
 int project32(cudaStream_t st, long long n4, const float4* const* v, int nv, const double* d, const double* sig2, const float4* w,
-              float4* out, double* dots, double* nrm2, double* scratch, uint2* out16, const double* nest, float* sc_out) {
+              float4* out, double* dots, double* nrm2, const Reduce& R, double* sig2_out, uint2* out16, const double* nest,
+              float* sc_out) {
     if (nv < 1) {
         set_error("project32: empty basis");
         return STG_E_INVALID;
     }
-    unsigned g = rgrid(n4);
     if (nv <= MAXV) {
         Tab t{};
         for (int q = 0; q < nv; q++) t.p[q] = v[q];
-        dispatch_nv<ProjL>(nv, st, n4, t, d, sig2, w, out, scratch, dots != nullptr, out16, nest, sc_out);
-        STG_LAUNCH_CK();
-        if (dots)
-            rcols_df(st, scratch, (int)g, MAXV + 1, nv + 1, dots, nrm2);  // the dots, and |out|^2 in column nv
-        else
-            rcols_df(st, scratch + nv, (int)g, MAXV + 1, 1, nrm2);
+        // the dots, and |out|^2 in column nv
+        dispatch_nv<ProjL>(nv, st, n4, t, d, sig2, w, out, R.part, dots != nullptr, out16, nest, sc_out,
+                           fin_of(R, dots ? 0 : nv, nv, dots, nrm2, sig2_out));
         STG_LAUNCH_CK();
         return STG_OK;
     }
@@ -621,14 +592,13 @@ int project32(cudaStream_t st, long long n4, const float4* const* v, int nv, con
         Tab t{};
         for (int q = 0; q < nb; q++) t.p[q] = v[j0 + q];
         const bool last = j0 + nb >= nv;  // the last chunk writes the FP16 copy
-        dispatch_nv<ProjL>(nb, st, n4, t, d + j0, sig2 + j0, j0 == 0 ? w : out, out, scratch, false, last ? out16 : nullptr, nest,
-                           sc_out);
+        Fin fin = fin_of(R, nb, nb, nullptr, nrm2, sig2_out);
+        if (!last || dots) fin.counter = nullptr;
+        dispatch_nv<ProjL>(nb, st, n4, t, d + j0, sig2 + j0, j0 == 0 ? w : out, out, R.part, false, last ? out16 : nullptr, nest,
+                           sc_out, fin);
         STG_LAUNCH_CK();
     }
-    if (dots) return multidot32(st, n4, v, nv, out, dots, scratch, nrm2);
-    rcols_df(st, scratch + (nv - ((nv - 1) / MAXV) * MAXV), (int)g, MAXV + 1, 1, nrm2);
-    STG_LAUNCH_CK();
-    return STG_OK;
+    return dots ? multidot32(st, n4, v, nv, out, dots, R, nrm2, sig2_out) : STG_OK;
 }
 
 int scale32(cudaStream_t st, long long n4, float4* x, const double* nrm2, float4* out, float* sc) {

@@ -123,12 +123,18 @@ struct stg_ctx {
     // Krylov (FP32)
     int m = 0;
     std::vector<float4*> V, Z;
+    float4 *vslab = nullptr, *zslab = nullptr;  // the vectors' memory
+    uint2* slab16 = nullptr;
     // FP16 copies of the basis V (3D, opts.basis16) read by the multi-dot passes, and their
     // scales (device)
     std::vector<uint2*> V16;
     float* dsc16 = nullptr;
     float4* w = nullptr;
     double *dscr = nullptr, *dh = nullptr, *dnrm = nullptr, *dy = nullptr, *dsig2 = nullptr;
+    // dh (2 (m + 2) dots) and dnrm (8 norms) are one array, mirrored in pinned host memory by
+    // the kernels that reduce into it
+    double* hres = nullptr;
+    unsigned* dcount = nullptr;
     // host-order staging (cells + 3 face arrays)
     double* stage = nullptr;
     int* istage = nullptr;

@@ -108,28 +108,34 @@ int axpy_multi_32to64(cudaStream_t st, long long n4, const float4* const* z, con
                       float4* xh = nullptr, float4* xl = nullptr, float4* e = nullptr);
 // first index of the last group of vectors axpy_multi_32to64 sums in one pass
 int axpy_last_chunk(int nz);
+// Scratch of the basis passes below: partials (1216 x 17 double-float pairs), the count of
+// blocks done (0 between launches), and the device array that holds every result with its
+// pinned host mirror, which the passes write too
+struct Reduce {
+    double* part;
+    unsigned* counter;
+    const double* dev;
+    double* host;
+};
 // h[j] = <v_j, w> for j < nv (FP32 per-thread partials, double-float block and grid sums),
-// and <w, w> into *ww when ww != nullptr
-
-int multidot32(cudaStream_t st, long long n4, const float4* const* v, int nv, const float4* w, double* h, double* scratch,
-               double* ww);
+// and <w, w> into *ww when ww != nullptr (and 1 / <w, w> into *sig2, see project32)
+int multidot32(cudaStream_t st, long long n4, const float4* const* v, int nv, const float4* w, double* h, const Reduce& R,
+               double* ww, double* sig2 = nullptr);
 // w = v - A z (Laplacian form, slot layout of g) fused with h[q] = <V_q, w> (q < nv) and
 // <w, w> into *ww (device). With V16 the first 16 dots read the vectors' FP16 copies
 // instead, scaled back by 1 / sc[q] (sc on the device).
 int shift_multidot32(cudaStream_t st, const Geom& g, float vol, const float4* v, const float4* z, const uint8_t* m, const float4* P,
-                     long long n4, const float4* const* V, int nv, float4* w, double* h, double* scratch, double* ww,
+                     long long n4, const float4* const* V, int nv, float4* w, double* h, const Reduce& R, double* ww,
                      const uint2* const* V16 = nullptr, const float* sc = nullptr);
-// w -= sum_j h[j] v_j ; then returns ||w||^2 into nrm2 (device)
-int multiaxpy32_norm(cudaStream_t st, long long n4, const float4* const* v, int nv, const double* h, float4* w, double* nrm2,
-                     double* scratch);
 // Classical Gram-Schmidt projection on unnormalised basis vectors in one pass:
 // out = w - sum_q sig2[q] d[q] v_q (d, sig2 on the device; out may alias w); ||out||^2
-// into *nrm2 and, when dots != nullptr, <v_q, out> into dots[0..nv) (device). With out16,
+// into *nrm2, its reciprocal into *sig2_out (1 where ||out||^2 lies outside [1e-8, 1e8]) and,
+// when dots != nullptr, <v_q, out> into dots[0..nv) (device). With out16,
 // also the FP16 copy of out, scaled for an out of squared norm at most *nest, the scale to
 // *sc_out (nest, sc_out on the device).
 int project32(cudaStream_t st, long long n4, const float4* const* v, int nv, const double* d, const double* sig2, const float4* w,
-              float4* out, double* dots, double* nrm2, double* scratch, uint2* out16 = nullptr, const double* nest = nullptr,
-              float* sc_out = nullptr);
+              float4* out, double* dots, double* nrm2, const Reduce& R, double* sig2_out, uint2* out16 = nullptr,
+              const double* nest = nullptr, float* sc_out = nullptr);
 // out = x / sqrt(*nrm2); with sc, the scale of x's FP16 copy follows (*sc *= sqrt(*nrm2))
 int scale32(cudaStream_t st, long long n4, float4* x, const double* nrm2, float4* out, float* sc = nullptr);
 // deterministic sum of nparts partials -> *out

@@ -577,9 +577,11 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
         // first cancelled nearly all of w: ||V_{j+1}|| < 0.1 ||w||) V_{j+1} -= sum sig^2 d2 V.
         // The looser trigger than the usual 0.7 costs orthogonality of order 1e-6 in FP32,
         // far below the 1e-4 an inner solve is asked for; the FP64 refinement decides.
-        sig[0] = 1.0;
-        const double one = 1.0;
-        STG_CK(cudaMemcpyAsync(h->dsig2, &one, sizeof(double), cudaMemcpyHostToDevice, h->st));
+        sig[0] = 1.0;  // (dsig2[0] is 1 from the start)
+        const Reduce red{h->dscr, h->dcount, h->dh, h->hres};
+        const double* hd = h->hres;            // dots of the first pass, of the second, norms
+        const double* hd2 = h->hres + m + 2;
+        const double* hn2 = h->hres + 2 * (m + 2);
         double prev_est = beta;
         // Learned warm start (warm_start 2): the first refinement step of a warm-started solve
         // is one FGMRES step whose preconditioner is the learned correction, i.e. the
@@ -609,31 +611,26 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
                 const int nh = h16 ? std::min(j + 1, 16) : 0;  // dots read from the FP16 copies
                 PROF(h, 6, (65.0 + 16.0 * (j + 1) - 8.0 * nh) * F.g.box(),
                      shift_multidot32(h->st, F.g, (float)F.vol, h->V[j], h->Z[j], F.m, F.P32, n4, h->V.data(), j + 1, h->w, h->dh,
-                                      h->dscr, h->dnrm + 1, h16 ? h->V16.data() : nullptr, h->dsc16));
+                                      red, h->dnrm + 1, h16 ? h->V16.data() : nullptr, h->dsc16));
             } else {
                 STG_TRY(h->shift32(h, h->V[j], h->Z[j], h->w));
-                PROF(h, 6, 16.0 * (j + 2) * n4, multidot32(h->st, n4, h->V.data(), j + 1, h->w, h->dh, h->dscr, h->dnrm + 1));
+                PROF(h, 6, 16.0 * (j + 2) * n4, multidot32(h->st, n4, h->V.data(), j + 1, h->w, h->dh, red, h->dnrm + 1));
             }
             // the new vector's FP16 copy is scaled for a norm up to ||w|| (the projection only
             // shortens w); a second projection rewrites it for its own input's norm
             PROF(h, 6, (16.0 * (j + 3) + (h16 ? 8.0 : 0.0)) * n4,
-                 project32(h->st, n4, h->V.data(), j + 1, h->dh, h->dsig2, h->w, h->V[j + 1], h->dh + m + 2, h->dnrm, h->dscr,
+                 project32(h->st, n4, h->V.data(), j + 1, h->dh, h->dsig2, h->w, h->V[j + 1], h->dh + m + 2, h->dnrm, red, h->dsig2 + j + 1,
                            h16 ? h->V16[j + 1] : nullptr, h->dnrm + 1, h->dsc16 + j + 1));
-            std::vector<double> h1(j + 1), h2(j + 1, 0.0);
-            double nrm[2] = {0, 0};
-            STG_CK(cudaMemcpyAsync(h1.data(), h->dh, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, h->st));
-            STG_CK(cudaMemcpyAsync(h2.data(), h->dh + m + 2, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, h->st));
-            STG_CK(cudaMemcpyAsync(nrm, h->dnrm, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
             STG_CK(cudaStreamSynchronize(h->st));
-            double nw2 = nrm[0];
-            if (nrm[0] < 0.01 * nrm[1]) {
+            std::vector<double> h1(hd, hd + j + 1), h2(j + 1, 0.0);
+            double nw2 = hn2[0];
+            if (hn2[0] < 0.01 * hn2[1]) {
+                std::copy(hd2, hd2 + j + 1, h2.begin());
                 PROF(h, 6, (16.0 * (j + 3) + (h16 ? 8.0 : 0.0)) * n4,
-                     project32(h->st, n4, h->V.data(), j + 1, h->dh + m + 2, h->dsig2, h->V[j + 1], h->V[j + 1], nullptr, h->dnrm,
-                               h->dscr, h16 ? h->V16[j + 1] : nullptr, h->dnrm, h->dsc16 + j + 1));
-                STG_CK(cudaMemcpyAsync(&nw2, h->dnrm, sizeof(double), cudaMemcpyDeviceToHost, h->st));
+                     project32(h->st, n4, h->V.data(), j + 1, h->dh + m + 2, h->dsig2, h->V[j + 1], h->V[j + 1], nullptr, h->dnrm, red,
+                               h->dsig2 + j + 1, h16 ? h->V16[j + 1] : nullptr, h->dnrm, h->dsc16 + j + 1));
                 STG_CK(cudaStreamSynchronize(h->st));
-            } else {
-                std::fill(h2.begin(), h2.end(), 0.0);
+                nw2 = hn2[0];
             }
             S.inner_iters++;
             // A z_j = v_j - sum_q sig_q sig_j d_q v_q - (sig_j / sig_{j+1}) v_{j+1}
@@ -650,13 +647,9 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
                 // for a weak preconditioner on high-contrast designs): renormalise before FP32
                 // over- or underflows
                 PROF(h, 6, 32.0 * n4, scale32(h->st, n4, h->V[j + 1], h->dnrm, h->V[j + 1], h16 ? h->dsc16 + j + 1 : nullptr));
-                sig[j + 1] = 1.0;
-                const double one1 = 1.0;
-                STG_CK(cudaMemcpyAsync(h->dsig2 + j + 1, &one1, sizeof(double), cudaMemcpyHostToDevice, h->st));
+                sig[j + 1] = 1.0;  // as the projection left dsig2
             } else if (nw2 > 0) {
                 sig[j + 1] = 1.0 / std::sqrt(nw2);
-                const double s2 = 1.0 / nw2;
-                STG_CK(cudaMemcpyAsync(h->dsig2 + j + 1, &s2, sizeof(double), cudaMemcpyHostToDevice, h->st));
             }
             // Givens rotations on the new Hessenberg column
             for (int q = 0; q < j; q++) {
@@ -936,29 +929,40 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
         return fail(rc);
     h->V.assign(h->m + 1, nullptr);
     h->Z.assign(h->m, nullptr);
-    for (auto& p : h->V)
-        if ((rc = dalloc(&p, ns))) return fail(rc);
-    for (auto& p : h->Z)
-        if ((rc = dalloc(&p, ns))) return fail(rc);
+    // one allocation for V and one for Z: a cudaMalloc and a memset each per vector were most of
+    // a small handle's creation
+    const size_t vs = (ns + 15) / 16 * 16;  // vectors start on 256-byte boundaries
+    if ((rc = dalloc(&h->vslab, vs * h->V.size())) || (rc = dalloc(&h->zslab, vs * h->Z.size()))) return fail(rc);
+    for (size_t q = 0; q < h->V.size(); q++) h->V[q] = h->vslab + q * vs;
+    for (size_t q = 0; q < h->Z.size(); q++) h->Z[q] = h->zslab + q * vs;
     if (dim == 3 && h->opts.basis16) {
         // the FP16 copies only speed up the multi-dot: without room for them the handle
         // runs on the FP32 basis alone
         h->V16.assign(h->m + 1, nullptr);
-        bool ok = dalloc(&h->dsc16, (size_t)h->m + 1) == STG_OK;
-        for (auto& p : h->V16) ok = ok && dalloc(&p, ns) == STG_OK;
+        const bool ok = dalloc(&h->dsc16, (size_t)h->m + 1) == STG_OK && dalloc(&h->slab16, vs * h->V16.size()) == STG_OK;
+        for (size_t q = 0; ok && q < h->V16.size(); q++) h->V16[q] = h->slab16 + q * vs;
         if (!ok) {
-            for (auto p : h->V16) cudaFree(p);
+            cudaFree(h->slab16);
             cudaFree(h->dsc16);
             h->V16.clear();
+            h->slab16 = nullptr;
             h->dsc16 = nullptr;
             cudaGetLastError();
             set_error("%s", "");
         }
     }
-    if ((rc = dalloc(&h->dscr, 1216 * 18)) || (rc = dalloc(&h->dh, 2 * (h->m + 2))) || (rc = dalloc(&h->dnrm, 8)) ||
+    const size_t nres = 2 * ((size_t)h->m + 2) + 8;
+    if ((rc = dalloc(&h->dscr, 1216 * 18)) || (rc = dalloc(&h->dh, nres)) || (rc = dalloc(&h->dcount, 1)) ||
         (rc = dalloc(&h->dsig2, h->m + 2)) ||
         (rc = dalloc(&h->dy, h->m + 1)) || (rc = dalloc(&h->d_parts, (size_t)nparts + 1216)) || (rc = dalloc(&h->dflag, 1)))
         return fail(rc);
+    h->dnrm = h->dh + (nres - 8);
+    if (cudaHostAlloc((void**)&h->hres, sizeof(double) * nres, cudaHostAllocMapped) != cudaSuccess)
+        return fail(cuda_fail(cudaGetLastError(), "cudaHostAlloc", __FILE__, __LINE__));
+    memset(h->hres, 0, sizeof(double) * nres);
+    const double one = 1.0;  // the first basis vector of every refinement step is normalised
+    if (cudaMemcpy(h->dsig2, &one, sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+        return fail(cuda_fail(cudaGetLastError(), "create", __FILE__, __LINE__));
     if ((rc = dalloc(&h->stage, h->ncell + 3 * h->nface)) || (rc = dalloc(&h->istage, h->ncell + 3 * h->nface))) return fail(rc);
     if ((rc = dalloc(&h->d_design, h->ncell)) || (rc = dalloc(&h->d_phys, h->ncell)) || (rc = dalloc(&h->d_sens, h->ncell)) ||
         (rc = dalloc(&h->d_sens_design, h->ncell)) || (rc = dalloc(&h->d_vw, h->ncell)) || (rc = dalloc(&h->d_tmp, h->ncell)) ||
@@ -1002,15 +1006,17 @@ int stg_destroy(stg_t* h) {
     for (float4* p : {h->xh, h->xl, h->bh, h->bl, h->Plo}) cudaFree(p);
     cudaFree(h->d_pscale);
     cudaFree(h->d_pmax);
-    for (auto p : h->V) cudaFree(p);
-    for (auto p : h->V16) cudaFree(p);
+    cudaFree(h->vslab);
+    cudaFree(h->zslab);
+    cudaFree(h->slab16);
     cudaFree(h->dsc16);
-    for (auto p : h->Z) cudaFree(p);
-    for (double* p : {h->dscr, h->dh, h->dnrm, h->dy, h->dsig2, h->stage, h->d_design, h->d_phys, h->d_sens, h->d_sens_design, h->d_vw,
+    for (double* p : {h->dscr, h->dh, h->dy, h->dsig2, h->stage, h->d_design, h->d_phys, h->d_sens, h->d_sens_design, h->d_vw,
                       h->d_tmp, h->d_gauss, h->d_parts, h->d_wsum})
         cudaFree(p);
     cudaFree(h->istage);
     cudaFree(h->dflag);
+    cudaFree(h->dcount);
+    cudaFreeHost(h->hres);
     if (h->e0) cudaEventDestroy(h->e0);
     if (h->e1) cudaEventDestroy(h->e1);
     for (auto e : h->prof.pool) cudaEventDestroy(e);
