@@ -85,27 +85,45 @@ struct Fin {
     int col0, col1;
 };
 
+// NC: columns of a row that are read (a thread takes whole rows, so all its loads of a row are in
+// flight together; one column after the other took 15 us of a 1193-block pass).
+template <int NC>
 __device__ __forceinline__ void finish_cols(const float2* part, int stride, const Fin& f) {
     if (!f.counter) return;
     __shared__ bool mine;
+    __shared__ float2 sh[NC][TPB / 32];
     __threadfence();  // this block's partials before its count
     __syncthreads();
     if (threadIdx.x == 0) mine = atomicAdd(f.counter, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!mine) return;
     __threadfence();
-    const int lane = threadIdx.x & 31;
-    for (int q = f.col0 + (threadIdx.x >> 5); q <= f.col1; q += TPB / 32) {
-        float2 s = make_float2(0.f, 0.f);
-        for (int p = lane; p < (int)gridDim.x; p += 32) s = df_add(s, __ldcg(part + (long long)p * stride + q));
-        s = warp_sum_df(s);
-        if (lane == 0) {
-            const double v = (double)s.x + (double)s.y;
-            double* dst = (f.last && q == f.col1) ? f.last : f.out + q;
-            *dst = v;
-            if (f.host) f.host[dst - f.dev] = v;
-            if (f.sig2 && q == f.col1) *f.sig2 = v >= 1e-8 && v <= 1e8 ? 1.0 / v : 1.0;
-        }
+    float2 acc[NC];
+#pragma unroll
+    for (int q = 0; q < NC; q++) acc[q] = make_float2(0.f, 0.f);
+    for (int p = threadIdx.x; p < (int)gridDim.x; p += TPB) {
+        float2 v[NC];
+#pragma unroll
+        for (int q = 0; q < NC; q++) v[q] = __ldcg(part + (long long)p * stride + q);
+#pragma unroll
+        for (int q = 0; q < NC; q++) acc[q] = df_add(acc[q], v[q]);
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NC; q++) {
+        const float2 s = warp_sum_df(acc[q]);
+        if (lane == 0) sh[q][wid] = s;
+    }
+    __syncthreads();
+    const int q = threadIdx.x;
+    if (q >= f.col0 && q <= f.col1 && q < NC) {
+        float2 t = sh[q][0];
+        for (int w = 1; w < TPB / 32; w++) t = df_add(t, sh[q][w]);
+        const double v = (double)t.x + (double)t.y;
+        double* dst = (f.last && q == f.col1) ? f.last : f.out + q;
+        *dst = v;
+        if (f.host) f.host[dst - f.dev] = v;
+        if (f.sig2 && q == f.col1) *f.sig2 = v >= 1e-8 && v <= 1e8 ? 1.0 / v : 1.0;
     }
     if (threadIdx.x == 0) *f.counter = 0;
 }
@@ -274,7 +292,7 @@ __global__ void __launch_bounds__(TPB) k_multidot32(long long n4, Tab v, const f
         if (WW) acc[NV] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
     }
     block_sums_df<NV + 1>(acc, part + (long long)blockIdx.x * (MAXV + 1));
-    finish_cols(part, MAXV + 1, fin);
+    finish_cols<NV + 1>(part, MAXV + 1, fin);
 }
 
 // The FGMRES operator fused with the first multi-dot of the Arnoldi step, in the
@@ -320,7 +338,7 @@ __global__ void __launch_bounds__(TPB) k_shift_dots(Geom g, float vol, const flo
         for (int q = 0; q < NV; q++) acc[q] *= __frcp_rn(__ldg(sc + q));
     }
     block_sums_df<NV + 1>(acc, part + (long long)blockIdx.x * (MAXV + 1));
-    finish_cols(part, MAXV + 1, fin);
+    finish_cols<NV + 1>(part, MAXV + 1, fin);
 }
 
 // Projection step of classical Gram-Schmidt on unnormalised basis vectors:
@@ -367,7 +385,7 @@ __global__ void __launch_bounds__(TPB) k_proj32(long long n4, Tab v, const doubl
         acc[NV] += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
     }
     block_sums_df<NV + 1>(acc, part + (long long)blockIdx.x * (MAXV + 1));
-    finish_cols(part, MAXV + 1, fin);
+    finish_cols<NV + 1>(part, MAXV + 1, fin);
 }
 
 // sc (optional): the scale of x's FP16 copy, which keeps representing the scaled vector
@@ -414,6 +432,15 @@ __global__ void __launch_bounds__(TPB) k_dot64(long long n4, const d4* __restric
 unsigned rgrid(long long work) {
     long long g = (work + TPB - 1) / TPB;
     return (unsigned)(g < 1 ? 1 : (g > RGRID ? RGRID : g));
+}
+
+// Grid of the passes over the basis: their partials are summed by one block, so from two blocks
+// an SM on a thread takes up to four slots before the grid grows on to RGRID (64^3: 304 blocks
+// instead of 1193).
+unsigned kgrid(long long work) {
+    const long long g = (work + TPB - 1) / TPB, g4 = (work + 4 * TPB - 1) / (4 * TPB);
+    const long long two = 304;
+    return rgrid(TPB * (g <= two ? g : g4 < two ? two : g4));
 }
 
 }  // namespace
@@ -486,9 +513,9 @@ template <int NV>
 struct DotL {
     static void run(cudaStream_t st, long long n4, const Tab& t, const float4* w, double* part, bool ww, const Fin& fin) {
         if (ww)
-            k_multidot32<NV, true><<<rgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part), fin);
+            k_multidot32<NV, true><<<kgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part), fin);
         else
-            k_multidot32<NV, false><<<rgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part), fin);
+            k_multidot32<NV, false><<<kgrid(n4), TPB, 0, st>>>(n4, t, w, reinterpret_cast<float2*>(part), fin);
     }
 };
 template <int NV>
@@ -496,9 +523,9 @@ struct ProjL {
     static void run(cudaStream_t st, long long n4, const Tab& t, const double* d, const double* sig2, const float4* w, float4* out,
                     double* part, bool dots, uint2* out16, const double* nest, float* sc_out, const Fin& fin) {
         if (dots)
-            k_proj32<NV, true><<<rgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out, fin);
+            k_proj32<NV, true><<<kgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out, fin);
         else
-            k_proj32<NV, false><<<rgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out, fin);
+            k_proj32<NV, false><<<kgrid(n4), TPB, 0, st>>>(n4, t, d, sig2, w, out, reinterpret_cast<float2*>(part), out16, nest, sc_out, fin);
     }
 };
 
@@ -530,7 +557,7 @@ template <int NV>
 struct ShiftL {
     static void run(cudaStream_t st, const Geom& g, float vol, const float4* v, const float4* z, const uint8_t* m, const float4* P,
                     const Tab& t, const TabH& th, const float* sc, float4* w, double* part, const Fin& fin) {
-        const unsigned nb = rgrid(g.box());
+        const unsigned nb = kgrid(g.box());
         if (sc)
             k_shift_dots<NV, true><<<nb, TPB, 0, st>>>(g, vol, v, z, m, P, t, th, sc, w, reinterpret_cast<float2*>(part), fin);
         else

@@ -194,6 +194,11 @@ int ensure_setup(stg_t* h, bool reference);
 // runs body() through a CUDA-graph cache (solver.cu)
 int graphed(stg_t* h, GraphCache& G, long long key, const std::function<int()>& body, const std::function<void(bool)>& state);
 bool fast(const stg_t* h, const Level& L);
+int sweeps_per_colour(const stg_t* h);
+// the V-cycle of levels top .. 0 in one cluster launch (smallcycle.cu), where it applies; rhs:
+// the right-hand side of level top (null: its own r); the result is left in lv[top].xb
+bool small_cycle_ok(const stg_t* h, int top);
+int small_cycle(stg_t* h, int top, const float4* rhs);
 // one V-cycle out = M(rhs) and y = A x on the finest level (FP32, solver.cu)
 int precond3(stg_t* h, const float4* rhs, float4* out);
 int apply3(stg_t* h, const float4* x, float4* y);

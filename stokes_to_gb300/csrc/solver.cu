@@ -256,8 +256,14 @@ int vcycle_levels(stg_t* h, int top, const float4* rhs) {
     const bool mixed = h->opts.method == STG_METHOD_MIXED;
     const bool lin = h->opts.prolong == 1 && !h->reference_cycle;
     const int L = h->L;
+    int low = 0;  // levels low .. 0 run in one launch (0: the coarsest solve alone)
     for (int i = top; i >= 1; i--) {
         Level& F = h->lv[i];
+        if (small_cycle_ok(h, i)) {
+            low = i;
+            PROF(h, i == L - 1 ? 1 : 10, 0.0, small_cycle(h, i, i == L - 1 ? rhs : nullptr));
+            break;
+        }
         const float4* r = (i == L - 1) ? rhs : F.r;
         F.cur = 0;
         STG_TRY(smooth(h, F, r, false, true));
@@ -265,9 +271,11 @@ int vcycle_levels(stg_t* h, int top, const float4* rhs) {
         PROF(h, 2, 49.0 * F.g.box() + 17.0 * C.g.box(), restrict_resid32(h->st, C.g, F.g, (float)F.vol, r, F.x(), F.m, F.P32, C.m, C.r, fast(h, F)));
     }
     Level& C0 = h->lv[0];
-    C0.cur = 0;
-    PROF(h, 7, 0.0, dense_apply32(h->st, h->dense, C0.g, L == 1 ? rhs : C0.r, C0.x()));
-    for (int i = 1; i <= top; i++) {
+    if (low == 0) {
+        C0.cur = 0;
+        PROF(h, 7, 0.0, dense_apply32(h->st, h->dense, C0.g, L == 1 ? rhs : C0.r, C0.x()));
+    }
+    for (int i = low + 1; i <= top; i++) {
         Level& F = h->lv[i];
         Level& C = h->lv[i - 1];
         const float4* r = (i == L - 1) ? rhs : F.r;
@@ -354,7 +362,7 @@ int coarse_cycle(stg_t* h) {
 // finest right-hand side is `rhs`, the result is left in fine(h).x().
 int vcycle(stg_t* h, const float4* rhs) {
     const int L = h->L;
-    if (L == 1) return vcycle_levels(h, 0, rhs);
+    if (L == 1 || small_cycle_ok(h, L - 1)) return vcycle_levels(h, L - 1, rhs);
     const bool mixed = h->opts.method == STG_METHOD_MIXED;
     Level& F = h->lv[L - 1];
     Level& C = h->lv[L - 2];

@@ -20,6 +20,7 @@
 
 #include "alpha.cuh"
 #include "ctx.h"
+#include "rowdot.cuh"
 
 namespace stg {
 
@@ -684,11 +685,22 @@ __global__ void __launch_bounds__(TPB) k2v_gemv(const __grid_constant__ V2 v) {
 // 8^2, 18 passes): a design iteration with about 34 V-cycles 12.2 -> 5.65 ms; 512^2, two levels
 // above the cluster's: a solve of 46 V-cycles 22.3 -> 8.7 ms.
 constexpr int VT = 512;  // threads of a cluster's block
+constexpr int CLUSTER_ND = 320;  // coarsest unknowns of a solve inside the cluster (8^2)
 __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, int top, int parts, const float* rhs, float* out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-    const int t0 = blockIdx.x * VT + threadIdx.x, step = gridDim.x * VT;
+    // consecutive warps in different blocks: the small levels then use every SM of the cluster
+    const int t0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), step = gridDim.x * VT;
+    const int lane = threadIdx.x & 31, warps = step >> 5;
+    RowDots<CLUSTER_ND, 2> rows;
+    int at = -1;  // the thread's entry of the coarsest right-hand side
+    auto ahead = [&] {
+        if (!(parts & 2)) return;
+        rows.load(v.inv, v.ld, t0 >> 5, warps, lane);
+        if (threadIdx.x < CLUSTER_ND) at = __ldg(v.map + threadIdx.x);
+    };
     if (parts & 1) {
+        if (top == 0) ahead();
         if (rhs) {
             pad_in(v, v.lv[top], rhs, t0, step);
             cl.sync();
@@ -700,11 +712,30 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
             sweep2<true, false>(L, 1, L.xa, C, nullptr, L.xb, t0, step);
             cl.sync();
             restrict2(L, L.xb, C, t0, step);
+            if (i == 1) ahead();
             cl.sync();
         }
     }
-    if (parts & 2) {
-        for (int row = t0 >> 5; row < v.nd; row += step >> 5) gemv_row2(v, row, threadIdx.x & 31);
+    if (parts & 2) {  // (always with part 1)
+        __shared__ double rd[CLUSTER_ND];
+        static_assert(CLUSTER_ND <= VT, "one entry of the right-hand side a thread");
+        const Lv2& L = v.lv[0];
+        if (threadIdx.x < CLUSTER_ND) rd[threadIdx.x] = at >= 0 ? (double)ldv2(L.r + at) : 0.0;
+        __syncthreads();
+        for (int first = t0 >> 5;;) {
+            double s[2];
+            rows.dot(rd, lane, s);
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int row = first + k * warps;
+                if (lane != k || row >= CLUSTER_ND) continue;
+                const int a = __ldg(v.map + row);
+                if (a >= 0) L.xa[a] = (float)s[k];
+            }
+            first += 2 * warps;
+            if (first >= CLUSTER_ND) break;
+            rows.load(v.inv, v.ld, first, warps, lane);
+        }
         cl.sync();
     }
     if (parts & 4) {
@@ -892,7 +923,7 @@ int setup2(stg_t* h) {
 // coarsest solve when its inverse is small, run in one cluster launch (128^2: 8192 cells a
 // colour, one for each thread of 16 blocks; at 256^2 a pass of one cluster would take longer
 // than a launch of the whole GPU); larger ones a launch a pass, replayed as a CUDA graph.
-constexpr int CLUSTER_N = 128, CLUSTER_ND = 512;
+constexpr int CLUSTER_N = 128;
 
 int launch_cluster2(stg_t* h, int top, int parts, const float* rhs, float* out) {
     cudaLaunchConfig_t cfg = {};
@@ -916,7 +947,7 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
     const unsigned gs = g1(v.fine.size());
     int top = fine;  // finest level of the cluster part
     while (top > 0 && v.lv[top].n > CLUSTER_N) top--;
-    const bool whole = top == fine, small = v.nd <= CLUSTER_ND;
+    const bool whole = top == fine, small = v.nd == CLUSTER_ND;
     if (whole && small) return launch_cluster2(h, top, 7, rhs, out);
     if (!whole || top == 0) {
         k2v_in<<<gs, TPB, 0, h->st>>>(v, rhs);
