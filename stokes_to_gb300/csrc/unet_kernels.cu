@@ -45,6 +45,7 @@ __device__ __forceinline__ void vox(int n, int v, int& i, int& j, int& k) {
 
 // forward 3x3x3 convolution; CIN multiple of 16, COUT multiple of 8 (<= 64); F32: FP32
 // output (used for gradients), else BF16
+// COUT: output channels of a warp, a slice of the layer's cout starting at COUT blockIdx.y
 template <int COUT, bool F32>
 __global__ void __launch_bounds__(32 * WPB) k_conv3_fwd(const __nv_bfloat16* __restrict__ in, int cin, int ldin,
                                                         const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
@@ -54,6 +55,8 @@ __global__ void __launch_bounds__(32 * WPB) k_conv3_fwd(const __nv_bfloat16* __r
     const int V = n * n * n;
     const int v0 = (blockIdx.x * WPB + warp) * 16;
     if (v0 >= V) return;
+    const int cb = COUT * blockIdx.y;
+    w += (size_t)cb * cin;
     const int vr0 = v0 + gid, vr1 = v0 + gid + 8;
     const bool in0 = vr0 < V, in1 = vr1 < V;  // rows past the grid (V not a multiple of 16) stay zero
     int i0, j0, k0, i1, j1, k1;
@@ -71,6 +74,7 @@ __global__ void __launch_bounds__(32 * WPB) k_conv3_fwd(const __nv_bfloat16* __r
         const __nv_bfloat16* p0 = in + (size_t)(ok0 ? (a0i * n + a0j) * n + a0k : 0) * ldin;
         const __nv_bfloat16* p1 = in + (size_t)(ok1 ? (a1i * n + a1j) * n + a1k : 0) * ldin;
         const __nv_bfloat16* wt = w + (size_t)t * wtap;
+#pragma unroll 4
         for (int c0 = 0; c0 < cin; c0 += 16) {
             uint32_t a[4];
             a[0] = ok0 ? ld_pair(p0 + c0 + 2 * tig) : 0u;
@@ -87,7 +91,7 @@ __global__ void __launch_bounds__(32 * WPB) k_conv3_fwd(const __nv_bfloat16* __r
     }
 #pragma unroll
     for (int f = 0; f < NF; f++) {
-        const int co = f * 8 + 2 * tig;
+        const int co = cb + f * 8 + 2 * tig;
         const float b0 = bias ? bias[co] : 0.f, b1 = bias ? bias[co + 1] : 0.f;
         float y00 = acc[f][0] + b0, y01 = acc[f][1] + b1, y10 = acc[f][2] + b0, y11 = acc[f][3] + b1;
         if (relu) {
@@ -170,14 +174,38 @@ __global__ void __launch_bounds__(32 * WPB) k_conv3_dw(const __nv_bfloat16* __re
     }
 }
 
-// db[co] += sum_v dy[v][co] (one block per 32 channels x voxel chunk)
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dy, int cout, int lddy, float* __restrict__ db, int V, int chunk) {
-    const int co = blockIdx.y * 32 + (threadIdx.x & 31);
-    if (co >= cout) return;
-    const int vbeg = blockIdx.x * chunk, vend = min(vbeg + chunk, V);
-    float s = 0.f;
-    for (int v = vbeg + (threadIdx.x >> 5); v < vend; v += blockDim.x >> 5) s += __bfloat162float(dy[(size_t)v * lddy + co]);
-    atomicAdd(db + co, s);
+// db[co] += sum_v dy[v][co]: a thread reads eight channels of a voxel at a time (16 bytes),
+// cout / 8 neighbouring threads (a power of two) a voxel. Bound: the reading of dy; at 32^3 x 16
+// 230 us as one chain of 512 dependent 2-byte loads a thread in 8 blocks, now 5 us.
+__global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restrict__ dy, int cout, int lddy, float* __restrict__ db,
+                                                   int V) {
+    __shared__ float sh[8][64];
+    const int tpv = cout >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = lane & (tpv - 1), vpb = 256 / tpv;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int v = blockIdx.x * vpb + threadIdx.x / tpv; v < V; v += gridDim.x * vpb) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(dy + (size_t)v * lddy + 8 * grp));
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[u]));
+            acc[2 * u] += f.x;
+            acc[2 * u + 1] += f.y;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        for (int o = 16; o >= tpv; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+        if (lane < tpv) sh[warp][8 * grp + u] = acc[u];
+    }
+    __syncthreads();
+    if (threadIdx.x < cout) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) t += sh[w][threadIdx.x];
+        atomicAdd(db + threadIdx.x, t);
+    }
 }
 
 // Wf[t][ci][co] = W[26 - t][co][ci]  (BF16 working weights for the backward-data pass)
@@ -430,6 +458,9 @@ constexpr size_t TC_FLOOR_TWO = 78 * 1024, TC_FLOOR_ONE = 118 * 1024;
 // J with the most useful rows per M-tile row, then as many planes per CTA as the tensor
 // memory holds (256 columns with two CTAs per SM, 512 with one); J = 0 when no plan fits
 // (small grids use the mma.sync kernel)
+// Small grids: fewer planes per CTA, until there is a CTA for every SM (each output's sum has
+// the same order, so the result is the same). At 32^3 x 16 channels P 4 -> 1, 24 -> 96 CTAs, 67
+// -> 26 us a layer.
 TcPlan tc_plan(int n, int cout) {
     TcPlan best;
     for (int tier = 0; tier < 2 && !best.J; tier++) {
@@ -454,6 +485,8 @@ TcPlan tc_plan(int n, int cout) {
         }
     }
     if (best.J) {
+        const int jb = (n + best.J - 1) / best.J;
+        while (best.P > 1 && (n + best.P - 1) / best.P * jb < 152) best.P--;
         int c = 32;
         while (c < best.P * best.T * cout) c <<= 1;
         best.ncols = c;
@@ -476,7 +509,7 @@ int launch_tc(const TcPlan& P, cudaStream_t st, const __nv_bfloat16* in, int cin
 }
 
 template <int C>
-void launch_fwd(int nblk, cudaStream_t st, const __nv_bfloat16* in, int cin, int ldin, const __nv_bfloat16* w, const float* bias,
+void launch_fwd(dim3 nblk, cudaStream_t st, const __nv_bfloat16* in, int cin, int ldin, const __nv_bfloat16* w, const float* bias,
                 void* out, int ldout, int n, int relu, bool f32, int wtap) {
     if (f32)
         k_conv3_fwd<C, true><<<nblk, 32 * WPB, 0, st>>>(in, cin, ldin, w, bias, out, ldout, n, relu, wtap);
@@ -543,7 +576,15 @@ int conv3_forward(cudaStream_t st, const __nv_bfloat16* in, int cin, int ldin, c
             return STG_OK;
         }
     }
-    const int nblk = (int)(((V + 15) / 16 + WPB - 1) / WPB);
+    dim3 nblk((unsigned)(((V + 15) / 16 + WPB - 1) / WPB));
+    if (nblk.x < 152 && cout % 16 == 0) {
+        // few voxels: a warp takes 16 output channels, so that more of them share the chain of
+        // loads (8^3, 64 -> 64 channels: 93 us with 64 channels a warp in 8 blocks, now 32)
+        nblk.y = (unsigned)(cout / 16);
+        launch_fwd<16>(nblk, st, in, cin, ldin, w, bias, out, ldout, n, relu, f32_out, wtap);
+        STG_LAUNCH_CK();
+        return STG_OK;
+    }
     switch (cout) {
         case 8: launch_fwd<8>(nblk, st, in, cin, ldin, w, bias, out, ldout, n, relu, f32_out, wtap); break;
         case 16: launch_fwd<16>(nblk, st, in, cin, ldin, w, bias, out, ldout, n, relu, f32_out, wtap); break;
@@ -560,12 +601,16 @@ int conv3_forward(cudaStream_t st, const __nv_bfloat16* in, int cin, int ldin, c
 
 int conv3_backward_weights(cudaStream_t st, const __nv_bfloat16* x, int cin, int ldx, const __nv_bfloat16* dy, int cout, int lddy,
                            float* dw, float* db, int n) {
-    if (n < 1 || cin % 8 || cin < 8 || (cin > 64 && cin != 96) || cout % 16 || cout < 16 || ldx % 2 || lddy % 2) {
+    if (n < 1 || cin % 8 || cin < 8 || (cin > 64 && cin != 96) || (cout != 16 && cout != 32 && cout != 64) || ldx % 2 || lddy % 8 ||
+        ((uintptr_t)dy & 15)) {
         set_error("conv3_backward_weights: unsupported shape (cin %d, cout %d)", cin, cout);
         return STG_E_INVALID;
     }
     const int V = n * n * n;
-    const int chunk = 1024;  // voxels per warp
+    // voxels per warp: a chain of loads and MMAs, so as short as leaves 16 warps an SM in all
+    // (32^3 x 16 channels: 256 instead of 1024, 68 -> 31 us; 8^3, 64 channels: 32, 48 -> 9 us)
+    int chunk = 1024;
+    while (chunk > 32 && (long long)((V + chunk - 1) / chunk) * 27 * (cout / 16) < 2432) chunk >>= 1;
     const int nchunk = (V + chunk - 1) / chunk;
     dim3 grid((nchunk + WPB - 1) / WPB, 27, cout / 16);
     switch (cin) {
@@ -581,9 +626,8 @@ int conv3_backward_weights(cudaStream_t st, const __nv_bfloat16* x, int cin, int
     }
     STG_LAUNCH_CK();
     if (db) {
-        const int bchunk = 4096;
-        dim3 g2((V + bchunk - 1) / bchunk, (cout + 31) / 32);
-        k_bias_grad<<<g2, 256, 0, st>>>(dy, cout, lddy, db, V, bchunk);
+        const int per = 4 * 2048 / cout;  // voxels of a block: four a thread
+        k_bias_grad<<<std::min(152, (V + per - 1) / per), 256, 0, st>>>(dy, cout, lddy, db, V);
         STG_LAUNCH_CK();
     }
     return STG_OK;
