@@ -515,6 +515,98 @@ __global__ void k_mask_to_blocked(Geom g, Blocked B, const uint8_t* __restrict__
     out[t] = s >= 0 ? ((m[s] >> comp) & 1) : 1;
 }
 
+// A x or E x (ENERGY) on vectors in the reference's blocked layout, on levels that admit the
+// Laplacian form. The form asks for vectors that are zero on fixed faces; A and E read those
+// faces as zero themselves (fix_f u of stencil.cuh), so masking them on loading makes it hold
+// for any vector; a fixed row is the identity (A) or zero (E).
+// A block takes a 4 x 4 x 16 (i, j, k) tile: four 64-entry blocks of each kind, read with a
+// one-slot halo into shared memory by component, written back in the blocked order.
+// Bound: the FP64 pipe (two operations per SM and clock): 40 operations a slot (E: 27) against
+// 90 of the 13-slot stencil, and no slot copies (96^3, A and E together: 417 -> 156 us, conversions
+// through the slots included before).
+constexpr int OI = 4, OJ = 4, OK_ = 16;                      // tile
+constexpr int HI = OI + 2, HJ = OJ + 2, HK = OK_ + 2, HN = HI * HJ * HK;  // with halo
+__device__ __forceinline__ long long blocked_index(const Blocked& B, int c, int x, int y, int z) {
+    const int nb = B.n >> 2, bx = x >> 2, by = y >> 2, bz = z >> 2, ix = x & 3, iy = y & 3, iz = z & 3;
+    if (c == 0) return (((long long)bz * nb + by) * nb + bx) * 64 + iz * 16 + iy * 4 + ix;
+    const int d = c - 1, nbx = nb + (d == 0), nby = nb + (d == 1);
+    const int in = d == 0 ? ix * 16 + iz * 4 + iy : d == 1 ? iy * 16 + iz * 4 + ix : iz * 16 + iy * 4 + ix;
+    return B.cell_size() + d * B.face_size() + (((long long)bz * nby + by) * nbx + bx) * 64 + in;
+}
+template <bool ENERGY>
+__global__ void __launch_bounds__(TPB) k_op_blocked(Geom g, Blocked B, double vol, const double* __restrict__ in,
+                                                    const uint8_t* __restrict__ m, const d4* __restrict__ P, double* __restrict__ out) {
+    __shared__ double sx[4][HN];
+    __shared__ double so[4][TPB];
+    const int n = g.n, tid = threadIdx.x;
+    const int i0 = blockIdx.z * OI, j0 = blockIdx.y * OJ, k0 = blockIdx.x * OK_;
+    // kinds this tile holds: cells and the faces of each axis (one block more along the axis)
+    const bool fi = i0 < n, fj = j0 < n, fk = k0 < n;
+    const bool has[4] = {fi && fj && fk, fj && fk, fi && fk, fi && fj};
+    if (!(has[0] || has[1] || has[2] || has[3])) return;
+    for (int e = tid; e < HN; e += TPB) {
+        const int c = e % HK, b = (e / HK) % HJ, a = e / (HK * HJ);
+        const int i = i0 - 1 + a, j = j0 - 1 + b, k = k0 - 1 + c;
+        const bool box = i >= 0 && j >= 0 && k >= 0 && i <= n && j <= n && k <= n;
+        const uint8_t mm = box ? __ldg(m + g.slot(i, j, k)) : (uint8_t)MALL;
+        sx[0][e] = (!ENERGY && box && cell_ok(n, i, j, k)) ? __ldg(in + blocked_index(B, 0, i, j, k)) : 0.0;
+        sx[1][e] = (mm & MU) ? 0.0 : __ldg(in + blocked_index(B, 1, i, j, k));
+        sx[2][e] = (mm & MV) ? 0.0 : __ldg(in + blocked_index(B, 2, i, j, k));
+        sx[3][e] = (mm & MW) ? 0.0 : __ldg(in + blocked_index(B, 3, i, j, k));
+    }
+    __syncthreads();
+    {
+        const int c = tid & (OK_ - 1), b = (tid >> 4) & 3, a = tid >> 6;
+        const int i = i0 + a, j = j0 + b, k = k0 + c;
+        double o[4] = {0.0, 0.0, 0.0, 0.0};
+        if (i <= n && j <= n && k <= n) {
+            const int e = ((a + 1) * HJ + b + 1) * HK + c + 1;
+            constexpr int DI = HJ * HK, DJ = HK;
+            const int s = g.slot(i, j, k);
+            const uint8_t mm = __ldg(m + s);
+            double pen[4];
+            load4(P, s, pen[0], pen[1], pen[2], pen[3]);
+            auto lap = [&](int q) {
+                return 6.0 * sx[q][e] - (sx[q][e - DI] + sx[q][e + DI]) - (sx[q][e - DJ] + sx[q][e + DJ]) - (sx[q][e - 1] + sx[q][e + 1]);
+            };
+            if (ENERGY) {
+                if (cell_ok(n, i, j, k)) o[0] = pen[0] * __ldg(in + blocked_index(B, 0, i, j, k));
+                if (!(mm & MU)) o[1] = vol * lap(1) + pen[1] * sx[1][e];
+                if (!(mm & MV)) o[2] = vol * lap(2) + pen[2] * sx[2][e];
+                if (!(mm & MW)) o[3] = vol * lap(3) + pen[3] * sx[3][e];
+            } else {
+                const double p = sx[0][e];
+                if (cell_ok(n, i, j, k))
+                    o[0] = vol * ((sx[1][e + DI] - sx[1][e]) + (sx[2][e + DJ] - sx[2][e]) + (sx[3][e + 1] - sx[3][e])) + pen[0] * p;
+                // (fixed rows: the value read, below)
+                if (!(mm & MU)) o[1] = vol * (lap(1) - (p - sx[0][e - DI])) + pen[1] * sx[1][e];
+                if (!(mm & MV)) o[2] = vol * (lap(2) - (p - sx[0][e - DJ])) + pen[2] * sx[2][e];
+                if (!(mm & MW)) o[3] = vol * (lap(3) - (p - sx[0][e - 1])) + pen[3] * sx[3][e];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) so[q][tid] = o[q];
+    }
+    __syncthreads();
+    // blocked order: thread t writes entry t % 64 of block t / 64 (along k) of each kind
+    const int q = tid >> 6, t = tid & 63, a0 = t & 3, a1 = (t >> 2) & 3, a2 = t >> 4;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const int kb = k0 + 4 * q;
+        if (!has[c] || (c == 3 ? kb > n : kb >= n)) continue;
+        // (i, j, k) offsets of entry t in a block of this kind (internal.cuh Blocked)
+        const int a = c == 1 ? a2 : a0, b = c == 0 ? a1 : c == 1 ? a0 : c == 2 ? a2 : a1, e = c == 0 ? a2 : c == 1 ? a1 : c == 2 ? a1 : a2;
+        const int i = i0 + a, j = j0 + b, k = kb + e;
+        const long long at = blocked_index(B, c, i, j, k);
+        double v = so[c][(a << 6) | (b << 4) | (4 * q + e)];
+        if (c > 0) {
+            const bool pad = !face_ok(n, c - 1, i, j, k);
+            if (pad || (__ldg(m + g.slot(i, j, k)) & (1 << c))) v = ENERGY ? 0.0 : __ldg(in + at);  // identity rows of A
+        }
+        out[at] = v;
+    }
+}
+
 __global__ void k_vol_slots(Geom g, const uint8_t* __restrict__ m, double cell_vol, double vol, d4* __restrict__ out) {
     long long t = (long long)blockIdx.x * TPB + threadIdx.x;
     if (t >= g.box()) return;
@@ -931,6 +1023,17 @@ int blocked_to_slots64(cudaStream_t st, const Geom& g, const double* in, d4* out
 int slots_to_blocked64(cudaStream_t st, const Geom& g, const d4* in, double* out, const double* pad_src) {
     Blocked B{g.n};
     k_slots_to_blocked64<<<grid_for(B.size(), TPB), TPB, 0, st>>>(g, B, reinterpret_cast<const double*>(in), out, pad_src);
+    STG_LAUNCH_CK();
+    return STG_OK;
+}
+
+int op_blocked(cudaStream_t st, const Geom& g, double vol, const double* in, const uint8_t* m, const d4* P, double* out, bool energy) {
+    Blocked B{g.n};
+    const dim3 grid((g.n + 4 + OK_ - 1) / OK_, g.n / OJ + 1, g.n / OI + 1);
+    if (energy)
+        k_op_blocked<true><<<grid, TPB, 0, st>>>(g, B, vol, in, m, P, out);
+    else
+        k_op_blocked<false><<<grid, TPB, 0, st>>>(g, B, vol, in, m, P, out);
     STG_LAUNCH_CK();
     return STG_OK;
 }

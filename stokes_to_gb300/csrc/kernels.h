@@ -87,6 +87,9 @@ int penalty_from_field(cudaStream_t st, const Geom& g, const double* cell, const
 // reference blocked layout <-> slots. pad_identity: blocked padding entries copy in->out.
 int blocked_to_slots64(cudaStream_t st, const Geom& g, const double* in, d4* out);
 int slots_to_blocked64(cudaStream_t st, const Geom& g, const d4* in, double* out, const double* pad_src);
+// out = A in (or E in) in the blocked layout, any vector, on a level that admits the Laplacian
+// form; in and out must not overlap
+int op_blocked(cudaStream_t st, const Geom& g, double vol, const double* in, const uint8_t* m, const d4* P, double* out, bool energy);
 int mask_to_blocked(cudaStream_t st, const Geom& g, const uint8_t* m, uint8_t* out);
 // descriptor vol per unknown: cell_vol on free cells, vol on free faces, 0 on fixed / absent
 int vol_slots(cudaStream_t st, const Geom& g, const uint8_t* m, double cell_vol, double vol, d4* out);

@@ -1466,6 +1466,13 @@ int stg_density_noise(stg_t* h, uint64_t seed, double sigma, double* out) {
 }
 
 // ---------------------------------------------------------------- LinearMapping adapters
+// The operators run in the blocked layout itself where the level has the Laplacian form and the
+// caller's vectors are apart (they may be the same: then they go through the slots).
+static bool apart(const Level& L, const double* a, const double* b) {
+    const Blocked B{L.g.n};
+    return a + B.size() <= b || b + B.size() <= a;
+}
+
 int stg_apply_A_device(stg_t* h, int level, double* d_Ap, const double* d_p) {
     STG_TRY(check_handle(h));
     if (level < 0 || level >= h->L || !d_Ap || !d_p) {
@@ -1479,6 +1486,11 @@ int stg_apply_A_device(stg_t* h, int level, double* d_Ap, const double* d_p) {
         return STG_OK;
     }
     Level& L = h->lv[level];
+    if (h->lap_ok && !h->gen && apart(L, d_Ap, d_p)) {
+        STG_TRY(op_blocked(h->st, L.g, L.vol, d_p, L.m, L.P64, d_Ap, false));
+        STG_CK(cudaStreamSynchronize(h->st));
+        return STG_OK;
+    }
     STG_TRY(ensure_adapter(L));
     STG_TRY(blocked_to_slots64(h->st, L.g, d_p, L.t0));
     if (h->gen)
@@ -1499,6 +1511,11 @@ int stg_apply_E_device(stg_t* h, double* d_Ap, const double* d_p) {
         return STG_OK;
     }
     Level& L = fine(h);
+    if (h->lap_ok && !h->gen && apart(L, d_Ap, d_p)) {
+        STG_TRY(op_blocked(h->st, L.g, L.vol, d_p, L.m, L.P64, d_Ap, true));
+        STG_CK(cudaStreamSynchronize(h->st));
+        return STG_OK;
+    }
     STG_TRY(ensure_adapter(L));
     STG_TRY(blocked_to_slots64(h->st, L.g, d_p, L.t0));
     if (h->gen)
