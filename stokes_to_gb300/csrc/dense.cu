@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "fp64bits.cuh"
 #include "kernels.h"
 #include "stencil.cuh"
 
@@ -214,104 +215,147 @@ __device__ __forceinline__ void gj_all(int nd, double* a, double* b, int* info) 
 __global__ void __launch_bounds__(TPB) k_gj_all(int nd, double* a, double* b, int* info) { gj_all(nd, a, b, info); }
 
 // ---------------------------------------------------------------- block inversion
-// The coarsest matrix is a saddle point [K B^T; B C]: K (faces) symmetric positive
-// definite, C (cells) the cell penalties plus, on a closed domain, ones everywhere. With
-// the ones moved to one bordering unknown l,
+// The coarsest matrix is a symmetric saddle point [K B^T; B C]: K (faces) positive definite, C
+// (cells) the cell penalties plus, on a closed domain, ones everywhere. With the ones moved to
+// one bordering unknown l,
 //   M = [K B^T 0; B C0 e; 0 e^T -1],   C0 = C - e e^T  (its Schur complement over l is A),
 // elimination in the order faces, cells, l meets positive pivots on the faces and negative
 // ones on the cells, which is stable without a pivot search; only the last block, which
-// holds l and the last cells, pivots inside itself. So the inverse is formed block by block:
-// for a diagonal block k of B unknowns, D = M_kk^-1 and M_ij -= M_ik D M_kj, in place: 2 N^3
-// FP64 operations instead of 4 nd^3, no pivot search over a strided column, and one grid
-// barrier a step. The faces of different axes are uncoupled until cells are eliminated, so
-// one step eliminates a block of every axis at once (S blocks), and tiles that are zero are
-// skipped. Every block of the grid inverts the M_kk for itself (a warp each, the tile in
-// registers), which saves a second barrier. A pivot of the wrong sign (a negative penalty)
-// or faces that are coupled across axes (open boundaries) end the attempt, in every block
-// alike, and the pivoted elimination above runs on the untouched [A | I] instead.
+// holds l and the last cells, pivots inside itself. So the inverse is formed block by block, in
+// place: for a diagonal block p of B unknowns and D = M_pp^-1,
+//   M_ij -= M_ip D M_pj,  M_pj = D M_pj,  M_ip = -M_ip D,  M_pp = D.
+// The faces of different axes are uncoupled until cells are eliminated, so one step takes a block
+// of every axis (S pivots). M stays symmetric up to signs (M_ji = M_ij^T, negated where just
+// one of i and j has been eliminated), so only the tiles i <= j are kept and updated, and the
+// column panel M_ip is the row panel's transpose: N^3 FP64 operations, less the tiles that are
+// zero, instead of the pivoted elimination's 4 nd^3.
+// A step: every block of the grid inverts the S pivot tiles for itself; the products E = D M_pj
+// are shared out; grid barrier; the tiles are shared out; grid barrier.
+// A pivot of the wrong sign (a negative penalty), faces that are coupled across axes (open
+// boundaries) or a matrix that is not symmetric end the attempt, in every block alike, and the
+// pivoted elimination above runs on the untouched [A | I] instead.
 //
-// Bound: for nd = 304 the chain of 10 barriers and 16 x 16 inversions (whole set-up of a
-// 16^3 handle 2.2 -> 0.42 ms against the pivoted elimination, one pivot per barrier), for nd =
-// 2112 the FP64 pipe, two FMAs per SM and clock (set-up at 96^2 276 -> 14.6 ms; 2 nd^3
-// operations take 15 ms, the skipped zero tiles save a third of them). Tile width: 16 keeps
-// the chain of small inversions short, 32 halves the panel traffic where the products dominate.
+// Bound: the FP64 pipe, two FMAs per SM and clock, at nd = 2112 (set-up of a 96^2 handle: 276 ms
+// pivoted, 14.6 with full square updates and FP64 tile inverses, 8.2 now); at nd = 304 the chain
+// of 10 steps of about 25 us (whole set-up of a 16^3 handle 2.2 ms pivoted, 0.36 now). Tile
+// width: 16 keeps the chain of small inversions short, 32 halves the panel traffic where the
+// products dominate.
+
+// Inverse of an FP64 tile to about 2^-44 in double-float arithmetic by one warp: the FP64 pipe's
+// latency makes a pivot of the same elimination cost 1900 clocks, the FP32 pipe's 300. Lane: row
+// lane / LPR, columns CE (lane % LPR) .. in registers. s becomes the inverse, hi its FP32 values.
+struct D2 {
+    float h, l;
+};
+__device__ __forceinline__ D2 d2_norm(float h, float l) {
+    const float t = h + l;
+    return D2{t, l - (t - h)};
+}
+__device__ __forceinline__ D2 d2_mul(D2 a, D2 b) {
+    const float p = a.h * b.h;
+    return d2_norm(p, fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p))));
+}
+__device__ __forceinline__ D2 d2_sub(D2 a, D2 b) {  // a - b
+    const float t = a.h - b.h, bb = t - a.h;
+    return d2_norm(t, ((a.h - (t - bb)) - (b.h + bb)) + (a.l - b.l));
+}
+__device__ __forceinline__ D2 d2_inv(D2 a) {
+    const float r = __fdividef(1.f, a.h);  // a few 2^-24 off; the residual below is exact to second order
+    const float e = fmaf(-a.l, r, fmaf(-a.h, r, 1.f));  // 1 - a r
+    return d2_norm(r, r * fmaf(e, e, e));
+}
+__device__ __forceinline__ D2 d2_shfl(D2 a, int src) {
+    return D2{__shfl_sync(0xffffffffu, a.h, src), __shfl_sync(0xffffffffu, a.l, src)};
+}
+
 template <int B>
-__device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], bool local_pivot, bool positive) {
-    // one warp; lane: row lane / LPR, columns CE (lane % LPR) .. of the tile
+__device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[B][B + 1], bool local_pivot, bool positive) {
     constexpr int LPR = 32 / B, CE = B / LPR;
     const int lane = threadIdx.x & 31, r = lane / LPR, h = lane % LPR;
-    double a[CE];
+    D2 a[CE];
 #pragma unroll
-    for (int c = 0; c < CE; c++) a[c] = s[r][h * CE + c];
+    for (int c = 0; c < CE; c++) split_bits(s[r][h * CE + c], a[c].h, a[c].l);
     int col = 0;  // lane q: the pivot row of step q
     bool ok = true;
-#pragma unroll
+    // the columns rotate by one a step, so that the pivot column is always the first and the loop
+    // stays small (unrolled over the pivots it ran from instruction-cache misses: 186 thousand
+    // clocks a 32 x 32 tile); B steps bring them back in order
+#pragma unroll 1
     for (int q = 0; q < B; q++) {
-        double f = __shfl_sync(0xffffffffu, a[q % CE], r * LPR + q / CE);  // column q of the own row
-        int p = q;
+        D2 f = d2_shfl(a[0], r * LPR);  // the pivot column's entry of the own row
         if (local_pivot) {
-            double best = (r >= q) ? fabs(f) : -1.0;
+            float best = (r >= q) ? fabsf(f.h) : -1.f;
             int bi = r;
             for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
                 const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (ob > best || (ob == best && oi < bi)) {
                     best = ob;
                     bi = oi;
                 }
             }
-            p = bi;
+            const int p = bi;
             if (p != q) {  // exchange rows p and q
                 const int src = (r == q ? p : r == p ? q : r) * LPR + h;
 #pragma unroll
-                for (int c = 0; c < CE; c++) a[c] = __shfl_sync(0xffffffffu, a[c], src);
-                f = __shfl_sync(0xffffffffu, f, src);
+                for (int c = 0; c < CE; c++) a[c] = d2_shfl(a[c], src);
+                f = d2_shfl(f, src);
             }
             if (lane == q) col = p;
         }
-        const double piv = __shfl_sync(0xffffffffu, f, q * LPR);
+        const D2 piv = d2_shfl(f, q * LPR);
         // NaN and infinity fail as well
-        const double want = local_pivot ? fabs(piv) : (positive ? piv : -piv);
-        ok = ok && want > 0.0 && want < 1e300;
-        const double inv = 1.0 / piv;
-        const double g = r == q ? -inv : f * inv;
+        const float want = local_pivot ? fabsf(piv.h) : (positive ? piv.h : -piv.h);
+        ok = ok && want > 0.f && want < 1e37f;
+        const D2 inv = d2_inv(piv);
+        const D2 g = r == q ? D2{-inv.h, -inv.l} : d2_mul(f, inv);
+        const D2 own{-g.h, -g.l};  // the pivot column's new entry
+        D2 first = own;            // the first column's, which moves to the end
 #pragma unroll
         for (int c = 0; c < CE; c++) {
-            const double row = __shfl_sync(0xffffffffu, a[c], q * LPR + h);
-            a[c] = (r == q ? 0.0 : a[c]) - g * row;
+            const D2 row = d2_shfl(a[c], q * LPR + h);
+            const D2 v = d2_sub(r == q ? D2{0.f, 0.f} : a[c], d2_mul(g, row));
+            if (c > 0)
+                a[c - 1] = v;
+            else if (h > 0)
+                first = v;  // (on the row's first lane it is the pivot column)
         }
-        if (h == q / CE) a[q % CE] = -g;
+        // the row's lanes hand their first column on: lane h takes lane h + 1's, the last the pivot's
+        a[CE - 1] = LPR > 1 ? d2_shfl(first, r * LPR + (h + 1) % LPR) : first;
     }
-    if (local_pivot) {  // undo the row exchanges on the columns, last first
 #pragma unroll
-        for (int c = 0; c < CE; c++) s[r][h * CE + c] = a[c];
-        __syncwarp();
+    for (int c = 0; c < CE; c++) {
+        s[r][h * CE + c] = f2d_bits(a[c].h) + f2d_bits(a[c].l);
+        hi[r][h * CE + c] = a[c].h;
+    }
+    __syncwarp();
+    if (local_pivot) {  // undo the row exchanges on the columns, last first
         for (int q = B - 1; q >= 0; q--) {
             const int p = __shfl_sync(0xffffffffu, col, q);
             if (p != q && h == 0) {
                 const double t = s[r][q];
                 s[r][q] = s[r][p];
                 s[r][p] = t;
+                const float u = hi[r][q];
+                hi[r][q] = hi[r][p];
+                hi[r][p] = u;
             }
             __syncwarp();
         }
-    } else {
-#pragma unroll
-        for (int c = 0; c < CE; c++) s[r][h * CE + c] = a[c];
     }
     return ok;
 }
 
 // perm[q], q < N: the unknown at position q, -1 for a decoupled filler, -2 for l. The
 // positions hold S face sections of TF tiles each (one axis a section), then the cells' tiles.
-// ws: N^2 + 4 S B N doubles (the pivoted elimination's second buffer). R: tiles of one column
-// a block updates with one product D M_kj.
-template <int B, int R, int S>
+// ws: N^2 + 3 S B N doubles (the pivoted elimination's second buffer).
+template <int B, int S>
 __global__ void __launch_bounds__(TPB) k_inv_blocks(int nd, int N, int TF, const int* __restrict__ perm, int closed, double* a,
                                                     double* ws, int* info) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    __shared__ double sD[S][B][B + 1], sE[S][B][B + 1], sA[B][B + 1];
+    __shared__ double sD[S][B][B + 1], sE[B][B + 1], sA[B][B + 1];
+    __shared__ float sH[S][B][B + 1], sF[B][B + 1];
     __shared__ int s_bad;
     const int T = N / B, tid = threadIdx.x, TC = S * TF, cell0 = TC * B;
     constexpr int EPT = B * B / TPB;  // tile elements of a thread: rows r0 + e (TPB / B), column c0
@@ -322,141 +366,179 @@ __global__ void __launch_bounds__(TPB) k_inv_blocks(int nd, int N, int TF, const
     const int steps = TF + (T - TC);
     auto pivots = [&](int k) { return k < TF ? S : 1; };
     auto pivot = [&](int k, int q) { return k < TF ? q * TF + k : TC + (k - TF); };
-    // panels of step k: column tiles M_ip (w = 0) and row tiles M_pj (w = 1) of pivot q
-    auto panel = [&](int k, int w, int q) { return ws + (long long)N * N + (long long)(((k & 1) * 2 + w) * S + q) * B * N; };
-    auto put = [&](int i, int j, int r, int k, double v) {  // element (r, c0) of tile (i, j), and the panels of step k
-        M[(long long)(i * B + r) * N + j * B + c0] = v;
-        const int o = r * B + c0;
-        for (int q = 0; q < pivots(k); q++) {
-            const int pv = pivot(k, q);
-            if (j == pv) panel(k, 0, q)[(long long)i * B * B + o] = v;
-            if (i == pv) panel(k, 1, q)[(long long)j * B * B + o] = v;
-        }
-    };
-    auto in_panel = [&](int i, int j, int k) {
+    auto pivot_of = [&](int k, int i) {  // i is pivot .. of step k, or -1
         for (int q = 0; q < pivots(k); q++)
-            if (i == pivot(k, q) || j == pivot(k, q)) return true;
-        return false;
+            if (i == pivot(k, q)) return q;
+        return -1;
     };
-    // the bordered matrix in the elimination order; *info counts faces coupled across axes
-    for (int t = blockIdx.x; t < T * T; t += gridDim.x) {
-        const int i = t / T, j = t % T;
-        const bool apart = i < TC && j < TC && i / TF != j / TF;
+    // M_ip = sign(i) M_pi^T for a pivot p of step k: -1 where i is already eliminated
+    auto sign = [&](int k, int i) { return (i < TC ? (k >= TF || i % TF < k) : i - TC < k - TF) ? -1.0 : 1.0; };
+    // while faces are eliminated, pivot q of section q is coupled to its own section and the cells only
+    auto apart = [&](int k, int q, int i) { return k < TF && i < TC && i / TF != q; };
+    // panels: row tiles M_pj of pivot q of step k (two parities), and E = D M_pj
+    auto panel = [&](int k, int q, int j) { return ws + (long long)N * N + ((long long)((k & 1) * S + q) * N + (long long)j * B) * B; };
+    auto epanel = [&](int q, int j) { return ws + (long long)N * N + ((long long)(2 * S + q) * N + (long long)j * B) * B; };
+    auto put = [&](int i, int j, int r, int k, double v) {  // element (r, c0) of tile i <= j, and the panels of step k
+        M[(long long)(i * B + r) * N + j * B + c0] = v;
+        const int pi = pivot_of(k, i), pj = pivot_of(k, j);
+        if (pi >= 0) panel(k, pi, j)[r * B + c0] = v;
+        if (pj >= 0 && i != j) panel(k, pj, i)[c0 * B + r] = sign(k, i) * v;
+    };
+    auto tile_of = [&](int t, int& i, int& j) {  // t-th of the tiles i <= j
+        j = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+        while (j * (j + 1) / 2 > t) j--;
+        while ((j + 1) * (j + 2) / 2 <= t) j++;
+        i = t - j * (j + 1) / 2;
+    };
+    const int tiles = T * (T + 1) / 2;
+    // the bordered matrix in the elimination order; *info = -1: not of the form
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        int i, j;
+        tile_of(t, i, j);
+        const bool ap = i < TC && j < TC && i / TF != j / TF;
 #pragma unroll
         for (int e = 0; e < EPT; e++) {
             const int r = r0 + e * RS, x = i * B + r, y = j * B + c0;
             const int px = __ldg(perm + x), py = __ldg(perm + y);
             double v;
-            if (px >= 0 && py >= 0)
-                v = a[(long long)px * 2 * nd + py] - (closed && x >= cell0 && y >= cell0 ? 1.0 : 0.0);
-            else if (x == y)
+            if (px >= 0 && py >= 0) {
+                v = a[(long long)px * 2 * nd + py];
+                if (fabs(v - a[(long long)py * 2 * nd + px]) > 1e-12 * fabs(v)) atomicExch(info, -1);
+                if (closed && x >= cell0 && y >= cell0) v -= 1.0;
+            } else if (x == y)
                 v = x >= cell0 ? -1.0 : 1.0;  // l, or a filler with its section's sign
             else
                 v = (closed && ((px == -2 && py >= 0 && y >= cell0) || (py == -2 && px >= 0 && x >= cell0))) ? 1.0 : 0.0;
-            if (apart && v != 0.0) atomicExch(info, -1);
+            if (ap && v != 0.0) atomicExch(info, -1);
             put(i, j, r, 0, v);
         }
     }
     grid.sync();
-    const int G = (T + R - 1) / R;
     bool good = __ldcg(info) == 0;
+    auto load = [&](double (&s)[B][B + 1], const double* tile) {  // false: all zero
+        bool nz = false;
+#pragma unroll
+        for (int e = 0; e < EPT; e++) {
+            const int r = r0 + e * RS;
+            const double v = __ldcg(tile + r * B + c0);
+            nz = nz || v != 0.0;
+            s[r][c0] = v;
+        }
+        return __syncthreads_or(nz) != 0;
+    };
+    auto product = [&](const double (&x)[B][B + 1], const double (&y)[B][B + 1], int r) {  // row r of x y
+        double acc = 0.0;
+#pragma unroll
+        for (int q = 0; q < B; q++) acc += x[r][q] * y[q][c0];
+        return acc;
+    };
+    auto product_t = [&](const double (&x)[B][B + 1], const double (&y)[B][B + 1], int r) {  // row r of x^T y
+        double acc = 0.0;
+#pragma unroll
+        for (int q = 0; q < B; q++) acc += x[q][r] * y[q][c0];
+        return acc;
+    };
     for (int k = 0; k < steps && good; k++) {
         const int np = pivots(k);
         const bool last = k == steps - 1;
-        auto load = [&](double (&s)[B][B + 1], const double* tile) {  // false: all zero
-            bool nz = false;
-#pragma unroll
-            for (int e = 0; e < EPT; e++) {
-                const int r = r0 + e * RS;
-                const double v = __ldcg(tile + r * B + c0);
-                nz = nz || v != 0.0;
-                s[r][c0] = v;
-            }
-            return __syncthreads_or(nz) != 0;
-        };
-        auto product = [&](const double (&x)[B][B + 1], const double (&y)[B][B + 1], int r) {
-            double acc = 0.0;
-#pragma unroll
-            for (int q = 0; q < B; q++) acc += x[r][q] * y[q][c0];
-            return acc;
-        };
         if (tid == 0) s_bad = 0;
-        for (int q = 0; q < np; q++) load(sD[q], panel(k, 0, q) + (long long)pivot(k, q) * B * B);
+        for (int q = 0; q < np; q++) load(sD[q], panel(k, q, pivot(k, q)));
         if (tid < 32 * np) {
-            const bool ok = tile_inverse<B>(sD[tid / 32], last, k < TF);
+            const bool ok = tile_inverse<B>(sD[tid / 32], sH[tid / 32], last, k < TF);
             if (!__all_sync(0xffffffffu, ok) && (tid & 31) == 0) atomicExch(&s_bad, 1);
         }
         __syncthreads();
         good = s_bad == 0;
         if (!good) break;
-        for (int item = blockIdx.x; item < T * G; item += gridDim.x) {
-            const int j = item % T, g0 = (item / T) * R;
-            int jp = -1;  // j is pivot tile jp of this step
-            for (int q = 0; q < np; q++)
-                if (j == pivot(k, q)) jp = q;
-            unsigned enz = 0;  // bit q: D_q M_pj is not zero
-            if (jp < 0) {
+        // Newton steps X += X (I - M_pp X) bring it to FP64 (one, unless the tile is ill-conditioned):
+        // the residual in FP64, the correction, at most 2^-20 of X, in FP32
+        for (int q = 0; q < np && good; q++) {
+            load(sA, panel(k, q, pivot(k, q)));
+            bool rough = true;
+            for (int it = 0; it < 3 && rough; it++) {
+                bool big = false;
 #pragma unroll
-                for (int q = 0; q < S; q++) {
-                    if (q >= np) break;
-                    if (load(sA, panel(k, 1, q) + (long long)j * B * B)) {
-                        enz |= 1u << q;
+                for (int e = 0; e < EPT; e++) {
+                    const int r = r0 + e * RS;
+                    const float f = (float)((r == c0 ? 1.0 : 0.0) - product(sA, sD[q], r));
+                    big = big || !(fabsf(f) < 1e-8f);
+                    sF[r][c0] = f;
+                }
+                rough = __syncthreads_or(big) != 0;  // this step leaves the square of the residual
 #pragma unroll
-                        for (int e = 0; e < EPT; e++) sE[q][r0 + e * RS][c0] = product(sD[q], sA, r0 + e * RS);
+                for (int e = 0; e < EPT; e++) {
+                    const int r = r0 + e * RS;
+                    float f = 0.f;
+#pragma unroll
+                    for (int u = 0; u < B; u++) f = fmaf(sH[q][r][u], sF[u][c0], f);
+                    sD[q][r][c0] += (double)f;
+                }
+                __syncthreads();
+            }
+            good = !rough;
+        }
+        if (!good) break;
+        for (int item = blockIdx.x; item < T * np; item += gridDim.x) {
+            const int j = item / np, q = item - j * np;
+            if (pivot_of(k, j) >= 0 || apart(k, q, j)) continue;
+            const bool nz = load(sA, panel(k, q, j));
+#pragma unroll
+            for (int e = 0; e < EPT; e++) {
+                const int r = r0 + e * RS;
+                epanel(q, j)[r * B + c0] = nz ? product(sD[q], sA, r) : 0.0;
+            }
+            __syncthreads();
+        }
+        grid.sync();
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+            int i, j;
+            tile_of(t, i, j);
+            const int ip = pivot_of(k, i), jp = pivot_of(k, j);
+            const bool keep = last || pivot_of(k + 1, i) >= 0 || pivot_of(k + 1, j) >= 0;  // written even when unchanged
+            double v[EPT];
+            bool changed = true;
+            if (ip >= 0 && jp >= 0) {
+#pragma unroll
+                for (int e = 0; e < EPT; e++) v[e] = ip == jp ? sD[ip][r0 + e * RS][c0] : 0.0;
+            } else if (ip >= 0) {
+#pragma unroll
+                for (int e = 0; e < EPT; e++) v[e] = apart(k, ip, j) ? 0.0 : __ldcg(epanel(ip, j) + (r0 + e * RS) * B + c0);
+            } else if (jp >= 0) {
+                const double sg = -sign(k, i);
+                const bool nz = !apart(k, jp, i) && load(sA, panel(k, jp, i));
+#pragma unroll
+                for (int e = 0; e < EPT; e++) v[e] = nz ? sg * product_t(sA, sD[jp], r0 + e * RS) : 0.0;
+            } else {
+                changed = keep;
+#pragma unroll
+                for (int e = 0; e < EPT; e++) v[e] = __ldcg(M + (long long)(i * B + r0 + e * RS) * N + j * B + c0);
+                const double sg = sign(k, i);
+                for (int q = 0; q < np; q++) {
+                    if (apart(k, q, i) || apart(k, q, j)) continue;
+                    if (load(sA, panel(k, q, i)) && load(sE, epanel(q, j))) {
+                        changed = true;
+#pragma unroll
+                        for (int e = 0; e < EPT; e++) v[e] -= sg * product_t(sA, sE, r0 + e * RS);
                     }
                     __syncthreads();
                 }
             }
-            for (int i = g0; i < g0 + R && i < T; i++) {
-                const bool keep = last || in_panel(i, j, k + 1);  // written even when unchanged
-                int ip = -1;
-                for (int q = 0; q < np; q++)
-                    if (i == pivot(k, q)) ip = q;
-                if (jp < 0 && ip < 0 && !enz && !keep) continue;
-                double v[EPT];
-                bool changed = true;
-                if (jp >= 0) {
-                    if (ip == jp) {
+            if (changed) {
 #pragma unroll
-                        for (int e = 0; e < EPT; e++) v[e] = sD[jp][r0 + e * RS][c0];
-                    } else {  // (another pivot's row: zero, and stays zero)
-                        load(sA, panel(k, 0, jp) + (long long)i * B * B);
-#pragma unroll
-                        for (int e = 0; e < EPT; e++) v[e] = -product(sA, sD[jp], r0 + e * RS);
+                for (int e = 0; e < EPT; e++) {
+                    const int r = r0 + e * RS;
+                    if (!last) {
+                        put(i, j, r, k + 1, v[e]);
+                        continue;
                     }
-                } else if (ip >= 0) {
-#pragma unroll
-                    for (int e = 0; e < EPT; e++) v[e] = (enz >> ip & 1) ? sE[ip][r0 + e * RS][c0] : 0.0;
-                } else {
-                    changed = keep;
-#pragma unroll
-                    for (int e = 0; e < EPT; e++) v[e] = M[(long long)(i * B + r0 + e * RS) * N + j * B + c0];
-#pragma unroll
-                    for (int q = 0; q < S; q++) {
-                        if (q >= np) break;
-                        if (!(enz >> q & 1)) continue;
-                        if (load(sA, panel(k, 0, q) + (long long)i * B * B)) {
-                            changed = true;
-#pragma unroll
-                            for (int e = 0; e < EPT; e++) v[e] -= product(sA, sE[q], r0 + e * RS);
-                        }
-                        __syncthreads();
+                    const int px = __ldg(perm + i * B + r), py = __ldg(perm + j * B + c0);
+                    if (px >= 0 && py >= 0) {
+                        a[(long long)px * 2 * nd + nd + py] = v[e];
+                        if (i != j) a[(long long)py * 2 * nd + nd + px] = v[e];
                     }
                 }
-                if (changed) {
-#pragma unroll
-                    for (int e = 0; e < EPT; e++) {
-                        const int r = r0 + e * RS;
-                        if (!last) {
-                            put(i, j, r, k + 1, v[e]);
-                            continue;
-                        }
-                        const int px = __ldg(perm + i * B + r), py = __ldg(perm + j * B + c0);
-                        if (px >= 0 && py >= 0) a[(long long)px * 2 * nd + nd + py] = v[e];
-                    }
-                }
-                __syncthreads();
             }
+            __syncthreads();
         }
         if (!last) grid.sync();
     }
@@ -665,22 +747,19 @@ void inv_order_free(InvOrder& O) {
 }
 
 int inv_blocks(cudaStream_t st, int nd, const InvOrder& O, int closed, double* a, double* b, int* info, const double** inv) {
-    const int B = inv_tile(nd), R = B == 16 ? 3 : 8;
+    const int B = inv_tile(nd);
     int dev = 0, sms = 0, per_sm = 0, N = O.N, TF = O.TF;
     STG_CK(cudaGetDevice(&dev));
     STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // tiles per work item: one round of items over the SMs at nd = 304 (three tiles), an
-    // eighth of the products spent on D M_kj at larger sizes
-    const void* fn = O.S == 3 ? (B == 16 ? (const void*)k_inv_blocks<16, 3, 3> : (const void*)k_inv_blocks<32, 8, 3>)
-                              : (B == 16 ? (const void*)k_inv_blocks<16, 3, 2> : (const void*)k_inv_blocks<32, 8, 2>);
+    const void* fn = O.S == 3 ? (B == 16 ? (const void*)k_inv_blocks<16, 3> : (const void*)k_inv_blocks<32, 3>)
+                              : (B == 16 ? (const void*)k_inv_blocks<16, 2> : (const void*)k_inv_blocks<32, 2>);
     STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, 0));
     // the pivoted elimination leaves its result in the first buffer for an even nd (the cells
     // and padded faces of a grid whose size is a multiple of 4 are always even in number)
-    const bool fits = (long long)N * N + 4ll * O.S * B * N <= 2ll * nd * nd && (nd & 1) == 0;
+    const bool fits = (long long)N * N + 3ll * O.S * B * N <= 2ll * nd * nd && (nd & 1) == 0;
     if (!fits || per_sm < 1 || sms < 1 || O.S < 2 || O.S > 3) return gj_invert(st, nd, a, b, info, inv, true);
     STG_CK(cudaMemsetAsync(info, 0, sizeof(int), st));
-    const int T = N / B, items = T * ((T + R - 1) / R);
-    const int g = items < sms ? items : sms;
+    const int T = N / B, tiles = T * (T + 1) / 2, g = tiles < sms ? tiles : sms;
     const int* perm = O.perm;
     void* args[] = {&nd, &N, &TF, &perm, &closed, &a, &b, &info};
     STG_CK(cudaLaunchCooperativeKernel(fn, dim3((unsigned)g), dim3(TPB), args, 0, st));
