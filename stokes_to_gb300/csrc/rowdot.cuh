@@ -1,8 +1,9 @@
 // Rows of the coarsest inverse times the right-hand side, inside a V-cycle that one cluster runs
-// (smallcycle.cu, solver2d.cu): a warp takes R rows, their entries are loaded ahead of the
-// barrier that completes the right-hand side, and the rows' FP64 chains run interleaved (one
-// row after the other, with its loads behind the barrier, took 15 us of a 37 us cycle at 304
-// unknowns; the FP64 pipe alone needs 2.4 us on 16 SMs).
+// (smallcycle.cu, solver2d.cu). Half a warp takes a row: the FP64 pipe does two lanes per SM and
+// clock, so the product's cost is its warp instructions, ND / 16 FMAs and four additions of the
+// half-warp sum for two rows (a whole warp a row: ND / 32 and five for one). The entries are
+// loaded ahead of the barrier that completes the right-hand side. One row after the other, with
+// its loads behind the barrier, took 15 us of a 37 us cycle at 304 unknowns.
 #pragma once
 #include "internal.cuh"
 
@@ -10,32 +11,37 @@ namespace stg {
 
 template <int ND, int R>
 struct RowDots {
-    static constexpr int Q = (ND + 31) / 32;
+    static constexpr int Q = (ND + 15) / 16;
+    static constexpr int HALVES = (ND + R - 1) / R;  // half-warps that have rows: h, h + HALVES, ...
     double v[R][Q];
-    // rows first, first + stride, ... of the row-major inverse
-    __device__ __forceinline__ void load(const double* inv, int ld, int first, int stride, int lane) {
+    __device__ __forceinline__ void load(const double* inv, int ld, int h, int lane) {
+        if (h >= HALVES) return;
 #pragma unroll
         for (int k = 0; k < R; k++) {
-            const int row = first + k * stride;
+            const int row = h + k * HALVES;
 #pragma unroll
             for (int q = 0; q < Q; q++) {
-                const int c = lane + 32 * q;
+                const int c = (lane & 15) + 16 * q;
                 v[k][q] = row < ND && c < ND ? __ldg(inv + (long long)row * ld + c) : 0.0;
             }
         }
     }
-    // out[k] = row k . rd (valid in every lane); rd: ND values in shared memory
+    // out[k] = row h + k HALVES times rd (valid in every lane of the half); rd: ND values in
+    // shared memory; called by whole warps with h < HALVES in at least one half
     __device__ __forceinline__ void dot(const double* rd, int lane, double (&out)[R]) const {
+        double a[R][2];
 #pragma unroll
-        for (int k = 0; k < R; k++) out[k] = 0.0;
+        for (int k = 0; k < R; k++) a[k][0] = a[k][1] = 0.0;
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-            const int c = lane + 32 * q;
+            const int c = (lane & 15) + 16 * q;
             const double b = c < ND ? rd[c] : 0.0;
 #pragma unroll
-            for (int k = 0; k < R; k++) out[k] += v[k][q] * b;
+            for (int k = 0; k < R; k++) a[k][q & 1] += v[k][q] * b;
         }
-        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < R; k++) out[k] = a[k][0] + a[k][1];
+        for (int o = 8; o > 0; o >>= 1)
 #pragma unroll
             for (int k = 0; k < R; k++) out[k] += __shfl_xor_sync(0xffffffffu, out[k], o);
     }

@@ -187,8 +187,9 @@ __global__ void __launch_bounds__(CT) k_small_cycle(const __grid_constant__ SCyc
     cg::cluster_group cl = cg::this_cluster();
     const int t0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), step = gridDim.x * CT;
     // this warp's rows of the coarsest inverse and this thread's entries of its right-hand side
-    const int lane = threadIdx.x & 31, warps = step >> 5;
-    RowDots<ND, 3> rows;
+    using Rows = RowDots<ND, 2>;
+    const int lane = threadIdx.x & 31, half = t0 >> 4;
+    Rows rows;
     int at[(ND + CT - 1) / CT];  // offset of entry threadIdx.x + q CT in the coarsest vector
     for (int i = S.top; i >= 1; i--) {
         const SLevel &L = S.lv[i], &C = S.lv[i - 1];
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(CT) k_small_cycle(const __grid_constant__ SCyc
         }
         small_restrict(L, x, C, t0, step);
         if (i == 1) {
-            rows.load(S.inv, S.ld, t0 >> 5, warps, lane);
+            rows.load(S.inv, S.ld, half, lane);
 #pragma unroll
             for (int q = 0; q < (ND + CT - 1) / CT; q++) {
                 const int c = threadIdx.x + q * CT;
@@ -220,17 +221,15 @@ __global__ void __launch_bounds__(CT) k_small_cycle(const __grid_constant__ SCyc
         for (int q = 0; q < (ND + CT - 1) / CT; q++)
             if (threadIdx.x + q * CT < ND) rd[threadIdx.x + q * CT] = (double)__ldcg(reinterpret_cast<const float*>(L.r) + at[q]);
         __syncthreads();
-        for (int first = t0 >> 5;;) {
-            double s[3];
+        if (t0 >> 5 < (Rows::HALVES + 1) / 2) {
+            double s[2];
             rows.dot(rd, lane, s);
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const int row = first + k * warps;
-                if (lane == k && row < ND) reinterpret_cast<float*>(L.xa)[4ll * __ldg(S.slot_of + row) + __ldg(S.comp_of + row)] = (float)s[k];
+            for (int k = 0; k < 2; k++) {
+                const int row = half + k * Rows::HALVES;
+                if ((lane & 15) == k && half < Rows::HALVES && row < ND)
+                    reinterpret_cast<float*>(L.xa)[4ll * __ldg(S.slot_of + row) + __ldg(S.comp_of + row)] = (float)s[k];
             }
-            first += 3 * warps;
-            if (first >= ND) break;
-            rows.load(S.inv, S.ld, first, warps, lane);
         }
         cl.sync();
     }
@@ -255,30 +254,37 @@ __global__ void __launch_bounds__(CT) k_small_cycle(const __grid_constant__ SCyc
 
 }  // namespace
 
-// Blocks of the cluster: 16 where the device grants it, else the portable 8; 0: none. Per device.
-static int cluster_blocks(int dev) {
-    static int blocks[MAX_DEVICES];
-    static bool known[MAX_DEVICES] = {};
-    if (known[dev]) return blocks[dev];
-    blocks[dev] = 0;
-    if (cudaFuncSetAttribute(k_small_cycle, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
-        for (int c = 16; c >= 8 && !blocks[dev]; c /= 2) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)c);
-            cfg.blockDim = dim3(CT);
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)c;
-            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int can = 0;
-            if (cudaOccupancyMaxActiveClusters(&can, k_small_cycle, &cfg) == cudaSuccess && can > 0) blocks[dev] = c;
-        }
+// Blocks of the cluster (more than the portable eight: the coarsest solve's rows need the warps of
+// all of them)
+constexpr int BLOCKS = 16;
+static_assert(RowDots<ND, 2>::HALVES <= BLOCKS * CT / 16, "a half-warp for every pair of rows");
+
+static cudaLaunchConfig_t config(cudaStream_t st, cudaLaunchAttribute (&at)[1]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(BLOCKS);
+    cfg.blockDim = dim3(CT);
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = BLOCKS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// whether the device runs such a cluster
+static bool cluster_ok(int dev) {
+    static int state[MAX_DEVICES] = {};  // 0 unknown, 1 no, 2 yes
+    if (!state[dev]) {
+        int can = 0;
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = config(nullptr, at);
+        const bool ok = cudaFuncSetAttribute(k_small_cycle, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&can, k_small_cycle, &cfg) == cudaSuccess && can > 0;
+        cudaGetLastError();
+        state[dev] = ok ? 2 : 1;
     }
-    cudaGetLastError();
-    known[dev] = true;
-    return blocks[dev];
+    return state[dev] == 2;
 }
 
 // Levels of 8 and 16 cells an axis over the 4^3 coarsest one: at 32^3 a cluster's pass takes as
@@ -289,7 +295,7 @@ bool small_cycle_ok(const stg_t* h, int top) {
     if (top < 1 || top >= MAXS || L.g.n > 16 || (L.g.n & (L.g.n - 1)) || h->dense.nd != ND || h->reference_cycle || !fast(h, L) || !L.P16 || h->opts.prolong == 1)
         return false;
     const int dev = device_slot();
-    return dev >= 0 && cluster_blocks(dev) > 0;
+    return dev >= 0 && cluster_ok(dev);
 }
 
 int small_cycle(stg_t* h, int top, const float4* rhs) {
@@ -309,17 +315,8 @@ int small_cycle(stg_t* h, int top, const float4* rhs) {
                          reinterpret_cast<const uint2*>(L.P16), h->d_pscale + i, L.P32, L.m};
         L.cur = i == 0 ? 0 : 1;
     }
-    const int blocks = cluster_blocks(device_slot());
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(CT);
-    cfg.stream = h->st;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)blocks;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = config(h->st, at);
     STG_CK(cudaLaunchKernelEx(&cfg, k_small_cycle, S));
     count_launch();
     return STG_OK;

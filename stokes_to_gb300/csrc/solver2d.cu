@@ -691,12 +691,13 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
     cg::cluster_group cl = cg::this_cluster();
     // consecutive warps in different blocks: the small levels then use every SM of the cluster
     const int t0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), step = gridDim.x * VT;
-    const int lane = threadIdx.x & 31, warps = step >> 5;
-    RowDots<CLUSTER_ND, 2> rows;
+    using Rows = RowDots<CLUSTER_ND, 1>;
+    const int lane = threadIdx.x & 31, half = t0 >> 4;
+    Rows rows;
     int at = -1;  // the thread's entry of the coarsest right-hand side
     auto ahead = [&] {
         if (!(parts & 2)) return;
-        rows.load(v.inv, v.ld, t0 >> 5, warps, lane);
+        rows.load(v.inv, v.ld, half, lane);
         if (threadIdx.x < CLUSTER_ND) at = __ldg(v.map + threadIdx.x);
     };
     if (parts & 1) {
@@ -722,19 +723,13 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
         const Lv2& L = v.lv[0];
         if (threadIdx.x < CLUSTER_ND) rd[threadIdx.x] = at >= 0 ? (double)ldv2(L.r + at) : 0.0;
         __syncthreads();
-        for (int first = t0 >> 5;;) {
-            double s[2];
+        if (t0 >> 5 < (Rows::HALVES + 1) / 2) {
+            double s[1];
             rows.dot(rd, lane, s);
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int row = first + k * warps;
-                if (lane != k || row >= CLUSTER_ND) continue;
-                const int a = __ldg(v.map + row);
-                if (a >= 0) L.xa[a] = (float)s[k];
+            if ((lane & 15) == 0 && half < CLUSTER_ND) {
+                const int a = __ldg(v.map + half);
+                if (a >= 0) L.xa[a] = (float)s[0];
             }
-            first += 2 * warps;
-            if (first >= CLUSTER_ND) break;
-            rows.load(v.inv, v.ld, first, warps, lane);
         }
         cl.sync();
     }
@@ -947,7 +942,7 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
     const unsigned gs = g1(v.fine.size());
     int top = fine;  // finest level of the cluster part
     while (top > 0 && v.lv[top].n > CLUSTER_N) top--;
-    const bool whole = top == fine, small = v.nd == CLUSTER_ND;
+    const bool whole = top == fine, small = v.nd == CLUSTER_ND && h->c2->cluster * VT / 16 >= CLUSTER_ND;  // a half-warp a row
     if (whole && small) return launch_cluster2(h, top, 7, rhs, out);
     if (!whole || top == 0) {
         k2v_in<<<gs, TPB, 0, h->st>>>(v, rhs);
