@@ -9,25 +9,27 @@
 // table of filter weight sums) lives in the fixed array below, which every GPU that
 // loads this library holds until the process exits.
 //
-// The bisection and the volume sums are the ones of stg_oc_update (same kernels'
-// arithmetic, same reduction grid and order), with the filter volume weights
-// vw_j = sum_i w_ij / W_i formed on the fly instead of being read from a buffer, so both
-// entry points return the same design and multiplier. W_i depends only on how far cell i
-// lies from each pair of domain faces (clamped at the filter radius R), so it is read
+// The bisection and each cell's arithmetic are the ones of stg_oc_update, with the filter
+// volume weights vw_j = sum_i w_ij / W_i formed on the fly instead of being read from a
+// buffer, so both entry points return the same design and multiplier (the volumes' block
+// sums are added in another order: they agree to rounding). 1 / W_i depends only on how far
+// cell i lies from each pair of domain faces (clamped at the filter radius R), so it is read
 // from a table of (R+1)^6 classes built once per call, in the summation order of the
-// handle's filter; a probe then costs (2R+1)^3 table reads per cell.
+// handle's filter; a probe then costs (2R+1)^3 table reads and multiply-adds per cell, and
+// no division among them.
 #include <climits>
 #include <cmath>
 #include <mutex>
 
 #include "kernels.h"
+#include "oc.cuh"
 
 namespace stg {
 
 namespace {
 
 constexpr int TPB = 256;
-constexpr int OC_GRID = 1216;                 // reduction grid (8 x 152 SMs), as stg_oc_update
+constexpr int OC_GRID = 1216;                 // reduction grid (8 x 152 SMs)
 constexpr int NOALLOC_MAX_N = 1024;           // largest design: 1024^3 cells
 constexpr int NOALLOC_MAX_R = 3;              // largest filter radius index: rmin <= 4
 constexpr int NOALLOC_CLASSES = 4096;         // (R+1)^6 weight-sum classes at R = 3
@@ -73,9 +75,9 @@ __device__ __forceinline__ int axis_class(int i, int n, int R) {
     return lo * (R + 1) + hi;
 }
 
-// W for every class: sum of the positive weights over the offsets the class allows, in
-// the loop order of the handle's weight-sum kernel (a, then b, then c), so the sums are
-// bit-identical to the ones stg_oc_update reads
+// 1 / W for every class, W the sum of the positive weights over the offsets the class allows,
+// in the loop order of the handle's weight-sum kernel (a, then b, then c), so the values are
+// bit-identical to the ones behind the weights that stg_oc_update reads
 __global__ void k_wsum_classes(int R, WTabNA T, double* __restrict__ wc) {
     const int per = (R + 1) * (R + 1);
     const int ncls = per * per * per;
@@ -93,7 +95,7 @@ __global__ void k_wsum_classes(int R, WTabNA T, double* __restrict__ wc) {
                 const double w = T.w[((a + R) * D + (b + R)) * D + (c + R)];
                 if (w > 0) s += w;
             }
-    wc[t] = s;
+    wc[t] = 1.0 / s;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -101,8 +103,8 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// One bisection probe: x_new(lambda) and per-block partials of sum vw x_new (into
-// scratch). vw_j = sum_i w_ij / W_i, summed in the handle filter's transpose order. x and
+// One bisection probe, the per-block partials of sum vw x_new(lambda) (into scratch), or with
+// xnew x_new itself. vw_j = sum_i w_ij / W_i, summed in the handle filter's transpose order. x and
 // xnew may be the same array (each element is read before it is written by one thread).
 __global__ void k_oc_noalloc(int n, int R, WTabNA T, const double* __restrict__ wclass_g, const double* x,
                              const double* __restrict__ dc, double lam, double move, double lo, double hi, double* xnew,
@@ -115,7 +117,7 @@ __global__ void k_oc_noalloc(int n, int R, WTabNA T, const double* __restrict__ 
     __syncthreads();
     const int D = 2 * R + 1;
     const long long nc = (long long)n * n * n;
-    const double inv_n = 1.0 / (double)nc;
+    const double inv_n = 1.0 / (double)nc, isl = rsqrt(lam);
     double acc = 0;
     for (long long t = (long long)blockIdx.x * TPB + threadIdx.x; t < nc; t += (long long)gridDim.x * TPB) {
         const int k = (int)(t % n), j = (int)((t / n) % n), i = (int)(t / ((long long)n * n));
@@ -133,17 +135,15 @@ __global__ void k_oc_noalloc(int n, int R, WTabNA T, const double* __restrict__ 
                     if (kk < 0 || kk >= n) continue;
                     const double w = T.w[((a + R) * D + (b + R)) * D + (c + R)];
                     if (w <= 0) continue;
-                    vw += w * 1.0 / wcls[cb + axis_class(kk, n, R)];
+                    vw += w * wcls[cb + axis_class(kk, n, R)];
                 }
             }
         }
         const double xi = x[t];
-        const double dv = vw * inv_n;
-        const double B = fmax(0.0, -dc[t]) / (dv * lam);
-        double xn = xi * sqrt(B);
-        xn = fmin(fmin(hi, xi + move), fmax(fmax(lo, xi - move), xn));
-        if (xnew) xnew[t] = xn;
-        acc += vw * xn;
+        if (xnew)
+            xnew[t] = oc_new(xi, dc[t], vw * inv_n, lam, move, lo, hi);
+        else
+            acc += vw * fmin(fmin(hi, xi + move), fmax(fmax(lo, xi - move), oc_scale(xi, dc[t], vw * inv_n) * isl));
     }
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
@@ -191,7 +191,7 @@ extern "C" int stg_oc_update_noalloc(int n, double rmin, const double* d_x, cons
     const int grid = (int)g;
     double* part = scratch;                 // OC_GRID partials
     double* sum = scratch + SCR_SUM;        // reduced volume
-    double* wclass = scratch + SCR_WCLASS;  // W per class
+    double* wclass = scratch + SCR_WCLASS;  // 1 / W per class
     const int ncls = (R + 1) * (R + 1) * (R + 1) * (R + 1) * (R + 1) * (R + 1);
     k_wsum_classes<<<(ncls + 127) / 128, 128, 0, st>>>(R, T, wclass);
     STG_LAUNCH_CK();

@@ -6,8 +6,12 @@
 #include <cooperative_groups.h>
 #include <math.h>
 
+#include <algorithm>
+#include <utility>
+
 #include "alpha.cuh"
 #include "kernels.h"
+#include "oc.cuh"
 #include "stencil.cuh"
 
 namespace stg {
@@ -63,10 +67,10 @@ __global__ void k_sensitivity(Geom g, const double* __restrict__ rho, stg_alpha 
 
 // Linear hat filter: out_i = sum_j w_ij in_j / W_i (forward) or sum_j w_ji in_j / W_j
 // (transpose), w_ij = max(0, rmin - |c_i - c_j|) over cells inside the domain, W_i =
-// sum_j w_ij. W is computed once per call by k_filter_wsum, so the transpose reads it
-// instead of re-summing every neighbour's weights. dim 2 runs the same loops with a
-// single k plane (nz = 1, no k offsets). Loop order and arithmetic are the same in both
-// kernels, so W_i and the sums are identical wherever they are formed.
+// sum_j w_ij. W (for the transpose in_j / W_j) is computed once per call by k_filter_wsum, so
+// the transpose reads it instead of re-summing every neighbour's weights. dim 2 runs the same
+// loops with a single k plane (nz = 1, no k offsets). Loop order and arithmetic are the same in
+// both kernels, so W_i and the sums are identical wherever they are formed.
 __device__ __forceinline__ double hat_w(double rmin, int a, int b, int c) { return rmin - sqrt((double)(a * a + b * b + c * c)); }
 
 // the weights rmin - |o| of every offset o, computed once on the host (IEEE sqrt, so the
@@ -81,8 +85,11 @@ __device__ __forceinline__ double weight(const WTab& T, double rmin, int R, int 
     return hat_w(rmin, a, b, c);
 }
 
+// in (the transpose): in_t / W_t instead of W_t, the value every neighbour's sum takes, so one
+// FP64 division a cell rather than one a neighbour (64^3, radius 1.5: the transpose was 71 us,
+// now 31)
 template <bool TAB>
-__global__ void k_filter_wsum(int n, int nz, double rmin, int R, int Rz, WTab T, double* __restrict__ W) {
+__global__ void k_filter_wsum(int n, int nz, double rmin, int R, int Rz, WTab T, const double* __restrict__ in, double* __restrict__ W) {
     long long t = (long long)blockIdx.x * TPB + threadIdx.x;
     if (t >= (long long)n * n * nz) return;
     int k = (int)(t % nz), j = (int)((t / nz) % n), i = (int)(t / ((long long)n * nz));
@@ -95,7 +102,7 @@ __global__ void k_filter_wsum(int n, int nz, double rmin, int R, int Rz, WTab T,
                 double w = weight<TAB>(T, rmin, R, Rz, a, b, c);
                 if (w > 0) s += w;
             }
-    W[t] = s;
+    W[t] = in ? in[t] / s : s;
 }
 
 template <bool TAB>
@@ -113,10 +120,7 @@ __global__ void k_filter(int n, int nz, double rmin, int R, int Rz, WTab T, cons
                 double w = weight<TAB>(T, rmin, R, Rz, a, b, c);
                 if (w <= 0) continue;
                 const long long q = ((long long)ii * n + jj) * nz + kk;
-                if (transpose)
-                    s += w * in[q] / W[q];
-                else
-                    s += w * in[q];
+                s += w * (transpose ? W[q] : in[q]);
             }
     out[t] = transpose ? s : s / W[t];
 }
@@ -124,31 +128,6 @@ __global__ void k_filter(int n, int nz, double rmin, int R, int Rz, WTab T, cons
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// One bisection probe of the OC update: x_new(lambda) and its filtered volume partials.
-__global__ void k_oc(int ncell, const double* __restrict__ x, const double* __restrict__ dc, const double* __restrict__ vw,
-                     double lam, double move, double lo, double hi, double* __restrict__ xnew, double* __restrict__ part) {
-    __shared__ double sh[TPB / 32];
-    double acc = 0;
-    double inv_n = 1.0 / ncell;
-    for (long long t = (long long)blockIdx.x * TPB + threadIdx.x; t < ncell; t += (long long)gridDim.x * TPB) {
-        double xi = x[t];
-        double dv = vw[t] * inv_n;
-        double B = fmax(0.0, -dc[t]) / (dv * lam);
-        double xn = xi * sqrt(B);
-        xn = fmin(fmin(hi, xi + move), fmax(fmax(lo, xi - move), xn));
-        if (xnew) xnew[t] = xn;
-        acc += vw[t] * xn;
-    }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0;
-        for (int w = 0; w < TPB / 32; w++) s += sh[w];
-        part[blockIdx.x] = s;
-    }
 }
 
 // seeded density: U[0,1) from a SplitMix64 hash of (seed, Field index)
@@ -176,95 +155,144 @@ __global__ void k_blur(int n, long long nc, long long stride, const double* __re
     out[t] = clip ? fmin(1.0, fmax(0.0, acc)) : acc;
 }
 
+// The OC update searches the multiplier l at which the filtered volume sum vw x_new(l) meets the
+// target: the bracket [0, 1e9] widened by decades while its upper end still overshoots, then
+// bisected to relative width 1e-9 (at most 200 steps), all in one launch. What bounds it is the
+// FP64 unit, which each quarter of an SM has half a lane of: 64 clocks for any FP64 instruction
+// of a warp, more than ninety until its result is there. Therefore
+// - x_new = clamp(s / sqrt(l)) with s formed once (oc_scale), four instructions a cell and probe
+//   where the root and the division of oc_new take fifty;
+// - a block has one warp for each quarter where registers can hold the cells (OC_T): the
+//   sums over warps and blocks, the bracket and 1 / sqrt(l), which every warp forms alike, then
+//   cost no quarter more than once;
+// - 1 / sqrt(l) of both possible next probes is formed while the blocks' sums travel.
+// Before and after, an update: 64^2 cells 271 us, now 112; 64^3 1010 us, now 299 (cells in
+// registers); 128^3 4.41 ms, now 1.71 (cells read for each probe).
+constexpr int OC_CB = 16;          // blocks of the cluster form
+constexpr int OC_CR = 8, OC_GR = 16;  // cells a thread holds, cluster and grid form
+constexpr int OC_MAX_BLOCKS = 1216;
+template <int R>
+constexpr int OC_T = R ? 128 : 512;
+constexpr int OC_CLUSTER_MAX = OC_CB * OC_T<OC_CR> * OC_CR;
 
-// x_new(lambda) of the OC update for the cells of this thread (grid-stride, as k_oc) and
-// the block's part of the filtered volume sum_j vw_j x_new_j.
-__device__ __forceinline__ double oc_block_volume(int ncell, const double* __restrict__ x, const double* __restrict__ dc,
-                                                  const double* __restrict__ vw, double lam, double move, double lo,
-                                                  double hi, double* __restrict__ xnew, double* sh) {
-    double acc = 0;
-    const double inv_n = 1.0 / ncell;
-    for (long long t = (long long)blockIdx.x * TPB + threadIdx.x; t < ncell; t += (long long)gridDim.x * TPB) {
-        const double xi = x[t];
-        const double dv = vw[t] * inv_n;
-        const double B = fmax(0.0, -dc[t]) / (dv * lam);
-        double xn = xi * sqrt(B);
-        xn = fmin(fmin(hi, xi + move), fmax(fmax(lo, xi - move), xn));
-        if (xnew) xnew[t] = xn;
-        acc += vw[t] * xn;
+// The bracket; every warp has the same sums and takes the same steps.
+struct OcBracket {
+    double l1 = 0.0, l2 = 1e9, lam = 1e9;
+    int widened = 0, steps = 0;
+    bool widen = true;
+
+    // the next probe after an overshooting volume, or after another (the bracket's end permitting)
+    __device__ __forceinline__ double candidate(bool over) const {
+        const double up = widen ? 10.0 * l2 : l2;
+        if (widen && over && widened + 1 < 60) return up;
+        return 0.5 * ((over ? lam : l1) + (over ? up : lam));
     }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    double r = 0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < TPB / 32; w++) r += sh[w];
-    __syncthreads();
-    return r;  // valid in thread 0
-}
-
-// Sum of the block partials in the order of the partial reduction kernel (threads stride
-// over the parts, warp tree, warps in order), formed by every block alike so that all
-// blocks take the same bisection decision.
-__device__ __forceinline__ double oc_reduce(const double* part, int nparts, double* sh) {
-    double s = 0;
-    for (int p = threadIdx.x; p < nparts; p += TPB) s += part[p];
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0;
-        for (int w = 0; w < TPB / 32; w++) r += sh[w];
-        sh[TPB / 32] = r;
+    // takes the volume's answer; false once the bracket is narrow enough
+    __device__ __forceinline__ bool step(bool over) {
+        const double next = candidate(over);
+        if (widen) {
+            if (over) {
+                l1 = l2;
+                l2 *= 10.0;
+                widen = ++widened < 60;
+            } else {
+                widen = false;
+            }
+        } else {
+            (over ? l1 : l2) = lam;
+            steps++;
+        }
+        lam = next;
+        return widen || ((l2 - l1) > 1e-9 * (l1 + l2) && steps < 200);
     }
-    __syncthreads();
-    const double r = sh[TPB / 32];
-    __syncthreads();
-    return r;
-}
+};
 
-// The whole OC update in one cooperative launch: the multiplier bracket [0, 1e9] widened
-// by decades while its upper end still overshoots the volume, then bisection to relative
-// width 1e-9 (at most 200 steps), then x_new at the midpoint. One grid-wide barrier per
-// probe; the partials alternate between two buffers so a probe never overwrites the ones
-// the previous probe's reduction still reads.
-__global__ void __launch_bounds__(TPB) k_oc_bisect(int ncell, const double* __restrict__ x, const double* __restrict__ dc,
-                                                   const double* __restrict__ vw, double target, double move, double lo,
-                                                   double hi, double* __restrict__ xnew, double* __restrict__ part,
-                                                   double* __restrict__ lambda_out) {
+// What a probe needs of a cell, formed once.
+struct OcCell {
+    double s, lo, hi, vw;
+    __device__ __forceinline__ double volume(double t) const { return vw * fmin(hi, fmax(lo, s * t)); }
+};
+
+// The update by the blocks of one cluster (CLUSTER: at most OC_CLUSTER_MAX cells; each warp's
+// sum goes straight into every block's shared memory) or of a cooperative launch (through part).
+// Both have two buffers of sums, so that a probe never overwrites those that the previous one's
+// reduction still reads. A thread holds its cells in R registers each, at most, or, R = 0, reads
+// them for each probe with s in xnew (it reads and writes its own cells only).
+template <bool CLUSTER, int R>
+__global__ void __launch_bounds__(OC_T<R>) k_oc_bisect(int ncell, const double* __restrict__ x, const double* __restrict__ dc,
+                                                             const double* __restrict__ vw, double target, double move,
+                                                             double lo, double hi, double* xnew, double* __restrict__ part,
+                                                             double* __restrict__ lambda_out) {
     namespace cg = cooperative_groups;
+    constexpr int T = OC_T<R>, W = T / 32;
+    __shared__ double sum[2][CLUSTER ? OC_CB * W : W];
+    const cg::cluster_group cluster = cg::this_cluster();
     cg::grid_group grid = cg::this_grid();
-    __shared__ double sh[TPB / 32 + 1];
-    const int nparts = gridDim.x;
-    int buf = 0;
-    auto volume = [&](double lam) {
-        const double b = oc_block_volume(ncell, x, dc, vw, lam, move, lo, hi, nullptr, sh);
-        double* pp = part + buf * nparts;
-        if (threadIdx.x == 0) pp[blockIdx.x] = b;
-        grid.sync();
-        const double v = oc_reduce(pp, nparts, sh);
-        buf ^= 1;
-        return v;
-    };
-    double l1 = 0.0, l2 = 1e9;
-    for (int k = 0; k < 60; k++) {
-        if (volume(l2) <= target) break;
-        l1 = l2;
-        l2 *= 10.0;
+    const int nblk = gridDim.x, rank = blockIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double inv_n = 1.0 / ncell;
+    const long long q0 = (long long)rank * T + threadIdx.x, dq = (long long)nblk * T;
+    OcCell c[R ? R : 1];
+    // the rounds that have cells: the same for the block, so that a probe branches past the others
+    const int held = (int)min((long long)R, (ncell - (long long)rank * T + dq - 1) / dq);
+    if (R) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const long long q = q0 + r * dq;
+            c[r] = OcCell{0.0, 0.0, 0.0, 0.0};
+            if (q < ncell) {
+                const double xi = x[q], w = vw[q];
+                c[r] = OcCell{oc_scale(xi, dc[q], w * inv_n), fmax(lo, xi - move), fmin(hi, xi + move), w};
+            }
+        }
+    } else {
+        for (long long q = q0; q < ncell; q += dq) xnew[q] = oc_scale(x[q], dc[q], vw[q] * inv_n);
     }
-    const double tol = 1e-9;
-    int steps = 0;
-    while ((l2 - l1) > tol * (l1 + l2) && steps < 200) {
-        const double lmid = 0.5 * (l1 + l2);
-        if (volume(lmid) > target)
-            l1 = lmid;
-        else
-            l2 = lmid;
-        steps++;
+    if (CLUSTER) cluster.sync();  // every block runs before its shared memory is written
+    OcBracket br;
+    double t = rsqrt(br.lam);
+    bool more = true;
+    for (int buf = 0; more; buf ^= 1) {
+        double acc = 0.0, tc, v = 0.0;
+        if (R) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (r == held) break;
+                acc += c[r].volume(t);
+            }
+        } else {
+            for (long long q = q0; q < ncell; q += dq) {
+                const double xi = x[q];
+                acc += OcCell{xnew[q], fmax(lo, xi - move), fmin(hi, xi + move), vw[q]}.volume(t);
+            }
+        }
+        acc = warp_sum(acc);
+        if (CLUSTER) {
+            if (lane < OC_CB) cluster.map_shared_rank(&sum[buf][0], lane)[rank * W + warp] = acc;
+            auto token = cluster.barrier_arrive();
+            tc = rsqrt(br.candidate(lane == 1));
+            cluster.barrier_wait(std::move(token));
+#pragma unroll
+            for (int p = 0; p < OC_CB * W; p += 32) v += sum[buf][p + lane];
+        } else {
+            if (lane == 0) sum[buf][warp] = acc;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int w = 0; w < W; w++) v += sum[buf][w];
+                part[buf * OC_MAX_BLOCKS + rank] = v;
+                v = 0.0;
+            }
+            auto token = grid.barrier_arrive();
+            tc = rsqrt(br.candidate(lane == 1));
+            grid.barrier_wait(std::move(token));
+            for (int p = lane; p < nblk; p += 32) v += part[buf * OC_MAX_BLOCKS + p];
+        }
+        const bool over = warp_sum(v) > target;
+        t = __shfl_sync(0xffffffffu, tc, over ? 1 : 0);
+        more = br.step(over);
     }
-    const double lmid = 0.5 * (l1 + l2);
-    oc_block_volume(ncell, x, dc, vw, lmid, move, lo, hi, xnew, sh);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *lambda_out = lmid;
+    for (long long q = q0; q < ncell; q += dq) xnew[q] = oc_new(x[q], dc[q], vw[q] * inv_n, br.lam, move, lo, hi);
+    if (rank == 0 && threadIdx.x == 0) *lambda_out = br.lam;
 }
 
 }  // namespace
@@ -298,9 +326,9 @@ int density_filter(cudaStream_t st, int dim, int n, double rmin, const double* i
                 for (int c = -Rz; c <= Rz; c++)
                     T.w[((a + R) * (2 * R + 1) + (b + R)) * (2 * Rz + 1) + (c + Rz)] = rmin - sqrt((double)(a * a + b * b + c * c));
     if (tab)
-        k_filter_wsum<true><<<grid_for(nc, TPB), TPB, 0, st>>>(n, nz, rmin, R, Rz, T, W);
+        k_filter_wsum<true><<<grid_for(nc, TPB), TPB, 0, st>>>(n, nz, rmin, R, Rz, T, transpose ? in : nullptr, W);
     else
-        k_filter_wsum<false><<<grid_for(nc, TPB), TPB, 0, st>>>(n, nz, rmin, R, Rz, T, W);
+        k_filter_wsum<false><<<grid_for(nc, TPB), TPB, 0, st>>>(n, nz, rmin, R, Rz, T, transpose ? in : nullptr, W);
     STG_LAUNCH_CK();
     if (tab)
         k_filter<true><<<grid_for(nc, TPB), TPB, 0, st>>>(n, nz, rmin, R, Rz, T, in, W, out, transpose);
@@ -310,35 +338,48 @@ int density_filter(cudaStream_t st, int dim, int n, double rmin, const double* i
     return STG_OK;
 }
 
-int oc_volume(cudaStream_t st, int ncell, const double* x, const double* dc, const double* vw, double lam, double move,
-              double lo, double hi, double* xnew, double* parts, int* nparts) {
-    long long g = (ncell + TPB - 1) / TPB;
-    if (g > 1216) g = 1216;
-    if (g < 1) g = 1;
-    *nparts = (int)g;
-    k_oc<<<(unsigned)g, TPB, 0, st>>>(ncell, x, dc, vw, lam, move, lo, hi, xnew, parts);
-    STG_LAUNCH_CK();
-    return STG_OK;
-}
-
 int oc_update_device(cudaStream_t st, int ncell, const double* x, const double* dc, const double* vw, double frac,
                      double move, double lo, double hi, double* xnew, double* parts, double* lambda_out) {
-    // the grid of the probe kernel (k_oc), capped at what can be co-resident
-    long long g = (ncell + TPB - 1) / TPB;
-    if (g > 1216) g = 1216;
-    if (g < 1) g = 1;
+    double target = frac * ncell;
+    void* args[] = {&ncell, &x, &dc, &vw, &target, &move, &lo, &hi, &xnew, &parts, &lambda_out};
+    // one cluster while its threads hold at most eight cells each: a cluster barrier is 0.3 us and
+    // one over the device 1.3, but the cells of a probe take 1.3 us of sixteen SMs' FP64 units at
+    // the line (16384 cells: 178 us an update) and next to none of all of them
+    const void* kernel = (const void*)k_oc_bisect<true, OC_CR>;
+    if (ncell <= OC_CLUSTER_MAX) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(OC_CB);
+        cfg.blockDim = dim3(OC_T<OC_CR>);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = OC_CB;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) {
+            STG_CK(cudaLaunchKernelExC(&cfg, kernel, args));
+            return STG_OK;
+        }
+        cudaGetLastError();
+    }
+    // as many blocks as have cells, one on each SM
     int dev = 0, sms = 0, per_sm = 0;
     STG_CK(cudaGetDevice(&dev));
     STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_oc_bisect, TPB, 0));
+    if (sms > OC_MAX_BLOCKS) sms = OC_MAX_BLOCKS;
+    const bool held = ncell <= (long long)sms * OC_T<OC_GR> * OC_GR;
+    const int threads = held ? OC_T<OC_GR> : OC_T<0>;
+    kernel = held ? (const void*)k_oc_bisect<false, OC_GR> : (const void*)k_oc_bisect<false, 0>;
+    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
     if (per_sm < 1) {
         set_error("the OC bisection kernel cannot be made resident");
         return STG_E_CUDA;
     }
-    if (g > (long long)sms * per_sm) g = (long long)sms * per_sm;
-    double target = frac * ncell;
-    void* args[] = {&ncell, &x, &dc, &vw, &target, &move, &lo, &hi, &xnew, &parts, &lambda_out};
-    STG_CK(cudaLaunchCooperativeKernel((const void*)k_oc_bisect, dim3((unsigned)g), dim3(TPB), args, 0, st));
+    const unsigned g = (unsigned)std::min(((long long)ncell + threads - 1) / threads, (long long)sms);
+    STG_CK(cudaLaunchCooperativeKernel(kernel, dim3(g), dim3(threads), args, 0, st));
     return STG_OK;
 }
 
