@@ -238,9 +238,23 @@ int sweeps_per_colour(const stg_t* h) {
     return h->boost ? std::max(s, 2) : s;
 }
 
+// The two sweeps from x = 0 run as one launch where there is one a colour and both are the solver's
+// own uniform-form sweeps (sweep.cu, MODE 3: the faster at every size from 24^3, where the small
+// cycle ends).
+bool fuse_pair(const stg_t* h, const Level& L) {
+    return !h->reference_cycle && sweeps_per_colour(h) == 1 && fast(h, L) && L.P16 && sweep_tma_available();
+}
+
 // C: the coarse level whose correction the first sweep injects (fuse_prolong)
 int smooth(stg_t* h, Level& L, const float4* r, bool post, bool x_is_zero, Level* C = nullptr) {
     const int per = sweeps_per_colour(h);
+    if (x_is_zero && fuse_pair(h, L)) {
+        PROF(h, &L == &fine(h) ? 1 : 10, 40.0 * L.g.box(),
+             sweep32(h->st, L.g, (float)L.vol, r, nullptr, L.other(), L.m, L.P32, post ? 1 : 0, true, L.P16,
+                     h->d_pscale + (&L - h->lv.data()), nullptr, nullptr, true));
+        L.cur ^= 1;
+        return STG_OK;
+    }
     int s = 0;
     for (int c = 0; c < 2; c++) {
         const int flag = post ? 1 - c : c;

@@ -987,13 +987,53 @@ __global__ void __launch_bounds__(NT, 3) k_sweep_tma(const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------- sweep by cells
+// The penalties of a cell's unknowns p, u, v, w and of its high faces from the staged FP16 planes
+// (Q: the cell's slot, Qn: the next plane's).
+template <int RW>
+__device__ __forceinline__ void cell_penalty(const uint2* Q, const uint2* Qn, float psc, float raw[7]) {
+    const uint2 po = *Q;
+    const __half* Hn = reinterpret_cast<const __half*>(Qn);
+    const __half* Hh = reinterpret_cast<const __half*>(Q);
+    const float2 pa = __half22float2(*reinterpret_cast<const __half2*>(&po.x)),
+                 pz = __half22float2(*reinterpret_cast<const __half2*>(&po.y));
+    // a fixed face's copy is infinite: its e in cell_solve is 0, and x is 0 there, so any finite
+    // penalty gives the same residual
+    raw[0] = pa.x * psc;
+    raw[1] = pa.y * psc;
+    raw[2] = pz.x * psc;
+    raw[3] = pz.y * psc;
+    raw[4] = __half2float(Hn[1]) * psc;
+    raw[5] = __half2float(Hh[4 * RW + 2]) * psc;
+    raw[6] = __half2float(Hh[4 + 3]) * psc;
+}
+
+// Block solve of a cell with the residuals res: adds the step to its faces and returns the
+// pressure's. e = 1 / diagonal of the free faces (6 vol + P), 0 on fixed ones.
+__device__ __forceinline__ float cell_solve(float vol, float v6, const float raw[7], const float res[7], float lo[3], float hi[3]) {
+    float el[3], eh[3], num = res[0], den = 2.f * raw[0];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        el[d] = __fdividef(1.f, v6 + raw[1 + d]);
+        eh[d] = __fdividef(1.f, v6 + raw[4 + d]);
+        num += vol * (res[1 + d] * el[d] - res[4 + d] * eh[d]);
+        den -= vol * vol * (el[d] + eh[d]);
+    }
+    const float dp = den != 0.f ? __fdividef(num, den) : 0.f, vdp = vol * dp;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        lo[d] += (res[1 + d] + vdp) * el[d];
+        hi[d] += (res[4 + d] - vdp) * eh[d];
+    }
+    return dp;
+}
+
 // The solver's own Laplacian-form sweep (FP16 penalty copy), one thread per red cell: the
 // cell's pressure and six faces are exactly the unknowns its block solve changes, and every
 // face belongs to one red cell, so a thread forms the seven residuals, solves and updates
 // without exchanging residuals or pressure updates with other threads, without a halo of
 // redundant residuals, and without the black pressures' rows, which nothing uses.
 //
-// A block covers TK (k) x TJ (j) slots, TK TJ = 512, and marches along i; a thread owns the
+// A block covers TK (k) x TJ (j) slots, TK TJ = 256, and marches along i; a thread owns the
 // slot pair (k0 + 2 kk, k0 + 2 kk + 1) of its row, one red and one black slot in every plane.
 // Planes of x (one slot more on the low and two on the high side), r and P are staged by one
 // TMA box load each, a plane ahead of their use (x ring of five planes, r and P of three).
@@ -1009,54 +1049,77 @@ __global__ void __launch_bounds__(NT, 3) k_sweep_tma(const __grid_constant__ CUt
 //
 // MODE 0: x = 0 (the first sweep: the residual is r); 1: x from memory; 2: x + the parent
 // coarse value (the injection: a fine fixed unknown's parent is fixed, so its value is 0),
-// added to every plane of x once it has landed.
+// added to every plane of x once it has landed; 3 (PAIR): the first two sweeps, colour flag from
+// x = 0 and then the other, in one launch. All that a cell of the second colour needs of x are
+// its six neighbours, cells of the first. So r and P are staged with one cell more on every
+// side, half of the warps form the first colour's cells two planes ahead (p and low faces, high
+// faces: sixteen bytes each, twelve loads instead of nineteen for the six neighbours), and the
+// others run the second colour from there: r and P are read once, and the first sweep's x is
+// neither written nor read.
 //
-// Bound: HBM at 256^3 (MODE 1 moves 0.98 GB in 185 us, 5.3 TB/s or 0.78 of the measured copy;
-// the form with one thread a slot, residuals exchanged through shared memory and 17 instead of
-// 5.7 warp instructions a slot took 290 us; MODE 0 131 us, MODE 2 204 us), shared-memory loads
-// next (19 of x a cell, 70 % of the L1 rate). Staging x by component instead, with 4-byte
-// asynchronous copies (255 us) or through registers (270 us), was slower: the transposing
-// stores and the scattered loads of r and P then bound it.
-template <int TK>
+// Bound: the chain of a plane (land, work, barrier), which four blocks an SM overlap, three of
+// PAIR; at 256^3 HBM too (MODE 1 moves 0.98 GB in 180 us, 5.4 TB/s or 0.80 of the measured
+// copy; MODE 2 197 us). The form with one thread a slot, residuals exchanged through shared
+// memory and 17 instead of 5.7 warp instructions a slot took 290 us; tiles of 512 slots with
+// half as many blocks 186 and 204 us. PAIR takes 216 us at 256^3, 33 at 128^3, 9.6 at 64^3 and
+// 5.2 at 32^3 against 316, 44, 13.9 and 8.8 of MODE 0 and MODE 1 one after the other; with
+// 256-cell tiles in slot order and two blocks an SM it took 250 us, with loads three planes ahead
+// 240, with two warps more for the cells around the tile 239.
+// Staging x by component instead, with 4-byte asynchronous copies (255 us for MODE 1) or through
+// registers (270 us), was slower: the transposing stores and the scattered loads of r and P
+// then bound it.
+template <int TK, bool PAIR = false>
 struct CellTile {
-    static constexpr int TJ = 512 / TK, LR = TK / 2;       // rows, pairs of a row
+    static constexpr int NT = 128;            // threads with a pair of slots
+    static constexpr int TJ = 2 * NT / TK, LR = TK / 2;    // rows, pairs of a row
     static constexpr int PW = LR < 16 ? LR : 16;           // pairs of a row in one warp
     static constexpr int XW = TK + 4, XR = TJ + 3;         // staged x: k0 - 2 .. k0 + TK + 1, j0 - 1 .. j0 + TJ + 1
-    static constexpr int RW = TK + 2, RR = TJ + 1;         // staged r and P: k0 .. (P: k0 - 1 ..), j0 .. j0 + TJ
+    static constexpr int O = PAIR ? 1 : 0;                 // PAIR: r and P of one cell more on every side
+    static constexpr int RW = TK + 2 + 2 * O, RR = TJ + 1 + 2 * O;  // staged r and P: k0 - O .. (P: k0 - 1 ..), j0 - O .. j0 + TJ + O
     static constexpr int XPL = (XW * XR + 7) / 8 * 8;      // ring slots, 128-byte multiples (in slots)
     static constexpr int RPL = (RW * RR + 7) / 8 * 8, PPL = (RW * RR + 15) / 16 * 16;
     static constexpr unsigned XB = XW * XR * 16, RB = RW * RR * 16, PB = RW * RR * 8;  // box bytes
     static constexpr int NX = (XW * XR + NT - 1) / NT;     // staged x slots of a thread (MODE 2)
-    static constexpr int XRING = 5, RRING = 3;
+    static constexpr int XRING = 5, RRING = PAIR ? 5 : 3;
+    // PAIR: first-colour cells by row and pair, low and high halves; a row is four slots off a
+    // multiple of 128 bytes, as the two rows of a warp have to be
+    static constexpr int FW = LR + 4, FPL = FW * (TJ + 2), FRING = 4;
     static constexpr int VN = 2 * (TJ + 1) * LR, WN = (2 * TJ * (LR + 1) + 1) / 2 * 2;  // sv, sw (floats)
-    static constexpr int smem(bool x) { return (x ? XRING * XPL * 16 : 0) + RRING * (RPL * 16 + PPL * 8) + 4 * (VN + WN) + 8; }
+    static constexpr int HALO = 2 * LR + TJ;               // PAIR: first-colour cells around the tile
+    static constexpr int THREADS = PAIR ? 2 * NT : NT;
+    static constexpr int smem(bool x) { return (PAIR ? FRING * FPL * 32 : x ? XRING * XPL * 16 : 0) + RRING * (RPL * 16 + PPL * 8) + 4 * (VN + WN) + 8; }
     static_assert((RRING * PPL * 8 + 4 * VN) % 8 == 0, "the mbarrier lies on an 8-byte boundary");
+    static_assert(!PAIR || (FW % 8 == 4 && FPL % 4 == 0), "the staged planes start on 128 bytes");
 };
 
 template <int TK, int MODE>
-__global__ void __launch_bounds__(NT, 2) k_sweep_cell(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmr,
-                                                      const __grid_constant__ CUtensorMap tmp, Geom g, float vol,
-                                                      float4* __restrict__ xout, const float* __restrict__ pscale, int flag,
-                                                      int chunk, int* __restrict__ err, const float4* __restrict__ xc, int c_plane,
-                                                      int c_sz) {
-    using C = CellTile<TK>;
-    constexpr int TJ = C::TJ, XW = C::XW, RW = C::RW;
+__global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 3 : 4) k_sweep_cell(
+    const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmr,
+    const __grid_constant__ CUtensorMap tmp, Geom g, float vol,
+    float4* __restrict__ xout, const float* __restrict__ pscale, int flag,
+    int chunk, int* __restrict__ err, const float4* __restrict__ xc, int c_plane,
+    int c_sz) {
+    constexpr bool PAIR = MODE == 3, STAGE_X = MODE == 1 || MODE == 2;
+    using C = CellTile<TK, PAIR>;
+    constexpr int NT = C::NT, TJ = C::TJ, XW = C::XW, RW = C::RW, FW = C::FW;
     // (no static shared memory: the TMA destinations start at the window's aligned origin)
     extern __shared__ __align__(1024) unsigned char cell_smem[];
     float4* sx = reinterpret_cast<float4*>(cell_smem);
-    float4* sr = sx + (MODE ? C::XRING * C::XPL : 0);
+    float4* sr = sx + (PAIR ? 2 * C::FRING * C::FPL : MODE ? C::XRING * C::XPL : 0);
     uint2* sp = reinterpret_cast<uint2*>(sr + C::RRING * C::RPL);
     float (*sv)[TJ + 1][C::LR] = reinterpret_cast<float (*)[TJ + 1][C::LR]>(sp + C::RRING * C::PPL);  // [2]
     float (*sw)[TJ][C::LR + 1] = reinterpret_cast<float (*)[TJ][C::LR + 1]>(reinterpret_cast<float*>(sv) + C::VN);  // [2]
     unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(reinterpret_cast<float*>(sw) + C::WN);
-    const int n = g.n, tid = threadIdx.x, lane = tid & 31, pr = lane >> 1;
+    const int n = g.n, tid = threadIdx.x, ct = tid & (NT - 1), lane = tid & 31, pr = lane >> 1;
     constexpr int WR = 32 / C::PW, WK = C::LR / C::PW;  // rows of a warp, warps side by side in k
-    const int wid = tid >> 5;
+    const int wid = ct >> 5;
     const int tj = (wid / WK) * WR + 2 * (pr / C::PW) + (lane & 1), kk = (wid % WK) * C::PW + pr % C::PW;
     const int k0 = blockIdx.x * TK, j0 = blockIdx.y * TJ, i0 = blockIdx.z * chunk;
     const int i1 = min(i0 + chunk, n);
     const int j = j0 + tj, kp0 = k0 + 2 * kk;
-    const bool live = j < n && kp0 < n;
+    const bool first = PAIR && tid >= NT;  // forms the first colour's cells
+    const bool live = j < n && kp0 < n && !first;
+    const int colour = PAIR ? flag ^ 1 : flag;  // written by the others
     const int plane = g.sy * g.sz;
     const float psc = __ldg(pscale), v6 = 6.f * vol;
 
@@ -1068,9 +1131,9 @@ __global__ void __launch_bounds__(NT, 2) k_sweep_cell(const __grid_constant__ CU
     auto xslot = [&](int p) { return ((p + C::XRING) % C::XRING) * C::XPL; };
     auto load_x = [&](int p) { tma3(bx + 16u * xslot(p), &tmx, 2 * (k0 - 1), j0, p + 1, bar); };
     auto load_rp = [&](int p) {
-        const int s = p % C::RRING;
-        tma3(br + 16u * (s * C::RPL), &tmr, 2 * (k0 + 1), j0 + 1, p + 1, bar);
-        tma3(bp_ + 8u * (s * C::PPL), &tmp, k0, j0 + 1, p + 1, bar);
+        const int s = (p + C::RRING) % C::RRING;
+        tma3(br + 16u * (s * C::RPL), &tmr, 2 * (k0 + 1 - C::O), j0 + 1 - C::O, p + 1, bar);
+        tma3(bp_ + 8u * (s * C::PPL), &tmp, k0, j0 + 1 - C::O, p + 1, bar);
     };
     unsigned phase = 0;
     auto wait_loads = [&]() {
@@ -1118,11 +1181,10 @@ __global__ void __launch_bounds__(NT, 2) k_sweep_cell(const __grid_constant__ CU
     }
     __syncthreads();
     if (tid == 0) {
-        arm_tx(bar, (MODE ? 4 * C::XB : 0) + 2 * (C::RB + C::PB));
-        if (MODE)
+        arm_tx(bar, (STAGE_X ? 4 * C::XB : 0) + (PAIR ? 5 : 2) * (C::RB + C::PB));
+        if (STAGE_X)
             for (int p = i0 - 1; p <= i0 + 2; p++) load_x(p);
-        load_rp(i0);
-        load_rp(i0 + 1);
+        for (int p = PAIR ? i0 - 1 : i0; p <= (PAIR ? i0 + 3 : i0 + 1); p++) load_rp(p);
     }
     if (MODE == 2) fetch_coarse(i0 - 1);
     if (__syncthreads_or(!wait_loads())) return fail(err);
@@ -1134,11 +1196,54 @@ __global__ void __launch_bounds__(NT, 2) k_sweep_cell(const __grid_constant__ CU
         __syncthreads();
     }
 
+    // PAIR: the first colour's cells of plane p in the tile and around it, from x = 0 (0 outside
+    // the domain): pressure and low faces, high faces; pair -1 and LR are the cells beside a row
+    auto fcell = [&](int p) { return sx + 2 * (p & (C::FRING - 1)) * C::FPL; };
+    auto first_cell = [&](int p, int row, int c) {
+        const int jj = j0 + row, k = k0 + c;
+        float dp = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+        if (p >= 0 && p < n && jj >= 0 && jj < n && k >= 0 && k < n) {
+            const int sl = (p + C::RRING) % C::RRING, sn = sl + 1 < C::RRING ? sl + 1 : 0, ro = (row + 1) * RW + c + 1;
+            const float4* R = sr + sl * C::RPL + ro;
+            float raw[7];
+            cell_penalty<RW>(sp + sl * C::PPL + ro, sp + sn * C::PPL + ro, psc, raw);
+            const float4 r0 = *R;
+            const float res[7] = {r0.x, r0.y, r0.z, r0.w, sr[sn * C::RPL + ro].y, R[RW].z, R[1].w};
+            dp = cell_solve(vol, v6, raw, res, lo, hi);
+        }
+        float4* F = fcell(p) + (row + 1) * FW + ((c + 2) >> 1);
+        F[0] = make_float4(dp, lo[0], lo[1], lo[2]);
+        F[C::FPL] = make_float4(hi[0], hi[1], hi[2], 0.f);
+    };
+    auto first_tile = [&](int p) { first_cell(p, tj, 2 * kk + ((p + j + flag) & 1)); };
+    auto first_halo = [&](int p) {
+        if (ct < 2 * C::LR) {  // the rows below and above
+            const int row = ct < C::LR ? -1 : TJ;
+            first_cell(p, row, 2 * (ct % C::LR) + ((p + j0 + row + flag) & 1));
+        } else if (ct < C::HALO) {  // one cell of each row, left or right of it
+            const int row = ct - 2 * C::LR;
+            first_cell(p, row, (p + j0 + row + flag) & 1 ? -1 : TK);
+        }
+    };
+    auto first_plane = [&](int p) {
+        first_tile(p);
+        first_halo(p);
+    };
+    if (PAIR) {
+        if (first) {
+            first_plane(i0);
+            first_plane(i0 + 1);
+        } else {
+            first_tile(i0 - 1);  // (nothing needs the cells around it)
+        }
+        __syncthreads();
+    }
+
     float ukeep = 0.f;               // u of this plane's black slot: the last plane's cell's high face
     float bp = 0.f, bu = 0.f;        // p and u of the last plane's black slot
     const bool own_v = tj > 0 || j0 == 0;  // the black slots' v is this block's
     auto write_black = [&](int i) {  // black slot of plane i
-        const int q = (i + j + flag) & 1;
+        const int q = (i + j + colour) & 1;
         const int s = g.slot(i, j, kp0 + 1 - q);
         const bool own_u = i > i0 || i0 == 0, own_w = q == 0 || kk > 0 || k0 == 0;
         const float bv = tj > 0 ? sv[i & 1][tj][kk] : 0.f;
@@ -1157,82 +1262,95 @@ __global__ void __launch_bounds__(NT, 2) k_sweep_cell(const __grid_constant__ CU
     int base = xslot(i0), rs = i0 % C::RRING;  // ring slots of plane i
     for (int i = i0; i < i1; i++) {
         const bool more = i + 1 < i1;
-        // x(i + 3) into the slot of x(i - 2), r and P of i + 2 into those of i - 1
+        // x(i + 3) into the slot of x(i - 2), r and P of i + 2 (PAIR: i + 4) into those of i - 1
         if (more && tid == 0) {
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            arm_tx(bar, (MODE ? C::XB : 0) + C::RB + C::PB);
-            if (MODE) load_x(i + 3);
-            load_rp(i + 2);
+            arm_tx(bar, (STAGE_X ? C::XB : 0) + C::RB + C::PB);
+            if (STAGE_X) load_x(i + 3);
+            load_rp(PAIR ? i + 4 : i + 2);
         }
         if (MODE == 2 && more && ((i + 3) & 1) == 0) fetch_coarse(i + 3);  // an odd plane's parents are the last plane's
         if (i > i0 && live) write_black(i - 1);
         const int rn = rs + 1 < C::RRING ? rs + 1 : 0;  // ring slot of r and P of plane i + 1
+        if (PAIR && first && more) first_plane(i + 2);
         if (live) {
-            const int q = (i + j + flag) & 1;  // red: (i + j + k + flag) even, k0 even
-            const int ro = tj * RW + 2 * kk + q;
+            const int q = (i + j + colour) & 1;  // red: (i + j + k + colour) even, k0 even
+            const int ro = (tj + C::O) * RW + 2 * kk + q + C::O;
             const float4* R = sr + rs * C::RPL + ro;
-            const uint2* Q = sp + rs * C::PPL + ro + 1;
-            const uint2 po = *Q;
-            const __half* Qn = reinterpret_cast<const __half*>(sp + rn * C::PPL + ro + 1);
-            const __half* Qh = reinterpret_cast<const __half*>(Q);
-            const float2 pa = __half22float2(*reinterpret_cast<const __half2*>(&po.x)),
-                         pz = __half22float2(*reinterpret_cast<const __half2*>(&po.y));
-            // a fixed face's copy is infinite: its e below is 0, and x is 0 there, so any finite
-            // penalty gives the same residual
-            const float raw[7] = {pa.x * psc, pa.y * psc, pz.x * psc, pz.y * psc,
-                                  __half2float(Qn[1]) * psc, __half2float(Qh[4 * RW + 2]) * psc, __half2float(Qh[4 + 3]) * psc};
+            float raw[7];
+            cell_penalty<RW>(sp + rs * C::PPL + ro + 1 - C::O, sp + rn * C::PPL + ro + 1 - C::O, psc, raw);
             const float4 r0 = *R;
             float res[7] = {r0.x, r0.y, r0.z, r0.w, sr[rn * C::RPL + ro].y, R[RW].z, R[1].w};
             float p0 = 0.f, pb = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
             if (MODE) {
-                constexpr int XP = C::XPL, XL = (C::XRING - 1) * XP;
-                const float4* B = sx + base + (tj + 1) * XW + 2 * kk + q + 2;
-                const float4* A = B + (base >= XP ? -XP : XL);                             // plane i - 1
-                const float4* D = B + (base < XL ? XP : -XL);                              // plane i + 1
-                const float4* E = B + (base < XL - XP ? 2 * XP : -(C::XRING - 2) * XP);    // plane i + 2
-                // the rows of stencil.cuh lap_core, low face at the cell's slot, high face one on
-                const float4 c = B[0], xm = A[0], xp = D[0], ym = B[-XW], yp = B[XW], zm = B[-1], zp = B[1];
-                const float4 xy = D[XW], xz = D[1], yz = B[XW + 1];
-                p0 = c.x;
-                pb = q ? zm.x : zp.x;
-                lo[0] = c.y;
-                lo[1] = c.z;
-                lo[2] = c.w;
-                hi[0] = xp.y;
-                hi[1] = yp.z;
-                hi[2] = zp.w;
-                const float lu = 6.f * c.y - (xm.y + xp.y) - (ym.y + yp.y) - (zm.y + zp.y);
-                const float hu = 6.f * xp.y - (c.y + E[0].y) - (D[-XW].y + xy.y) - (D[-1].y + xz.y);
-                const float lv = 6.f * c.z - (xm.z + xp.z) - (ym.z + yp.z) - (zm.z + zp.z);
-                const float hv = 6.f * yp.z - (A[XW].z + xy.z) - (c.z + B[2 * XW].z) - (B[XW - 1].z + yz.z);
-                const float lw = 6.f * c.w - (xm.w + xp.w) - (ym.w + yp.w) - (zm.w + zp.w);
-                const float hw = 6.f * zp.w - (A[1].w + xz.w) - (B[1 - XW].w + yz.w) - (c.w + B[2].w);
+                float lu, hu, lv, hv, lw, hw, pw, pe, ps, pn, pd, pu;  // pressures west (i - 1) .. up (k + 1)
+                if constexpr (PAIR) {
+                    // x = 0 but for what the first colour wrote: the six neighbours
+                    const float4* F = fcell(i) + (tj + 1) * FW + kk + 1;
+                    const float4 *W = fcell(i - 1) + (tj + 1) * FW + kk + 1, *E = fcell(i + 1) + (tj + 1) * FW + kk + 1;
+                    const float4 wl = W[0], wh = W[C::FPL], el = E[0], eh = E[C::FPL], sl = F[-FW], sh = F[C::FPL - FW], nl = F[FW],
+                                 nh = F[C::FPL + FW], dl = F[q - 1], dh = F[C::FPL + q - 1], ul = F[q], uh = F[C::FPL + q];
+                    pw = wl.x;
+                    pe = el.x;
+                    ps = sl.x;
+                    pn = nl.x;
+                    pd = dl.x;
+                    pu = ul.x;
+                    pb = q ? pd : pu;
+                    lo[0] = wh.x;
+                    lo[1] = sh.y;
+                    lo[2] = dh.z;
+                    hi[0] = el.y;
+                    hi[1] = nl.z;
+                    hi[2] = ul.w;
+                    lu = 6.f * wh.x - (wl.y + el.y) - (sl.y + nl.y) - (dl.y + ul.y);
+                    hu = 6.f * el.y - (wh.x + eh.x) - (sh.x + nh.x) - (dh.x + uh.x);
+                    lv = 6.f * sh.y - (wl.z + el.z) - (sl.z + nl.z) - (dl.z + ul.z);
+                    hv = 6.f * nl.z - (wh.y + eh.y) - (sh.y + nh.y) - (dh.y + uh.y);
+                    lw = 6.f * dh.z - (wl.w + el.w) - (sl.w + nl.w) - (dl.w + ul.w);
+                    hw = 6.f * ul.w - (wh.z + eh.z) - (sh.z + nh.z) - (dh.z + uh.z);
+                } else {
+                    constexpr int XP = C::XPL, XL = (C::XRING - 1) * XP;
+                    const float4* B = sx + base + (tj + 1) * XW + 2 * kk + q + 2;
+                    const float4* A = B + (base >= XP ? -XP : XL);                             // plane i - 1
+                    const float4* D = B + (base < XL ? XP : -XL);                              // plane i + 1
+                    const float4* E = B + (base < XL - XP ? 2 * XP : -(C::XRING - 2) * XP);    // plane i + 2
+                    // the rows of stencil.cuh lap_core, low face at the cell's slot, high face one on
+                    const float4 c = B[0], xm = A[0], xp = D[0], ym = B[-XW], yp = B[XW], zm = B[-1], zp = B[1];
+                    const float4 xy = D[XW], xz = D[1], yz = B[XW + 1];
+                    p0 = c.x;
+                    pb = q ? zm.x : zp.x;
+                    lo[0] = c.y;
+                    lo[1] = c.z;
+                    lo[2] = c.w;
+                    hi[0] = xp.y;
+                    hi[1] = yp.z;
+                    hi[2] = zp.w;
+                    lu = 6.f * c.y - (xm.y + xp.y) - (ym.y + yp.y) - (zm.y + zp.y);
+                    hu = 6.f * xp.y - (c.y + E[0].y) - (D[-XW].y + xy.y) - (D[-1].y + xz.y);
+                    lv = 6.f * c.z - (xm.z + xp.z) - (ym.z + yp.z) - (zm.z + zp.z);
+                    hv = 6.f * yp.z - (A[XW].z + xy.z) - (c.z + B[2 * XW].z) - (B[XW - 1].z + yz.z);
+                    lw = 6.f * c.w - (xm.w + xp.w) - (ym.w + yp.w) - (zm.w + zp.w);
+                    hw = 6.f * zp.w - (A[1].w + xz.w) - (B[1 - XW].w + yz.w) - (c.w + B[2].w);
+                    pw = xm.x;
+                    pe = xp.x;
+                    ps = ym.x;
+                    pn = yp.x;
+                    pd = zm.x;
+                    pu = zp.x;
+                }
                 float pen[7];
 #pragma unroll
                 for (int d = 0; d < 7; d++) pen[d] = fminf(raw[d], 1e38f);
                 res[0] -= vol * ((hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2])) + pen[0] * p0;
-                res[1] -= vol * (lu - (p0 - xm.x)) + pen[1] * lo[0];
-                res[2] -= vol * (lv - (p0 - ym.x)) + pen[2] * lo[1];
-                res[3] -= vol * (lw - (p0 - zm.x)) + pen[3] * lo[2];
-                res[4] -= vol * (hu - (xp.x - p0)) + pen[4] * hi[0];
-                res[5] -= vol * (hv - (yp.x - p0)) + pen[5] * hi[1];
-                res[6] -= vol * (hw - (zp.x - p0)) + pen[6] * hi[2];
+                res[1] -= vol * (lu - (p0 - pw)) + pen[1] * lo[0];
+                res[2] -= vol * (lv - (p0 - ps)) + pen[2] * lo[1];
+                res[3] -= vol * (lw - (p0 - pd)) + pen[3] * lo[2];
+                res[4] -= vol * (hu - (pe - p0)) + pen[4] * hi[0];
+                res[5] -= vol * (hv - (pn - p0)) + pen[5] * hi[1];
+                res[6] -= vol * (hw - (pu - p0)) + pen[6] * hi[2];
             }
-            // block solve: e = 1 / diagonal of the free faces (6 vol + P), 0 on fixed ones
-            float el[3], eh[3], num = res[0], den = 2.f * raw[0];
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                el[d] = __fdividef(1.f, v6 + raw[1 + d]);
-                eh[d] = __fdividef(1.f, v6 + raw[4 + d]);
-                num += vol * (res[1 + d] * el[d] - res[4 + d] * eh[d]);
-                den -= vol * vol * (el[d] + eh[d]);
-            }
-            const float dp = den != 0.f ? __fdividef(num, den) : 0.f, vdp = vol * dp;
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                lo[d] += (res[1 + d] + vdp) * el[d];
-                hi[d] += (res[4 + d] - vdp) * eh[d];
-            }
+            const float dp = cell_solve(vol, v6, raw, res, lo, hi);
             const int k = kp0 + q;
             const int s = g.slot(i, j, k);
             xout[s] = make_float4(p0 + dp, lo[0], lo[1], lo[2]);
@@ -1310,10 +1428,9 @@ int g_sms[MAX_DEVICES] = {};
 // plane after plane (its prologue costs about four), and the blocks run in waves of SMs x
 // resident blocks, so the chunk minimises waves x (chunk + 4), the longest chain of planes an
 // SM works through (n = 256: 37 planes in three waves, n = 128: 15 in one, n = 64: 2 in one).
-int cell_chunk(int dev, int n, int tk, int resident) {
+int cell_chunk(int dev, int n, int tk, int tj, int resident) {
     if (!g_sms[dev] && cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sms[dev] = 0;
     const long long slots = (long long)resident * (g_sms[dev] > 0 ? g_sms[dev] : 152);
-    const int tj = 512 / tk;
     const long long plane_blocks = (long long)((n + tk - 1) / tk) * ((n + tj - 1) / tj);
     int best = 1;
     long long best_cost = -1;
@@ -1340,28 +1457,33 @@ bool cell_map(EncodeTiled enc, CUtensorMap* map, const void* base, const Geom& g
 
 template <int TK>
 int launch_cell(cudaStream_t st, int dev, EncodeTiled enc, const Geom& g, float vol, const float4* r, const float4* xin, float4* xout,
-                const __half* P16, const float* psc, int flag, const float4* xc, const Geom* gc, bool* done) {
+                const __half* P16, const float* psc, int flag, const float4* xc, const Geom* gc, bool pair, bool* done) {
     using C = CellTile<TK>;
+    using CP = CellTile<TK, true>;
     static bool set[MAX_DEVICES] = {};
     if (!set[dev]) {
         STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(false)));
         STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(true)));
         STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(true)));
+        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, CP::smem(true)));
         set[dev] = true;
     }
     CUtensorMap mx{}, mr{}, mp{};
-    *done = cell_map(enc, &mr, r, g, 2, C::RW, C::RR) && cell_map(enc, &mp, P16, g, 1, C::RW, C::RR) &&
+    const int rw = pair ? CP::RW : C::RW, rr = pair ? CP::RR : C::RR;
+    *done = cell_map(enc, &mr, r, g, 2, rw, rr) && cell_map(enc, &mp, P16, g, 1, rw, rr) &&
             (!xin || cell_map(enc, &mx, xin, g, 2, C::XW, C::XR));
     if (!*done) return STG_OK;
-    const int chunk = cell_chunk(dev, g.n, TK, xin ? 2 : 4);
-    const dim3 grid((g.n + TK - 1) / TK, (g.n + C::TJ - 1) / C::TJ, (g.n + chunk - 1) / chunk);
+    const int tj = pair ? CP::TJ : C::TJ, chunk = cell_chunk(dev, g.n, TK, tj, pair ? 3 : xin ? 4 : 8);
+    const dim3 grid((g.n + TK - 1) / TK, (g.n + tj - 1) / tj, (g.n + chunk - 1) / chunk);
     int* err = g_sweep_err[dev];
-    if (!xin)
-        k_sweep_cell<TK, 0><<<grid, NT, C::smem(false), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+    if (pair)
+        k_sweep_cell<TK, 3><<<grid, CP::THREADS, CP::smem(true), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+    else if (!xin)
+        k_sweep_cell<TK, 0><<<grid, C::NT, C::smem(false), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
     else if (!xc)
-        k_sweep_cell<TK, 1><<<grid, NT, C::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+        k_sweep_cell<TK, 1><<<grid, C::NT, C::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
     else
-        k_sweep_cell<TK, 2><<<grid, NT, C::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, xc, gc->sy * gc->sz, gc->sz);
+        k_sweep_cell<TK, 2><<<grid, C::NT, C::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, xc, gc->sy * gc->sz, gc->sz);
     STG_LAUNCH_CK();
     return STG_OK;
 }
@@ -1388,7 +1510,7 @@ int sweep_status(cudaStream_t st, int* timed_out) {
 }
 
 int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const float4* xin, float4* xout, const uint8_t* m,
-            const float4* P, int flag, bool lap, const __half* P16, const float* p16_scale, const float4* xc, const Geom* gc) {
+            const float4* P, int flag, bool lap, const __half* P16, const float* p16_scale, const float4* xc, const Geom* gc, bool pair) {
     const int dev = device_slot();
     if (dev < 0) {
         set_error("sweep32: device ordinal beyond %d", MAX_DEVICES - 1);
@@ -1403,15 +1525,15 @@ int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const fl
         g_attr_set[dev] = true;
     }
     if (lap && P16 && p16_scale && encoder()) {
-        // the solver's own sweeps; narrower tiles (with more rows) where a row has fewer slots
+        // the solver's own sweeps; a narrower tile (with more rows) where a row has fewer slots
         STG_TRY(sweep_err_init(dev));
         bool done = false;
-        const auto go = g.n > 32 ? launch_cell<64> : g.n > 16 ? launch_cell<32> : launch_cell<16>;
-        STG_TRY(go(st, dev, encoder(), g, vol, r, xin, xout, P16, p16_scale, flag, xc, gc, &done));
+        const auto go = g.n > 16 ? launch_cell<32> : launch_cell<16>;
+        STG_TRY(go(st, dev, encoder(), g, vol, r, xin, xout, P16, p16_scale, flag, xc, gc, pair, &done));
         if (done) return STG_OK;
     }
-    if (xc) {
-        set_error("sweep32: the fused prolongation needs the TMA sweep by cells");
+    if (xc || pair) {
+        set_error("sweep32: the fused prolongation and the pair of sweeps need the TMA sweep by cells");
         return STG_E_UNSUPPORTED;
     }
     // planes per block: long marches on big grids (prologue amortised), short ones on the

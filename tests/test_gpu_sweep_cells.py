@@ -1,6 +1,7 @@
 """The solver's sweep by cells (sweep.cu k_sweep_cell) at the sizes where its tiles end: part
-tiles in k and j (24 of 32, 48 and 96 of 64 slots; levels 12 to 96), whole ones of every
-width, chunks of one plane, both sweep counts, and fixed faces inside the domain. A sweep that
+tiles in k and j (12 of 16, 24 and 48 of 32 slots; levels 12 to 96), whole ones of both
+widths, chunks of one plane, one sweep a colour (the first two in one launch) and two, and
+fixed faces inside the domain. A sweep that
 loses an unknown at an edge, or moves a fixed one, leaves a V-cycle that no longer
 converges at the smooth densities' rate: the solve must reach its FP64 tolerance within 30
 V-cycles (18 to 20 are usual), with the residual confirmed by the FP64 operator and
