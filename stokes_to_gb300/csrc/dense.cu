@@ -604,6 +604,7 @@ int dense_init(DenseCoarse& D, const Geom& g) {
     STG_CK(cudaMalloc(&D.dense_of, sizeof(int) * dense_of.size()));
     STG_CK(cudaMalloc(&D.A, sizeof(double) * 2 * nd * nd));
     STG_CK(cudaMalloc(&D.Ainv, sizeof(double) * 2 * nd * nd));
+    if (n == 4) STG_CK(cudaMalloc(&D.inv2, sizeof(float2) * nd * nd));
     STG_CK(cudaMalloc(&D.piv, sizeof(int) * nd));
     STG_CK(cudaMalloc(&D.info, sizeof(int)));
     STG_CK(cudaMalloc(&D.probe, sizeof(d4) * g.nslot));
@@ -627,6 +628,7 @@ void dense_free(DenseCoarse& D) {
     cudaFree(D.dense_of);
     cudaFree(D.A);
     cudaFree(D.Ainv);
+    cudaFree(D.inv2);
     cudaFree(D.piv);
     cudaFree(D.info);
     cudaFree(D.probe);

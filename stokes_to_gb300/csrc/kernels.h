@@ -161,6 +161,7 @@ struct DenseCoarse {
     double* A = nullptr;       // two row-major nd x 2nd buffers for Gauss-Jordan on [A | I]
     double* Ainv = nullptr;
     const double* inv = nullptr;  // the inverse: right half of the final buffer, row stride 2 nd
+    float2* inv2 = nullptr;    // its entries as sums of two floats, nd x nd (smallcycle.cu)
     int* piv = nullptr;
     int* info = nullptr;
     d4* probe = nullptr;       // probe vector and its image (slots)

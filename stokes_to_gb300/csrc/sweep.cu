@@ -28,6 +28,7 @@
 
 #include <type_traits>
 
+#include "cell.cuh"
 #include "kernels.h"
 #include "stencil.cuh"
 
@@ -987,46 +988,6 @@ __global__ void __launch_bounds__(NT, 3) k_sweep_tma(const __grid_constant__ CUt
 }
 
 // ---------------------------------------------------------------- sweep by cells
-// The penalties of a cell's unknowns p, u, v, w and of its high faces from the staged FP16 planes
-// (Q: the cell's slot, Qn: the next plane's).
-template <int RW>
-__device__ __forceinline__ void cell_penalty(const uint2* Q, const uint2* Qn, float psc, float raw[7]) {
-    const uint2 po = *Q;
-    const __half* Hn = reinterpret_cast<const __half*>(Qn);
-    const __half* Hh = reinterpret_cast<const __half*>(Q);
-    const float2 pa = __half22float2(*reinterpret_cast<const __half2*>(&po.x)),
-                 pz = __half22float2(*reinterpret_cast<const __half2*>(&po.y));
-    // a fixed face's copy is infinite: its e in cell_solve is 0, and x is 0 there, so any finite
-    // penalty gives the same residual
-    raw[0] = pa.x * psc;
-    raw[1] = pa.y * psc;
-    raw[2] = pz.x * psc;
-    raw[3] = pz.y * psc;
-    raw[4] = __half2float(Hn[1]) * psc;
-    raw[5] = __half2float(Hh[4 * RW + 2]) * psc;
-    raw[6] = __half2float(Hh[4 + 3]) * psc;
-}
-
-// Block solve of a cell with the residuals res: adds the step to its faces and returns the
-// pressure's. e = 1 / diagonal of the free faces (6 vol + P), 0 on fixed ones.
-__device__ __forceinline__ float cell_solve(float vol, float v6, const float raw[7], const float res[7], float lo[3], float hi[3]) {
-    float el[3], eh[3], num = res[0], den = 2.f * raw[0];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        el[d] = __fdividef(1.f, v6 + raw[1 + d]);
-        eh[d] = __fdividef(1.f, v6 + raw[4 + d]);
-        num += vol * (res[1 + d] * el[d] - res[4 + d] * eh[d]);
-        den -= vol * vol * (el[d] + eh[d]);
-    }
-    const float dp = den != 0.f ? __fdividef(num, den) : 0.f, vdp = vol * dp;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        lo[d] += (res[1 + d] + vdp) * el[d];
-        hi[d] += (res[4 + d] - vdp) * eh[d];
-    }
-    return dp;
-}
-
 // The solver's own Laplacian-form sweep (FP16 penalty copy), one thread per red cell: the
 // cell's pressure and six faces are exactly the unknowns its block solve changes, and every
 // face belongs to one red cell, so a thread forms the seven residuals, solves and updates
@@ -1282,73 +1243,17 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
             const float4 r0 = *R;
             float res[7] = {r0.x, r0.y, r0.z, r0.w, sr[rn * C::RPL + ro].y, R[RW].z, R[1].w};
             float p0 = 0.f, pb = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
-            if (MODE) {
-                float lu, hu, lv, hv, lw, hw, pw, pe, ps, pn, pd, pu;  // pressures west (i - 1) .. up (k + 1)
-                if constexpr (PAIR) {
-                    // x = 0 but for what the first colour wrote: the six neighbours
-                    const float4* F = fcell(i) + (tj + 1) * FW + kk + 1;
-                    const float4 *W = fcell(i - 1) + (tj + 1) * FW + kk + 1, *E = fcell(i + 1) + (tj + 1) * FW + kk + 1;
-                    const float4 wl = W[0], wh = W[C::FPL], el = E[0], eh = E[C::FPL], sl = F[-FW], sh = F[C::FPL - FW], nl = F[FW],
-                                 nh = F[C::FPL + FW], dl = F[q - 1], dh = F[C::FPL + q - 1], ul = F[q], uh = F[C::FPL + q];
-                    pw = wl.x;
-                    pe = el.x;
-                    ps = sl.x;
-                    pn = nl.x;
-                    pd = dl.x;
-                    pu = ul.x;
-                    pb = q ? pd : pu;
-                    lo[0] = wh.x;
-                    lo[1] = sh.y;
-                    lo[2] = dh.z;
-                    hi[0] = el.y;
-                    hi[1] = nl.z;
-                    hi[2] = ul.w;
-                    lu = 6.f * wh.x - (wl.y + el.y) - (sl.y + nl.y) - (dl.y + ul.y);
-                    hu = 6.f * el.y - (wh.x + eh.x) - (sh.x + nh.x) - (dh.x + uh.x);
-                    lv = 6.f * sh.y - (wl.z + el.z) - (sl.z + nl.z) - (dl.z + ul.z);
-                    hv = 6.f * nl.z - (wh.y + eh.y) - (sh.y + nh.y) - (dh.y + uh.y);
-                    lw = 6.f * dh.z - (wl.w + el.w) - (sl.w + nl.w) - (dl.w + ul.w);
-                    hw = 6.f * ul.w - (wh.z + eh.z) - (sh.z + nh.z) - (dh.z + uh.z);
-                } else {
-                    constexpr int XP = C::XPL, XL = (C::XRING - 1) * XP;
-                    const float4* B = sx + base + (tj + 1) * XW + 2 * kk + q + 2;
-                    const float4* A = B + (base >= XP ? -XP : XL);                             // plane i - 1
-                    const float4* D = B + (base < XL ? XP : -XL);                              // plane i + 1
-                    const float4* E = B + (base < XL - XP ? 2 * XP : -(C::XRING - 2) * XP);    // plane i + 2
-                    // the rows of stencil.cuh lap_core, low face at the cell's slot, high face one on
-                    const float4 c = B[0], xm = A[0], xp = D[0], ym = B[-XW], yp = B[XW], zm = B[-1], zp = B[1];
-                    const float4 xy = D[XW], xz = D[1], yz = B[XW + 1];
-                    p0 = c.x;
-                    pb = q ? zm.x : zp.x;
-                    lo[0] = c.y;
-                    lo[1] = c.z;
-                    lo[2] = c.w;
-                    hi[0] = xp.y;
-                    hi[1] = yp.z;
-                    hi[2] = zp.w;
-                    lu = 6.f * c.y - (xm.y + xp.y) - (ym.y + yp.y) - (zm.y + zp.y);
-                    hu = 6.f * xp.y - (c.y + E[0].y) - (D[-XW].y + xy.y) - (D[-1].y + xz.y);
-                    lv = 6.f * c.z - (xm.z + xp.z) - (ym.z + yp.z) - (zm.z + zp.z);
-                    hv = 6.f * yp.z - (A[XW].z + xy.z) - (c.z + B[2 * XW].z) - (B[XW - 1].z + yz.z);
-                    lw = 6.f * c.w - (xm.w + xp.w) - (ym.w + yp.w) - (zm.w + zp.w);
-                    hw = 6.f * zp.w - (A[1].w + xz.w) - (B[1 - XW].w + yz.w) - (c.w + B[2].w);
-                    pw = xm.x;
-                    pe = xp.x;
-                    ps = ym.x;
-                    pn = yp.x;
-                    pd = zm.x;
-                    pu = zp.x;
-                }
-                float pen[7];
-#pragma unroll
-                for (int d = 0; d < 7; d++) pen[d] = fminf(raw[d], 1e38f);
-                res[0] -= vol * ((hi[0] - lo[0]) + (hi[1] - lo[1]) + (hi[2] - lo[2])) + pen[0] * p0;
-                res[1] -= vol * (lu - (p0 - pw)) + pen[1] * lo[0];
-                res[2] -= vol * (lv - (p0 - ps)) + pen[2] * lo[1];
-                res[3] -= vol * (lw - (p0 - pd)) + pen[3] * lo[2];
-                res[4] -= vol * (hu - (pe - p0)) + pen[4] * hi[0];
-                res[5] -= vol * (hv - (pn - p0)) + pen[5] * hi[1];
-                res[6] -= vol * (hw - (pu - p0)) + pen[6] * hi[2];
+            if (PAIR) {
+                const int o = (tj + 1) * FW + kk + 1;
+                neighbour_residual<FW, C::FPL>(fcell(i - 1) + o, fcell(i) + o, fcell(i + 1) + o, q, vol, raw, p0, lo, hi, res, pb);
+            } else if (MODE) {
+                constexpr int XP = C::XPL, XL = (C::XRING - 1) * XP;
+                const float4* B = sx + base + (tj + 1) * XW + 2 * kk + q + 2;
+                const float4* A = B + (base >= XP ? -XP : XL);                             // plane i - 1
+                const float4* D = B + (base < XL ? XP : -XL);                              // plane i + 1
+                const float4* E = B + (base < XL - XP ? 2 * XP : -(C::XRING - 2) * XP);    // plane i + 2
+                slot_residual<XW>(A, B, D, E, vol, raw, p0, lo, hi, res);
+                pb = q ? B[-1].x : B[1].x;
             }
             const float dp = cell_solve(vol, v6, raw, res, lo, hi);
             const int k = kp0 + q;

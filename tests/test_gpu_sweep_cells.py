@@ -35,7 +35,7 @@ def solve_and_check(oracle, stg, n, b, fp, limit, **opts):
     s.close()
 
 
-@pytest.mark.parametrize("n,sweeps,method", [(8, 1, 0), (16, 2, 0), (24, 1, 0), (32, 1, 1), (48, 2, 0), (64, 1, 0), (96, 1, 0),
+@pytest.mark.parametrize("n,sweeps,method", [(8, 1, 0), (16, 2, 0), (16, 1, 0), (16, 1, 1), (24, 1, 0), (32, 1, 1), (48, 2, 0), (64, 1, 0), (96, 1, 0),
                                              (96, 1, 1)])
 def test_solve_at_tile_edges(oracle, stg, n, sweeps, method):
     b, rho, phys, fp = problem(oracle, n, seed=2)
