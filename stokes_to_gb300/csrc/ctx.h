@@ -199,8 +199,6 @@ int sweeps_per_colour(const stg_t* h);
 // the right-hand side of level top (null: its own r); the result is left in lv[top].xb
 bool small_cycle_ok(const stg_t* h, int top);
 int small_cycle(stg_t* h, int top, const float4* rhs);
-// the coarsest inverse's entries as small_cycle reads them, after each inversion
-int split_inverse(cudaStream_t st, DenseCoarse& D);
 // one V-cycle out = M(rhs) and y = A x on the finest level (FP32, solver.cu)
 int precond3(stg_t* h, const float4* rhs, float4* out);
 int apply3(stg_t* h, const float4* x, float4* y);

@@ -582,6 +582,22 @@ __global__ void k_gemv(int nd, const double* __restrict__ Ainv, int ld, const do
 
 }  // namespace
 
+namespace {
+__global__ void k_split_inverse(int nd, const double* __restrict__ inv, int ld, float2* __restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nd * nd) return;
+    const double a = inv[(long long)(t / nd) * ld + t % nd];
+    const float hi = (float)a;
+    out[t] = make_float2(hi, (float)(a - (double)hi));
+}
+}  // namespace
+
+int split_inverse(cudaStream_t st, int nd, const double* inv, int ld, float2* out) {
+    k_split_inverse<<<(nd * nd + 255) / 256, 256, 0, st>>>(nd, inv, ld, out);
+    STG_LAUNCH_CK();
+    return STG_OK;
+}
+
 int dense_init(DenseCoarse& D, const Geom& g) {
     std::vector<int> slot_of, comp_of, dense_of((size_t)g.nslot * 4, -1);
     const int n = g.n;

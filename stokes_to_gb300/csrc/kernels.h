@@ -170,6 +170,8 @@ struct DenseCoarse {
     InvOrder order;
 };
 int dense_init(DenseCoarse& D, const Geom& g);
+// the entries of an nd x nd inverse (row stride ld) as sums of two floats, row-major nd x nd
+int split_inverse(cudaStream_t st, int nd, const double* inv, int ld, float2* out);
 void dense_free(DenseCoarse& D);
 // DirectSolve3D::update: probe assembly + (closed) all-ones p-block + inversion (invert
 // false: the assembly only, for a caller that captures it in a CUDA graph and then calls

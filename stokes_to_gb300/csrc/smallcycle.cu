@@ -299,44 +299,6 @@ struct CycleShared {
 static_assert(ND % 16 == 0 && DOT_ROWS <= 2 * 16 && ND <= 512, "two rows a warp of half a block");
 static_assert(sizeof(CycleShared) <= 227 * 1024, "the shared memory of an SM");
 
-// sum of ND products a b over the lanes of a warp: a = hi + lo
-struct DfSum {
-    float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void add(float v) {  // exact: s + err = s + v
-        const float t = s + v, z = t - s;
-        c += (s - (t - z)) + (v - z);
-        s = t;
-    }
-    __device__ __forceinline__ void fma(float2 a, float b) {
-        const float p = __fmul_rn(a.x, b), e = fmaf(a.x, b, -p);  // a.x b = p + e
-        add(p);
-        c += fmaf(a.y, b, e);
-    }
-    __device__ __forceinline__ float warp_total() {
-        for (int o = 16; o > 0; o >>= 1) {
-            const float v = __shfl_xor_sync(0xffffffffu, s, o), d = __shfl_xor_sync(0xffffffffu, c, o);
-            const float t = s + v, z = t - s;
-            c = (c + d) + ((s - (t - z)) + (v - z));
-            s = t;
-        }
-        return s + c;
-    }
-};
-
-__global__ void k_split_inverse(const double* __restrict__ inv, int ld, float2* __restrict__ out) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ND * ND) return;
-    const double a = inv[(long long)(t / ND) * ld + t % ND];
-    const float hi = (float)a;
-    out[t] = make_float2(hi, (float)(a - (double)hi));
-}
-
-__device__ __forceinline__ void copy8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 // a cell's right-hand side from slots in shared memory (pitches RW, RP)
 template <int RW, int RP>
 __device__ __forceinline__ void cell_rhs(const float4* R, float res[7]) {
@@ -679,13 +641,6 @@ bool small_cycle_ok(const stg_t* h, int top) {
         return false;
     const int dev = device_slot();
     return dev >= 0 && cluster_ok(dev, false);
-}
-
-int split_inverse(cudaStream_t st, DenseCoarse& D) {
-    if (!D.inv2 || D.nd != ND) return STG_OK;
-    k_split_inverse<<<(ND * ND + 255) / 256, 256, 0, st>>>(D.inv, 2 * D.nd, D.inv2);
-    STG_LAUNCH_CK();
-    return STG_OK;
 }
 
 int small_cycle(stg_t* h, int top, const float4* rhs) {

@@ -181,7 +181,7 @@ int update(stg_t* h) {
                  },
                  [](bool) {}));
     PROF(h, 8, 0.0, inv_blocks(h->st, h->dense.nd, h->dense.order, h->closed ? 1 : 0, h->dense.A, h->dense.Ainv, h->dense.info, &h->dense.inv));
-    if (h->L > 2) PROF(h, 8, 0.0, split_inverse(h->st, h->dense));
+    if (h->L > 2 && h->dense.inv2) PROF(h, 8, 0.0, split_inverse(h->st, h->dense.nd, h->dense.inv, 2 * h->dense.nd, h->dense.inv2));
     h->updated = true;
     return STG_OK;
 }

@@ -513,6 +513,7 @@ struct V2 {
     G2d fine, coarse;
     int L;
     const double* inv;  // coarsest inverse, row stride ld, blocked coarse order
+    float2* inv2;       // its entries as sums of two floats, nd x nd (k2v_cycle; null: not used)
     int nd, ld;
     const int* map;     // blocked coarse index -> padded offset (-1: padding)
 };
@@ -545,26 +546,33 @@ __device__ __forceinline__ float ldv2(const float* p) { return __ldcg(p); }
 
 // One colour of the smoother, cells t0, t0 + step, ...: xo = x + P_c (r - A x); HX false: x = 0.
 // PRO: x is first corrected by the parent values of xc on level C (a fixed face's parent is
-// fixed, so its value is 0). The other colour's pressures are copied.
-template <bool HX, bool PRO>
+// fixed, so its value is 0). The other colour's pressures are copied. SM: the level's vectors and
+// coefficients are in shared memory; CS: xc is.
+template <bool HX, bool PRO, bool SM = false, bool CS = SM>
 __device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, const Lv2& C, const float* xc, float* xo, int t0,
                                        int step) {
     const int h = L.n >> 1, S = L.S, NS = L.NS;
+    auto var = [](const float* p) { return SM ? *p : ldv2(p); };
+    auto coef = [](const float* p) { return SM ? *p : __ldg(p); };
+    auto mask = [](const uint8_t* p) { return SM ? *p : __ldg(p); };
     for (int t = t0; t < L.n * h; t += step) {
         const int y = t / h, xx = 2 * (t - y * h) + ((y + flag) & 1);
         const int i = L.at(xx, y);
         const int ob = (xx & 1) ? i - 1 : i + 1;  // the pair's other cell
         auto V = [&](int c, int a, int b) {
-            float v = ldv2(x + c * NS + i + b * S + a);
-            if (PRO) v += ldv2(xc + c * C.NS + C.at((xx + a) >> 1, (y + b) >> 1));
+            float v = var(x + c * NS + i + b * S + a);
+            if (PRO) {
+                const float* e = xc + c * C.NS + C.at((xx + a) >> 1, (y + b) >> 1);
+                v += CS ? *e : ldv2(e);
+            }
             return v;
         };
-        const uint8_t m0 = __ldg(L.m + i), m1 = __ldg(L.m + i + 1), m2 = __ldg(L.m + i + S);
+        const uint8_t m0 = mask(L.m + i), m1 = mask(L.m + i + 1), m2 = mask(L.m + i + S);
         const bool fa = m0 & 1, fb = (m1 & 1) || xx + 1 == L.n, fc = m0 & 2, fd = (m2 & 2) || y + 1 == L.n;
-        const float Pp = __ldg(L.P + i), Pa = __ldg(L.P + NS + i), Pb = __ldg(L.P + NS + i + 1), Pc = __ldg(L.P + 2 * NS + i),
-                    Pd = __ldg(L.P + 2 * NS + i + S);
-        float rp = ldv2(L.r + i), ra = ldv2(L.r + NS + i), rb = ldv2(L.r + NS + i + 1), rc = ldv2(L.r + 2 * NS + i),
-              rd = ldv2(L.r + 2 * NS + i + S);
+        const float Pp = coef(L.P + i), Pa = coef(L.P + NS + i), Pb = coef(L.P + NS + i + 1), Pc = coef(L.P + 2 * NS + i),
+                    Pd = coef(L.P + 2 * NS + i + S);
+        float rp = var(L.r + i), ra = var(L.r + NS + i), rb = var(L.r + NS + i + 1), rc = var(L.r + 2 * NS + i),
+              rd = var(L.r + 2 * NS + i + S);
         float p = 0.f, ua = 0.f, ub = 0.f, vc = 0.f, vd = 0.f, pb = 0.f;
         if (HX) {
             p = V(0, 0, 0);
@@ -611,24 +619,28 @@ __device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, c
 
 // C.r = the 4-child sums of r - A x, 0 on fixed coarse faces; one coarse cell and its two low
 // faces a thread (the faces at X, Y = n are fixed: 0, as allocated)
+template <bool SM = false>
 __device__ __forceinline__ void restrict2(const Lv2& L, const float* x, const Lv2& C, int t0, int step) {
     const int S = L.S, NS = L.NS;
+    auto var = [](const float* p) { return SM ? *p : ldv2(p); };
+    auto coef = [](const float* p) { return SM ? *p : __ldg(p); };
+    auto mask = [](const uint8_t* p) { return SM ? *p : __ldg(p); };
     for (int t = t0; t < C.n * C.n; t += step) {
         const int Y = t / C.n, X = t - Y * C.n, o = C.at(X, Y);
         float sp = 0.f, su = 0.f, sw = 0.f;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const int i = L.at(2 * X + (q & 1), 2 * Y + (q >> 1));
-            const uint8_t m = __ldg(L.m + i);
+            const uint8_t m = mask(L.m + i);
             const float *xp = x + i, *xu = x + NS + i, *xv = x + 2 * NS + i;
-            const float p = ldv2(xp), u = ldv2(xu), v = ldv2(xv), ub = ldv2(xu + 1), vd = ldv2(xv + S);
-            const float lu = 4.f * u - (ldv2(xu - 1) + ub) - (ldv2(xu - S) + ldv2(xu + S));
-            const float lv = 4.f * v - (ldv2(xv - 1) + ldv2(xv + 1)) - (ldv2(xv - S) + vd);
-            sp += ldv2(L.r + i) - (L.vol * ((ub - u) + (vd - v)) + __ldg(L.P + i) * p);
-            if (!(m & 1)) su += ldv2(L.r + NS + i) - (L.vol * (lu - (p - ldv2(xp - 1))) + __ldg(L.P + NS + i) * u);
-            if (!(m & 2)) sw += ldv2(L.r + 2 * NS + i) - (L.vol * (lv - (p - ldv2(xp - S))) + __ldg(L.P + 2 * NS + i) * v);
+            const float p = var(xp), u = var(xu), v = var(xv), ub = var(xu + 1), vd = var(xv + S);
+            const float lu = 4.f * u - (var(xu - 1) + ub) - (var(xu - S) + var(xu + S));
+            const float lv = 4.f * v - (var(xv - 1) + var(xv + 1)) - (var(xv - S) + vd);
+            sp += var(L.r + i) - (L.vol * ((ub - u) + (vd - v)) + coef(L.P + i) * p);
+            if (!(m & 1)) su += var(L.r + NS + i) - (L.vol * (lu - (p - var(xp - 1))) + coef(L.P + NS + i) * u);
+            if (!(m & 2)) sw += var(L.r + 2 * NS + i) - (L.vol * (lv - (p - var(xp - S))) + coef(L.P + 2 * NS + i) * v);
         }
-        const uint8_t mc = __ldg(C.m + o);
+        const uint8_t mc = mask(C.m + o);
         C.r[o] = sp;
         C.r[C.NS + o] = (mc & 1) ? 0.f : su;
         C.r[2 * C.NS + o] = (mc & 2) ? 0.f : sw;
@@ -641,10 +653,11 @@ __device__ __forceinline__ void pad_in(const V2& v, const Lv2& L, const float* r
         if (a >= 0) L.r[a] = __ldg(rhs + t);
     }
 }
+template <bool SM = false>
 __device__ __forceinline__ void pad_out(const V2& v, const Lv2& L, const float* x, float* out, int t0, int step) {
     for (int t = t0; t < v.fine.size(); t += step) {
         const int a = pad_index(v.fine, L, t);
-        out[t] = a >= 0 ? ldv2(x + a) : 0.f;
+        out[t] = a < 0 ? 0.f : SM ? x[a] : ldv2(x + a);
     }
 }
 
@@ -679,29 +692,17 @@ __global__ void __launch_bounds__(TPB) k2v_gemv(const __grid_constant__ V2 v) {
 }
 
 // The V-cycle of levels top .. 0 by one thread-block cluster, a cluster barrier between the
-// passes (about 1 us a pass against 2 to 4 us for a kernel of a graph): parts 1 the way down, 2
-// the coarsest solve, 4 the way up. rhs / out: blocked finest vectors when top is the finest.
-// A level's passes are a few loads deep for each thread, so latency bounds it. 64^2 (levels to
-// 8^2, 18 passes): a design iteration with about 34 V-cycles 12.2 -> 5.65 ms; 512^2, two levels
-// above the cluster's: a solve of 46 V-cycles 22.3 -> 8.7 ms.
+// passes: parts 1 the way down, 4 the way up, with the coarsest solve (a larger inverse than
+// k2v_cycle takes) between them. rhs / out: blocked finest vectors when top is the finest.
+// A level's passes are a few loads deep for each thread, so latency bounds it: 2.25 us a pass
+// (96^2: two launches of 18 us a V-cycle).
 constexpr int VT = 512;  // threads of a cluster's block
-constexpr int CLUSTER_ND = 320;  // coarsest unknowns of a solve inside the cluster (8^2)
 __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, int top, int parts, const float* rhs, float* out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     // consecutive warps in different blocks: the small levels then use every SM of the cluster
     const int t0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), step = gridDim.x * VT;
-    using Rows = RowDots<CLUSTER_ND, 1>;
-    const int lane = threadIdx.x & 31, half = t0 >> 4;
-    Rows rows;
-    int at = -1;  // the thread's entry of the coarsest right-hand side
-    auto ahead = [&] {
-        if (!(parts & 2)) return;
-        rows.load(v.inv, v.ld, half, lane);
-        if (threadIdx.x < CLUSTER_ND) at = __ldg(v.map + threadIdx.x);
-    };
     if (parts & 1) {
-        if (top == 0) ahead();
         if (rhs) {
             pad_in(v, v.lv[top], rhs, t0, step);
             cl.sync();
@@ -713,25 +714,8 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
             sweep2<true, false>(L, 1, L.xa, C, nullptr, L.xb, t0, step);
             cl.sync();
             restrict2(L, L.xb, C, t0, step);
-            if (i == 1) ahead();
-            cl.sync();
+            if (i > 1) cl.sync();
         }
-    }
-    if (parts & 2) {  // (always with part 1)
-        __shared__ double rd[CLUSTER_ND];
-        static_assert(CLUSTER_ND <= VT, "one entry of the right-hand side a thread");
-        const Lv2& L = v.lv[0];
-        if (threadIdx.x < CLUSTER_ND) rd[threadIdx.x] = at >= 0 ? (double)ldv2(L.r + at) : 0.0;
-        __syncthreads();
-        if (t0 >> 5 < (Rows::HALVES + 1) / 2) {
-            double s[1];
-            rows.dot(rd, lane, s);
-            if ((lane & 15) == 0 && half < CLUSTER_ND) {
-                const int a = __ldg(v.map + half);
-                if (a >= 0) L.xa[a] = (float)s[0];
-            }
-        }
-        cl.sync();
     }
     if (parts & 4) {
         for (int i = 1; i <= top; i++) {
@@ -743,6 +727,133 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
         }
         if (out) pad_out(v, v.lv[top], top == 0 ? v.lv[0].xa : v.lv[top].xb, out, t0, step);
     }
+}
+
+// The same with the coarsest solve, for an 8^2 coarsest level. Every block has the levels of at
+// most 32 cells an axis to itself, in shared memory, so that their passes meet at block barriers;
+// only the levels above, the coarsest right-hand side's sixteenth of rows a block and its solution
+// cross the cluster. Bound: latency, 2.2 us for a pass through L2 and 0.5 for one in shared memory.
+// 64^2 (levels to 8^2): 32.4 us a cycle, with all passes through L2 and the coarsest product on the
+// FP64 pipe 41.2; 128^2: 42.7 and 51.6.
+constexpr int CYCLE_ND = 320, CYCLE_BLOCKS = 16, CYCLE_LEVELS = 3;  // coarsest unknowns; levels of 8, 16 and 32
+__host__ __device__ constexpr int cycle_mask(int NS) { return (NS + 15) / 16 * 16; }  // bytes of a level's mask: the next vectors lie on 16
+constexpr int cycle_smem() {
+    int s = 0;
+    for (int n = 8; n <= 32; n *= 2) s += (n + 4) * (n + 3) * 12 * 4 + cycle_mask((n + 4) * (n + 3));
+    return s;
+}
+__global__ void __launch_bounds__(VT) k2v_cycle(const __grid_constant__ V2 v, int top, const float* rhs, float* out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char cycle_window[];
+    __shared__ Lv2 lv[CYCLE_LEVELS];
+    __shared__ float rd[CYCLE_ND];
+    const int tid = threadIdx.x, b = blockIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t0 = (warp * CYCLE_BLOCKS + b) * 32 + lane, step = CYCLE_BLOCKS * VT;
+    const int in = min(top, CYCLE_LEVELS - 1);  // levels in .. 0 are the block's own
+    {
+        unsigned char* at = cycle_window;
+        for (int i = 0; i <= in; i++) {
+            const Lv2& G = v.lv[i];
+            float* f = reinterpret_cast<float*>(at);
+            uint8_t* m = at + 12 * 4 * G.NS;
+            if (tid == 0) {
+                lv[i] = G;
+                lv[i].r = f;
+                lv[i].xa = f + 3 * G.NS;
+                lv[i].xb = f + 6 * G.NS;
+                lv[i].P = f + 9 * G.NS;
+                lv[i].m = m;
+            }
+            // (NS is a multiple of 4)
+            for (int t = tid; t < 9 * G.NS / 4; t += VT) reinterpret_cast<float4*>(f)[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int t = tid; t < 3 * G.NS / 4; t += VT) copy16(f + 9 * G.NS + 4 * t, G.P + 4 * t);
+            for (int t = tid; t < G.NS / 4; t += VT) copy4(m + 4 * t, G.m + 4 * t);
+            at = m + cycle_mask(G.NS);
+        }
+    }
+    // the block's rows of the coarsest inverse, a warp a row
+    constexpr int ROWS = CYCLE_ND / CYCLE_BLOCKS, Q = CYCLE_ND / 32, H = (ROWS + VT / 32 - 1) / (VT / 32);
+    static_assert(CYCLE_ND % 32 == 0 && CYCLE_ND <= VT, "whole rows a warp, an entry a thread");
+    float2 a[H][Q];
+#pragma unroll
+    for (int k = 0; k < H; k++)
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int r = warp + k * (VT / 32);
+            a[k][q] = r < ROWS ? __ldg(v.inv2 + (b + CYCLE_BLOCKS * r) * CYCLE_ND + lane + 32 * q) : make_float2(0.f, 0.f);
+        }
+    const int at = tid < CYCLE_ND ? __ldg(v.map + tid) : -1;
+    __syncthreads();
+    auto started = cl.barrier_arrive();  // (cleared: other blocks may write here)
+    if (top > in) {
+        cl.barrier_wait(std::move(started));
+        if (rhs) {
+            pad_in(v, v.lv[top], rhs, t0, step);
+            cl.sync();
+        }
+        for (int i = top; i > in; i--) {
+            const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
+            sweep2<false, false>(L, 0, nullptr, C, nullptr, L.xa, t0, step);
+            cl.sync();
+            sweep2<true, false>(L, 1, L.xa, C, nullptr, L.xb, t0, step);
+            cl.sync();
+            restrict2(L, L.xb, C, t0, step);
+            cl.sync();
+        }
+        const float4* r = reinterpret_cast<const float4*>(v.lv[in].r);
+        for (int t = tid; t < 3 * v.lv[in].NS / 4; t += VT) reinterpret_cast<float4*>(lv[in].r)[t] = __ldcg(r + t);
+    } else {
+        pad_in(v, lv[top], rhs, tid, VT);
+        cl.barrier_wait(std::move(started));
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    for (int i = in; i >= 1; i--) {
+        const Lv2 &L = lv[i], &C = lv[i - 1];
+        sweep2<false, false, true>(L, 0, nullptr, C, nullptr, L.xa, tid, VT);
+        __syncthreads();
+        sweep2<true, false, true>(L, 1, L.xa, C, nullptr, L.xb, tid, VT);
+        __syncthreads();
+        restrict2<true>(L, L.xb, C, tid, VT);
+        __syncthreads();
+    }
+    if (tid < CYCLE_ND) rd[tid] = at >= 0 ? lv[0].r[at] : 0.f;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < H; k++) {
+        const int r = warp + k * (VT / 32);
+        if (r >= ROWS) break;
+        DfSum sum;
+#pragma unroll
+        for (int q = 0; q < Q; q++) sum.fma(a[k][q], rd[lane + 32 * q]);
+        const float x = sum.warp_total();
+        const int o = __ldg(v.map + b + CYCLE_BLOCKS * r);
+        if (lane < CYCLE_BLOCKS && o >= 0) cl.map_shared_rank(lv[0].xa, lane)[o] = x;
+    }
+    cl.sync();
+    for (int i = 1; i <= in; i++) {
+        const Lv2 &L = lv[i], &C = lv[i - 1];
+        sweep2<true, true, true>(L, 1, L.xb, C, i == 1 ? C.xa : C.xb, L.xa, tid, VT);
+        __syncthreads();
+        sweep2<true, false, true>(L, 0, L.xa, C, nullptr, L.xb, tid, VT);
+        __syncthreads();
+    }
+    for (int i = in + 1; i <= top; i++) {
+        const Lv2& L = v.lv[i];
+        if (i == in + 1)
+            sweep2<true, true, false, true>(L, 1, L.xb, lv[in], lv[in].xb, L.xa, t0, step);
+        else
+            sweep2<true, true>(L, 1, L.xb, v.lv[i - 1], v.lv[i - 1].xb, L.xa, t0, step);
+        cl.sync();
+        sweep2<true, false>(L, 0, L.xa, v.lv[i - 1], nullptr, L.xb, t0, step);
+        if (i < top || out) cl.sync();
+    }
+    if (!out) return;
+    if (top > in)
+        pad_out(v, v.lv[top], v.lv[top].xb, out, t0, step);
+    else
+        pad_out<true>(v, lv[top], top == 0 ? lv[0].xa : lv[top].xb, out, t0, step);
 }
 
 }  // namespace
@@ -906,6 +1017,7 @@ int setup2(stg_t* h) {
         STG_TRY(inv_blocks(h->st, lv[0].g.size(), h->c2->order, h->closed ? 1 : 0, h->c2->aug0, h->c2->aug1, h->c2->info, &h->c2->inv));
     V2& v = h->c2->v;
     v.inv = h->c2->inv;
+    if (v.inv2) STG_TRY(split_inverse(h->st, v.nd, v.inv, v.ld, v.inv2));
     for (int i = 0; i < v.L; i++) {  // a face's vol doubles a level down, as lap does
         v.lv[i].lap = (float)lv[i].lap;
         v.lv[i].vol = (float)std::ldexp(h->vol2d, v.L - 1 - i);
@@ -914,24 +1026,33 @@ int setup2(stg_t* h) {
     return STG_OK;
 }
 
-// The solver's V-cycle in the Laplacian form. Levels of at most 128 cells an axis, and the
-// coarsest solve when its inverse is small, run in one cluster launch (128^2: 8192 cells a
-// colour, one for each thread of 16 blocks; at 256^2 a pass of one cluster would take longer
-// than a launch of the whole GPU); larger ones a launch a pass, replayed as a CUDA graph.
+// The solver's V-cycle in the Laplacian form. Levels of at most 128 cells an axis run in one
+// cluster launch, with the coarsest solve when that level is 8^2 (128^2: 8192 cells a colour, one
+// for each thread of 16 blocks; at 256^2 a pass of one cluster would take longer than a launch
+// of the whole GPU); larger ones a launch a pass, replayed as a CUDA graph.
 constexpr int CLUSTER_N = 128;
 
-int launch_cluster2(stg_t* h, int top, int parts, const float* rhs, float* out) {
+cudaLaunchConfig_t config2(cudaStream_t st, int blocks, bool cycle, cudaLaunchAttribute (&at)[1]) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)h->c2->cluster);
+    cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(VT);
-    cfg.stream = h->st;
-    cudaLaunchAttribute at[1];
+    cfg.dynamicSmemBytes = cycle ? cycle_smem() : 0;
+    cfg.stream = st;
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)h->c2->cluster;
+    at[0].val.clusterDim.x = (unsigned)blocks;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    STG_CK(cudaLaunchKernelEx(&cfg, k2v_cluster, h->c2->v, top, parts, rhs, out));
+    return cfg;
+}
+// parts 7: the whole cycle of levels top .. 0 (k2v_cycle)
+int launch_cluster2(stg_t* h, int top, int parts, const float* rhs, float* out) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = config2(h->st, parts == 7 ? CYCLE_BLOCKS : h->c2->cluster, parts == 7, at);
+    if (parts == 7)
+        STG_CK(cudaLaunchKernelEx(&cfg, k2v_cycle, h->c2->v, top, rhs, out));
+    else
+        STG_CK(cudaLaunchKernelEx(&cfg, k2v_cluster, h->c2->v, top, parts, rhs, out));
     count_launch();
     return STG_OK;
 }
@@ -942,7 +1063,7 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
     const unsigned gs = g1(v.fine.size());
     int top = fine;  // finest level of the cluster part
     while (top > 0 && v.lv[top].n > CLUSTER_N) top--;
-    const bool whole = top == fine, small = v.nd == CLUSTER_ND && h->c2->cluster * VT / 16 >= CLUSTER_ND;  // a half-warp a row
+    const bool whole = top == fine, small = v.inv2 != nullptr;
     if (whole && small) return launch_cluster2(h, top, 7, rhs, out);
     if (!whole || top == 0) {
         k2v_in<<<gs, TPB, 0, h->st>>>(v, rhs);
@@ -1094,18 +1215,19 @@ int create2d(stg_t* h) {
         STG_LAUNCH_CK();
         // blocks of one cluster: 16 where the device grants it, else the portable 8
         STG_CK(cudaFuncSetAttribute(k2v_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        int can = 0;
+        cudaLaunchAttribute at[1];
         for (int c = 16; c >= 8 && !h->c2->cluster; c /= 2) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)c);
-            cfg.blockDim = dim3(VT);
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)c;
-            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int can = 0;
+            const cudaLaunchConfig_t cfg = config2(nullptr, c, false, at);
             if (cudaOccupancyMaxActiveClusters(&can, k2v_cluster, &cfg) == cudaSuccess && can > 0) h->c2->cluster = c;
+            cudaGetLastError();
+        }
+        if (nd == CYCLE_ND) {
+            STG_CK(cudaFuncSetAttribute(k2v_cycle, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            STG_CK(cudaFuncSetAttribute(k2v_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, cycle_smem()));
+            const cudaLaunchConfig_t cfg = config2(nullptr, CYCLE_BLOCKS, true, at);
+            if (h->c2->cluster && cudaOccupancyMaxActiveClusters(&can, k2v_cycle, &cfg) == cudaSuccess && can > 0)
+                STG_TRY(dalloc(&v.inv2, (size_t)nd * nd));
             cudaGetLastError();
         }
     }
@@ -1141,6 +1263,7 @@ void destroy2d(stg_t* h) {
     cudaFree(h->c2->pad);
     cudaFree(h->c2->padm);
     cudaFree(h->c2->map);
+    cudaFree(h->c2->v.inv2);
     delete h->c2;
     h->c2 = nullptr;
 }
