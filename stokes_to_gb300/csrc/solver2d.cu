@@ -617,33 +617,41 @@ __device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, c
     }
 }
 
-// C.r = the 4-child sums of r - A x, 0 on fixed coarse faces; one coarse cell and its two low
-// faces a thread (the faces at X, Y = n are fixed: 0, as allocated)
+// C.r = the 4-child sums of r - A x, 0 on fixed coarse faces (the faces at X, Y = n are fixed: 0,
+// as allocated). A lane per fine cell and its two low faces, the children of a coarse cell in
+// neighbouring lanes (levels have n^2 a multiple of 32): bound by latency, so the loads of one
+// child in a chain, not of four (512^2 children 6.7 us, 256^2 4.4; a thread a coarse cell took 10.9
+// and 10.6).
 template <bool SM = false>
 __device__ __forceinline__ void restrict2(const Lv2& L, const float* x, const Lv2& C, int t0, int step) {
     const int S = L.S, NS = L.NS;
     auto var = [](const float* p) { return SM ? *p : ldv2(p); };
     auto coef = [](const float* p) { return SM ? *p : __ldg(p); };
     auto mask = [](const uint8_t* p) { return SM ? *p : __ldg(p); };
-    for (int t = t0; t < C.n * C.n; t += step) {
-        const int Y = t / C.n, X = t - Y * C.n, o = C.at(X, Y);
-        float sp = 0.f, su = 0.f, sw = 0.f;
+    for (int t = t0; t < L.n * L.n; t += step) {
+        const int ch = t & 3, c = t >> 2, Y = c / C.n, X = c - Y * C.n, o = C.at(X, Y);
+        const int i = L.at(2 * X + (ch & 1), 2 * Y + (ch >> 1));
+        const uint8_t m = mask(L.m + i), mc = mask(C.m + o);
+        const float *xp = x + i, *xu = x + NS + i, *xv = x + 2 * NS + i;
+        const float p = var(xp), u = var(xu), v = var(xv), ub = var(xu + 1), vd = var(xv + S);
+        const float lu = 4.f * u - (var(xu - 1) + ub) - (var(xu - S) + var(xu + S));
+        const float lv = 4.f * v - (var(xv - 1) + var(xv + 1)) - (var(xv - S) + vd);
+        float sp = var(L.r + i) - (L.vol * ((ub - u) + (vd - v)) + coef(L.P + i) * p);
+        float su = var(L.r + NS + i) - (L.vol * (lu - (p - var(xp - 1))) + coef(L.P + NS + i) * u);
+        float sw = var(L.r + 2 * NS + i) - (L.vol * (lv - (p - var(xp - S))) + coef(L.P + 2 * NS + i) * v);
+        if (m & 1) su = 0.f;
+        if (m & 2) sw = 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int i = L.at(2 * X + (q & 1), 2 * Y + (q >> 1));
-            const uint8_t m = mask(L.m + i);
-            const float *xp = x + i, *xu = x + NS + i, *xv = x + 2 * NS + i;
-            const float p = var(xp), u = var(xu), v = var(xv), ub = var(xu + 1), vd = var(xv + S);
-            const float lu = 4.f * u - (var(xu - 1) + ub) - (var(xu - S) + var(xu + S));
-            const float lv = 4.f * v - (var(xv - 1) + var(xv + 1)) - (var(xv - S) + vd);
-            sp += var(L.r + i) - (L.vol * ((ub - u) + (vd - v)) + coef(L.P + i) * p);
-            if (!(m & 1)) su += var(L.r + NS + i) - (L.vol * (lu - (p - var(xp - 1))) + coef(L.P + NS + i) * u);
-            if (!(m & 2)) sw += var(L.r + 2 * NS + i) - (L.vol * (lv - (p - var(xp - S))) + coef(L.P + 2 * NS + i) * v);
+        for (int d = 1; d <= 2; d <<= 1) {
+            sp += __shfl_xor_sync(0xffffffffu, sp, d);
+            su += __shfl_xor_sync(0xffffffffu, su, d);
+            sw += __shfl_xor_sync(0xffffffffu, sw, d);
         }
-        const uint8_t mc = mask(C.m + o);
-        C.r[o] = sp;
-        C.r[C.NS + o] = (mc & 1) ? 0.f : su;
-        C.r[2 * C.NS + o] = (mc & 2) ? 0.f : sw;
+        if (ch == 0) {
+            C.r[o] = sp;
+            C.r[C.NS + o] = (mc & 1) ? 0.f : su;
+            C.r[2 * C.NS + o] = (mc & 2) ? 0.f : sw;
+        }
     }
 }
 
@@ -675,20 +683,30 @@ __global__ void __launch_bounds__(TPB) k2v_in(const __grid_constant__ V2 v, cons
 __global__ void __launch_bounds__(TPB) k2v_out(const __grid_constant__ V2 v, float* __restrict__ out) {
     pad_out(v, v.lv[v.L - 1], v.L == 1 ? v.lv[0].xa : v.lv[v.L - 1].xb, out, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
 }
-__device__ __forceinline__ void gemv_row2(const V2& v, int row, int lane) {
-    const Lv2& L = v.lv[0];
-    double s = 0;
-    for (int c = lane; c < v.nd; c += 32) {
-        const int a = __ldg(v.map + c);
-        if (a >= 0) s += __ldg(v.inv + (long long)row * v.ld + c) * (double)ldv2(L.r + a);
-    }
-    s = warp_sum(s);
-    const int a = __ldg(v.map + row);
-    if (lane == 0 && a >= 0) L.xa[a] = (float)s;
-}
+// The coarsest solve, a warp a row, the right-hand side gathered into shared memory (as FP64: a
+// conversion costs the FP64 unit as much as the multiply-add) and four loads of the row in flight.
+// Bound: the FP64 unit, 64 clocks a warp instruction and quarter of an SM. 24^2 (2112 unknowns):
+// 19.1 us, with the gather in the loop 43.5.
 __global__ void __launch_bounds__(TPB) k2v_gemv(const __grid_constant__ V2 v) {
-    const int row = (blockIdx.x * TPB + threadIdx.x) >> 5;
-    if (row < v.nd) gemv_row2(v, row, threadIdx.x & 31);
+    extern __shared__ double gv_r[];
+    const Lv2& L = v.lv[0];
+    for (int c = threadIdx.x; c < v.nd; c += TPB) {
+        const int a = __ldg(v.map + c);
+        gv_r[c] = a >= 0 ? (double)ldv2(L.r + a) : 0.0;
+    }
+    __syncthreads();
+    const int row = (blockIdx.x * TPB + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= v.nd) return;
+    const double* in = v.inv + (long long)row * v.ld;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int c = lane;
+    for (; c + 96 < v.nd; c += 128)
+#pragma unroll
+        for (int q = 0; q < 4; q++) s[q] += __ldg(in + c + 32 * q) * gv_r[c + 32 * q];
+    for (; c < v.nd; c += 32) s[0] += __ldg(in + c) * gv_r[c];
+    const double x = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+    const int a = __ldg(v.map + row);
+    if (lane == 0 && a >= 0) L.xa[a] = (float)x;
 }
 
 // The V-cycle of levels top .. 0 by one thread-block cluster, a cluster barrier between the
@@ -733,8 +751,8 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
 // most 32 cells an axis to itself, in shared memory, so that their passes meet at block barriers;
 // only the levels above, the coarsest right-hand side's sixteenth of rows a block and its solution
 // cross the cluster. Bound: latency, 2.2 us for a pass through L2 and 0.5 for one in shared memory.
-// 64^2 (levels to 8^2): 32.4 us a cycle, with all passes through L2 and the coarsest product on the
-// FP64 pipe 41.2; 128^2: 42.7 and 51.6.
+// 64^2 (levels to 8^2): 30.9 us a cycle, with all passes through L2 and the coarsest product on the
+// FP64 pipe 39.7; 128^2: 39.8 and 48.7.
 constexpr int CYCLE_ND = 320, CYCLE_BLOCKS = 16, CYCLE_LEVELS = 3;  // coarsest unknowns; levels of 8, 16 and 32
 __host__ __device__ constexpr int cycle_mask(int NS) { return (NS + 15) / 16 * 16; }  // bytes of a level's mask: the next vectors lie on 16
 constexpr int cycle_smem() {
@@ -1077,14 +1095,14 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
             STG_LAUNCH_CK();
             k2v_sweep<true, false><<<gb, TPB, 0, h->st>>>(L, 1, L.xa, C, nullptr, L.xb);
             STG_LAUNCH_CK();
-            k2v_restrict<<<g1((long long)C.n * C.n), TPB, 0, h->st>>>(L, L.xb, C);
+            k2v_restrict<<<g1((long long)L.n * L.n), TPB, 0, h->st>>>(L, L.xb, C);
             STG_LAUNCH_CK();
         }
         if (small) {
             STG_TRY(launch_cluster2(h, top, 7, nullptr, nullptr));
         } else {
             if (top > 0) STG_TRY(launch_cluster2(h, top, 1, nullptr, nullptr));
-            k2v_gemv<<<g1(32ll * v.nd), TPB, 0, h->st>>>(v);
+            k2v_gemv<<<g1(32ll * v.nd), TPB, sizeof(double) * v.nd, h->st>>>(v);
             STG_LAUNCH_CK();
             if (top > 0) STG_TRY(launch_cluster2(h, top, 4, nullptr, nullptr));
         }
@@ -1100,7 +1118,7 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
     };
     if (whole && top > 0) {  // the levels fit a cluster, the coarsest inverse does not
         STG_TRY(launch_cluster2(h, top, 1, rhs, nullptr));
-        k2v_gemv<<<g1(32ll * v.nd), TPB, 0, h->st>>>(v);
+        k2v_gemv<<<g1(32ll * v.nd), TPB, sizeof(double) * v.nd, h->st>>>(v);
         STG_LAUNCH_CK();
         return launch_cluster2(h, top, 4, nullptr, out);
     }
@@ -1215,6 +1233,7 @@ int create2d(stg_t* h) {
         STG_LAUNCH_CK();
         // blocks of one cluster: 16 where the device grants it, else the portable 8
         STG_CK(cudaFuncSetAttribute(k2v_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        STG_CK(cudaFuncSetAttribute(k2v_gemv, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * (int)sizeof(double)));
         int can = 0;
         cudaLaunchAttribute at[1];
         for (int c = 16; c >= 8 && !h->c2->cluster; c /= 2) {
