@@ -26,7 +26,14 @@ namespace {
 
 constexpr int TPB = 256;
 
-__global__ void k_probe(Geom g, int kind, int flag, d4* __restrict__ probe) {
+__device__ __forceinline__ void probe_of(int q, int& kind, int& flag) {
+    kind = q < 2 ? 0 : 1;
+    flag = q < 2 ? q : q - 2;
+}
+__global__ void k_probe(Geom g, int first, d4* __restrict__ probe) {
+    int kind, flag;
+    probe_of(first + blockIdx.y, kind, flag);
+    probe += (long long)blockIdx.y * g.nslot;
     long long t = (long long)blockIdx.x * TPB + threadIdx.x;
     if (t >= g.box()) return;
     int i, j, k;
@@ -44,10 +51,13 @@ __global__ void k_probe(Geom g, int kind, int flag, d4* __restrict__ probe) {
 }
 
 // Scatter one probe image into the dense matrix (column-major, nd x nd).
-__global__ void k_scatter(Geom g, int kind, int flag, int nd, const int* __restrict__ slot_of, const int* __restrict__ comp_of,
+__global__ void k_scatter(Geom g, int first, int nd, const int* __restrict__ slot_of, const int* __restrict__ comp_of,
                           const int* __restrict__ dense_of, const d4* __restrict__ image, double* __restrict__ A) {
     int row = blockIdx.x * TPB + threadIdx.x;
     if (row >= nd) return;
+    int kind, flag;
+    probe_of(first + blockIdx.y, kind, flag);
+    image += (long long)blockIdx.y * g.nslot;
     const int n = g.n;
     int s = slot_of[row], c = comp_of[row];
     // logical coordinates of the slot
@@ -623,8 +633,8 @@ int dense_init(DenseCoarse& D, const Geom& g) {
     if (n == 4) STG_CK(cudaMalloc(&D.inv2, sizeof(float2) * nd * nd));
     STG_CK(cudaMalloc(&D.piv, sizeof(int) * nd));
     STG_CK(cudaMalloc(&D.info, sizeof(int)));
-    STG_CK(cudaMalloc(&D.probe, sizeof(d4) * g.nslot));
-    STG_CK(cudaMalloc(&D.image, sizeof(d4) * g.nslot));
+    STG_CK(cudaMalloc(&D.probe, sizeof(d4) * g.nslot * PROBES));
+    STG_CK(cudaMalloc(&D.image, sizeof(d4) * g.nslot * PROBES));
     STG_CK(cudaMalloc(&D.rd, sizeof(double) * nd));
     std::vector<std::vector<int>> faces(3);
     std::vector<int> cells;
@@ -633,8 +643,8 @@ int dense_init(DenseCoarse& D, const Geom& g) {
     STG_CK(cudaMemcpy(D.slot_of, slot_of.data(), sizeof(int) * nd, cudaMemcpyHostToDevice));
     STG_CK(cudaMemcpy(D.comp_of, comp_of.data(), sizeof(int) * nd, cudaMemcpyHostToDevice));
     STG_CK(cudaMemcpy(D.dense_of, dense_of.data(), sizeof(int) * dense_of.size(), cudaMemcpyHostToDevice));
-    STG_CK(cudaMemset(D.probe, 0, sizeof(d4) * g.nslot));
-    STG_CK(cudaMemset(D.image, 0, sizeof(d4) * g.nslot));
+    STG_CK(cudaMemset(D.probe, 0, sizeof(d4) * g.nslot * PROBES));
+    STG_CK(cudaMemset(D.image, 0, sizeof(d4) * g.nslot * PROBES));
     return STG_OK;
 }
 
@@ -662,15 +672,12 @@ int dense_setup_v(cudaStream_t st, DenseCoarse& D, const Geom& g, const d4* V, c
     const int nd = D.nd;
     k_aug_init<<<grid_for(2ll * nd * nd, TPB), TPB, 0, st>>>(nd, D.A);
     STG_LAUNCH_CK();
-    for (int kind = 0; kind < 2; kind++) {
-        int nflags = kind == 0 ? 2 : 7;
-        for (int f = 0; f < nflags; f++) {
-            k_probe<<<grid_for(g.box(), TPB), TPB, 0, st>>>(g, kind, f, D.probe);
-            STG_LAUNCH_CK();
-            STG_TRY(op64v(st, g, D.probe, m, P64, V, nullptr, D.image, 0, nullptr, nullptr));
-            k_scatter<<<grid_for(nd, TPB), TPB, 0, st>>>(g, kind, f, nd, D.slot_of, D.comp_of, D.dense_of, D.image, D.A);
-            STG_LAUNCH_CK();
-        }
+    for (int q = 0; q < PROBES; q++) {
+        k_probe<<<grid_for(g.box(), TPB), TPB, 0, st>>>(g, q, D.probe);
+        STG_LAUNCH_CK();
+        STG_TRY(op64v(st, g, D.probe, m, P64, V, nullptr, D.image, 0, nullptr, nullptr));
+        k_scatter<<<grid_for(nd, TPB), TPB, 0, st>>>(g, q, nd, D.slot_of, D.comp_of, D.dense_of, D.image, D.A);
+        STG_LAUNCH_CK();
     }
     if (closed) {
         k_closed<<<grid_for((long long)nd * nd, TPB), TPB, 0, st>>>(nd, D.comp_of, D.A);
@@ -685,16 +692,12 @@ int dense_setup(cudaStream_t st, DenseCoarse& D, const Geom& g, double vol, cons
     const int nd = D.nd;
     k_aug_init<<<grid_for(2ll * nd * nd, TPB), TPB, 0, st>>>(nd, D.A);
     STG_LAUNCH_CK();
-    for (int kind = 0; kind < 2; kind++) {
-        int nflags = kind == 0 ? 2 : 7;
-        for (int f = 0; f < nflags; f++) {
-            k_probe<<<grid_for(g.box(), TPB), TPB, 0, st>>>(g, kind, f, D.probe);
-            STG_LAUNCH_CK();
-            STG_TRY(op64(st, g, vol, D.probe, m, P64, nullptr, D.image, 0, nullptr, nullptr));
-            k_scatter<<<grid_for(nd, TPB), TPB, 0, st>>>(g, kind, f, nd, D.slot_of, D.comp_of, D.dense_of, D.image, D.A);
-            STG_LAUNCH_CK();
-        }
-    }
+    // all probes at once: three launches of a few us each, nine times three took 95 us of a set-up
+    k_probe<<<dim3(grid_for(g.box(), TPB), PROBES), TPB, 0, st>>>(g, 0, D.probe);
+    STG_LAUNCH_CK();
+    STG_TRY(op64(st, g, vol, D.probe, m, P64, nullptr, D.image, 0, nullptr, nullptr, false, PROBES));
+    k_scatter<<<dim3(grid_for(nd, TPB), PROBES), TPB, 0, st>>>(g, 0, nd, D.slot_of, D.comp_of, D.dense_of, D.image, D.A);
+    STG_LAUNCH_CK();
     if (closed) {
         k_closed<<<grid_for((long long)nd * nd, TPB), TPB, 0, st>>>(nd, D.comp_of, D.A);
         STG_LAUNCH_CK();

@@ -38,6 +38,10 @@ __global__ void __launch_bounds__(TPB) k_op64(Geom g, double vol, const d4* __re
                                               const d4* __restrict__ P, const d4* __restrict__ b, d4* __restrict__ out,
                                               double* __restrict__ part) {
     long long t = (long long)blockIdx.x * TPB + threadIdx.x;
+    if (MODE == 0) {  // a batch of vectors, one after the other
+        x += (long long)blockIdx.y * g.nslot;
+        out += (long long)blockIdx.y * g.nslot;
+    }
     double acc = 0.0;
     if (t < g.box()) {
         int i, j, k;
@@ -865,13 +869,13 @@ int half_square64(cudaStream_t st, long long n4, const d4* x, d4* out) {
 }
 
 int op64(cudaStream_t st, const Geom& g, double vol, const d4* x, const uint8_t* m, const d4* P, const d4* b, d4* out,
-         int mode, double* part, int* nblocks_out, bool lap) {
+         int mode, double* part, int* nblocks_out, bool lap, int batch) {
     unsigned nb = grid_for(g.box(), TPB);
     if (nblocks_out) *nblocks_out = (int)nb;
     if (mode == 0 && lap)
-        k_op64<0, true><<<nb, TPB, 0, st>>>(g, vol, x, m, P, b, out, part);
+        k_op64<0, true><<<dim3(nb, batch), TPB, 0, st>>>(g, vol, x, m, P, b, out, part);
     else if (mode == 0)
-        k_op64<0, false><<<nb, TPB, 0, st>>>(g, vol, x, m, P, b, out, part);
+        k_op64<0, false><<<dim3(nb, batch), TPB, 0, st>>>(g, vol, x, m, P, b, out, part);
     else if (mode == 1 && !x && lap)  // r = b with x = 0: no operator pass
         k_op64<3, true><<<nb, TPB, 0, st>>>(g, vol, x, m, P, b, out, part);
     else if (mode == 1 && !x)

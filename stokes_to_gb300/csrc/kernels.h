@@ -19,7 +19,7 @@ namespace stg {
 // it when the level satisfies the Laplacian-form conditions and its vectors are zero on
 // fixed unknowns.
 int op64(cudaStream_t st, const Geom& g, double vol, const d4* x, const uint8_t* m, const d4* P, const d4* b, d4* out,
-         int mode, double* part, int* nblocks_out, bool lap = false);
+         int mode, double* part, int* nblocks_out, bool lap = false, int batch = 1);
 // rr = r - A x in FP32 (x == nullptr means x = 0, so rr = r)
 int resid32(cudaStream_t st, const Geom& g, float vol, const float4* r, const float4* x, const uint8_t* m, const float4* P,
             float4* rr, bool lap = false);
@@ -153,6 +153,7 @@ struct InvOrder {
     int N = 0, S = 0, TF = 0;
     int* perm = nullptr;
 };
+constexpr int PROBES = 9;  // coloured vectors that expose the coarsest matrix: two of cells, seven of faces
 struct DenseCoarse {
     int nd = 0;                // number of unknowns present at the coarsest level
     int* slot_of = nullptr;    // dense index -> slot
@@ -164,7 +165,7 @@ struct DenseCoarse {
     float2* inv2 = nullptr;    // its entries as sums of two floats, nd x nd (smallcycle.cu)
     int* piv = nullptr;
     int* info = nullptr;
-    d4* probe = nullptr;       // probe vector and its image (slots)
+    d4* probe = nullptr;       // PROBES probe vectors and their images (slots)
     d4* image = nullptr;
     double* rd = nullptr;      // gathered right-hand side (nd)
     InvOrder order;

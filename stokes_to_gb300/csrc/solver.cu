@@ -170,7 +170,7 @@ int update(stg_t* h) {
     for (int i = 0; i < h->L; i++) PROF(h, 8, 0.0, to_f16(h->st, h->lv[i].g, h->lv[i].P32, h->lv[i].m, h->d_pscale + i, h->lv[i].P16));
     // low words of the finest penalty for the double-float residual (P32 holds the high)
     PROF(h, 8, 0.0, split64(h->st, fine(h).g.nslot, fine(h).P64, nullptr, h->Plo));
-    // the coarsest matrix's assembly (27 small launches) reads and writes fixed buffers:
+    // the coarsest matrix's assembly (a few small launches) reads and writes fixed buffers:
     // replayed as a CUDA graph; its inversion is one cooperative launch
     GraphCache& G = h->sgraph;
     PROF(h, 8, 0.0,
