@@ -76,6 +76,7 @@ struct stg_ctx {
     stg_opts opts{};
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    cudaEvent_t ecol = nullptr;  // a Krylov column is in pinned memory
     // second stream and events for host copies that overlap the set-up (stg_set_rhs)
     cudaStream_t cst = nullptr;
     cudaEvent_t ec0 = nullptr, ec1 = nullptr;

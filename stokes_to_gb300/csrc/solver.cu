@@ -397,6 +397,11 @@ int vcycle(stg_t* h, const float4* rhs) {
 }
 
 // ---------------------------------------------------------------- FP64 refinement + FGMRES
+// Finest slots (quarters of the unknowns) up to which the next V-cycle is launched ahead of the
+// host's wait. 16^3 (6.9e3): a solve 1.20 -> 1.15 ms, 64^2 (3.3e3): a design step 5 % faster;
+// from 64^3 (3.0e5) and 512^2 (2.0e5) on the V-cycles lost at the end of a refinement step cost
+// what the others gain (1 % either way there, 128^3 3 % slower).
+constexpr long long AHEAD_SLOTS = 1 << 16;
 int residual64(stg_t* h, const d4* b, const d4* x, d4* r, double* nrm2_host) {
     Level& F = fine(h);
     int nb = 0;
@@ -612,9 +617,20 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
         // residual that minimises the new residual (never worse than the plain warm start)
         const bool predict = h->opts.warm_start == 2 && outer == 0 && !x_zero;
         const int msteps = predict ? 1 : m;
+        // The next step's V-cycle goes out before the host has this step's column: its input is
+        // on the device, and the host's wait, the small least-squares update and the launches pass
+        // while it runs. It is lost when the column ends the refinement step, so it is not sent
+        // when the last reduction would reach the target once more, nor where a V-cycle takes
+        // longer than what a step can gain (AHEAD_SLOTS). A vector that a second projection or a
+        // rescaling changes gets its V-cycle again.
+        const bool can_ahead = !predict && !h->net_on && !h->gen && !h->prof.on && n4 <= AHEAD_SLOTS;
+        bool ahead = false;  // Z[j]'s V-cycle is on its way
+        double last_est = beta;
         for (int j = 0; j < msteps; j++) {
             const bool aug_step = j >= m - have_aug;  // Z[j] holds a stored correction
-            if (predict) {
+            if (ahead) {
+                ahead = false;
+            } else if (predict) {
                 S.learned_iters++;
                 const bool keep = h->net_on;
                 h->net_on = true;
@@ -644,10 +660,18 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
             PROF(h, 6, (16.0 * (j + 3) + (h16 ? 8.0 : 0.0)) * n4,
                  project32(h->st, n4, h->V.data(), j + 1, h->dh, h->dsig2, h->w, h->V[j + 1], h->dh + m + 2, h->dnrm, red, h->dsig2 + j + 1,
                            h16 ? h->V16[j + 1] : nullptr, h->dnrm + 1, h->dsc16 + j + 1));
-            STG_CK(cudaStreamSynchronize(h->st));
+            if (can_ahead && j + 1 < msteps && j + 1 < m - have_aug && (j == 0 || prev_est * prev_est > itol * beta * last_est)) {
+                STG_CK(cudaEventRecord(h->ecol, h->st));
+                STG_TRY(h->precond(h, h->V[j + 1], h->Z[j + 1]));
+                ahead = true;
+                STG_CK(cudaEventSynchronize(h->ecol));
+            } else {
+                STG_CK(cudaStreamSynchronize(h->st));
+            }
             std::vector<double> h1(hd, hd + j + 1), h2(j + 1, 0.0);
             double nw2 = hn2[0];
             if (hn2[0] < 0.01 * hn2[1]) {
+                ahead = false;
                 std::copy(hd2, hd2 + j + 1, h2.begin());
                 PROF(h, 6, (16.0 * (j + 3) + (h16 ? 8.0 : 0.0)) * n4,
                      project32(h->st, n4, h->V.data(), j + 1, h->dh + m + 2, h->dsig2, h->V[j + 1], h->V[j + 1], nullptr, h->dnrm, red,
@@ -669,6 +693,7 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
                 // the unnormalised basis drifts in scale by the gain of A M each step (large
                 // for a weak preconditioner on high-contrast designs): renormalise before FP32
                 // over- or underflows
+                ahead = false;
                 PROF(h, 6, 32.0 * n4, scale32(h->st, n4, h->V[j + 1], h->dnrm, h->V[j + 1], h16 ? h->dsc16 + j + 1 : nullptr));
                 sig[j + 1] = 1.0;  // as the projection left dsig2
             } else if (nw2 > 0) {
@@ -701,6 +726,7 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
                 h->net_on = false;
                 S.fallbacks++;
             }
+            last_est = prev_est;
             prev_est = est;
             if (est <= itol * beta || hn == 0.0) break;
         }
@@ -905,6 +931,7 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
     }
     h->st = h->own_st;
     cudaEventCreate(&h->e0);
+    cudaEventCreateWithFlags(&h->ecol, cudaEventDisableTiming);
     cudaEventCreate(&h->e1);
     if (cudaStreamCreateWithFlags(&h->cst, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ec0, cudaEventDisableTiming) != cudaSuccess ||
@@ -1041,6 +1068,7 @@ int stg_destroy(stg_t* h) {
     cudaFree(h->dcount);
     cudaFreeHost(h->hres);
     if (h->e0) cudaEventDestroy(h->e0);
+    if (h->ecol) cudaEventDestroy(h->ecol);
     if (h->e1) cudaEventDestroy(h->e1);
     for (auto e : h->prof.pool) cudaEventDestroy(e);
     if (h->own_st) cudaStreamDestroy(h->own_st);
