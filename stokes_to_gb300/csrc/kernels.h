@@ -30,7 +30,7 @@ int apply32(cudaStream_t st, const Geom& g, float vol, const float4* x, const ui
 // residual: xout = xin + SHATTER(B^-1 GATHER(r - A xin)) (sweep.cu). xin == nullptr: xin = 0.
 // xc (coarse x on gc): xin is first corrected by the injected coarse value (the
 // prolongation fused into the sweep; needs xin, lap and P16, else STG_E_UNSUPPORTED). pair:
-// the sweeps of colour flag and then of the other, from xin = nullptr (needs lap and P16).
+// the sweeps of colour flag and then of the other (needs lap and P16).
 int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const float4* xin, float4* xout, const uint8_t* m,
             const float4* P, int flag, bool lap = false, const __half* P16 = nullptr, const float* p16_scale = nullptr,
             const float4* xc = nullptr, const Geom* gc = nullptr, bool pair = false);

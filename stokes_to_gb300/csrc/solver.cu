@@ -246,14 +246,25 @@ bool fuse_pair(const stg_t* h, const Level& L) {
     return !h->reference_cycle && sweeps_per_colour(h) == 1 && fast(h, L) && L.P16 && sweep_tma_available();
 }
 
-// C: the coarse level whose correction the first sweep injects (fuse_prolong)
-int smooth(stg_t* h, Level& L, const float4* r, bool post, bool x_is_zero, Level* C = nullptr) {
+// ... and the two after the coarse correction, up to 64 cells an axis (sweep.cu, MODE 4): two launches
+// against one take 17.4 and 15.8 us at 64^3, 9.6 and 8.0 at 32^3, with the gap between them another
+// 1 us; but 59 and 66 at 128^3, 377 and 420 at 256^3, where two blocks an SM overlap too little.
+constexpr int POST_PAIR_N = 64;
+bool fuse_post(const stg_t* h, const Level& L) { return fuse_pair(h, L) && L.g.n <= POST_PAIR_N; }
+
+// C: the coarse level whose correction the first sweep injects (fuse_prolong); pair: the two
+// post-sweeps may be one launch, with one change of buffer
+int smooth(stg_t* h, Level& L, const float4* r, bool post, bool x_is_zero, Level* C = nullptr, bool pair = false) {
     const int per = sweeps_per_colour(h);
-    if (x_is_zero && fuse_pair(h, L)) {
-        PROF(h, &L == &fine(h) ? 1 : 10, 40.0 * L.g.box(),
-             sweep32(h->st, L.g, (float)L.vol, r, nullptr, L.other(), L.m, L.P32, post ? 1 : 0, true, L.P16,
-                     h->d_pscale + (&L - h->lv.data()), nullptr, nullptr, true));
-        L.cur ^= 1;
+    // both sweeps in one launch; before the coarse correction the result stays in the first
+    // buffer where the post-smoother's pair, with its one change of buffer, follows
+    const bool post_pair = fuse_post(h, L);
+    if (x_is_zero ? fuse_pair(h, L) : pair && post_pair) {
+        float4* out = x_is_zero && post_pair ? L.x() : L.other();
+        PROF(h, &L == &fine(h) ? 1 : 10, (x_is_zero ? 40.0 : C ? 58.0 : 56.0) * L.g.box(),
+             sweep32(h->st, L.g, (float)L.vol, r, x_is_zero ? nullptr : L.x(), out, L.m, L.P32, post ? 1 : 0, true, L.P16,
+                     h->d_pscale + (&L - h->lv.data()), C ? C->x() : nullptr, C ? &C->g : nullptr, true));
+        if (out == L.other()) L.cur ^= 1;
         return STG_OK;
     }
     int s = 0;
@@ -295,7 +306,7 @@ int vcycle_levels(stg_t* h, int top, const float4* rhs) {
         Level& C = h->lv[i - 1];
         const float4* r = (i == L - 1) ? rhs : F.r;
         if (fuse_prolong(h, F)) {
-            STG_TRY(smooth(h, F, r, true, false, &C));
+            STG_TRY(smooth(h, F, r, true, false, &C, true));
             continue;
         }
         if (mixed) {
@@ -304,7 +315,7 @@ int vcycle_levels(stg_t* h, int top, const float4* rhs) {
         } else {
             PROF(h, 3, 16.0 * C.g.box() + 33.0 * F.g.box(), prolong_add32(h->st, F.g, C.g, C.x(), F.m, F.x(), lin));
         }
-        STG_TRY(smooth(h, F, r, true, false));
+        STG_TRY(smooth(h, F, r, true, false, nullptr, true));
     }
     return STG_OK;
 }
@@ -385,7 +396,7 @@ int vcycle(stg_t* h, const float4* rhs) {
     STG_TRY(smooth(h, F, rhs, false, true));
     PROF(h, 2, 49.0 * F.g.box() + 17.0 * C.g.box(), restrict_resid32(h->st, C.g, F.g, (float)F.vol, rhs, F.x(), F.m, F.P32, C.m, C.r, fast(h, F)));
     STG_TRY(coarse_cycle(h));
-    if (fuse_prolong(h, F)) return smooth(h, F, rhs, true, false, &C);
+    if (fuse_prolong(h, F)) return smooth(h, F, rhs, true, false, &C, true);
     const bool lin = h->opts.prolong == 1 && !h->reference_cycle;
     if (mixed) {
         PROF(h, 3, 24.0 * C.g.box(), to_bf16(h->st, C.g, C.x(), C.xbf));
@@ -393,7 +404,7 @@ int vcycle(stg_t* h, const float4* rhs) {
     } else {
         PROF(h, 3, 16.0 * C.g.box() + 33.0 * F.g.box(), prolong_add32(h->st, F.g, C.g, C.x(), F.m, F.x(), lin));
     }
-    return smooth(h, F, rhs, true, false);
+    return smooth(h, F, rhs, true, false, nullptr, true);
 }
 
 // ---------------------------------------------------------------- FP64 refinement + FGMRES

@@ -1016,7 +1016,9 @@ __global__ void __launch_bounds__(NT, 3) k_sweep_tma(const __grid_constant__ CUt
 // side, half of the warps form the first colour's cells two planes ahead (p and low faces, high
 // faces: sixteen bytes each, twelve loads instead of nineteen for the six neighbours), and the
 // others run the second colour from there: r and P are read once, and the first sweep's x is
-// neither written nor read.
+// neither written nor read; 4: the same from x, with the parents where xc is given (the two sweeps
+// after the coarse correction): x lands with two slots more on every side, and the first colour's
+// cells hand on the pressure of the pair's other cell too.
 //
 // Bound: the chain of a plane (land, work, barrier), which four blocks an SM overlap, three of
 // PAIR; at 256^3 HBM too (MODE 1 moves 0.98 GB in 180 us, 5.4 TB/s or 0.80 of the measured
@@ -1026,21 +1028,23 @@ __global__ void __launch_bounds__(NT, 3) k_sweep_tma(const __grid_constant__ CUt
 // 5.2 at 32^3 against 316, 44, 13.9 and 8.8 of MODE 0 and MODE 1 one after the other; with
 // 256-cell tiles in slot order and two blocks an SM it took 250 us, with loads three planes ahead
 // 240, with two warps more for the cells around the tile 239.
+// MODE 4 holds two blocks an SM: 15.8 us at 64^3 and 8.0 at 32^3 against 17.4 and 9.6 of MODE 2
+// and MODE 1, but 420 at 256^3 against 377 (solver.cu fuse_post).
 // Staging x by component instead, with 4-byte asynchronous copies (255 us for MODE 1) or through
 // registers (270 us), was slower: the transposing stores and the scattered loads of r and P
 // then bound it.
-template <int TK, bool PAIR = false>
+template <int TK, bool PAIR = false, bool WIDE = false>
 struct CellTile {
     static constexpr int NT = 128;            // threads with a pair of slots
     static constexpr int TJ = 2 * NT / TK, LR = TK / 2;    // rows, pairs of a row
     static constexpr int PW = LR < 16 ? LR : 16;           // pairs of a row in one warp
-    static constexpr int XW = TK + 4, XR = TJ + 3;         // staged x: k0 - 2 .. k0 + TK + 1, j0 - 1 .. j0 + TJ + 1
+    // staged x: k0 - 2 .. k0 + TK + 1, j0 - 1 .. j0 + TJ + 1; WIDE (PAIR with x): one cell more on every side
+    static constexpr int OX = WIDE ? 1 : 0, XW = TK + 4 + 2 * OX, XR = TJ + 3 + 2 * OX;
     static constexpr int O = PAIR ? 1 : 0;                 // PAIR: r and P of one cell more on every side
     static constexpr int RW = TK + 2 + 2 * O, RR = TJ + 1 + 2 * O;  // staged r and P: k0 - O .. (P: k0 - 1 ..), j0 - O .. j0 + TJ + O
     static constexpr int XPL = (XW * XR + 7) / 8 * 8;      // ring slots, 128-byte multiples (in slots)
     static constexpr int RPL = (RW * RR + 7) / 8 * 8, PPL = (RW * RR + 15) / 16 * 16;
     static constexpr unsigned XB = XW * XR * 16, RB = RW * RR * 16, PB = RW * RR * 8;  // box bytes
-    static constexpr int NX = (XW * XR + NT - 1) / NT;     // staged x slots of a thread (MODE 2)
     static constexpr int XRING = 5, RRING = PAIR ? 5 : 3;
     // PAIR: first-colour cells by row and pair, low and high halves; a row is four slots off a
     // multiple of 128 bytes, as the two rows of a warp have to be
@@ -1048,25 +1052,28 @@ struct CellTile {
     static constexpr int VN = 2 * (TJ + 1) * LR, WN = (2 * TJ * (LR + 1) + 1) / 2 * 2;  // sv, sw (floats)
     static constexpr int HALO = 2 * LR + TJ;               // PAIR: first-colour cells around the tile
     static constexpr int THREADS = PAIR ? 2 * NT : NT;
-    static constexpr int smem(bool x) { return (PAIR ? FRING * FPL * 32 : x ? XRING * XPL * 16 : 0) + RRING * (RPL * 16 + PPL * 8) + 4 * (VN + WN) + 8; }
+    static constexpr int NX = (XW * XR + THREADS - 1) / THREADS;  // staged x slots of a thread (with parents)
+    static constexpr int smem(bool x) { return (PAIR ? FRING * FPL * 32 : 0) + (x ? XRING * XPL * 16 : 0) + RRING * (RPL * 16 + PPL * 8) + 4 * (VN + WN) + 8; }
     static_assert((RRING * PPL * 8 + 4 * VN) % 8 == 0, "the mbarrier lies on an 8-byte boundary");
     static_assert(!PAIR || (FW % 8 == 4 && FPL % 4 == 0), "the staged planes start on 128 bytes");
 };
 
 template <int TK, int MODE>
-__global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 3 : 4) k_sweep_cell(
+__global__ void __launch_bounds__(CellTile<TK, MODE >= 3>::THREADS, MODE == 3 ? 3 : MODE == 4 ? 2 : 4) k_sweep_cell(
     const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmr,
     const __grid_constant__ CUtensorMap tmp, Geom g, float vol,
     float4* __restrict__ xout, const float* __restrict__ pscale, int flag,
     int chunk, int* __restrict__ err, const float4* __restrict__ xc, int c_plane,
     int c_sz) {
-    constexpr bool PAIR = MODE == 3, STAGE_X = MODE == 1 || MODE == 2;
-    using C = CellTile<TK, PAIR>;
+    constexpr bool PAIR = MODE >= 3, STAGE_X = MODE == 1 || MODE == 2 || MODE == 4;
+    using C = CellTile<TK, PAIR, MODE == 4>;
+    const bool parents = MODE == 2 || (MODE == 4 && xc);
     constexpr int NT = C::NT, TJ = C::TJ, XW = C::XW, RW = C::RW, FW = C::FW;
     // (no static shared memory: the TMA destinations start at the window's aligned origin)
     extern __shared__ __align__(1024) unsigned char cell_smem[];
-    float4* sx = reinterpret_cast<float4*>(cell_smem);
-    float4* sr = sx + (PAIR ? 2 * C::FRING * C::FPL : MODE ? C::XRING * C::XPL : 0);
+    float4* sf = reinterpret_cast<float4*>(cell_smem);
+    float4* sx = sf + (PAIR ? 2 * C::FRING * C::FPL : 0);
+    float4* sr = sx + (STAGE_X ? C::XRING * C::XPL : 0);
     uint2* sp = reinterpret_cast<uint2*>(sr + C::RRING * C::RPL);
     float (*sv)[TJ + 1][C::LR] = reinterpret_cast<float (*)[TJ + 1][C::LR]>(sp + C::RRING * C::PPL);  // [2]
     float (*sw)[TJ][C::LR + 1] = reinterpret_cast<float (*)[TJ][C::LR + 1]>(reinterpret_cast<float*>(sv) + C::VN);  // [2]
@@ -1090,7 +1097,7 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
     const unsigned bx = (unsigned)__cvta_generic_to_shared(sx), br = (unsigned)__cvta_generic_to_shared(sr),
                    bp_ = (unsigned)__cvta_generic_to_shared(sp);
     auto xslot = [&](int p) { return ((p + C::XRING) % C::XRING) * C::XPL; };
-    auto load_x = [&](int p) { tma3(bx + 16u * xslot(p), &tmx, 2 * (k0 - 1), j0, p + 1, bar); };
+    auto load_x = [&](int p) { tma3(bx + 16u * xslot(p), &tmx, 2 * (k0 - 1), j0 - C::OX, p + 1, bar); };
     auto load_rp = [&](int p) {
         const int s = (p + C::RRING) % C::RRING;
         tma3(br + 16u * (s * C::RPL), &tmr, 2 * (k0 + 1 - C::O), j0 + 1 - C::O, p + 1, bar);
@@ -1106,11 +1113,11 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
     // MODE 2: the parent values of the thread's share of a staged plane, and adding them
     float4 cv[C::NX];
     int co[C::NX];  // offset in a coarse plane, -1: none
-    if (MODE == 2) {
+    if (parents) {
 #pragma unroll
         for (int q = 0; q < C::NX; q++) {
-            const int e = tid + q * NT, jj = j0 - 1 + e / XW, k = k0 - 2 + e % XW;
-            co[q] = e < XW * C::XR && k >= -1 && jj <= n + 1 && k <= n + 1 ? ((jj >> 1) + 1) * c_sz + ((k >> 1) + 1) : -1;
+            const int e = tid + q * C::THREADS, jj = j0 - 1 - C::OX + e / XW, k = k0 - 2 + e % XW;
+            co[q] = e < XW * C::XR && k >= -1 && jj >= -1 && jj <= n + 1 && k <= n + 1 ? ((jj >> 1) + 1) * c_sz + ((k >> 1) + 1) : -1;
         }
     }
     auto fetch_coarse = [&](int p) {
@@ -1127,12 +1134,12 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
 #pragma unroll
         for (int q = 0; q < C::NX; q++) {
             if (co[q] < 0) continue;
-            float4 v = dst[q * NT];
+            float4 v = dst[q * C::THREADS];
             v.x += cv[q].x;
             v.y += cv[q].y;
             v.z += cv[q].z;
             v.w += cv[q].w;
-            dst[q * NT] = v;
+            dst[q * C::THREADS] = v;
         }
     };
 
@@ -1142,39 +1149,48 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
     }
     __syncthreads();
     if (tid == 0) {
-        arm_tx(bar, (STAGE_X ? 4 * C::XB : 0) + (PAIR ? 5 : 2) * (C::RB + C::PB));
+        arm_tx(bar, (STAGE_X ? (4 + C::OX) * C::XB : 0) + (PAIR ? 5 : 2) * (C::RB + C::PB));
         if (STAGE_X)
-            for (int p = i0 - 1; p <= i0 + 2; p++) load_x(p);
+            for (int p = i0 - 1 - C::OX; p <= i0 + 2; p++) load_x(p);
         for (int p = PAIR ? i0 - 1 : i0; p <= (PAIR ? i0 + 3 : i0 + 1); p++) load_rp(p);
     }
-    if (MODE == 2) fetch_coarse(i0 - 1);
-    if (__syncthreads_or(!wait_loads())) return fail(err);
-    if (MODE == 2) {
-        for (int p = i0 - 1; p <= i0 + 2; p++) {
-            if (p > i0 - 1 && ((p & 1) == 0)) fetch_coarse(p);  // planes 2 P and 2 P + 1 share their parents
+    auto add_parents = [&](int first_plane, int last_plane) {  // planes 2 P and 2 P + 1 share their parents
+        for (int p = first_plane; p <= last_plane; p++) {
+            if (p > first_plane && ((p & 1) == 0)) fetch_coarse(p);
             add_coarse(p);
         }
+    };
+    if (parents) fetch_coarse(i0 - 1 - C::OX);
+    if (__syncthreads_or(!wait_loads())) return fail(err);
+    if (parents) {
+        add_parents(i0 - 1 - C::OX, i0 + 2);
         __syncthreads();
     }
 
-    // PAIR: the first colour's cells of plane p in the tile and around it, from x = 0 (0 outside
-    // the domain): pressure and low faces, high faces; pair -1 and LR are the cells beside a row
-    auto fcell = [&](int p) { return sx + 2 * (p & (C::FRING - 1)) * C::FPL; };
+    // PAIR: the first colour's cells of plane p in the tile and around it (0 outside the domain):
+    // pressure and low faces, high faces and the pressure of the pair's other cell; pair -1 and
+    // LR are the cells beside a row
+    auto fcell = [&](int p) { return sf + 2 * (p & (C::FRING - 1)) * C::FPL; };
     auto first_cell = [&](int p, int row, int c) {
         const int jj = j0 + row, k = k0 + c;
-        float dp = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+        float p0 = 0.f, po = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
         if (p >= 0 && p < n && jj >= 0 && jj < n && k >= 0 && k < n) {
             const int sl = (p + C::RRING) % C::RRING, sn = sl + 1 < C::RRING ? sl + 1 : 0, ro = (row + 1) * RW + c + 1;
             const float4* R = sr + sl * C::RPL + ro;
             float raw[7];
             cell_penalty<RW>(sp + sl * C::PPL + ro, sp + sn * C::PPL + ro, psc, raw);
             const float4 r0 = *R;
-            const float res[7] = {r0.x, r0.y, r0.z, r0.w, sr[sn * C::RPL + ro].y, R[RW].z, R[1].w};
-            dp = cell_solve(vol, v6, raw, res, lo, hi);
+            float res[7] = {r0.x, r0.y, r0.z, r0.w, sr[sn * C::RPL + ro].y, R[RW].z, R[1].w};
+            if (MODE == 4) {
+                const float4* B = sx + (row + 2) * XW + c + 2;
+                slot_residual<XW>(B + xslot(p - 1), B + xslot(p), B + xslot(p + 1), B + xslot(p + 2), vol, raw, p0, lo, hi, res);
+                po = B[xslot(p) + (c & 1 ? -1 : 1)].x;
+            }
+            p0 += cell_solve(vol, v6, raw, res, lo, hi);
         }
         float4* F = fcell(p) + (row + 1) * FW + ((c + 2) >> 1);
-        F[0] = make_float4(dp, lo[0], lo[1], lo[2]);
-        F[C::FPL] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        F[0] = make_float4(p0, lo[0], lo[1], lo[2]);
+        F[C::FPL] = make_float4(hi[0], hi[1], hi[2], po);
     };
     auto first_tile = [&](int p) { first_cell(p, tj, 2 * kk + ((p + j + flag) & 1)); };
     auto first_halo = [&](int p) {
@@ -1191,12 +1207,24 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
         first_halo(p);
     };
     if (PAIR) {
-        if (first) {
+        if (first)
             first_plane(i0);
-            first_plane(i0 + 1);
-        } else {
+        else
             first_tile(i0 - 1);  // (nothing needs the cells around it)
+        if (MODE == 4) {  // x of two planes more, in place of the first two
+            __syncthreads();
+            if (tid == 0) {
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                arm_tx(bar, 2 * C::XB);
+                load_x(i0 + 3);
+                load_x(i0 + 4);
+            }
+            if (parents && ((i0 + 3) & 1) == 0) fetch_coarse(i0 + 3);
+            const bool ok = wait_loads();
+            if (parents) add_parents(i0 + 3, i0 + 4);
+            if (__syncthreads_or(!ok)) return fail(err);
         }
+        if (first) first_plane(i0 + 1);
         __syncthreads();
     }
 
@@ -1223,14 +1251,14 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
     int base = xslot(i0), rs = i0 % C::RRING;  // ring slots of plane i
     for (int i = i0; i < i1; i++) {
         const bool more = i + 1 < i1;
-        // x(i + 3) into the slot of x(i - 2), r and P of i + 2 (PAIR: i + 4) into those of i - 1
+        // x(i + 3) into the slot of x(i - 2) (PAIR: i + 5, i), r and P of i + 2 (i + 4) into those of i - 1
         if (more && tid == 0) {
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             arm_tx(bar, (STAGE_X ? C::XB : 0) + C::RB + C::PB);
-            if (STAGE_X) load_x(i + 3);
+            if (STAGE_X) load_x(PAIR ? i + 5 : i + 3);
             load_rp(PAIR ? i + 4 : i + 2);
         }
-        if (MODE == 2 && more && ((i + 3) & 1) == 0) fetch_coarse(i + 3);  // an odd plane's parents are the last plane's
+        if (parents && more && ((i + 3) & 1) == 0) fetch_coarse(PAIR ? i + 5 : i + 3);  // an odd plane's parents are the last plane's
         if (i > i0 && live) write_black(i - 1);
         const int rn = rs + 1 < C::RRING ? rs + 1 : 0;  // ring slot of r and P of plane i + 1
         if (PAIR && first && more) first_plane(i + 2);
@@ -1245,6 +1273,7 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
             float p0 = 0.f, pb = 0.f, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
             if (PAIR) {
                 const int o = (tj + 1) * FW + kk + 1;
+                if (MODE == 4) p0 = fcell(i)[C::FPL + o].w;
                 neighbour_residual<FW, C::FPL>(fcell(i - 1) + o, fcell(i) + o, fcell(i + 1) + o, q, vol, raw, p0, lo, hi, res, pb);
             } else if (MODE) {
                 constexpr int XP = C::XPL, XL = (C::XRING - 1) * XP;
@@ -1273,7 +1302,7 @@ __global__ void __launch_bounds__(CellTile<TK, MODE == 3>::THREADS, MODE == 3 ? 
         rs = rn;
         if (!more) break;
         const bool ok = wait_loads();
-        if (MODE == 2) add_coarse(i + 3);
+        if (parents) add_coarse(PAIR ? i + 5 : i + 3);
         if (__syncthreads_or(!ok)) return fail(err);
     }
     __syncthreads();
@@ -1365,24 +1394,29 @@ int launch_cell(cudaStream_t st, int dev, EncodeTiled enc, const Geom& g, float 
                 const __half* P16, const float* psc, int flag, const float4* xc, const Geom* gc, bool pair, bool* done) {
     using C = CellTile<TK>;
     using CP = CellTile<TK, true>;
+    using CX = CellTile<TK, true, true>;
     static bool set[MAX_DEVICES] = {};
     if (!set[dev]) {
         STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(false)));
         STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(true)));
         STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(true)));
-        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, CP::smem(true)));
+        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, CP::smem(false)));
+        STG_CK(cudaFuncSetAttribute(k_sweep_cell<TK, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, CX::smem(true)));
         set[dev] = true;
     }
     CUtensorMap mx{}, mr{}, mp{};
     const int rw = pair ? CP::RW : C::RW, rr = pair ? CP::RR : C::RR;
     *done = cell_map(enc, &mr, r, g, 2, rw, rr) && cell_map(enc, &mp, P16, g, 1, rw, rr) &&
-            (!xin || cell_map(enc, &mx, xin, g, 2, C::XW, C::XR));
+            (!xin || cell_map(enc, &mx, xin, g, 2, pair ? CX::XW : C::XW, pair ? CX::XR : C::XR));
     if (!*done) return STG_OK;
-    const int tj = pair ? CP::TJ : C::TJ, chunk = cell_chunk(dev, g.n, TK, tj, pair ? 3 : xin ? 4 : 8);
+    const int tj = pair ? CP::TJ : C::TJ, chunk = cell_chunk(dev, g.n, TK, tj, pair ? (xin ? 2 : 3) : xin ? 4 : 8);
     const dim3 grid((g.n + TK - 1) / TK, (g.n + tj - 1) / tj, (g.n + chunk - 1) / chunk);
     int* err = g_sweep_err[dev];
-    if (pair)
-        k_sweep_cell<TK, 3><<<grid, CP::THREADS, CP::smem(true), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+    if (pair && !xin)
+        k_sweep_cell<TK, 3><<<grid, CP::THREADS, CP::smem(false), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
+    else if (pair)
+        k_sweep_cell<TK, 4><<<grid, CX::THREADS, CX::smem(true), st>>>(mx, mr, mp, g, vol, xout, psc, flag, chunk, err, xc,
+                                                                        xc ? gc->sy * gc->sz : 0, xc ? gc->sz : 0);
     else if (!xin)
         k_sweep_cell<TK, 0><<<grid, C::NT, C::smem(false), st>>>(mr, mr, mp, g, vol, xout, psc, flag, chunk, err, nullptr, 0, 0);
     else if (!xc)
