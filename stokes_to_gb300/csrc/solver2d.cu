@@ -547,10 +547,13 @@ __device__ __forceinline__ float ldv2(const float* p) { return __ldcg(p); }
 // One colour of the smoother, cells t0, t0 + step, ...: xo = x + P_c (r - A x); HX false: x = 0.
 // PRO: x is first corrected by the parent values of xc on level C (a fixed face's parent is
 // fixed, so its value is 0). The other colour's pressures are copied. SM: the level's vectors and
-// coefficients are in shared memory; CS: xc is.
-template <bool HX, bool PRO, bool SM = false, bool CS = SM>
+// coefficients are in shared memory; CS: xc is. IN (red, x = 0): r comes from the blocked vector
+// of g instead, and goes to L.r on the way; OUT (red): the result goes to the blocked vector xo.
+// Either leaves out the faces on the domain boundary that lie at black cells (fixed: r is 0 there
+// and so is x; out_border).
+template <bool HX, bool PRO, bool SM = false, bool CS = SM, bool IN = false, bool OUT = false>
 __device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, const Lv2& C, const float* xc, float* xo, int t0,
-                                       int step) {
+                                       int step, const G2d g = G2d(), const float* blocked = nullptr) {
     const int h = L.n >> 1, S = L.S, NS = L.NS;
     auto var = [](const float* p) { return SM ? *p : ldv2(p); };
     auto coef = [](const float* p) { return SM ? *p : __ldg(p); };
@@ -571,8 +574,26 @@ __device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, c
         const bool fa = m0 & 1, fb = (m1 & 1) || xx + 1 == L.n, fc = m0 & 2, fd = (m2 & 2) || y + 1 == L.n;
         const float Pp = coef(L.P + i), Pa = coef(L.P + NS + i), Pb = coef(L.P + NS + i + 1), Pc = coef(L.P + 2 * NS + i),
                     Pd = coef(L.P + 2 * NS + i + S);
-        float rp = var(L.r + i), ra = var(L.r + NS + i), rb = var(L.r + NS + i + 1), rc = var(L.r + 2 * NS + i),
-              rd = var(L.r + 2 * NS + i + S);
+        float rp, ra, rb, rc, rd;
+        if (IN) {
+            rp = __ldg(blocked + g.cell(xx, y));
+            ra = __ldg(blocked + g.face(xx, y, 0));
+            rb = __ldg(blocked + g.face(xx + 1, y, 0));
+            rc = __ldg(blocked + g.face(xx, y, 1));
+            rd = __ldg(blocked + g.face(xx, y + 1, 1));
+            L.r[i] = rp;
+            L.r[ob] = __ldg(blocked + g.cell(xx ^ 1, y));
+            L.r[NS + i] = ra;
+            L.r[NS + i + 1] = rb;
+            L.r[2 * NS + i] = rc;
+            L.r[2 * NS + i + S] = rd;
+        } else {
+            rp = var(L.r + i);
+            ra = var(L.r + NS + i);
+            rb = var(L.r + NS + i + 1);
+            rc = var(L.r + 2 * NS + i);
+            rd = var(L.r + 2 * NS + i + S);
+        }
         float p = 0.f, ua = 0.f, ub = 0.f, vc = 0.f, vd = 0.f, pb = 0.f;
         if (HX) {
             p = V(0, 0, 0);
@@ -608,12 +629,20 @@ __device__ __forceinline__ void sweep2(const Lv2& L, int flag, const float* x, c
         const float schur = Pp - (ga * wa + gb * wb + gc * wc + gd * wd);
         const float num = rp - (ga * za + gb * zb + gc * zc + gd * zd);
         const float dp = schur != 0.f ? num / schur : 0.f;  // a cell between four fixed faces keeps its pressure
-        xo[i] = p + dp;
-        xo[ob] = pb;
-        xo[NS + i] = ua + (za - dp * wa);
-        xo[NS + i + 1] = ub + (zb - dp * wb);
-        xo[2 * NS + i] = vc + (zc - dp * wc);
-        xo[2 * NS + i + S] = vd + (zd - dp * wd);
+        xo[OUT ? g.cell(xx, y) : i] = p + dp;
+        xo[OUT ? g.cell(xx ^ 1, y) : ob] = pb;
+        xo[OUT ? g.face(xx, y, 0) : NS + i] = ua + (za - dp * wa);
+        xo[OUT ? g.face(xx + 1, y, 0) : NS + i + 1] = ub + (zb - dp * wb);
+        xo[OUT ? g.face(xx, y, 1) : 2 * NS + i] = vc + (zc - dp * wc);
+        xo[OUT ? g.face(xx, y + 1, 1) : 2 * NS + i + S] = vd + (zd - dp * wd);
+    }
+}
+
+// 0 in the blocked vector's padding and on the faces of the domain boundary (fixed)
+__device__ __forceinline__ void out_border(const G2d& g, float* out, int t0, int step) {
+    for (int t = t0; t < 18 * g.n; t += step) {
+        const int q = t % g.n, c = t / g.n % 9, d = t / (9 * g.n), a = c ? g.n + c - 1 : 0;
+        out[d ? g.face(q, a, 1) : g.face(a, q, 0)] = 0.f;
     }
 }
 
@@ -674,6 +703,19 @@ template <bool HX, bool PRO>
 __global__ void __launch_bounds__(TPB) k2v_sweep(Lv2 L, int flag, const float* x, Lv2 C, const float* xc, float* xo) {
     sweep2<HX, PRO>(L, flag, x, C, xc, xo, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
 }
+// the finest level's first sweep, from the blocked right-hand side, and its last, to the blocked
+// result (512^2: 5.3 and 7.3 us; the sweeps 4.5 and 5.9 with a pass of its own for either
+// conversion, 5.6 and 5.9)
+__global__ void __launch_bounds__(TPB) k2v_sweep_in(const __grid_constant__ V2 v, const float* __restrict__ rhs) {
+    const Lv2& L = v.lv[v.L - 1];
+    sweep2<false, false, false, false, true>(L, 0, nullptr, L, nullptr, L.xa, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB, v.fine, rhs);
+}
+__global__ void __launch_bounds__(TPB) k2v_sweep_out(const __grid_constant__ V2 v, float* __restrict__ out) {
+    const Lv2& L = v.lv[v.L - 1];
+    const int t0 = blockIdx.x * TPB + threadIdx.x, step = gridDim.x * TPB;
+    sweep2<true, false, false, false, false, true>(L, 0, L.xa, L, nullptr, out, t0, step, v.fine);
+    out_border(v.fine, out, t0, step);
+}
 __global__ void __launch_bounds__(TPB) k2v_restrict(Lv2 L, const float* x, Lv2 C) {
     restrict2(L, x, C, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
 }
@@ -681,7 +723,7 @@ __global__ void __launch_bounds__(TPB) k2v_in(const __grid_constant__ V2 v, cons
     pad_in(v, v.lv[v.L - 1], rhs, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
 }
 __global__ void __launch_bounds__(TPB) k2v_out(const __grid_constant__ V2 v, float* __restrict__ out) {
-    pad_out(v, v.lv[v.L - 1], v.L == 1 ? v.lv[0].xa : v.lv[v.L - 1].xb, out, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+    pad_out(v, v.lv[0], v.lv[0].xa, out, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);  // (one level)
 }
 // The coarsest solve, a warp a row, the right-hand side gathered into shared memory (as FP64: a
 // conversion costs the FP64 unit as much as the multiply-add) and four loads of the row in flight.
@@ -721,13 +763,12 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
     // consecutive warps in different blocks: the small levels then use every SM of the cluster
     const int t0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), step = gridDim.x * VT;
     if (parts & 1) {
-        if (rhs) {
-            pad_in(v, v.lv[top], rhs, t0, step);
-            cl.sync();
-        }
         for (int i = top; i >= 1; i--) {
             const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
-            sweep2<false, false>(L, 0, nullptr, C, nullptr, L.xa, t0, step);
+            if (i == top && rhs)
+                sweep2<false, false, false, false, true>(L, 0, nullptr, C, nullptr, L.xa, t0, step, v.fine, rhs);
+            else
+                sweep2<false, false>(L, 0, nullptr, C, nullptr, L.xa, t0, step);
             cl.sync();
             sweep2<true, false>(L, 1, L.xa, C, nullptr, L.xb, t0, step);
             cl.sync();
@@ -740,10 +781,14 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
             const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
             sweep2<true, true>(L, 1, L.xb, C, i == 1 ? C.xa : C.xb, L.xa, t0, step);
             cl.sync();
-            sweep2<true, false>(L, 0, L.xa, C, nullptr, L.xb, t0, step);
-            cl.sync();
+            if (i == top && out) {
+                sweep2<true, false, false, false, false, true>(L, 0, L.xa, C, nullptr, out, t0, step, v.fine);
+                out_border(v.fine, out, t0, step);
+            } else {
+                sweep2<true, false>(L, 0, L.xa, C, nullptr, L.xb, t0, step);
+            }
+            if (i < top) cl.sync();
         }
-        if (out) pad_out(v, v.lv[top], top == 0 ? v.lv[0].xa : v.lv[top].xb, out, t0, step);
     }
 }
 
@@ -751,8 +796,9 @@ __global__ void __launch_bounds__(VT) k2v_cluster(const __grid_constant__ V2 v, 
 // most 32 cells an axis to itself, in shared memory, so that their passes meet at block barriers;
 // only the levels above, the coarsest right-hand side's sixteenth of rows a block and its solution
 // cross the cluster. Bound: latency, 2.2 us for a pass through L2 and 0.5 for one in shared memory.
-// 64^2 (levels to 8^2): 30.9 us a cycle, with all passes through L2 and the coarsest product on the
-// FP64 pipe 39.7; 128^2: 39.8 and 48.7.
+// 64^2 (levels to 8^2): 25.9 us a cycle; with all passes through L2, the coarsest product on the
+// FP64 pipe and passes of their own for the blocked vectors 39.7; 128^2 below larger levels: 39.8
+// and 48.7.
 constexpr int CYCLE_ND = 320, CYCLE_BLOCKS = 16, CYCLE_LEVELS = 3;  // coarsest unknowns; levels of 8, 16 and 32
 __host__ __device__ constexpr int cycle_mask(int NS) { return (NS + 15) / 16 * 16; }  // bytes of a level's mask: the next vectors lie on 16
 constexpr int cycle_smem() {
@@ -806,13 +852,12 @@ __global__ void __launch_bounds__(VT) k2v_cycle(const __grid_constant__ V2 v, in
     auto started = cl.barrier_arrive();  // (cleared: other blocks may write here)
     if (top > in) {
         cl.barrier_wait(std::move(started));
-        if (rhs) {
-            pad_in(v, v.lv[top], rhs, t0, step);
-            cl.sync();
-        }
         for (int i = top; i > in; i--) {
             const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
-            sweep2<false, false>(L, 0, nullptr, C, nullptr, L.xa, t0, step);
+            if (i == top && rhs)
+                sweep2<false, false, false, false, true>(L, 0, nullptr, C, nullptr, L.xa, t0, step, v.fine, rhs);
+            else
+                sweep2<false, false>(L, 0, nullptr, C, nullptr, L.xa, t0, step);
             cl.sync();
             sweep2<true, false>(L, 1, L.xa, C, nullptr, L.xb, t0, step);
             cl.sync();
@@ -864,14 +909,15 @@ __global__ void __launch_bounds__(VT) k2v_cycle(const __grid_constant__ V2 v, in
         else
             sweep2<true, true>(L, 1, L.xb, v.lv[i - 1], v.lv[i - 1].xb, L.xa, t0, step);
         cl.sync();
-        sweep2<true, false>(L, 0, L.xa, v.lv[i - 1], nullptr, L.xb, t0, step);
-        if (i < top || out) cl.sync();
+        if (i == top && out) {
+            sweep2<true, false, false, false, false, true>(L, 0, L.xa, v.lv[i - 1], nullptr, out, t0, step, v.fine);
+            out_border(v.fine, out, t0, step);
+        } else {
+            sweep2<true, false>(L, 0, L.xa, v.lv[i - 1], nullptr, L.xb, t0, step);
+        }
+        if (i < top) cl.sync();
     }
-    if (!out) return;
-    if (top > in)
-        pad_out(v, v.lv[top], v.lv[top].xb, out, t0, step);
-    else
-        pad_out<true>(v, lv[top], top == 0 ? lv[0].xa : lv[top].xb, out, t0, step);
+    if (top == in && out) pad_out<true>(v, lv[top], top == 0 ? lv[0].xa : lv[top].xb, out, t0, step);
 }
 
 }  // namespace
@@ -1083,7 +1129,12 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
     while (top > 0 && v.lv[top].n > CLUSTER_N) top--;
     const bool whole = top == fine, small = v.inv2 != nullptr;
     if (whole && small) return launch_cluster2(h, top, 7, rhs, out);
-    if (!whole || top == 0) {
+    // the finest level's first and last pass take the caller's vectors and stay outside the graph
+    const unsigned gf = g1((long long)v.lv[fine].n * v.lv[fine].n / 2);
+    if (!whole) {
+        k2v_sweep_in<<<gf, TPB, 0, h->st>>>(v, rhs);
+        STG_LAUNCH_CK();
+    } else if (top == 0) {
         k2v_in<<<gs, TPB, 0, h->st>>>(v, rhs);
         STG_LAUNCH_CK();
     }
@@ -1091,8 +1142,10 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
         for (int i = fine; i > top; i--) {
             const Lv2 &L = v.lv[i], &C = v.lv[i - 1];
             const unsigned gb = g1((long long)L.n * L.n / 2);
-            k2v_sweep<false, false><<<gb, TPB, 0, h->st>>>(L, 0, nullptr, C, nullptr, L.xa);
-            STG_LAUNCH_CK();
+            if (i < fine) {
+                k2v_sweep<false, false><<<gb, TPB, 0, h->st>>>(L, 0, nullptr, C, nullptr, L.xa);
+                STG_LAUNCH_CK();
+            }
             k2v_sweep<true, false><<<gb, TPB, 0, h->st>>>(L, 1, L.xa, C, nullptr, L.xb);
             STG_LAUNCH_CK();
             k2v_restrict<<<g1((long long)L.n * L.n), TPB, 0, h->st>>>(L, L.xb, C);
@@ -1111,8 +1164,10 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
             const unsigned gb = g1((long long)L.n * L.n / 2);
             k2v_sweep<true, true><<<gb, TPB, 0, h->st>>>(L, 1, L.xb, C, i == 1 ? C.xa : C.xb, L.xa);
             STG_LAUNCH_CK();
-            k2v_sweep<true, false><<<gb, TPB, 0, h->st>>>(L, 0, L.xa, C, nullptr, L.xb);
-            STG_LAUNCH_CK();
+            if (i < fine) {
+                k2v_sweep<true, false><<<gb, TPB, 0, h->st>>>(L, 0, L.xa, C, nullptr, L.xb);
+                STG_LAUNCH_CK();
+            }
         }
         return STG_OK;
     };
@@ -1124,7 +1179,10 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
     }
     // the vol of the levels is a kernel argument: part of the key through a counter of changes
     STG_TRY(graphed(h, h->vgraph, 2 + 2 * (long long)h->vol2d_changes + (v.inv == h->c2->aug0 + v.nd), body, [](bool) {}));
-    k2v_out<<<gs, TPB, 0, h->st>>>(v, out);
+    if (!whole)
+        k2v_sweep_out<<<gf, TPB, 0, h->st>>>(v, out);
+    else
+        k2v_out<<<gs, TPB, 0, h->st>>>(v, out);
     STG_LAUNCH_CK();
     return STG_OK;
 }
