@@ -143,6 +143,7 @@ struct stg_ctx {
     // design loop
     double *d_design = nullptr, *d_phys = nullptr, *d_sens = nullptr, *d_sens_design = nullptr, *d_vw = nullptr,
            *d_tmp = nullptr, *d_gauss = nullptr, *d_parts = nullptr, *d_wsum = nullptr;
+    size_t nparts = 0;  // doubles of d_parts
     double vw_rmin = -1.0;
     const double* phys_used = nullptr;
     // fine vector length in float4 / d4 units and the per-dimension hooks of solve_core

@@ -208,10 +208,11 @@ int sensitivity(cudaStream_t st, const Geom& g, const double* rho, const stg_alp
 // dim 2: cells (i,j) -> i*n + j; dim 3: (i*n + j)*n + k. W: scratch of n^dim doubles
 // (receives the row sums W_i, for the transpose in_i / W_i).
 int density_filter(cudaStream_t st, int dim, int n, double rmin, const double* in, double* out, int transpose, double* W);
-// The whole OC update (bracket, bisection, x_new) in one launch; parts: two buffers of up to
-// 1216 block partials; lambda_out: one device double. xnew is not x (it holds scratch).
+// The whole OC update (bracket, bisection, x_new) in one launch; parts: nparts doubles for block
+// sums, enough for every form with OC_PARTS (oc_form.h; fewer than the launch takes are refused);
+// lambda_out: one device double. xnew is not x (it holds scratch).
 int oc_update_device(cudaStream_t st, int ncell, const double* x, const double* dc, const double* vw, double frac,
-                     double move, double lo, double hi, double* xnew, double* parts, double* lambda_out);
+                     double move, double lo, double hi, double* xnew, double* parts, size_t nparts, double* lambda_out);
 int density_noise(cudaStream_t st, int dim, int n, uint64_t seed, const double* w, int R, double* out, double* tmp);
 
 }  // namespace stg

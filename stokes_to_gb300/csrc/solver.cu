@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "oc_form.h"
 
 namespace stg {
 
@@ -1013,9 +1014,10 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
         }
     }
     const size_t nres = 2 * ((size_t)h->m + 2) + 8;
+    h->nparts = (size_t)nparts + OC_PARTS;
     if ((rc = dalloc(&h->dscr, 1216 * 18)) || (rc = dalloc(&h->dh, nres)) || (rc = dalloc(&h->dcount, 1)) ||
         (rc = dalloc(&h->dsig2, h->m + 2)) ||
-        (rc = dalloc(&h->dy, h->m + 1)) || (rc = dalloc(&h->d_parts, (size_t)nparts + 1216)) || (rc = dalloc(&h->dflag, 1)))
+        (rc = dalloc(&h->dy, h->m + 1)) || (rc = dalloc(&h->d_parts, h->nparts)) || (rc = dalloc(&h->dflag, 1)))
         return fail(rc);
     h->dnrm = h->dh + (nres - 8);
     if (cudaHostAlloc((void**)&h->hres, sizeof(double) * nres, cudaHostAllocMapped) != cudaSuccess)
@@ -1459,9 +1461,9 @@ int stg_oc_update(stg_t* h, double rmin, const double* x, const double* dc, doub
     }
     // the multiplier grows with the sensitivities (with the objective, i.e. with the grid:
     // above 1e9 at 512^3): the bracket is widened by decades until its upper end
-    // undershoots, then bisected - all of it in one cooperative launch, with no host
-    // round trip per multiplier step
-    STG_TRY(oc_update_device(h->st, nc, h->d_design, ddc, h->d_vw, frac, move, lo, hi, h->d_tmp, h->d_parts, h->dnrm));
+    // undershoots, then bisected - all of it in one launch, with no host round trip per
+    // multiplier step
+    STG_TRY(oc_update_device(h->st, nc, h->d_design, ddc, h->d_vw, frac, move, lo, hi, h->d_tmp, h->d_parts, h->nparts, h->dnrm));
     STG_CK(cudaMemcpyAsync(h->d_design, h->d_tmp, sizeof(double) * h->ncell, cudaMemcpyDeviceToDevice, h->st));
     if (x_new) STG_CK(cudaMemcpyAsync(x_new, h->d_design, sizeof(double) * h->ncell, cudaMemcpyDeviceToHost, h->st));
     double lmid = 0;

@@ -12,6 +12,7 @@
 #include "alpha.cuh"
 #include "kernels.h"
 #include "oc.cuh"
+#include "oc_form.h"
 #include "stencil.cuh"
 
 namespace stg {
@@ -168,12 +169,6 @@ __global__ void k_blur(int n, long long nc, long long stride, const double* __re
 // - 1 / sqrt(l) of both possible next probes is formed while the blocks' sums travel.
 // Before and after, an update: 64^2 cells 271 us, now 112; 64^3 1010 us, now 299 (cells in
 // registers); 128^3 4.41 ms, now 1.71 (cells read for each probe).
-constexpr int OC_CB = 16;          // blocks of the cluster form
-constexpr int OC_CR = 8, OC_GR = 16;  // cells a thread holds, cluster and grid form
-constexpr int OC_MAX_BLOCKS = 1216;
-template <int R>
-constexpr int OC_T = R ? 128 : 512;
-constexpr int OC_CLUSTER_MAX = OC_CB * OC_T<OC_CR> * OC_CR;
 
 // The bracket; every warp has the same sums and takes the same steps.
 struct OcBracket {
@@ -279,13 +274,13 @@ __global__ void __launch_bounds__(OC_T<R>) k_oc_bisect(int ncell, const double* 
             __syncthreads();
             if (threadIdx.x == 0) {
                 for (int w = 0; w < W; w++) v += sum[buf][w];
-                part[buf * OC_MAX_BLOCKS + rank] = v;
+                part[buf * nblk + rank] = v;
                 v = 0.0;
             }
             auto token = grid.barrier_arrive();
             tc = rsqrt(br.candidate(lane == 1));
             grid.barrier_wait(std::move(token));
-            for (int p = lane; p < nblk; p += 32) v += part[buf * OC_MAX_BLOCKS + p];
+            for (int p = lane; p < nblk; p += 32) v += part[buf * nblk + p];
         }
         const bool over = warp_sum(v) > target;
         t = __shfl_sync(0xffffffffu, tc, over ? 1 : 0);
@@ -339,47 +334,45 @@ int density_filter(cudaStream_t st, int dim, int n, double rmin, const double* i
 }
 
 int oc_update_device(cudaStream_t st, int ncell, const double* x, const double* dc, const double* vw, double frac,
-                     double move, double lo, double hi, double* xnew, double* parts, double* lambda_out) {
+                     double move, double lo, double hi, double* xnew, double* parts, size_t nparts, double* lambda_out) {
     double target = frac * ncell;
     void* args[] = {&ncell, &x, &dc, &vw, &target, &move, &lo, &hi, &xnew, &parts, &lambda_out};
-    // one cluster while its threads hold at most eight cells each: a cluster barrier is 0.3 us and
-    // one over the device 1.3, but the cells of a probe take 1.3 us of sixteen SMs' FP64 units at
-    // the line (16384 cells: 178 us an update) and next to none of all of them
-    const void* kernel = (const void*)k_oc_bisect<true, OC_CR>;
-    if (ncell <= OC_CLUSTER_MAX) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(OC_CB);
-        cfg.blockDim = dim3(OC_T<OC_CR>);
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = OC_CB;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) {
-            STG_CK(cudaLaunchKernelExC(&cfg, kernel, args));
-            return STG_OK;
-        }
-        cudaGetLastError();
-    }
-    // as many blocks as have cells, one on each SM
     int dev = 0, sms = 0, per_sm = 0;
     STG_CK(cudaGetDevice(&dev));
     STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (sms > OC_MAX_BLOCKS) sms = OC_MAX_BLOCKS;
-    const bool held = ncell <= (long long)sms * OC_T<OC_GR> * OC_GR;
-    const int threads = held ? OC_T<OC_GR> : OC_T<0>;
-    kernel = held ? (const void*)k_oc_bisect<false, OC_GR> : (const void*)k_oc_bisect<false, 0>;
-    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(OC_CB);
+    cfg.blockDim = dim3(OC_T<OC_CR>);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = OC_CB;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const void* kernel = (const void*)k_oc_bisect<true, OC_CR>;
+    int clusters = 0;
+    if (ncell <= OC_CLUSTER_MAX && (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+                                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess)) {
+        clusters = 0;
+        cudaGetLastError();
+    }
+    const OcForm f = oc_form(ncell, sms, clusters > 0);
+    if ((size_t)f.parts() > nparts) {
+        set_error("oc_update_device: %d block sums in an array of %zu", f.parts(), nparts);
+        return STG_E_INVALID;
+    }
+    if (f.cluster) {
+        STG_CK(cudaLaunchKernelExC(&cfg, kernel, args));
+        return STG_OK;
+    }
+    kernel = f.held ? (const void*)k_oc_bisect<false, OC_GR> : (const void*)k_oc_bisect<false, 0>;
+    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, f.threads, 0));
     if (per_sm < 1) {
         set_error("the OC bisection kernel cannot be made resident");
         return STG_E_CUDA;
     }
-    const unsigned g = (unsigned)std::min(((long long)ncell + threads - 1) / threads, (long long)sms);
-    STG_CK(cudaLaunchCooperativeKernel(kernel, dim3(g), dim3(threads), args, 0, st));
+    STG_CK(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)f.blocks), dim3((unsigned)f.threads), args, 0, st));
     return STG_OK;
 }
 
