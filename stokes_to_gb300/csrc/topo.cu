@@ -282,7 +282,8 @@ __global__ void __launch_bounds__(OC_T<R>) k_oc_bisect(int ncell, const double* 
             grid.barrier_wait(std::move(token));
             for (int p = lane; p < nblk; p += 32) v += part[buf * nblk + p];
         }
-        const bool over = warp_sum(v) > target;
+        v = warp_sum(v);
+        const bool over = br.widen ? !(v <= target) : v > target;  // (a NaN target: the least design)
         t = __shfl_sync(0xffffffffu, tc, over ? 1 : 0);
         more = br.step(over);
     }

@@ -26,3 +26,15 @@ def test_oc_update_between_the_cluster_and_full_grids(stg, dim, n):
     assert abs(lam - ref_lam) <= 2e-9 * ref_lam
     assert np.max(np.abs(xn.ravel() - ref)) <= 1e-9
     assert lam2 == lam and np.array_equal(again, xn)
+
+
+@pytest.mark.parametrize("dim,n", [(3, 8), (3, 32), (2, 160)])
+def test_volume_that_cannot_be_compared_keeps_widening(stg, dim, n):
+    """A NaN fraction: no volume undershoots it, so the bracket is widened to its end (60
+    decades past 1e9) and bisected down to its lower one, and the design falls as far as it may."""
+    x = 0.05 + 0.9 * np.random.default_rng(n).random((n,) * dim)
+    s = stg.Solver(n, dim=dim)
+    xn, lam = s.oc_update(1.5, x, -np.ones((n,) * dim), float("nan"))
+    s.close()
+    assert abs(lam / 1e68 - 1.0) < 1e-8
+    assert np.max(np.abs(xn - np.maximum(0.0, x - 0.2))) <= 1e-30  # x sqrt(ncell / 1e68) at most
