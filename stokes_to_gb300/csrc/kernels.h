@@ -208,6 +208,9 @@ int sensitivity(cudaStream_t st, const Geom& g, const double* rho, const stg_alp
 // dim 2: cells (i,j) -> i*n + j; dim 3: (i*n + j)*n + k. W: scratch of n^dim doubles
 // (receives the row sums W_i, for the transpose in_i / W_i).
 int density_filter(cudaStream_t st, int dim, int n, double rmin, const double* in, double* out, int transpose, double* W);
+// Its launch form on the current device (oc_form.h)
+struct OcForm;
+int oc_form_here(long long ncell, OcForm* f);
 // The whole OC update (bracket, bisection, x_new) in one launch; parts: nparts doubles for block
 // sums, enough for every form with OC_PARTS (oc_form.h; fewer than the launch takes are refused);
 // lambda_out: one device double. xnew is not x (it holds scratch).

@@ -5,7 +5,7 @@ namespace stg {
 
 constexpr int OC_CB = 16;             // blocks of the cluster form
 constexpr int OC_CR = 8, OC_GR = 16;  // cells a thread holds, cluster and grid form
-constexpr int OC_MAX_BLOCKS = 608;    // blocks of the grid form at most
+constexpr int OC_MAX_BLOCKS = 304;    // blocks of the grid form at most
 // Doubles of block sums that an update needs at most: two buffers, so that a probe never
 // overwrites the sums that the previous one's reduction still reads.
 constexpr int OC_PARTS = 2 * OC_MAX_BLOCKS;

@@ -1014,7 +1014,8 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
         }
     }
     const size_t nres = 2 * ((size_t)h->m + 2) + 8;
-    h->nparts = (size_t)nparts + OC_PARTS;
+    h->nparts = (size_t)nparts + 1216;  // the passes over whole vectors have up to 1216 blocks
+    static_assert(OC_PARTS <= 1216, "block sums of the OC update");
     if ((rc = dalloc(&h->dscr, 1216 * 18)) || (rc = dalloc(&h->dh, nres)) || (rc = dalloc(&h->dcount, 1)) ||
         (rc = dalloc(&h->dsig2, h->m + 2)) ||
         (rc = dalloc(&h->dy, h->m + 1)) || (rc = dalloc(&h->d_parts, h->nparts)) || (rc = dalloc(&h->dflag, 1)))

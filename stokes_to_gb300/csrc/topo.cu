@@ -202,12 +202,6 @@ struct OcBracket {
     }
 };
 
-// What a probe needs of a cell, formed once.
-struct OcCell {
-    double s, lo, hi, vw;
-    __device__ __forceinline__ double volume(double t) const { return vw * fmin(hi, fmax(lo, s * t)); }
-};
-
 // The update by the blocks of one cluster (CLUSTER: at most OC_CLUSTER_MAX cells; each warp's
 // sum goes straight into every block's shared memory) or of a cooperative launch (through part).
 // Both have two buffers of sums, so that a probe never overwrites those that the previous one's
@@ -235,10 +229,7 @@ __global__ void __launch_bounds__(OC_T<R>) k_oc_bisect(int ncell, const double* 
         for (int r = 0; r < R; r++) {
             const long long q = q0 + r * dq;
             c[r] = OcCell{0.0, 0.0, 0.0, 0.0};
-            if (q < ncell) {
-                const double xi = x[q], w = vw[q];
-                c[r] = OcCell{oc_scale(xi, dc[q], w * inv_n), fmax(lo, xi - move), fmin(hi, xi + move), w};
-            }
+            if (q < ncell) c[r] = oc_cell(x[q], dc[q], vw[q], inv_n, move, lo, hi);
         }
     } else {
         for (long long q = q0; q < ncell; q += dq) xnew[q] = oc_scale(x[q], dc[q], vw[q] * inv_n);
@@ -253,12 +244,12 @@ __global__ void __launch_bounds__(OC_T<R>) k_oc_bisect(int ncell, const double* 
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 if (r == held) break;
-                acc += c[r].volume(t);
+                acc = c[r].add(t, acc);
             }
         } else {
             for (long long q = q0; q < ncell; q += dq) {
                 const double xi = x[q];
-                acc += OcCell{xnew[q], fmax(lo, xi - move), fmin(hi, xi + move), vw[q]}.volume(t);
+                acc = OcCell{xnew[q], fmax(lo, xi - move), fmin(hi, xi + move), vw[q]}.add(t, acc);
             }
         }
         acc = warp_sum(acc);
@@ -334,40 +325,55 @@ int density_filter(cudaStream_t st, int dim, int n, double rmin, const double* i
     return STG_OK;
 }
 
-int oc_update_device(cudaStream_t st, int ncell, const double* x, const double* dc, const double* vw, double frac,
-                     double move, double lo, double hi, double* xnew, double* parts, size_t nparts, double* lambda_out) {
-    double target = frac * ncell;
-    void* args[] = {&ncell, &x, &dc, &vw, &target, &move, &lo, &hi, &xnew, &parts, &lambda_out};
-    int dev = 0, sms = 0, per_sm = 0;
-    STG_CK(cudaGetDevice(&dev));
-    STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+static cudaLaunchConfig_t oc_cluster(cudaStream_t st, cudaLaunchAttribute (&at)[1]) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(OC_CB);
     cfg.blockDim = dim3(OC_T<OC_CR>);
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = OC_CB;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const void* kernel = (const void*)k_oc_bisect<true, OC_CR>;
-    int clusters = 0;
-    if (ncell <= OC_CLUSTER_MAX && (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-                                    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess)) {
-        clusters = 0;
-        cudaGetLastError();
+    return cfg;
+}
+
+int oc_form_here(long long ncell, OcForm* f) {
+    int dev = 0, sms = 0, clusters = 0;
+    STG_CK(cudaGetDevice(&dev));
+    STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (ncell <= OC_CLUSTER_MAX) {
+        const void* kernel = (const void*)k_oc_bisect<true, OC_CR>;
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = oc_cluster(nullptr, at);
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
+            clusters = 0;
+            cudaGetLastError();
+        }
     }
-    const OcForm f = oc_form(ncell, sms, clusters > 0);
+    *f = oc_form(ncell, sms, clusters > 0);
+    return STG_OK;
+}
+
+int oc_update_device(cudaStream_t st, int ncell, const double* x, const double* dc, const double* vw, double frac,
+                     double move, double lo, double hi, double* xnew, double* parts, size_t nparts, double* lambda_out) {
+    double target = frac * ncell;
+    void* args[] = {&ncell, &x, &dc, &vw, &target, &move, &lo, &hi, &xnew, &parts, &lambda_out};
+    OcForm f;
+    STG_TRY(oc_form_here(ncell, &f));
     if ((size_t)f.parts() > nparts) {
         set_error("oc_update_device: %d block sums in an array of %zu", f.parts(), nparts);
         return STG_E_INVALID;
     }
     if (f.cluster) {
-        STG_CK(cudaLaunchKernelExC(&cfg, kernel, args));
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = oc_cluster(st, at);
+        STG_CK(cudaLaunchKernelExC(&cfg, (const void*)k_oc_bisect<true, OC_CR>, args));
         return STG_OK;
     }
-    kernel = f.held ? (const void*)k_oc_bisect<false, OC_GR> : (const void*)k_oc_bisect<false, 0>;
+    int per_sm = 0;
+    const void* kernel = f.held ? (const void*)k_oc_bisect<false, OC_GR> : (const void*)k_oc_bisect<false, 0>;
     STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, f.threads, 0));
     if (per_sm < 1) {
         set_error("the OC bisection kernel cannot be made resident");
