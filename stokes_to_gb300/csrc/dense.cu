@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(TPB) k_gj_all(int nd, double* a, double* b, in
 //
 // Bound: the FP64 pipe, two FMAs per SM and clock, at nd = 2112 (set-up of a 96^2 handle: 276 ms
 // pivoted, 14.6 with full square updates and FP64 tile inverses, 8.2 now); at nd = 304 the chain
-// of 10 steps of about 25 us (whole set-up of a 16^3 handle 2.2 ms pivoted, 0.36 now). Tile
+// of 10 steps of about 25 us (whole set-up of a 16^3 handle 2.2 ms pivoted, 0.36 now); at
+// nd = 7344 (12^3: grids of 24, 48, 96) the set-up takes 0.173 s, 10.95 pivoted. Tile
 // width: 16 keeps the chain of small inversions short, 32 halves the panel traffic where the
 // products dominate.
 
@@ -356,6 +357,15 @@ __device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[
     return ok;
 }
 
+// Shared memory of a block: 59 KB for 32-wide tiles of three axes, so it is dynamic (a kernel's own
+// declaration ends at 48 KB)
+template <int B, int S>
+struct InvShared {
+    double D[S][B][B + 1], E[B][B + 1], A[B][B + 1];
+    float H[S][B][B + 1], F[B][B + 1];
+    int bad;
+};
+
 // perm[q], q < N: the unknown at position q, -1 for a decoupled filler, -2 for l. The
 // positions hold S face sections of TF tiles each (one axis a section), then the cells' tiles.
 // ws: N^2 + 3 S B N doubles (the pivoted elimination's second buffer).
@@ -364,9 +374,13 @@ __global__ void __launch_bounds__(TPB) k_inv_blocks(int nd, int N, int TF, const
                                                     double* ws, int* info) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    __shared__ double sD[S][B][B + 1], sE[B][B + 1], sA[B][B + 1];
-    __shared__ float sH[S][B][B + 1], sF[B][B + 1];
-    __shared__ int s_bad;
+    extern __shared__ __align__(16) unsigned char inv_window[];
+    InvShared<B, S>& W = *reinterpret_cast<InvShared<B, S>*>(inv_window);
+    auto& sD = W.D;
+    auto &sE = W.E, &sA = W.A;
+    auto& sH = W.H;
+    auto& sF = W.F;
+    int& s_bad = W.bad;
     const int T = N / B, tid = threadIdx.x, TC = S * TF, cell0 = TC * B;
     constexpr int EPT = B * B / TPB;  // tile elements of a thread: rows r0 + e (TPB / B), column c0
     const int c0 = tid % B, r0 = tid / B;
@@ -774,7 +788,10 @@ int inv_blocks(cudaStream_t st, int nd, const InvOrder& O, int closed, double* a
     STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const void* fn = O.S == 3 ? (B == 16 ? (const void*)k_inv_blocks<16, 3> : (const void*)k_inv_blocks<32, 3>)
                               : (B == 16 ? (const void*)k_inv_blocks<16, 2> : (const void*)k_inv_blocks<32, 2>);
-    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, 0));
+    const size_t smem = O.S == 3 ? (B == 16 ? sizeof(InvShared<16, 3>) : sizeof(InvShared<32, 3>))
+                                 : (B == 16 ? sizeof(InvShared<16, 2>) : sizeof(InvShared<32, 2>));
+    STG_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, smem));
     // the pivoted elimination leaves its result in the first buffer for an even nd (the cells
     // and padded faces of a grid whose size is a multiple of 4 are always even in number)
     const bool fits = (long long)N * N + 3ll * O.S * B * N <= 2ll * nd * nd && (nd & 1) == 0;
@@ -783,7 +800,7 @@ int inv_blocks(cudaStream_t st, int nd, const InvOrder& O, int closed, double* a
     const int T = N / B, tiles = T * (T + 1) / 2, g = tiles < sms ? tiles : sms;
     const int* perm = O.perm;
     void* args[] = {&nd, &N, &TF, &perm, &closed, &a, &b, &info};
-    STG_CK(cudaLaunchCooperativeKernel(fn, dim3((unsigned)g), dim3(TPB), args, 0, st));
+    STG_CK(cudaLaunchCooperativeKernel(fn, dim3((unsigned)g), dim3(TPB), args, smem, st));
     add_launches(1);
     *inv = a + nd;
     return STG_OK;
