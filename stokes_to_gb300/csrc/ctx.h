@@ -148,6 +148,7 @@ struct stg_ctx {
     const double* phys_used = nullptr;
     // fine vector length in float4 / d4 units and the per-dimension hooks of solve_core
     long long n4 = 0;
+    int coarsest = 0;  // unknowns of the coarsest inverse
     int (*setup)(stg_t*) = nullptr;
     int (*resid64)(stg_t*, const stg::d4* b, const stg::d4* x, stg::d4* r, double* nrm2_host) = nullptr;
     int (*precond)(stg_t*, const float4* rhs, float4* out) = nullptr;

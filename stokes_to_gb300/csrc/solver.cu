@@ -249,7 +249,8 @@ bool fuse_pair(const stg_t* h, const Level& L) {
 
 // ... and the two after the coarse correction, up to 64 cells an axis (sweep.cu, MODE 4): two launches
 // against one take 17.4 and 15.8 us at 64^3, 9.6 and 8.0 at 32^3, with the gap between them another
-// 1 us; but 59 and 66 at 128^3, 377 and 420 at 256^3, where two blocks an SM overlap too little.
+// 1 us (a solve's Krylov part at 48^3 3.41 and 3.36 ms); but 59 and 66 at 128^3, 377 and 420 at 256^3,
+// where two blocks an SM overlap too little. At 96^3 it is even (6.29 ms either way).
 constexpr int POST_PAIR_N = 64;
 bool fuse_post(const stg_t* h, const Level& L) { return fuse_pair(h, L) && L.g.n <= POST_PAIR_N; }
 
@@ -410,10 +411,14 @@ int vcycle(stg_t* h, const float4* rhs) {
 
 // ---------------------------------------------------------------- FP64 refinement + FGMRES
 // Finest slots (quarters of the unknowns) up to which the next V-cycle is launched ahead of the
-// host's wait. 16^3 (6.9e3): a solve 1.20 -> 1.15 ms, 64^2 (3.3e3): a design step 5 % faster;
-// from 64^3 (3.0e5) and 512^2 (2.0e5) on the V-cycles lost at the end of a refinement step cost
-// what the others gain (1 % either way there, 128^3 3 % slower).
+// host's wait: a solve without it and with it takes 1163 and 1090 us at 16^3 (6.9e3 slots), 1823 and
+// 1761 at 32^3 (4.4e4), 1600 and 1546 at 64^2 (3.3e3), 2839 and 2819 at 256^2 (5.0e4); from 512^2
+// (2.0e5: 4026 and 4078) and 64^3 (3.0e5: 3345 and 3308) on the V-cycles lost at the end of a
+// refinement step cost what the others gain (128^3 3 % slower). And coarsest unknowns up to
+// which: the product of a large coarsest inverse makes every V-cycle long, and the lost one with it
+// (24^3, 7344 unknowns: the Krylov part 2.60 and 2.66 ms; 192^2, 2112: 1.92 and 1.94).
 constexpr long long AHEAD_SLOTS = 1 << 16;
+constexpr int AHEAD_COARSEST = 512;
 int residual64(stg_t* h, const d4* b, const d4* x, d4* r, double* nrm2_host) {
     Level& F = fine(h);
     int nb = 0;
@@ -635,7 +640,8 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
         // when the last reduction would reach the target once more, nor where a V-cycle takes
         // longer than what a step can gain (AHEAD_SLOTS). A vector that a second projection or a
         // rescaling changes gets its V-cycle again.
-        const bool can_ahead = !predict && !h->net_on && !h->gen && !h->prof.on && n4 <= AHEAD_SLOTS;
+        const bool can_ahead = !predict && !h->net_on && !h->gen && !h->prof.on && n4 <= AHEAD_SLOTS &&
+                               h->coarsest <= AHEAD_COARSEST;
         bool ahead = false;  // Z[j]'s V-cycle is on its way
         double last_est = beta;
         for (int j = 0; j < msteps; j++) {
@@ -969,6 +975,7 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
     }
     if (dim == 3) {
         if ((rc = dense_init(h->dense, h->lv[0].g))) return fail(rc);
+        h->coarsest = h->dense.nd;
         Level& F = fine(h);
         h->n4 = (long long)F.g.nslot;
         h->setup = update;

@@ -1255,6 +1255,7 @@ int create2d(stg_t* h) {
         set_error("N = %d leaves a %d-unknown coarsest level (N / 8 must have a larger power-of-two factor)", n, nd);
         return STG_E_UNSUPPORTED;
     }
+    h->coarsest = nd;
     STG_TRY(dalloc(&h->c2->aug0, 2ull * nd * nd));
     STG_TRY(dalloc(&h->c2->aug1, 2ull * nd * nd));
     STG_TRY(dalloc(&h->c2->info, 1));
