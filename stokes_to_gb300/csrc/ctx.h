@@ -93,11 +93,10 @@ struct stg_ctx {
     bool gen = false;
     stg::d4* gtmp[3] = {nullptr, nullptr, nullptr};
     bool fixed_cells2d = false;  // 2D: the boundary fixes cells (identity rows among the pressures)
-    // 2D: the boundary admits the Laplacian form (solver2d.cu vcycle2_lap); the free faces' vol,
-    // and how often set_boundary changed it (captured graphs hold it)
+    // 2D: the boundary admits the Laplacian form (solver2d.cu vcycle2_lap); the free faces' vol
     bool lap2d = false;
     double vol2d = 1.0;
-    int vol2d_changes = 0;
+    int vol_changes = 0;  // how often set_boundary changed the vol, which captured graphs hold
     // the coarse levels hold the solver's own penalties (flow rule of kernels.cu k_coarsen)
     // rather than the reference's sums, which the component adapters reproduce
     bool hier_flow = false;

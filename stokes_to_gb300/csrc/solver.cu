@@ -175,7 +175,7 @@ int update(stg_t* h) {
     // replayed as a CUDA graph; its inversion is one cooperative launch
     GraphCache& G = h->sgraph;
     PROF(h, 8, 0.0,
-         graphed(h, G, h->closed ? 2 : 1,
+         graphed(h, G, (h->closed ? 2 : 1) + 4ll * h->vol_changes,
                  [&] {
                      return dense_setup(h->st, h->dense, h->lv[0].g, h->lv[0].vol, h->lv[0].m, h->lv[0].P64, h->closed ? 1 : 0,
                                         false);
@@ -373,7 +373,7 @@ int coarse_cycle(stg_t* h) {
     const long long key = (long long)per | ((long long)(h->opts.method == STG_METHOD_MIXED) << 3) |
                           ((long long)fast(h, h->lv[top]) << 4) | ((long long)(h->dense.inv == h->dense.Ainv) << 5) |
                           ((long long)h->L << 6) | ((long long)h->reference_cycle << 12) |  // adapters: FP32 sweeps
-                          ((long long)(h->opts.prolong == 1) << 13);
+                          ((long long)(h->opts.prolong == 1) << 13) | ((long long)h->vol_changes << 14);
     GraphCache& G = h->boost && !h->reference_cycle ? h->vgraph_boost : h->vgraph;
     return graphed(h, G, key, [&] { return vcycle_levels(h, top, nullptr); },
                    [&](bool save) {
@@ -1166,7 +1166,7 @@ int stg_set_boundary(stg_t* h, const double* cell_vol, const int32_t* cell_fixed
         h->lap2d = lap && !std::isnan(fv);
         if (h->lap2d && fv != h->vol2d) {
             h->vol2d = fv;
-            h->vol2d_changes++;
+            h->vol_changes++;
         }
         STG_TRY(set_boundary2d(h, dc, cell_fixed ? ist : nullptr, df[0], df[1], ist + h->ncell, ist + h->ncell + h->nface));
         h->closed = closed != 0;
@@ -1215,7 +1215,9 @@ int stg_set_boundary(stg_t* h, const double* cell_vol, const int32_t* cell_fixed
     h->lap_ok = bnd_fixed && !gen;
     double cv = cell_vol ? cell_vol[0] : 1.0;
     Level& F = fine(h);
-    F.vol = std::isnan(v) ? 0.0 : v;
+    if (std::isnan(v)) v = 0.0;
+    if (F.vol != v) h->vol_changes++;
+    F.vol = v;
     F.cell_vol = cv;
     int* ist = h->istage;
     const int* fi[3];

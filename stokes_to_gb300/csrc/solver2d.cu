@@ -1178,7 +1178,7 @@ int vcycle2_lap(stg_t* h, const float* rhs, float* out) {
         return launch_cluster2(h, top, 4, nullptr, out);
     }
     // the vol of the levels is a kernel argument: part of the key through a counter of changes
-    STG_TRY(graphed(h, h->vgraph, 2 + 2 * (long long)h->vol2d_changes + (v.inv == h->c2->aug0 + v.nd), body, [](bool) {}));
+    STG_TRY(graphed(h, h->vgraph, 2 + 2 * (long long)h->vol_changes + (v.inv == h->c2->aug0 + v.nd), body, [](bool) {}));
     if (!whole)
         k2v_sweep_out<<<gf, TPB, 0, h->st>>>(v, out);
     else
