@@ -134,6 +134,7 @@ struct stg_ctx {
     // dh (2 (m + 2) dots) and dnrm (8 norms) are one array, mirrored in pinned host memory by
     // the kernels that reduce into it
     double* hres = nullptr;
+    int* hflags = nullptr;  // two more words of it, for set_boundary2d
     unsigned* dcount = nullptr;
     // host-order staging (cells + 3 face arrays)
     double* stage = nullptr;
@@ -176,7 +177,7 @@ void destroy2d(stg_t* h);
 long long dof2d(const stg_t* h, int level);
 int level_n2d(const stg_t* h, int level);
 int set_boundary2d(stg_t* h, const double* cvol, const int* cfix, const double* fv0, const double* fv1, const int* ff0,
-                   const int* ff1);
+                   const int* ff1, double fv, bool* fixed_cells, bool* uniform);
 int set_penalty2d(stg_t* h, const double* cp, const double* f0, const double* f1);
 int set_density2d(stg_t* h, const double* rho, const stg_alpha& law);
 int field_to_vec2d(stg_t* h, const double* cell, const double* f0, const double* f1, d4* out);

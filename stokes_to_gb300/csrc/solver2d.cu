@@ -299,29 +299,41 @@ __global__ void k2_coarsen(G2d gc, G2d gf, const uint8_t* __restrict__ ff, const
     cpen32[t] = (float)p;
 }
 
-// fine descriptor from Field-order host inputs (staged on the device)
+// fine descriptor from Field-order host inputs (staged on the device). flags (pinned host memory):
+// flags[0] becomes 1 when a cell is fixed, flags[1] when a face on the domain boundary is free or a
+// free face's vol is not fv
 __global__ void k2_fine_descr(G2d g, const double* __restrict__ cvol, const int* __restrict__ cfix, const double* __restrict__ fv0,
-                              const double* __restrict__ fv1, const int* __restrict__ ff0, const int* __restrict__ ff1,
-                              uint8_t* __restrict__ fixed, double* __restrict__ vol) {
+                              const double* __restrict__ fv1, const int* __restrict__ ff0, const int* __restrict__ ff1, double fv,
+                              uint8_t* __restrict__ fixed, double* __restrict__ vol, int* __restrict__ flags) {
     int t = blockIdx.x * TPB + threadIdx.x;
-    if (t >= g.size()) return;
-    int kind, x, y;
-    g.decode(t, kind, x, y);
-    const int n = g.n;
-    uint8_t f = 0;
-    double v = 0;
-    if (kind < 0) {
-        f = cfix ? (cfix[x * n + y] != 0) : 0;
-        v = cvol ? cvol[x * n + y] : 0.0;
-    } else if (g.face_ok(x, y, kind)) {
-        int idx = kind == 0 ? x * n + y : x * (n + 1) + y;
-        f = (kind == 0 ? ff0 : ff1)[idx] != 0;
-        v = (kind == 0 ? fv0 : fv1)[idx];
-    } else {
-        f = 1;
+    bool cell_fixed = false, uneven = false;
+    if (t < g.size()) {
+        int kind, x, y;
+        g.decode(t, kind, x, y);
+        const int n = g.n;
+        uint8_t f = 0;
+        double v = 0;
+        if (kind < 0) {
+            f = cfix ? (cfix[x * n + y] != 0) : 0;
+            v = cvol ? cvol[x * n + y] : 0.0;
+            cell_fixed = f;
+        } else if (g.face_ok(x, y, kind)) {
+            int idx = kind == 0 ? x * n + y : x * (n + 1) + y;
+            f = (kind == 0 ? ff0 : ff1)[idx] != 0;
+            v = (kind == 0 ? fv0 : fv1)[idx];
+            const int c = kind == 0 ? x : y;
+            uneven = !f && (c == 0 || c == n || !(v == fv));
+        } else {
+            f = 1;
+        }
+        fixed[t] = f;
+        vol[t] = f ? 0.0 : v;
     }
-    fixed[t] = f;
-    vol[t] = f ? 0.0 : v;
+    const int any_fixed = __syncthreads_or(cell_fixed), any_uneven = __syncthreads_or(uneven);
+    if (threadIdx.x == 0) {
+        if (any_fixed) flags[0] = 1;
+        if (any_uneven) flags[1] = 1;
+    }
 }
 
 __global__ void k2_penalty_from_field(G2d g, const double* __restrict__ cp, const double* __restrict__ f0,
@@ -1351,11 +1363,15 @@ int level_n2d(const stg_t* h, int level) { return h->c2->lv[level].g.n; }
 
 // inputs are device staging copies of the Field-order host arrays
 int set_boundary2d(stg_t* h, const double* cvol, const int* cfix, const double* fv0, const double* fv1, const int* ff0,
-                   const int* ff1) {
+                   const int* ff1, double fv, bool* fixed_cells, bool* uniform) {
     Level2& F = fine2(h);
-    k2_fine_descr<<<g1(F.g.size()), TPB, 0, h->st>>>(F.g, cvol, cfix, fv0, fv1, ff0, ff1, F.fixed, F.vol);
+    h->hflags[0] = h->hflags[1] = 0;
+    k2_fine_descr<<<g1(F.g.size()), TPB, 0, h->st>>>(F.g, cvol, cfix, fv0, fv1, ff0, ff1, fv, F.fixed, F.vol, h->hflags);
     STG_LAUNCH_CK();
     STG_TRY(f64_to_f32(h->st, F.g.size() / 4, reinterpret_cast<const d4*>(F.vol), 1.0, reinterpret_cast<float4*>(F.vol32)));
+    STG_CK(cudaStreamSynchronize(h->st));
+    *fixed_cells = h->hflags[0] != 0;
+    *uniform = h->hflags[1] == 0;
     return STG_OK;
 }
 
