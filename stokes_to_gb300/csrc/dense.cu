@@ -252,7 +252,8 @@ __global__ void __launch_bounds__(TPB) k_gj_all(int nd, double* a, double* b, in
 // width: 16 keeps the chain of small inversions short, 32 halves the panel traffic where the
 // products dominate.
 
-// Inverse of an FP64 tile to about 2^-44 in double-float arithmetic by one warp: the FP64 pipe's
+// Inverse of an FP64 tile to about 2^-44 in double-float arithmetic (error-free sums after Knuth,
+// products after Dekker, with an FMA) by one warp: the FP64 pipe's
 // latency makes a pivot of the same elimination cost 1900 clocks, the FP32 pipe's 300. Lane: row
 // lane / LPR, columns CE (lane % LPR) .. in registers. s becomes the inverse, hi its FP32 values.
 struct D2 {
@@ -357,14 +358,26 @@ __device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[
     return ok;
 }
 
-// Shared memory of a block: 59 KB for 32-wide tiles of three axes, so it is dynamic (a kernel's own
-// declaration ends at 48 KB)
+// Shared memory of a block: 59 KB for 32-wide tiles of three axes, which makes it dynamic (a kernel's
+// own declarations end at 48 KB); the others declare their arrays one by one (as members of one
+// struct 6 registers more, and a set-up of 192^2 takes 7.77 instead of 7.73 ms)
 template <int B, int S>
 struct InvShared {
     double D[S][B][B + 1], E[B][B + 1], A[B][B + 1];
     float H[S][B][B + 1], F[B][B + 1];
     int bad;
+    static constexpr size_t dynamic() { return sizeof(InvShared) > 48 * 1024 ? sizeof(InvShared) : 0; }
 };
+template <class W, class T, int ID>  // member `in` of the window W, or array ID of type T of its own
+__device__ __forceinline__ T& inv_array(T W::*in) {
+    extern __shared__ __align__(16) unsigned char inv_window[];
+    if constexpr (W::dynamic() > 0) {
+        return reinterpret_cast<W*>(inv_window)->*in;
+    } else {
+        __shared__ T own;
+        return own;
+    }
+}
 
 // perm[q], q < N: the unknown at position q, -1 for a decoupled filler, -2 for l. The
 // positions hold S face sections of TF tiles each (one axis a section), then the cells' tiles.
@@ -374,13 +387,13 @@ __global__ void __launch_bounds__(TPB) k_inv_blocks(int nd, int N, int TF, const
                                                     double* ws, int* info) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    extern __shared__ __align__(16) unsigned char inv_window[];
-    InvShared<B, S>& W = *reinterpret_cast<InvShared<B, S>*>(inv_window);
-    auto& sD = W.D;
-    auto &sE = W.E, &sA = W.A;
-    auto& sH = W.H;
-    auto& sF = W.F;
-    int& s_bad = W.bad;
+    using W = InvShared<B, S>;
+    auto& sD = inv_array<W, double[S][B][B + 1], 0>(&W::D);
+    auto& sE = inv_array<W, double[B][B + 1], 1>(&W::E);
+    auto& sA = inv_array<W, double[B][B + 1], 2>(&W::A);
+    auto& sH = inv_array<W, float[S][B][B + 1], 3>(&W::H);
+    auto& sF = inv_array<W, float[B][B + 1], 4>(&W::F);
+    int& s_bad = inv_array<W, int, 5>(&W::bad);
     const int T = N / B, tid = threadIdx.x, TC = S * TF, cell0 = TC * B;
     constexpr int EPT = B * B / TPB;  // tile elements of a thread: rows r0 + e (TPB / B), column c0
     const int c0 = tid % B, r0 = tid / B;
@@ -788,9 +801,9 @@ int inv_blocks(cudaStream_t st, int nd, const InvOrder& O, int closed, double* a
     STG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const void* fn = O.S == 3 ? (B == 16 ? (const void*)k_inv_blocks<16, 3> : (const void*)k_inv_blocks<32, 3>)
                               : (B == 16 ? (const void*)k_inv_blocks<16, 2> : (const void*)k_inv_blocks<32, 2>);
-    const size_t smem = O.S == 3 ? (B == 16 ? sizeof(InvShared<16, 3>) : sizeof(InvShared<32, 3>))
-                                 : (B == 16 ? sizeof(InvShared<16, 2>) : sizeof(InvShared<32, 2>));
-    STG_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = O.S == 3 ? (B == 16 ? InvShared<16, 3>::dynamic() : InvShared<32, 3>::dynamic())
+                                 : (B == 16 ? InvShared<16, 2>::dynamic() : InvShared<32, 2>::dynamic());
+    if (smem) STG_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     STG_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TPB, smem));
     // the pivoted elimination leaves its result in the first buffer for an even nd (the cells
     // and padded faces of a grid whose size is a multiple of 4 are always even in number)
