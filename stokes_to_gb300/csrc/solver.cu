@@ -414,11 +414,11 @@ int vcycle(stg_t* h, const float4* rhs) {
 // host's wait: a solve without it and with it takes 1163 and 1090 us at 16^3 (6.9e3 slots), 1823 and
 // 1761 at 32^3 (4.4e4), 1600 and 1546 at 64^2 (3.3e3), 2839 and 2819 at 256^2 (5.0e4); from 512^2
 // (2.0e5: 4026 and 4078) and 64^3 (3.0e5: 3345 and 3308) on the V-cycles lost at the end of a
-// refinement step cost what the others gain (128^3 3 % slower). And coarsest unknowns up to
-// which: the product of a large coarsest inverse makes every V-cycle long, and the lost one with it
-// (24^3, 7344 unknowns: the Krylov part 2.60 and 2.66 ms; 192^2, 2112: 1.92 and 1.94).
-constexpr long long AHEAD_SLOTS = 1 << 16;
-constexpr int AHEAD_COARSEST = 512;
+// refinement step cost what the others gain (128^3 3 % slower). The product of a large coarsest
+// inverse makes every V-cycle longer, and the lost one with it: with 2112 unknowns the line lies lower
+// (48^2 8890 and 8869 us, 96^2 9482 and 9450, 192^2 9867 and 9907), with 5440 and more it never pays (80^2
+// 89.26 and 89.48 ms, 24^3 a Krylov part of 2.60 and 2.66).
+long long ahead_slots(int coarsest) { return coarsest <= 512 ? 1 << 16 : coarsest <= 4096 ? 1 << 13 : 0; }
 int residual64(stg_t* h, const d4* b, const d4* x, d4* r, double* nrm2_host) {
     Level& F = fine(h);
     int nb = 0;
@@ -638,10 +638,9 @@ int solve_core(stg_t* h, const d4* b, d4* x, stg_stats* stats) {
         // on the device, and the host's wait, the small least-squares update and the launches pass
         // while it runs. It is lost when the column ends the refinement step, so it is not sent
         // when the last reduction would reach the target once more, nor where a V-cycle takes
-        // longer than what a step can gain (AHEAD_SLOTS). A vector that a second projection or a
+        // longer than what a step can gain (ahead_slots). A vector that a second projection or a
         // rescaling changes gets its V-cycle again.
-        const bool can_ahead = !predict && !h->net_on && !h->gen && !h->prof.on && n4 <= AHEAD_SLOTS &&
-                               h->coarsest <= AHEAD_COARSEST;
+        const bool can_ahead = !predict && !h->net_on && !h->gen && !h->prof.on && n4 <= ahead_slots(h->coarsest);
         bool ahead = false;  // Z[j]'s V-cycle is on its way
         double last_est = beta;
         for (int j = 0; j < msteps; j++) {
