@@ -70,7 +70,8 @@ __device__ __forceinline__ void block_sums_df(const float (&v)[NV], float2* out)
 }
 
 // Where a reduction's sums go: the last block of the grid to store its partials adds columns
-// col0 .. col1 of the table up in a fixed order (one warp a column), so no second kernel runs.
+// col0 .. col1 of the table up in a fixed order (a thread takes whole rows, one thread a column
+// the warps' sums), so no second kernel runs.
 // Column q goes to out[q], the last one to *last when that is not null; every value also goes
 // to the host mirror, a pinned copy of the array that starts at dev, so the host reads it
 // after a stream synchronisation without a copy. sig2 (optional): 1 / the last column, or 1

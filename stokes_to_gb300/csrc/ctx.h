@@ -159,7 +159,7 @@ struct stg_ctx {
     struct MmaState* mma = nullptr;   // MMA optimizer state (mma.cu), created on first use
     GraphCache vgraph;                // the V-cycle below the finest level (3D) or all of it (2D)
     GraphCache vgraph_boost;          // the 3D one while `boost` raises the sweeps
-    GraphCache sgraph;                // the coarsest-level set-up (probes and Gauss-Jordan inverse)
+    GraphCache sgraph;                // the coarsest matrix's assembly (2D: the coarsening too)
     struct NetState* net = nullptr;   // learned preconditioner (unet.cu), stg_net_init
     bool net_on = false;              // LEARNED: the network is in use in the current refinement step
 };

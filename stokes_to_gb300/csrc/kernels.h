@@ -159,7 +159,7 @@ struct DenseCoarse {
     int* slot_of = nullptr;    // dense index -> slot
     int* comp_of = nullptr;    // dense index -> 0 p, 1 u, 2 v, 3 w
     int* dense_of = nullptr;   // slot*4+comp -> dense index or -1
-    double* A = nullptr;       // two row-major nd x 2nd buffers for Gauss-Jordan on [A | I]
+    double* A = nullptr;       // two row-major nd x 2nd buffers: [A | I], and the inversions' workspace
     double* Ainv = nullptr;
     const double* inv = nullptr;  // the inverse: right half of the final buffer, row stride 2 nd
     float2* inv2 = nullptr;    // its entries as sums of two floats, nd x nd (smallcycle.cu)

@@ -49,8 +49,10 @@ struct RowDots {
 
 // Sum of products a b over the lanes of a warp on the FP32 pipe: a = a.x + a.y (split_inverse), the
 // products and sums in double-float arithmetic. The FP64 pipe takes 64 clocks of a quarter of an SM
-// for an instruction of a warp, these eleven take one each. Rounded to FP32 the sum has the error of
-// an FP64 one (304 terms: 5.7e-8 at most, 2.1e-8 on average, rows over nine decades included).
+// for an instruction of a warp, these eleven take one each. (Error-free sum after Knuth, product
+// after Dekker with an FMA.) Rounded to FP32 the sums are those of an FP64 product, bit for bit, on the
+// inverses and V-cycle residuals of 3D grids of 8 to 32 and 2D ones of 16 to 128 cells (error
+// against 64 bits 5.9e-8 at most, 2.2e-8 on average, either way).
 struct DfSum {
     float s = 0.f, c = 0.f;
     __device__ __forceinline__ void add(float v) {  // exact: s + err = s + v

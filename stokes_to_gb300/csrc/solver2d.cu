@@ -11,7 +11,7 @@
 //   smoother   stoke/StokeFlowSmoothing.cu:8-209 (5-unknown box with two 2x2 velocity
 //              blocks, colours (x + y + flag) even, r-form with a residual update per colour)
 //   coarsest   stoke/StokeFlowDirectSolve.cpp:6-133 (analytic dense matrix), inverted on
-//              the GPU by Gauss-Jordan and applied as a GEMV
+//              the GPU by blocks (dense.cu; pivoted where cells are fixed), applied as a GEMV
 //   V-cycle    common_cpx/MultigridSolve.cpp:73-106 in FP32; Krylov as in 3D (solve_core).
 #include <cooperative_groups.h>
 
@@ -522,7 +522,7 @@ struct Lv2 {
 constexpr int MAXL2 = 12;
 struct V2 {
     Lv2 lv[MAXL2];
-    G2d fine, coarse;
+    G2d fine;
     int L;
     const double* inv;  // coarsest inverse, row stride ld, blocked coarse order
     float2* inv2;       // its entries as sums of two floats, nd x nd (k2v_cycle; null: not used)
@@ -1284,7 +1284,6 @@ int create2d(stg_t* h) {
         STG_TRY(dalloc(&h->c2->map, (size_t)nd));
         v.L = L;
         v.fine = lv[L - 1].g;
-        v.coarse = lv[0].g;
         v.nd = nd;
         v.ld = 2 * nd;
         v.map = h->c2->map;

@@ -1464,7 +1464,8 @@ int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const fl
         g_attr_set[dev] = true;
     }
     if (lap && P16 && p16_scale && encoder()) {
-        // the solver's own sweeps; a narrower tile (with more rows) where a row has fewer slots
+        // the solver's own sweeps; a narrower tile (with more rows) where a row has fewer slots: levels
+        // of 8 and 16 cells that no cluster launch takes (linear prolongation, smallcycle.cu small_cycle_ok)
         STG_TRY(sweep_err_init(dev));
         bool done = false;
         const auto go = g.n > 16 ? launch_cell<32> : launch_cell<16>;
