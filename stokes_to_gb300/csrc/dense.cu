@@ -288,7 +288,6 @@ __device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[
 #pragma unroll
     for (int c = 0; c < CE; c++) split_bits(s[r][h * CE + c], a[c].h, a[c].l);
     int col = 0;  // lane q: the pivot row of step q
-    bool ok = true;
     // the columns rotate by one a step, so that the pivot column is always the first and the loop
     // stays small (unrolled over the pivots it ran from instruction-cache misses: 186 thousand
     // clocks a 32 x 32 tile); B steps bring them back in order
@@ -296,7 +295,10 @@ __device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[
     for (int q = 0; q < B; q++) {
         D2 f = d2_shfl(a[0], r * LPR);  // the pivot column's entry of the own row
         if (local_pivot) {
-            float best = (r >= q) ? fabsf(f.h) : -1.f;
+            // (a NaN counts as infinity: every lane has to come to the same row, since the lanes
+            // exchange rows together)
+            const float v = fabsf(f.h);
+            float best = r < q ? -1.f : v <= 3e38f ? v : INFINITY;
             int bi = r;
             for (int o = 16; o > 0; o >>= 1) {
                 const float ob = __shfl_xor_sync(0xffffffffu, best, o);
@@ -316,9 +318,10 @@ __device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[
             if (lane == q) col = p;
         }
         const D2 piv = d2_shfl(f, q * LPR);
-        // NaN and infinity fail as well
+        // NaN and infinity fail as well. The pivot is the same in all lanes, so all leave: going on after
+        // a pivot of 0 (the last cell of a closed domain without its ones) would fill the tile with NaN.
         const float want = local_pivot ? fabsf(piv.h) : (positive ? piv.h : -piv.h);
-        ok = ok && want > 0.f && want < 1e37f;
+        if (!(want > 0.f && want < 1e37f)) return false;
         const D2 inv = d2_inv(piv);
         const D2 g = r == q ? D2{-inv.h, -inv.l} : d2_mul(f, inv);
         const D2 own{-g.h, -g.l};  // the pivot column's new entry
@@ -355,7 +358,7 @@ __device__ __forceinline__ bool tile_inverse(double (&s)[B][B + 1], float (&hi)[
             __syncwarp();
         }
     }
-    return ok;
+    return true;
 }
 
 // Shared memory of a block: 59 KB for 32-wide tiles of three axes, which makes it dynamic (a kernel's
