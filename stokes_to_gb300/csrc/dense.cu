@@ -167,7 +167,7 @@ __device__ __forceinline__ int gj_pivot(int nd, int k, const double* in) {
                 b = sv[w];
                 ii = si[w];
             }
-        sp = ii;
+        sp = ii < nd ? ii : k;  // a column of NaN has no largest entry: stay in the matrix
     }
     __syncthreads();
     return sp;
