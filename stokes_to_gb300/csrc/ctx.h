@@ -229,12 +229,15 @@ int mma_update(stg_t* h, const double* d_x, const double* d_df, double frac, dou
 int mma_reset(stg_t* h);
 void mma_free(stg_t* h);
 
+// Zeroed device memory, ready for work on st. (Cleared on st, not by cudaMemset: the handles' streams
+// don't wait for the default stream, where it would still be under way when the first kernel or
+// copy writes the array.)
 template <class T>
-int dalloc(T** p, size_t count) {
+int dalloc(cudaStream_t st, T** p, size_t count) {
     cudaError_t e = cudaMalloc((void**)p, sizeof(T) * (count ? count : 1));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
-    e = cudaMemset(*p, 0, sizeof(T) * (count ? count : 1));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemset", __FILE__, __LINE__);
+    e = cudaMemsetAsync(*p, 0, sizeof(T) * (count ? count : 1), st);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
     return STG_OK;
 }
 }  // namespace stg

@@ -638,7 +638,7 @@ int split_inverse(cudaStream_t st, int nd, const double* inv, int ld, float2* ou
     return STG_OK;
 }
 
-int dense_init(DenseCoarse& D, const Geom& g) {
+int dense_init(cudaStream_t st, DenseCoarse& D, const Geom& g) {
     std::vector<int> slot_of, comp_of, dense_of((size_t)g.nslot * 4, -1);
     const int n = g.n;
     for (int i = 0; i <= n; i++)
@@ -673,8 +673,8 @@ int dense_init(DenseCoarse& D, const Geom& g) {
     STG_CK(cudaMemcpy(D.slot_of, slot_of.data(), sizeof(int) * nd, cudaMemcpyHostToDevice));
     STG_CK(cudaMemcpy(D.comp_of, comp_of.data(), sizeof(int) * nd, cudaMemcpyHostToDevice));
     STG_CK(cudaMemcpy(D.dense_of, dense_of.data(), sizeof(int) * dense_of.size(), cudaMemcpyHostToDevice));
-    STG_CK(cudaMemset(D.probe, 0, sizeof(d4) * g.nslot * PROBES));
-    STG_CK(cudaMemset(D.image, 0, sizeof(d4) * g.nslot * PROBES));
+    STG_CK(cudaMemsetAsync(D.probe, 0, sizeof(d4) * g.nslot * PROBES, st));
+    STG_CK(cudaMemsetAsync(D.image, 0, sizeof(d4) * g.nslot * PROBES, st));
     return STG_OK;
 }
 

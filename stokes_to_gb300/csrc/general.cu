@@ -318,17 +318,17 @@ namespace {
 int gen_alloc(stg_t* h) {
     for (auto& L : h->lv) {
         const size_t ns = L.g.nslot;
-        if (!L.V64 && dalloc(&L.V64, ns)) return STG_E_CUDA;
-        if (!L.gr && (dalloc(&L.gr, ns) || dalloc(&L.gx, ns) || dalloc(&L.gp, ns) || dalloc(&L.gAp, ns))) return STG_E_CUDA;
+        if (!L.V64 && dalloc(h->st, &L.V64, ns)) return STG_E_CUDA;
+        if (!L.gr && (dalloc(h->st, &L.gr, ns) || dalloc(h->st, &L.gx, ns) || dalloc(h->st, &L.gp, ns) || dalloc(h->st, &L.gAp, ns))) return STG_E_CUDA;
         if (&L != &h->lv[0]) {
             const size_t nb = (size_t)L.g.n * L.g.n * L.g.n / 2;
             for (int c = 0; c < 2; c++)
-                if (!L.vblk[c] && (dalloc(&L.vblk[c], 49 * nb) || dalloc(&L.vpiv[c], 7 * nb))) return STG_E_CUDA;
+                if (!L.vblk[c] && (dalloc(h->st, &L.vblk[c], 49 * nb) || dalloc(h->st, &L.vpiv[c], 7 * nb))) return STG_E_CUDA;
         }
     }
     const size_t ns = fine(h).g.nslot;
     for (auto& p : h->gtmp)
-        if (!p && dalloc(&p, ns)) return STG_E_CUDA;
+        if (!p && dalloc(h->st, &p, ns)) return STG_E_CUDA;
     return STG_OK;
 }
 

@@ -170,7 +170,7 @@ struct DenseCoarse {
     double* rd = nullptr;      // gathered right-hand side (nd)
     InvOrder order;
 };
-int dense_init(DenseCoarse& D, const Geom& g);
+int dense_init(cudaStream_t st, DenseCoarse& D, const Geom& g);
 // the entries of an nd x nd inverse (row stride ld) as sums of two floats, row-major nd x nd
 int split_inverse(cudaStream_t st, int nd, const double* inv, int ld, float2* out);
 void dense_free(DenseCoarse& D);

@@ -209,8 +209,8 @@ int mma_update(stg_t* h, const double* d_x, const double* d_df, double frac, dou
         h->mma = new MmaState();
         MmaArrays& A = h->mma->A;
         for (double** p : {&A.low, &A.upp, &A.xold1, &A.xold2, &A.alpha, &A.beta, &A.p0, &A.q0, &A.p1, &A.q1})
-            STG_TRY(dalloc(p, (size_t)n));
-        STG_TRY(dalloc(&h->mma->part, 2 * MGRID));
+            STG_TRY(dalloc(h->st, p, (size_t)n));
+        STG_TRY(dalloc(h->st, &h->mma->part, 2 * MGRID));
         h->mma->hpart.resize(2 * MGRID);
     }
     MmaState& M = *h->mma;

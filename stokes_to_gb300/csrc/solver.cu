@@ -819,9 +819,9 @@ int choose_path(stg_t* h, const Level& L, const d4* x) {
     return STG_OK;
 }
 
-int ensure_adapter(Level& L) {
-    if (!L.t0) STG_TRY(dalloc(&L.t0, L.g.nslot));
-    if (!L.t1) STG_TRY(dalloc(&L.t1, L.g.nslot));
+int ensure_adapter(stg_t* h, Level& L) {
+    if (!L.t0) STG_TRY(dalloc(h->st, &L.t0, L.g.nslot));
+    if (!L.t1) STG_TRY(dalloc(h->st, &L.t1, L.g.nslot));
     return STG_OK;
 }
 
@@ -960,9 +960,9 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
         Level& L = h->lv[i];
         L.g = Geom::make(nn);
         size_t ns = L.g.nslot;
-        if ((rc = dalloc(&L.m, ns)) || (rc = dalloc(&L.P64, ns)) || (rc = dalloc(&L.P32, ns)) || (rc = dalloc(&L.r, ns)) ||
-            (rc = dalloc(&L.xa, ns)) || (rc = dalloc(&L.xb, ns)) || (rc = dalloc(&L.rr, ns)) ||
-            (rc = dalloc(&L.xbf, 4 * ns)) || (rc = dalloc(&L.P16, 4 * ns)))
+        if ((rc = dalloc(h->st, &L.m, ns)) || (rc = dalloc(h->st, &L.P64, ns)) || (rc = dalloc(h->st, &L.P32, ns)) || (rc = dalloc(h->st, &L.r, ns)) ||
+            (rc = dalloc(h->st, &L.xa, ns)) || (rc = dalloc(h->st, &L.xb, ns)) || (rc = dalloc(h->st, &L.rr, ns)) ||
+            (rc = dalloc(h->st, &L.xbf, 4 * ns)) || (rc = dalloc(h->st, &L.P16, 4 * ns)))
             return fail(rc);
         // halo and absent unknowns fixed; the box is rewritten by set_boundary / coarsen
         if ((rc = mask_from_field(h->st, L.g, nullptr, nullptr, nullptr, nullptr, L.m))) return fail(rc);
@@ -973,7 +973,7 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
         return fail(STG_E_INVALID);
     }
     if (dim == 3) {
-        if ((rc = dense_init(h->dense, h->lv[0].g))) return fail(rc);
+        if ((rc = dense_init(h->st, h->dense, h->lv[0].g))) return fail(rc);
         h->coarsest = h->dense.nd;
         Level& F = fine(h);
         h->n4 = (long long)F.g.nslot;
@@ -990,24 +990,24 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
         nparts = grid_for(4 * h->n4, 256);
     }
     const size_t ns = (size_t)h->n4;
-    if ((rc = dalloc(&h->b64, ns)) || (rc = dalloc(&h->x64, ns)) || (rc = dalloc(&h->r64, ns)) || (rc = dalloc(&h->t64, ns)) ||
-        (rc = dalloc(&h->lam64, ns)) || (rc = dalloc(&h->w, ns)) ||
-        (dim == 3 && ((rc = dalloc(&h->xh, ns)) || (rc = dalloc(&h->xl, ns)) || (rc = dalloc(&h->bh, ns)) || (rc = dalloc(&h->bl, ns)) ||
-                      (rc = dalloc(&h->Plo, ns)) || (rc = dalloc(&h->d_pscale, (size_t)h->L)) || (rc = dalloc(&h->d_pmax, 1)))))
+    if ((rc = dalloc(h->st, &h->b64, ns)) || (rc = dalloc(h->st, &h->x64, ns)) || (rc = dalloc(h->st, &h->r64, ns)) || (rc = dalloc(h->st, &h->t64, ns)) ||
+        (rc = dalloc(h->st, &h->lam64, ns)) || (rc = dalloc(h->st, &h->w, ns)) ||
+        (dim == 3 && ((rc = dalloc(h->st, &h->xh, ns)) || (rc = dalloc(h->st, &h->xl, ns)) || (rc = dalloc(h->st, &h->bh, ns)) || (rc = dalloc(h->st, &h->bl, ns)) ||
+                      (rc = dalloc(h->st, &h->Plo, ns)) || (rc = dalloc(h->st, &h->d_pscale, (size_t)h->L)) || (rc = dalloc(h->st, &h->d_pmax, 1)))))
         return fail(rc);
     h->V.assign(h->m + 1, nullptr);
     h->Z.assign(h->m, nullptr);
     // one allocation for V and one for Z: a cudaMalloc and a memset each per vector were most of
     // a small handle's creation
     const size_t vs = (ns + 15) / 16 * 16;  // vectors start on 256-byte boundaries
-    if ((rc = dalloc(&h->vslab, vs * h->V.size())) || (rc = dalloc(&h->zslab, vs * h->Z.size()))) return fail(rc);
+    if ((rc = dalloc(h->st, &h->vslab, vs * h->V.size())) || (rc = dalloc(h->st, &h->zslab, vs * h->Z.size()))) return fail(rc);
     for (size_t q = 0; q < h->V.size(); q++) h->V[q] = h->vslab + q * vs;
     for (size_t q = 0; q < h->Z.size(); q++) h->Z[q] = h->zslab + q * vs;
     if (dim == 3 && h->opts.basis16) {
         // the FP16 copies only speed up the multi-dot: without room for them the handle
         // runs on the FP32 basis alone
         h->V16.assign(h->m + 1, nullptr);
-        const bool ok = dalloc(&h->dsc16, (size_t)h->m + 1) == STG_OK && dalloc(&h->slab16, vs * h->V16.size()) == STG_OK;
+        const bool ok = dalloc(h->st, &h->dsc16, (size_t)h->m + 1) == STG_OK && dalloc(h->st, &h->slab16, vs * h->V16.size()) == STG_OK;
         for (size_t q = 0; ok && q < h->V16.size(); q++) h->V16[q] = h->slab16 + q * vs;
         if (!ok) {
             cudaFree(h->slab16);
@@ -1022,9 +1022,9 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
     const size_t nres = 2 * ((size_t)h->m + 2) + 8;
     h->nparts = (size_t)nparts + 1216;  // the passes over whole vectors have up to 1216 blocks
     static_assert(OC_PARTS <= 1216, "block sums of the OC update");
-    if ((rc = dalloc(&h->dscr, 1216 * 18)) || (rc = dalloc(&h->dh, nres)) || (rc = dalloc(&h->dcount, 1)) ||
-        (rc = dalloc(&h->dsig2, h->m + 2)) ||
-        (rc = dalloc(&h->dy, h->m + 1)) || (rc = dalloc(&h->d_parts, h->nparts)) || (rc = dalloc(&h->dflag, 1)))
+    if ((rc = dalloc(h->st, &h->dscr, 1216 * 18)) || (rc = dalloc(h->st, &h->dh, nres)) || (rc = dalloc(h->st, &h->dcount, 1)) ||
+        (rc = dalloc(h->st, &h->dsig2, h->m + 2)) ||
+        (rc = dalloc(h->st, &h->dy, h->m + 1)) || (rc = dalloc(h->st, &h->d_parts, h->nparts)) || (rc = dalloc(h->st, &h->dflag, 1)))
         return fail(rc);
     h->dnrm = h->dh + (nres - 8);
     if (cudaHostAlloc((void**)&h->hres, sizeof(double) * (nres + 1), cudaHostAllocMapped) != cudaSuccess)
@@ -1032,15 +1032,17 @@ int stg_create(int dim, int n, const stg_opts* opts, stg_t** out) {
     memset(h->hres, 0, sizeof(double) * (nres + 1));
     h->hflags = reinterpret_cast<int*>(h->hres + nres);
     const double one = 1.0;  // the first basis vector of every refinement step is normalised
-    if (cudaMemcpy(h->dsig2, &one, sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpyAsync(h->dsig2, &one, sizeof(double), cudaMemcpyHostToDevice, h->st) != cudaSuccess)
         return fail(cuda_fail(cudaGetLastError(), "create", __FILE__, __LINE__));
-    if ((rc = dalloc(&h->stage, h->ncell + 3 * h->nface)) || (rc = dalloc(&h->istage, h->ncell + 3 * h->nface))) return fail(rc);
-    if ((rc = dalloc(&h->d_design, h->ncell)) || (rc = dalloc(&h->d_phys, h->ncell)) || (rc = dalloc(&h->d_sens, h->ncell)) ||
-        (rc = dalloc(&h->d_sens_design, h->ncell)) || (rc = dalloc(&h->d_vw, h->ncell)) || (rc = dalloc(&h->d_tmp, h->ncell)) ||
-        (rc = dalloc(&h->d_wsum, h->ncell)) ||
-        (rc = dalloc(&h->d_gauss, 512)))
+    if ((rc = dalloc(h->st, &h->stage, h->ncell + 3 * h->nface)) || (rc = dalloc(h->st, &h->istage, h->ncell + 3 * h->nface))) return fail(rc);
+    if ((rc = dalloc(h->st, &h->d_design, h->ncell)) || (rc = dalloc(h->st, &h->d_phys, h->ncell)) || (rc = dalloc(h->st, &h->d_sens, h->ncell)) ||
+        (rc = dalloc(h->st, &h->d_sens_design, h->ncell)) || (rc = dalloc(h->st, &h->d_vw, h->ncell)) || (rc = dalloc(h->st, &h->d_tmp, h->ncell)) ||
+        (rc = dalloc(h->st, &h->d_wsum, h->ncell)) ||
+        (rc = dalloc(h->st, &h->d_gauss, 512)))
         return fail(rc);
-    if (cudaStreamSynchronize(h->st) != cudaSuccess) return fail(cuda_fail(cudaGetLastError(), "create", __FILE__, __LINE__));
+    // (the default stream: the tables that were copied there)
+    if (cudaStreamSynchronize(h->st) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess)
+        return fail(cuda_fail(cudaGetLastError(), "create", __FILE__, __LINE__));
     *out = h;
     return STG_OK;
 }
@@ -1232,7 +1234,7 @@ int stg_set_boundary(stg_t* h, const double* cell_vol, const int32_t* cell_fixed
     h->gen = gen;
     if (gen) {
         // per-slot vols (0 on fixed unknowns, as the reference's finish() leaves them)
-        if (!F.V64 && dalloc(&F.V64, F.g.nslot)) return STG_E_CUDA;
+        if (!F.V64 && dalloc(h->st, &F.V64, F.g.nslot)) return STG_E_CUDA;
         const double* dc = nullptr;
         const double* df[3] = {nullptr, nullptr, nullptr};
         STG_TRY(upload_fields(h, cell_vol, face_vol, &dc, df));
@@ -1554,7 +1556,7 @@ int stg_apply_A_device(stg_t* h, int level, double* d_Ap, const double* d_p) {
         STG_CK(cudaStreamSynchronize(h->st));
         return STG_OK;
     }
-    STG_TRY(ensure_adapter(L));
+    STG_TRY(ensure_adapter(h, L));
     STG_TRY(blocked_to_slots64(h->st, L.g, d_p, L.t0));
     if (h->gen)
         STG_TRY(op64v(h->st, L.g, L.t0, L.m, L.P64, L.V64, nullptr, L.t1, 0, nullptr, nullptr));
@@ -1579,7 +1581,7 @@ int stg_apply_E_device(stg_t* h, double* d_Ap, const double* d_p) {
         STG_CK(cudaStreamSynchronize(h->st));
         return STG_OK;
     }
-    STG_TRY(ensure_adapter(L));
+    STG_TRY(ensure_adapter(h, L));
     STG_TRY(blocked_to_slots64(h->st, L.g, d_p, L.t0));
     if (h->gen)
         STG_TRY(op64v(h->st, L.g, L.t0, L.m, L.P64, L.V64, nullptr, L.t1, 2, nullptr, nullptr));
@@ -1607,7 +1609,7 @@ int stg_vcycle_device(stg_t* h, double* d_out, const double* d_in) {
         return STG_OK;
     }
     Level& F = fine(h);
-    STG_TRY(ensure_adapter(F));
+    STG_TRY(ensure_adapter(h, F));
     STG_TRY(blocked_to_slots64(h->st, F.g, d_in, F.t0));
     if (h->gen) {
         STG_CK(cudaMemcpyAsync(F.gr, F.t0, sizeof(d4) * F.g.nslot, cudaMemcpyDeviceToDevice, h->st));
@@ -1639,12 +1641,12 @@ int stg_apply_op_device(stg_t* h, int op, int level, double* d_out, const double
         return STG_OK;
     }
     Level& L = h->lv[level];
-    STG_TRY(ensure_adapter(L));
+    STG_TRY(ensure_adapter(h, L));
     switch (op) {
         case STG_OP_RESTRICT: {
             if (level >= h->L - 1) break;
             Level& F = h->lv[level + 1];
-            STG_TRY(ensure_adapter(F));
+            STG_TRY(ensure_adapter(h, F));
             STG_TRY(blocked_to_slots64(h->st, F.g, d_in, F.t0));
             STG_TRY(restrict64(h->st, L.g, F.g, F.t0, L.m, L.t1));
             STG_TRY(slots_to_blocked64(h->st, L.g, L.t1, d_out, nullptr));
@@ -1654,7 +1656,7 @@ int stg_apply_op_device(stg_t* h, int op, int level, double* d_out, const double
         case STG_OP_PROLONG: {
             if (level >= h->L - 1) break;
             Level& F = h->lv[level + 1];
-            STG_TRY(ensure_adapter(F));
+            STG_TRY(ensure_adapter(h, F));
             STG_TRY(blocked_to_slots64(h->st, L.g, d_in, L.t0));
             STG_TRY(prolong64(h->st, F.g, L.g, L.t0, F.m, F.t1));
             STG_TRY(slots_to_blocked64(h->st, F.g, F.t1, d_out, nullptr));
@@ -1720,7 +1722,7 @@ int stg_level_descr_device(stg_t* h, int level, double* d_vol, double* d_penalty
         return STG_OK;
     }
     Level& L = h->lv[level];
-    STG_TRY(ensure_adapter(L));
+    STG_TRY(ensure_adapter(h, L));
     if (d_penalty) STG_TRY(slots_to_blocked64(h->st, L.g, L.P64, d_penalty, nullptr));
     if (d_fixed) STG_TRY(mask_to_blocked(h->st, L.g, L.m, d_fixed));
     if (d_vol) {

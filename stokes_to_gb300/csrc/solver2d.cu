@@ -1255,12 +1255,12 @@ int create2d(stg_t* h) {
     for (int i = L - 2; i >= 0; i--) lv[i].lap = 2.0 * lv[i + 1].lap;  // createSubSystem (StokeFlowSubSystem.cu:155)
     for (auto& V : lv) {
         size_t s = V.g.size();
-        STG_TRY(dalloc(&V.fixed, s));
-        STG_TRY(dalloc(&V.vol, s));
-        STG_TRY(dalloc(&V.pen, s));
-        STG_TRY(dalloc(&V.vol32, s));
-        STG_TRY(dalloc(&V.pen32, s));
-        for (float** q : {&V.r, &V.x, &V.p, &V.Ap, &V.rs, &V.d, &V.Ad}) STG_TRY(dalloc(q, s));
+        STG_TRY(dalloc(h->st, &V.fixed, s));
+        STG_TRY(dalloc(h->st, &V.vol, s));
+        STG_TRY(dalloc(h->st, &V.pen, s));
+        STG_TRY(dalloc(h->st, &V.vol32, s));
+        STG_TRY(dalloc(h->st, &V.pen32, s));
+        for (float** q : {&V.r, &V.x, &V.p, &V.Ap, &V.rs, &V.d, &V.Ad}) STG_TRY(dalloc(h->st, q, s));
     }
     const int nd = lv[0].g.size();
     if (nd > 8192) {
@@ -1268,9 +1268,9 @@ int create2d(stg_t* h) {
         return STG_E_UNSUPPORTED;
     }
     h->coarsest = nd;
-    STG_TRY(dalloc(&h->c2->aug0, 2ull * nd * nd));
-    STG_TRY(dalloc(&h->c2->aug1, 2ull * nd * nd));
-    STG_TRY(dalloc(&h->c2->info, 1));
+    STG_TRY(dalloc(h->st, &h->c2->aug0, 2ull * nd * nd));
+    STG_TRY(dalloc(h->st, &h->c2->aug1, 2ull * nd * nd));
+    STG_TRY(dalloc(h->st, &h->c2->info, 1));
     std::vector<std::vector<int>> faces(2);
     std::vector<int> cells;
     for (int q = 0; q < nd; q++) (q < lv[0].g.off(0) ? cells : faces[q >= lv[0].g.off(1)]).push_back(q);
@@ -1279,9 +1279,9 @@ int create2d(stg_t* h) {
         V2& v = h->c2->v;
         size_t nf = 0, nm = 0;
         for (auto& q : lv) nf += 12ull * (q.g.n + 4) * (q.g.n + 3), nm += (size_t)(q.g.n + 4) * (q.g.n + 3);
-        STG_TRY(dalloc(&h->c2->pad, nf));
-        STG_TRY(dalloc(&h->c2->padm, nm));
-        STG_TRY(dalloc(&h->c2->map, (size_t)nd));
+        STG_TRY(dalloc(h->st, &h->c2->pad, nf));
+        STG_TRY(dalloc(h->st, &h->c2->padm, nm));
+        STG_TRY(dalloc(h->st, &h->c2->map, (size_t)nd));
         v.L = L;
         v.fine = lv[L - 1].g;
         v.nd = nd;
@@ -1316,7 +1316,7 @@ int create2d(stg_t* h) {
             STG_CK(cudaFuncSetAttribute(k2v_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, cycle_smem()));
             const cudaLaunchConfig_t cfg = config2(nullptr, CYCLE_BLOCKS, true, at);
             if (h->c2->cluster && cudaOccupancyMaxActiveClusters(&can, k2v_cycle, &cfg) == cudaSuccess && can > 0)
-                STG_TRY(dalloc(&v.inv2, (size_t)nd * nd));
+                STG_TRY(dalloc(h->st, &v.inv2, (size_t)nd * nd));
             cudaGetLastError();
         }
     }

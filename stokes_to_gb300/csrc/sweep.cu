@@ -1428,10 +1428,10 @@ int launch_cell(cudaStream_t st, int dev, EncodeTiled enc, const Geom& g, float 
 }
 
 // the flag a TMA sweep sets when its wait gave up, per device
-int sweep_err_init(int dev) {
+int sweep_err_init(cudaStream_t st, int dev) {
     if (g_sweep_err[dev]) return STG_OK;
     STG_CK(cudaMalloc((void**)&g_sweep_err[dev], sizeof(int)));
-    STG_CK(cudaMemset(g_sweep_err[dev], 0, sizeof(int)));
+    STG_CK(cudaMemsetAsync(g_sweep_err[dev], 0, sizeof(int), st));
     return STG_OK;
 }
 
@@ -1466,7 +1466,7 @@ int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const fl
     if (lap && P16 && p16_scale && encoder()) {
         // the solver's own sweeps; a narrower tile (with more rows) where a row has fewer slots: levels
         // of 8 and 16 cells that no cluster launch takes (linear prolongation, smallcycle.cu small_cycle_ok)
-        STG_TRY(sweep_err_init(dev));
+        STG_TRY(sweep_err_init(st, dev));
         bool done = false;
         const auto go = g.n > 16 ? launch_cell<32> : launch_cell<16>;
         STG_TRY(go(st, dev, encoder(), g, vol, r, xin, xout, P16, p16_scale, flag, xc, gc, pair, &done));
@@ -1488,7 +1488,7 @@ int sweep32(cudaStream_t st, const Geom& g, float vol, const float4* r, const fl
         if (!g_tattr_set[dev]) {
             STG_CK(cudaFuncSetAttribute(k_sweep_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
             STG_CK(cudaFuncSetAttribute(k_sweep_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t));
-            STG_TRY(sweep_err_init(dev));
+            STG_TRY(sweep_err_init(st, dev));
             g_tattr_set[dev] = true;
         }
         CUtensorMap mx{}, mr{}, mp{};

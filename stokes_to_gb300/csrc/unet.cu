@@ -892,7 +892,7 @@ int stg_net_train(stg_t* h, int steps, double lr, uint64_t seed, float* losses) 
     STG_TRY(stg::net_buffers(N, h->n, true));
     std::vector<double> dl(steps > 0 ? steps : 1);
     double* d_losses = nullptr;
-    STG_TRY(stg::dalloc(&d_losses, dl.size()));
+    STG_TRY(stg::dalloc(h->st, &d_losses, dl.size()));
     int rc = STG_OK;
     for (int s = 0; s < steps && rc == STG_OK; s++) {
         const uint64_t sd = seed * 0x100000001B3ull + (uint64_t)s;

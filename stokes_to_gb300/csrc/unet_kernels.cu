@@ -557,7 +557,7 @@ int conv3_forward(cudaStream_t st, const __nv_bfloat16* in, int cin, int ldin, c
         if (P.J && dev >= 0) {
             if (!g_tc_err[dev]) {
                 STG_CK(cudaMalloc((void**)&g_tc_err[dev], sizeof(int)));
-                STG_CK(cudaMemset(g_tc_err[dev], 0, sizeof(int)));
+                STG_CK(cudaMemsetAsync(g_tc_err[dev], 0, sizeof(int), st));
             }
             int* const err = g_tc_err[dev];
             int rc = STG_OK;
